@@ -1,29 +1,32 @@
 // 3x3x3 convolution on the 5th-generation tensor cores (tcgen05, sm_103a).
 //
-// Implicit GEMM: M = 128 output voxels (a tile of 8 x 16 voxels in x, y at one
-// z), N = CO_T output channels, K = 27 taps x 16-channel slices.  The tile's
-// zero-padded halo (10 x 18 x 3 voxels) is stored "chunk-planar": channels
-// 0..7 of every halo voxel, 16 bytes each, then channels 8..15.  In that layout
-// the A operand of any tap is a K-major, no-swizzle shared-memory matrix:
-// 8 consecutive voxels of one x row form a core matrix (8 rows x 16 bytes,
-// contiguous), successive y rows are 10 voxels (160 bytes) apart (the stride
-// between 8-row groups) and the second 8 channels are one plane further (the
-// stride between K-adjacent core matrices).  So each tap is one
-// tcgen05.mma.kind::f16 (BF16 x BF16 -> FP32, M = 128, N = CO_T, K = 16)
-// reading the halo in place, accumulating in tensor memory.
+// Implicit GEMM: M = 128 output voxels (a tile of 8 x 16 voxels in x, y at one z), K = 27 taps x 16-channel slices.  A slab
+// (one z plane of the tile's zero-padded halo, 10 x 18 voxels, 16 channels) is stored "chunk-planar": channels 0..7 of
+// every voxel, 16 bytes each, then channels 8..15.  In that layout the A operand of any tap is a K-major, no-swizzle
+// shared-memory matrix: 8 consecutive voxels of one x row form a core matrix (8 rows x 16 bytes, contiguous), successive y
+// rows are 10 voxels (160 bytes) apart (the stride between 8-row groups) and the second 8 channels are one plane further
+// (the stride between K-adjacent core matrices), so each tap reads the halo in place.
 //
-// A CTA (4 warps) is persistent: it keeps the weights of its output-channel
-// group for every input slice in shared memory (same planar layout: the B
-// operand of tap t starts at row t * CO_T), walks its tiles slice by slice,
-// and copies the next slice's halo with cp.async (two buffers) while the
-// tensor cores work.
-// Thread 0 issues the MMAs and commits them to the mbarrier of the halo buffer
-// they read; that barrier gates both the buffer's reuse and, at the end of a
-// tile, the epilogue, where each warp reads its 32 accumulator rows with
-// tcgen05.ld (one voxel per thread), adds the bias, applies the activation and
-// mask, and stores the voxel's channels.  Every mbarrier wait is bounded: on
-// timeout the kernel raises a device error bit, stops issuing work, waits for
-// its copies and frees its tensor memory.
+// The three z taps share one MMA: a slab at z feeds the output planes z - 1, z and z + 1, whose accumulators are
+// neighbouring columns of tensor memory, so for every (dy, dx) one tcgen05.mma of N = 3 CO_T takes the slab's 4 KB window
+// for all three.  What bounds these layers is that window's way through shared memory, about 60 cycles an MMA however small
+// N is: 9 MMAs a slab and tile instead of 27, and every slab is copied once instead of three times.
+//
+// A CTA marches an item (a tile x up to 256 / CO_T planes, all accumulators in 256 columns) slice by slice, plane by plane,
+// so that the products of an output are added in the order slice, z tap, y tap, x tap.  Its output planes are drained while
+// the next ones are summed; two CTAs share an SM and hide each other's waits.  The weights of the CTA's output-channel
+// group stay in shared memory.
+//
+// Measured on GB300, us a launch, against one MMA of N = CO_T per tap with three halo planes copied for every output plane
+// (and mma.sync for 128 and more input channels); the results are the same bit for bit:
+//   16 -> 16 on 128^3   141 -> 55..72     48 -> 16 on 128^3   430 -> 107     16 -> 48 on 128^3   190 -> 102
+//   32 -> 32 on  64^3    51 -> 26         96 -> 32 on  64^3   339 -> 63
+//   64 -> 64 on  32^3    44 -> 20        192 -> 64 on  32^3   147 -> 49     128 -> 128 on 16^3   65 -> 17
+//
+// Warps: 0..3 epilogue, 4..7 copy the slabs (cp.async into a ring; the first input may be read through a nearest 2x
+// upsampling, so that neither the upsampled nor the concatenated tensor exists in memory), 8 issues the MMAs.  Every wait
+// is bounded: one that runs out (2 s) sets an abort word that ends all later waits at once; the roles then run through
+// their work without waiting (every access stays in its buffers), the kernel raises DF_TIMEOUT and frees its tensor memory.
 #include <algorithm>
 
 #include "vg_nn.cuh"
@@ -33,67 +36,83 @@ namespace nn {
 
 namespace {
 
-constexpr int kTX = 8, kTY = 16;                  // tile: 8 x 16 x 1 voxels = M 128
-constexpr int kHX = kTX + 2, kHY = kTY + 2;        // halo 10 x 18 x 3
-constexpr int kNH = kHX * kHY * 3;                 // 540 halo voxels
-constexpr int kPlane = kNH * 16;                   // bytes of one 8-channel plane of a halo slice
-constexpr int kHaloBytes = 2 * kPlane;             // one 16-channel slice
-constexpr size_t kUmmaWeightBytes = 100 * 1024;
-constexpr long long kWaitLimit = 1LL << 24;
-constexpr int kBufs = 2;                           // halo buffers in flight (3 costs a CTA per SM, measured slower)
+constexpr int kTX = 8, kTY = 16;                 // tile: 8 x 16 voxels = M 128
+constexpr int kHX = kTX + 2, kHY = kTY + 2;       // halo 10 x 18
+constexpr int kChunks = kHX * kHY * 2;            // 16-byte chunks of a slab
+constexpr unsigned kXPlane = kHX * kHY * 16;      // bytes of 8 channels of a slab
+constexpr unsigned kSlab = 2 * kXPlane;
+constexpr int kEpiWarps = 4, kCopyWarps = 4, kCopyThreads = kCopyWarps * 32;
+constexpr int kMmaWarp = kEpiWarps + kCopyWarps, kThreads = (kMmaWarp + 1) * 32;
+constexpr int kMaxSlabs = 8, kMinSlabs = 4;       // slabs in the ring
+constexpr int kCols = 256;                        // tensor-memory columns of a CTA
+constexpr int kMaxPlanes = 16;
+constexpr size_t kSmemTwo = 113 * 1024, kSmemOne = 226 * 1024;  // shared memory of a CTA at two and at one per SM
+constexpr size_t kTail = (2 * kMaxSlabs + 2 * kMaxPlanes) * 8 + 64;
+constexpr unsigned long long kWaitNs = 2000000000ull;
 
 __device__ __forceinline__ unsigned su32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
+__device__ __forceinline__ bool try_wait(unsigned mbar, unsigned parity) {
+  unsigned done;
+  asm volatile(
+      "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+      : "=r"(done)
+      : "r"(mbar), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+
+__device__ __forceinline__ void wait_phase(unsigned mbar, unsigned parity, volatile int* abort_word) {
+  for (int k = 0; k < 512; ++k)
+    if (try_wait(mbar, parity)) return;
+  unsigned long long t0, t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
+  while (!*abort_word) {
+    for (int k = 0; k < 16; ++k)
+      if (try_wait(mbar, parity)) return;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    if (t - t0 > kWaitNs) *abort_word = 1;
+  }
+}
+
+// One arrival for the warp, after all of its lanes.
+__device__ __forceinline__ void arrive(unsigned mbar) {
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
+}
+
+__device__ __forceinline__ void commit_to(unsigned mbar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
+}
+
+__device__ __forceinline__ bool elect_one() {
+  unsigned r;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(r));
+  return r != 0;
+}
+
 __device__ __forceinline__ void cp_async16(unsigned dst, const void* src, int src_bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(src_bytes));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
 }
 
-__device__ __forceinline__ uint64_t smem_desc(unsigned addr, unsigned lbo, unsigned sbo) {
-  return (uint64_t)((addr >> 4) & 0x3fff) | ((uint64_t)((lbo >> 4) & 0x3fff) << 16) |
-         ((uint64_t)((sbo >> 4) & 0x3fff) << 32) | ((uint64_t)1 << 46);  // no swizzle, version 1
+// No-swizzle K-major descriptors: the low word holds the address and the distance of the second 8 channels, the high word
+// the distance of 8-row groups (and the descriptor version).
+__device__ __forceinline__ unsigned desc_lo(unsigned addr, unsigned plane) {
+  return ((addr >> 4) & 0x3fff) | ((plane >> 4) << 16);
 }
+constexpr unsigned kDescHiA = ((kHX * 16u) >> 4) | (1u << 14), kDescHiB = (128u >> 4) | (1u << 14);
 
-// kind::f16 instruction descriptor: FP32 accumulate, BF16 A and B, both K-major.
+// kind::f16 instruction descriptor: FP32 accumulate, BF16 A and B, both K-major, M = 128.
 __host__ __device__ constexpr unsigned idesc_bf16(int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(n >> 3) << 17) | ((128u >> 4) << 24);
 }
 
-__device__ __forceinline__ bool mbar_wait(unsigned mbar, unsigned parity) {
-  for (long long it = 0; it < kWaitLimit; ++it) {
-    unsigned done;
-    asm volatile(
-        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
-        : "=r"(done)
-        : "r"(mbar), "r"(parity));
-    if (done) return true;
-  }
-  return false;
-}
-
-// Copies one 16-channel slice of the halo of the tile at (x0, y0, z0) into the
-// planar buffer at byte address dst (zero-filled outside the volume).
-__device__ __forceinline__ void issue_halo_planar(unsigned dst, const ConvIn& in, int x0, int y0, int z0, int ci0) {
-  for (int s = threadIdx.x; s < kNH; s += blockDim.x) {
-    const int ix = s % kHX, iy = (s / kHX) % kHY, iz = s / (kHX * kHY);
-    const int z = z0 + iz - 1, y = y0 + iy - 1, x = x0 + ix - 1;
-    const bool inside = z >= 0 && y >= 0 && x >= 0 && z < in.D && y < in.H && x < in.W;
-    const __nv_bfloat16* p = in.x1;  // a valid address when nothing is read
-    if (inside) {
-      if (ci0 < in.C1) {
-        if (in.up1) {
-          const int H1 = in.H >> 1, W1 = in.W >> 1;
-          p = in.x1 + (((size_t)(z >> 1) * H1 + (y >> 1)) * W1 + (x >> 1)) * in.C1 + ci0;
-        } else {
-          p = in.x1 + (((size_t)z * in.H + y) * in.W + x) * in.C1 + ci0;
-        }
-      } else {
-        p = in.x2 + (((size_t)z * in.H + y) * in.W + x) * in.C2 + (ci0 - in.C1);
-      }
-    }
-    const int nb = inside ? 16 : 0;
-    cp_async16(dst + s * 16, p, nb);
-    cp_async16(dst + kPlane + s * 16, p + 8, nb);
-  }
+__device__ __forceinline__ void mma(unsigned d, unsigned a_lo, unsigned b_lo, unsigned idesc, unsigned acc) {
+  asm volatile(
+      "{\n.reg .pred p;\n.reg .b64 da, db;\nsetp.ne.b32 p, %6, 0;\nmov.b64 da, {%1, %4};\nmov.b64 db, {%2, %5};\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n}" ::"r"(d),
+      "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(kDescHiA), "r"(kDescHiB), "r"(acc)
+      : "memory");
 }
 
 // 16 consecutive FP32 accumulator columns of this thread's TMEM lane.
@@ -105,177 +124,264 @@ __device__ __forceinline__ void tmem_ld16(unsigned taddr, unsigned* r) {
       : "r"(taddr));
 }
 
-// Epilogue of one tile: thread (warp w, lane l) owns accumulator row 32 w + l,
-// i.e. voxel (x0 + row % 8, y0 + row / 8, z0), and its CO_T channels.
-template <int CO_T>
-__device__ __forceinline__ void umma_epilogue(unsigned tmem, const ConvIn& in, const ConvOut& out, int x0, int y0,
-                                              int z0, int co0) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, m = warp * 32 + lane;
-  unsigned r[CO_T];
-#pragma unroll
-  for (int j = 0; j < CO_T / 16; ++j) tmem_ld16(tmem + ((unsigned)(warp * 32) << 16) + 16 * j, r + 16 * j);
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int q = 0; q < CO_T; ++q) asm volatile("" : "+r"(r[q]));  // uses stay after the wait
-  const size_t vox = ((size_t)z0 * in.H + (y0 + (m >> 3))) * in.W + (x0 + (m & 7));
-  const int Co = out.Co;
-#pragma unroll
-  for (int c8 = 0; c8 < CO_T / 8; ++c8) {
-    float v[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      float t = __uint_as_float(r[c8 * 8 + q]);
-      if (out.bias) t += out.bias[co0 + c8 * 8 + q];
-      if (out.relu) t = t > 0.f ? t : out.slope * t;
-      v[q] = t;
-    }
-    const size_t at = vox * Co + co0 + c8 * 8;
-    if (out.mask) {
-      const uint4 mk = *reinterpret_cast<const uint4*>(out.mask + at);
-      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&mk);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        if (!(__low2float(h[q]) > 0.f)) v[2 * q] *= out.mask_slope;
-        if (!(__high2float(h[q]) > 0.f)) v[2 * q + 1] *= out.mask_slope;
-      }
-    }
-    if (out.yf) {
-      float4* d = reinterpret_cast<float4*>(out.yf + at);
-      d[0] = make_float4(v[0], v[1], v[2], v[3]);
-      d[1] = make_float4(v[4], v[5], v[6], v[7]);
-    } else {
-      __align__(16) __nv_bfloat162 h[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) h[q] = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
-      *reinterpret_cast<uint4*>(out.y + at) = *reinterpret_cast<const uint4*>(h);
-    }
-  }
-}
+struct UmmaPlan {
+  int nxt, nyt;  // tiles along x and y
+  int zr, nz;    // planes per item, items along z
+  int ncog;      // output-channel groups
+  int slabs;     // slabs in the ring
+};
 
 template <int CO_T>
-__global__ void __launch_bounds__(128) k_conv3_umma(const ConvIn in, const __nv_bfloat16* __restrict__ wt,
-                                                    const ConvOut out, int ncog, int* __restrict__ err) {
+__global__ void __launch_bounds__(kThreads, 2) k_conv3_umma(const ConvIn in, const __nv_bfloat16* __restrict__ wt,
+                                                            const ConvOut out, const UmmaPlan P, int* __restrict__ err) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  constexpr int kPB = 27 * CO_T * 16;  // bytes of one 8-channel plane of one slice's weights
-  constexpr int kCols = CO_T <= 32 ? 32 : 64;
-  const int Ci = in.C1 + in.C2, nsl = Ci / 16, Co = out.Co;
-  const unsigned s_w = su32(smem);
-  const unsigned s_x = s_w + nsl * 2 * kPB;  // kBufs halo buffers
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + nsl * 2 * kPB + kBufs * kHaloBytes);
-  unsigned* tslot = reinterpret_cast<unsigned*>(bars + kBufs);
-  const int nxt = in.W / kTX, nyt = in.H / kTY, ntiles = nxt * nyt * in.D;
-  const int co0 = (blockIdx.x % ncog) * CO_T;
-  const int t0 = blockIdx.x / ncog, tstride = gridDim.x / ncog;
-  if (t0 >= ntiles) return;  // whole CTA, before any barrier
-  const int nst = ((ntiles - t0 + tstride - 1) / tstride) * nsl;
-  const int tid = threadIdx.x, warp = tid >> 5;
-  auto origin = [&](int st, int& x0, int& y0, int& z0) {
-    int t = t0 + (st / nsl) * tstride;
-    x0 = (t % nxt) * kTX;
-    t /= nxt;
-    y0 = (t % nyt) * kTY;
-    z0 = t / nyt;
-  };
-  // weights of this channel group: slice sl, plane c, row tap * CO_T + co
-  for (int i = tid; i < 27 * CO_T * nsl; i += blockDim.x) {
-    const int sl = i / (27 * CO_T), r = i % (27 * CO_T), tap = r / CO_T, co = r % CO_T;
-    const __nv_bfloat16* src = wt + ((size_t)tap * Co + co0 + co) * Ci + sl * 16;
-    const unsigned dst = s_w + sl * 2 * kPB + r * 16;
-    cp_async16(dst, src, 16);
-    cp_async16(dst + kPB, src + 8, 16);
-  }
-  {
-    int x0, y0, z0;
-    origin(0, x0, y0, z0);
-    issue_halo_planar(s_x, in, x0, y0, z0, 0);
+  constexpr int N = 3 * CO_T;
+  constexpr unsigned kWPlane = 9u * N * 16u;  // 8 channels of a slice's weights
+  const int Ci = in.C1 + in.C2, nsl = Ci / 16, Co = out.Co, H = in.H, W = in.W, D = in.D;
+  const unsigned wbytes = (unsigned)nsl * 2u * kWPlane;
+  const unsigned s_w = su32(smem), s_x = s_w + wbytes;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + wbytes + (size_t)P.slabs * kSlab);
+  const unsigned b_full = su32(bars), b_empty = b_full + 8 * kMaxSlabs, b_accf = b_empty + 8 * kMaxSlabs,
+                 b_acce = b_accf + 8 * kMaxPlanes;
+  unsigned* tslot = reinterpret_cast<unsigned*>(bars + 2 * kMaxSlabs + 2 * kMaxPlanes);
+  volatile int* abort_word = reinterpret_cast<volatile int*>(tslot + 1);
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const int co0 = (blockIdx.x % P.ncog) * CO_T;
+  const int item0 = blockIdx.x / P.ncog, item_step = gridDim.x / P.ncog, items = P.nxt * P.nyt * P.nz;
+
+  // weights of this channel group: slice, 8-channel chunk, (dy, dx), row j CO_T + co for dz = 1 - j
+  for (int i = tid; i < nsl * 9 * N * 2; i += kThreads) {
+    const int c = i & 1, r = i >> 1, n = r % N, q = r / N, yx = q % 9, sl = q / 9, j = n / CO_T, co = n % CO_T;
+    const __nv_bfloat16* src = wt + ((size_t)((2 - j) * 9 + yx) * Co + co0 + co) * Ci + sl * 16 + c * 8;
+    cp_async16(s_w + (unsigned)(sl * 2 + c) * kWPlane + (unsigned)(yx * N + n) * 16u, src, 16);
   }
   asm volatile("cp.async.commit_group;\n" ::);
   if (tid == 0) {
-    for (int b = 0; b < kBufs; ++b) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(su32(&bars[b])));
+    for (int b = 0; b < P.slabs; ++b) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(b_full + 8 * b), "r"(kCopyWarps));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(b_empty + 8 * b));
+    }
+    for (int p = 0; p < kMaxPlanes; ++p) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(b_accf + 8 * p));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(b_acce + 8 * p), "r"(kEpiWarps));
+    }
+    *abort_word = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::);
   }
-  if (warp == 0) {
+  if (warp == kMmaWarp) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su32(tslot)), "n"(kCols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
   }
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::);
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::);
   const unsigned tmem = *tslot;
-  bool failed = false;
-  for (int st = 0; st < nst; ++st) {
-    // stage s uses buffer s % kBufs and commits its MMAs to that buffer's
-    // barrier (phase s / kBufs); the buffer refilled below was last read by
-    // stage st + 1 - kBufs, whose MMAs have had a whole stage to finish
-    if (st + 1 >= kBufs && st + 1 < nst) {
-      const int old = st + 1 - kBufs;
-      const bool got = mbar_wait(su32(&bars[old % kBufs]), (old / kBufs) & 1);
-      if (!__syncthreads_and(got)) {
-        failed = true;
-        break;
+  auto item_of = [&](int it, int& x0, int& y0, int& z0, int& z1) {
+    x0 = (it % P.nxt) * kTX;
+    it /= P.nxt;
+    y0 = (it % P.nyt) * kTY;
+    z0 = (it / P.nyt) * P.zr;
+    z1 = min(z0 + P.zr, D);
+  };
+
+  if (warp >= kEpiWarps && warp < kMmaWarp) {
+    // ---- slab copies
+    constexpr int kPer = (kChunks + kCopyThreads - 1) / kCopyThreads;
+    const int t = tid - kEpiWarps * 32;
+    unsigned b = 0, phase = 1, pend = 0, pb = 0;  // ring position; slabs in flight and the oldest one's position
+    for (int it = item0; it < items; it += item_step) {
+      int x0, y0, z0, z1;
+      item_of(it, x0, y0, z0, z1);
+      for (int sl = 0; sl < nsl; ++sl) {
+        const int ci = sl * 16;
+        const bool one = ci < in.C1;
+        const int C = one ? in.C1 : in.C2, sh = one && in.up1 ? 1 : 0;
+        const __nv_bfloat16* base = one ? in.x1 + ci : in.x2 + (ci - in.C1);
+        // this thread's chunks: place in the plane (or outside the volume) and in the slab
+        int src[kPer];
+        unsigned dst[kPer];
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+          const int i = t + k * kCopyThreads, c = i & 1, v = i >> 1, y = y0 + v / kHX - 1, x = x0 + v % kHX - 1;
+          const bool inside = (unsigned)y < (unsigned)H && (unsigned)x < (unsigned)W;
+          src[k] = inside ? ((y >> sh) * (W >> sh) + (x >> sh)) * C + c * 8 : -1;
+          dst[k] = (unsigned)c * kXPlane + (unsigned)v * 16u;
+        }
+        const size_t plane = (size_t)(H >> sh) * (W >> sh) * C;
+        for (int zi = max(z0 - 1, 0); zi <= min(z1, D - 1); ++zi) {
+          wait_phase(b_empty + 8 * b, phase, abort_word);
+          const __nv_bfloat16* p = base + (size_t)(zi >> sh) * plane;
+          const unsigned to = s_x + b * kSlab;
+#pragma unroll
+          for (int k = 0; k < kPer; ++k)
+            if ((k + 1) * kCopyThreads <= kChunks || t + k * kCopyThreads < kChunks)
+              cp_async16(to + dst[k], p + max(src[k], 0), src[k] >= 0 ? 16 : 0);
+          asm volatile("cp.async.commit_group;\n" ::);
+          if (++b == (unsigned)P.slabs) {
+            b = 0;
+            phase ^= 1;
+          }
+          // the slab two copies back is complete: hand it to the tensor cores
+          if (++pend > 2) {
+            asm volatile("cp.async.wait_group 2;\n" ::: "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            arrive(b_full + 8 * pb);
+            pb = pb + 1 == (unsigned)P.slabs ? 0 : pb + 1;
+            --pend;
+          }
+        }
       }
     }
-    if (st + 1 < nst) {
-      int x0, y0, z0;
-      origin(st + 1, x0, y0, z0);
-      issue_halo_planar(s_x + ((st + 1) % kBufs) * kHaloBytes, in, x0, y0, z0, ((st + 1) % nsl) * 16);
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    for (; pend; --pend) {
+      arrive(b_full + 8 * pb);
+      pb = pb + 1 == (unsigned)P.slabs ? 0 : pb + 1;
     }
-    asm volatile("cp.async.commit_group;\n" ::);
-    asm volatile("cp.async.wait_group 1;\n" ::);
-    asm volatile("fence.proxy.async.shared::cta;" ::);
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::);
-    const int sl = st % nsl;
-    if (tid == 0) {
-      const unsigned xb = s_x + (st % kBufs) * kHaloBytes, wb = s_w + sl * 2 * kPB;
-      for (int tap = 0; tap < 27; ++tap) {
-        const int dz = tap / 9, dy = (tap / 3) % 3, dx = tap % 3;
-        const uint64_t ad = smem_desc(xb + ((dz * kHY + dy) * kHX + dx) * 16, kPlane, kHX * 16);
-        const uint64_t bd = smem_desc(wb + tap * CO_T * 16, kPB, 128);
-        const unsigned accumulate = (sl > 0 || tap > 0) ? 1u : 0u;
-        asm volatile(
-            "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(tmem),
-            "l"(ad), "l"(bd), "r"(idesc_bf16(CO_T)), "r"(accumulate));
+  } else if (warp == kMmaWarp) {
+    // ---- MMAs: a slab at zi into the output planes zi - 1 + j, j = 0, 1, 2 (dz = 1 - j), those of the item
+    unsigned b = 0, phase = 0;
+    unsigned pe = 0xffffffffu;  // parity to wait for before a plane is summed anew, by plane
+    for (int it = item0; it < items; it += item_step) {
+      int x0, y0, z0, z1;
+      item_of(it, x0, y0, z0, z1);
+      const int zf = max(z0 - 1, 0), zl = min(z1, D - 1);
+      for (int sl = 0; sl < nsl; ++sl) {
+        const unsigned w0 = desc_lo(s_w + (unsigned)sl * 2u * kWPlane, kWPlane);
+        for (int zi = zf; zi <= zl; ++zi) {
+          const int jlo = max(0, z0 - zi + 1), jhi = min(2, z1 - zi);
+          const int jnew = min(max(sl ? 3 : (zi == 0 ? 1 : 2), jlo), jhi + 1);  // planes from here on start with this slab
+          wait_phase(b_full + 8 * b, phase, abort_word);
+          for (int j = jnew; j <= jhi; ++j) {
+            const int k = zi - 1 + j - z0;
+            wait_phase(b_acce + 8 * k, (pe >> k) & 1, abort_word);
+            pe ^= 1u << k;
+          }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::);
+          const unsigned a0 = desc_lo(s_x + b * kSlab, kXPlane);
+          const unsigned d = tmem + (unsigned)((zi - 1 - z0 + jlo) * CO_T), wj = w0 + (unsigned)(jlo * CO_T);
+          const unsigned idesc = idesc_bf16(0) + ((unsigned)((jhi - jlo + 1) * CO_T / 8) << 17);
+          if (elect_one()) {
+            if (jnew > jhi) {
+              mma(d, a0, wj, idesc, 1u);
+            } else {  // the first tap pair overwrites in the planes that start here
+              if (jnew > jlo) mma(d, a0, wj, idesc_bf16(0) + ((unsigned)((jnew - jlo) * CO_T / 8) << 17), 1u);
+              mma(d + (unsigned)((jnew - jlo) * CO_T), a0, w0 + (unsigned)(jnew * CO_T),
+                  idesc_bf16(0) + ((unsigned)((jhi - jnew + 1) * CO_T / 8) << 17), 0u);
+            }
+#pragma unroll
+            for (int q = 1; q < 9; ++q) mma(d, a0 + (unsigned)((q / 3) * kHX + q % 3), wj + (unsigned)(q * N), idesc, 1u);
+            commit_to(b_empty + 8 * b);
+            if (sl == nsl - 1) {  // output planes whose last slab this was
+              if (zi - 1 >= z0) commit_to(b_accf + 8 * (zi - 1 - z0));
+              if (zi == D - 1 && zi < z1) commit_to(b_accf + 8 * (zi - z0));
+            }
+          }
+          __syncwarp();
+          if (++b == (unsigned)P.slabs) {
+            b = 0;
+            phase ^= 1;
+          }
+        }
       }
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-          su32(&bars[st % kBufs])));
     }
-    if (sl == nsl - 1) {
-      const bool got = mbar_wait(su32(&bars[st % kBufs]), (st / kBufs) & 1);
-      if (!__syncthreads_and(got)) {
-        failed = true;
-        break;
+  } else {
+    // ---- epilogue: thread (warp w, lane l) owns accumulator row 32 w + l, voxel (x0 + row % 8, y0 + row / 8)
+    const int m = warp * 32 + lane;
+    const float slope = out.relu ? out.slope : 1.f;  // v > 0 ? v : slope v = max(v, slope v) for slopes up to 1
+    unsigned pf = 0;
+    for (int it = item0; it < items; it += item_step) {
+      int x0, y0, z0, z1;
+      item_of(it, x0, y0, z0, z1);
+      size_t at0 = (((size_t)z0 * H + (y0 + (m >> 3))) * W + (x0 + (m & 7))) * Co + co0;
+      for (int zo = z0; zo < z1; ++zo, at0 += (size_t)H * W * Co) {
+        const int k = zo - z0;
+        wait_phase(b_accf + 8 * k, (pf >> k) & 1, abort_word);
+        pf ^= 1u << k;
+        __syncwarp();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::);
+        unsigned r[CO_T];
+#pragma unroll
+        for (int j = 0; j < CO_T / 16; ++j)
+          tmem_ld16(tmem + ((unsigned)(warp * 32) << 16) + (unsigned)(k * CO_T + 16 * j), r + 16 * j);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int q = 0; q < CO_T; ++q) asm volatile("" : "+r"(r[q]));  // uses stay after the wait
+        asm volatile("tcgen05.fence::before_thread_sync;" ::);
+        arrive(b_acce + 8 * k);
+#pragma unroll
+        for (int c8 = 0; c8 < CO_T / 8; ++c8) {
+          float v[8];
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            float t = __uint_as_float(r[c8 * 8 + q]);
+            if (out.bias) t += __ldg(out.bias + co0 + c8 * 8 + q);
+            v[q] = fmaxf(t, slope * t);
+          }
+          const size_t at = at0 + c8 * 8;
+          if (out.mask) {
+            const uint4 mk = *reinterpret_cast<const uint4*>(out.mask + at);
+            const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&mk);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              if (!(__low2float(h[q]) > 0.f)) v[2 * q] *= out.mask_slope;
+              if (!(__high2float(h[q]) > 0.f)) v[2 * q + 1] *= out.mask_slope;
+            }
+          }
+          if (out.yf) {
+            float4* d = reinterpret_cast<float4*>(out.yf + at);
+            d[0] = make_float4(v[0], v[1], v[2], v[3]);
+            d[1] = make_float4(v[4], v[5], v[6], v[7]);
+          } else {
+            __align__(16) __nv_bfloat162 h[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) h[q] = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
+            *reinterpret_cast<uint4*>(out.y + at) = *reinterpret_cast<const uint4*>(h);
+          }
+        }
       }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::);
-      int x0, y0, z0;
-      origin(st, x0, y0, z0);
-      umma_epilogue<CO_T>(tmem, in, out, x0, y0, z0, co0);
-      asm volatile("tcgen05.fence::before_thread_sync;" ::);
     }
-    __syncthreads();
   }
-  asm volatile("cp.async.wait_all;\n" ::);
-  if (failed && tid == 0) atomicOr(err, DF_TIMEOUT);
   asm volatile("tcgen05.fence::before_thread_sync;" ::);
   __syncthreads();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(kCols));
+  if (tid == 0 && *abort_word) atomicOr(err, DF_TIMEOUT);
+  if (warp == kMmaWarp) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::);
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(kCols));
+  }
 }
+
+constexpr size_t weight_bytes(int Ci, int co_t) { return (size_t)27 * Ci * co_t * 2; }
 
 template <int CO_T>
 vg_status launch_umma(Ctx* c, const ConvIn& in, const __nv_bfloat16* wt, const ConvOut& out) {
-  const int Ci = in.C1 + in.C2, ncog = out.Co / CO_T;
-  const size_t smem = (size_t)(Ci / 16) * 2 * 27 * CO_T * 16 + kBufs * kHaloBytes + 64;
+  const size_t wbytes = weight_bytes(in.C1 + in.C2, CO_T);
+  const bool two = wbytes + kMinSlabs * kSlab + kTail <= kSmemTwo;
+  UmmaPlan P;
+  P.nxt = in.W / kTX;
+  P.nyt = in.H / kTY;
+  P.ncog = out.Co / CO_T;
+  P.slabs = (int)std::min<size_t>(kMaxSlabs, ((two ? kSmemTwo : kSmemOne) - wbytes - kTail) / kSlab);
+  // planes per item: the fewest rounds of items over the CTAs, counting the two extra input planes of an item
+  const int ctas = std::max(1, (two ? 2 : 1) * sm_count() / P.ncog), zmax = std::min(in.D, kCols / CO_T);
+  double best = 1e30;
+  P.zr = 1;
+  for (int zr = 1; zr <= zmax; ++zr) {
+    const int nz = (in.D + zr - 1) / zr;
+    const double cost = (double)((P.nxt * P.nyt * nz + ctas - 1) / ctas) * (zr + 2);
+    if (cost < best - 1e-9) {
+      best = cost;
+      P.zr = zr;
+    }
+  }
+  P.nz = (in.D + P.zr - 1) / P.zr;
+  const size_t smem = wbytes + P.slabs * (size_t)kSlab + kTail;
   VG_CUDA(c, cudaFuncSetAttribute(k_conv3_umma<CO_T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   VG_CUDA(c, cudaFuncSetAttribute(k_conv3_umma<CO_T>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-  // CTAs per SM: shared memory (228 KB per SM, 1 KB reserved per CTA) and the
-  // 512 tensor-memory columns bound it; extra CTAs would only queue
-  constexpr int kCols = CO_T <= 32 ? 32 : 64;
-  const int per_sm = std::max(1, std::min<int>(std::min<int>((228 * 1024) / (int)(smem + 1024), 512 / kCols), 8));
-  const long items = (long)(in.W / kTX) * (in.H / kTY) * in.D * ncog;
-  long grid = std::min<long>(items, (long)std::max(per_sm, 1) * sm_count());
-  grid = std::max<long>(ncog, grid / ncog * ncog);
-  k_conv3_umma<CO_T><<<(unsigned)grid, 128, smem, c->stream>>>(in, wt, out, ncog, c->dflag);
+  const int grid = P.ncog * std::min(ctas, P.nxt * P.nyt * P.nz);
+  k_conv3_umma<CO_T><<<(unsigned)grid, kThreads, smem, c->stream>>>(in, wt, out, P, c->dflag);
   VG_LAUNCHED(c);
   VG_CUDA(c, cudaGetLastError());
   return VG_OK;
@@ -290,19 +396,18 @@ bool conv3_umma_fits(const ConvIn& in, int Co) {
 vg_status conv3_fwd_umma(Ctx* c, const ConvIn& in, const __nv_bfloat16* wt, const ConvOut& out, bool* handled) {
   *handled = false;
   if (!conv3_umma_fits(in, out.Co) || !c->dflag) return VG_OK;
-  const size_t Ci = (size_t)(in.C1 + in.C2);
-  const int cands[4] = {out.Co == 48 ? 48 : 64, 32, 16, 0};
-  for (int k = 0; cands[k]; ++k) {
-    const int co_t = cands[k];
-    if (out.Co % co_t || 27 * (size_t)co_t * Ci * 2 > kUmmaWeightBytes) continue;
-    *handled = true;
-    switch (co_t) {
-      case 64: return launch_umma<64>(c, in, wt, out);
-      case 48: return launch_umma<48>(c, in, wt, out);
-      case 32: return launch_umma<32>(c, in, wt, out);
-      default: return launch_umma<16>(c, in, wt, out);
-    }
+  const int Ci = in.C1 + in.C2;
+  auto fits = [&](int co_t, size_t smem) {
+    return out.Co % co_t == 0 && weight_bytes(Ci, co_t) + kMinSlabs * kSlab + kTail <= smem;
+  };
+  *handled = true;
+  // the widest group at two CTAs per SM, else at one
+  for (const size_t smem : {kSmemTwo, kSmemOne}) {
+    if (fits(48, smem) && out.Co % 32) return launch_umma<48>(c, in, wt, out);
+    if (fits(32, smem)) return launch_umma<32>(c, in, wt, out);
+    if (fits(16, smem)) return launch_umma<16>(c, in, wt, out);
   }
+  *handled = false;
   return VG_OK;
 }
 
