@@ -466,8 +466,12 @@ vg_status backward(Ctx* c, Net* N) {
     const LayerDesc& L = kNet[l];
     const int e = N->dims(L.level);
     const size_t nv = N->vox(L.level);
-    if ((st = conv3_wgrad(c, layer_input(N, l), N->g[l], L.co, N->grad + N->wofs[l])) != VG_OK) return st;
-    {
+    bool handled = false;
+    if ((st = conv3_wgrad_rows(c, layer_input(N, l), N->g[l], L.co, N->grad + N->wofs[l], N->grad + N->bofs[l],
+                               &handled)) != VG_OK)
+      return st;
+    if (!handled) {
+      if ((st = conv3_wgrad(c, layer_input(N, l), N->g[l], L.co, N->grad + N->wofs[l])) != VG_OK) return st;
       const int lanes = 256 / L.co;
       unsigned nb = (unsigned)std::min<size_t>((nv + lanes - 1) / lanes, 4 * (size_t)sm_count());
       k_colsum<<<nb, 256, 0, c->stream>>>(N->g[l], nv, L.co, N->grad + N->bofs[l]);

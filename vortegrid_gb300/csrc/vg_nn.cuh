@@ -46,6 +46,8 @@ vg_status conv3_fwd(Ctx* c, const ConvIn& in, const __nv_bfloat16* wt, const Con
 vg_status conv3_fwd_umma(Ctx* c, const ConvIn& in, const __nv_bfloat16* wt, const ConvOut& out, bool* handled);
 // dW[27][Co][Ci] += sum over voxels of dY (x) X_tap  (FP32, accumulated atomically)
 vg_status conv3_wgrad(Ctx* c, const ConvIn& in, const __nv_bfloat16* dy, int Co, float* dw);
+// The same, and db[Co] += sum over voxels of dY, over whole x rows (W = 16, 32, 64 or 128; vg_nn_wgrad.cu).
+vg_status conv3_wgrad_rows(Ctx* c, const ConvIn& in, const __nv_bfloat16* dy, int Co, float* dw, float* db, bool* handled);
 
 }  // namespace nn
 }  // namespace vg
