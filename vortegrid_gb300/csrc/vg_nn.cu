@@ -40,7 +40,7 @@ namespace nn {
 namespace {
 
 constexpr int kLayers = 15;
-constexpr int kRedBlocks = 304;  // partial sums of the norm reductions (a fixed width)
+constexpr int kRedBlocks = 608;  // partial sums of the norm reductions (a fixed width)
 constexpr float kSlope = 0.1f;  // leaky ReLU: v > 0 ? v : kSlope v
 
 struct LayerDesc {
@@ -115,21 +115,55 @@ __device__ __forceinline__ void block_sum_to(double v, double* dst) {
 __device__ __forceinline__ float ld(const float* p, size_t i) { return p[i]; }
 __device__ __forceinline__ float ld(const __nv_bfloat16* p, size_t i) { return __bfloat162float(p[i]); }
 
+// A running sum of squares as an unevaluated pair of floats: the square split exactly by an FMA, the sum error-free
+// (TwoSum), so that the pair keeps ~2^-46 relative accuracy without GB300's low-rate FP64 pipe (the sum over 129^3 x 3
+// values took 46 us in FP64, 17 us in pairs).
+struct PairSum {
+  float hi = 0.f, lo = 0.f;
+  __device__ __forceinline__ void add_square(float v) {
+    const float p = __fmul_rn(v, v), e = __fmaf_rn(v, v, -p);
+    const float t = __fadd_rn(hi, p), b = __fsub_rn(t, hi);
+    lo = __fadd_rn(lo, __fadd_rn(__fadd_rn(__fsub_rn(hi, __fsub_rn(t, b)), __fsub_rn(p, b)), e));
+    hi = t;
+  }
+  // Whether no square can have left the range of floats unseen; otherwise the caller sums in FP64.
+  __device__ __forceinline__ bool sound() const { return hi > 1e-22f && hi < 1e36f; }
+  __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
+};
+
 // Sum of squares of count values, one fixed partial per block (deterministic).
 template <typename T>
 __global__ void k_sumsq(const T* __restrict__ a, size_t count, double* __restrict__ partials) {
-  double s = 0.0;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x) {
-    const float v = ld(a, i);
-    s += (double)v * v;
+  PairSum s;
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (; i + 7 * stride < count; i += 8 * stride) {  // eight loads in flight
+    float v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = ld(a, i + k * stride);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) s.add_square(v[k]);
   }
-  block_sum_to(s, partials + blockIdx.x);
+  for (; i < count; i += stride) s.add_square(ld(a, i));
+  double v = s.value();
+  if (!s.sound()) {
+    v = 0.0;
+    for (i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += stride) v += (double)ld(a, i) * ld(a, i);
+  }
+  block_sum_to(v, partials + blockIdx.x);
+}
+
+// The sum of nb partials by one warp, in a fixed order (every lane returns it).
+__device__ __forceinline__ double warp_sum_partials(const double* __restrict__ partials, int nb) {
+  double s = 0.0;
+  for (int i = threadIdx.x; i < nb; i += 32) s += partials[i];
+  for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
 }
 
 __global__ void k_scales(const double* __restrict__ partials, int nb, double count, float h2k, float* scales) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double s = 0.0;
-  for (int i = 0; i < nb; ++i) s += partials[i];
+  const double s = warp_sum_partials(partials, nb);
+  if (threadIdx.x != 0) return;
   double rms = sqrt(s / count);
   if (!(rms > 0.0) || !isfinite(rms)) rms = 1.0;
   scales[0] = (float)(1.0 / rms);
@@ -195,29 +229,36 @@ __global__ void k_unpack_output(const float* __restrict__ out, int n, const floa
 template <typename T>
 __global__ void k_target_energy(const T* __restrict__ vp, int n, const float* __restrict__ scales,
                                 double* __restrict__ partials) {
-  double s = 0.0;
-  const size_t nv = (size_t)n * n * n;
+  PairSum s;
   const int np = n + 1;
   const float s_t = scales[1];
-  for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += (size_t)gridDim.x * blockDim.x) {
-    const int i = (int)(v % n), j = (int)((v / n) % n), k = (int)(v / ((size_t)n * n));
-    if (i && j && k) {
-      const size_t p = ((size_t)k * np + j) * np + i;
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const float t = ld(vp, 3 * p + c) * s_t;
-        s += (double)t * t;
+  double sum = 0.0;
+  // interior rows (j, k) dealt to the warps, a row's values to its lanes; in FP64 where pairs of floats are not sound
+  for (int pass = 0; pass < 2; ++pass) {
+    for (int r = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32; r < (n - 1) * (n - 1); r += gridDim.x * (blockDim.x / 32)) {
+      const int j = 1 + r % (n - 1), k = 1 + r / (n - 1);
+      const T* row = vp + 3 * (((size_t)k * np + j) * np);
+#pragma unroll 4
+      for (int x = 3 + (int)(threadIdx.x & 31); x < 3 * n; x += 32) {
+        const float t = ld(row, x) * s_t;
+        if (pass)
+          sum += (double)t * t;
+        else
+          s.add_square(t);
       }
     }
+    if (pass == 0 && s.sound()) {
+      sum = s.value();
+      break;
+    }
   }
-  block_sum_to(s, partials + blockIdx.x);
+  block_sum_to(sum, partials + blockIdx.x);
 }
 
 // e[1] = target energy (1 if zero), e[2] = 2 / e[1] (the loss gradient's scale)
 __global__ void k_finish_energy(const double* __restrict__ partials, int nb, float* e) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double s = 0.0;
-  for (int i = 0; i < nb; ++i) s += partials[i];
+  double s = warp_sum_partials(partials, nb);
+  if (threadIdx.x != 0) return;
   if (!(s > 0.0) || !isfinite(s)) s = 1.0;
   e[1] = (float)s;
   e[2] = (float)(2.0 / s);
@@ -230,7 +271,7 @@ template <typename T>
 __global__ void k_loss_grad(const float* __restrict__ out, const T* __restrict__ vp, int n,
                             const float* __restrict__ scales, const float* __restrict__ e,
                             __nv_bfloat16* __restrict__ g, double* __restrict__ partials) {
-  double s = 0.0;
+  PairSum s;
   const size_t nv = (size_t)n * n * n;
   const int np = n + 1;
   const float s_t = scales[1], gscale = e[2];
@@ -240,10 +281,9 @@ __global__ void k_loss_grad(const float* __restrict__ out, const T* __restrict__
     if (i && j && k) {
       const size_t p = ((size_t)k * np + j) * np + i;
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        d[c] = out[v * 16 + c] - ld(vp, 3 * p + c) * s_t;
-        s += (double)d[c] * d[c];
-      }
+      for (int c = 0; c < 3; ++c) d[c] = __ldg(out + v * 16 + c) - ld(vp, 3 * p + c) * s_t;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) s.add_square(d[c]);
     }
     __align__(16) __nv_bfloat162 h[8];
     h[0] = __floats2bfloat162_rn(d[0] * gscale, d[1] * gscale);
@@ -254,14 +294,26 @@ __global__ void k_loss_grad(const float* __restrict__ out, const T* __restrict__
     dst[0] = *reinterpret_cast<const uint4*>(&h[0]);
     dst[1] = *reinterpret_cast<const uint4*>(&h[4]);
   }
-  block_sum_to(s, partials + blockIdx.x);
+  double sum = s.value();
+  if (!s.sound()) {
+    sum = 0.0;
+    for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += (size_t)gridDim.x * blockDim.x) {
+      const int i = (int)(v % n), j = (int)((v / n) % n), k = (int)(v / ((size_t)n * n));
+      if (!i || !j || !k) continue;
+      const size_t p = ((size_t)k * np + j) * np + i;
+      for (int c = 0; c < 3; ++c) {
+        const float d = out[v * 16 + c] - ld(vp, 3 * p + c) * s_t;
+        sum += (double)d * d;
+      }
+    }
+  }
+  block_sum_to(sum, partials + blockIdx.x);
 }
 
 // e[0] = loss = sum of squared differences / target energy
 __global__ void k_finish_loss(const double* __restrict__ partials, int nb, float* e) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double s = 0.0;
-  for (int i = 0; i < nb; ++i) s += partials[i];
+  const double s = warp_sum_partials(partials, nb);
+  if (threadIdx.x != 0) return;
   e[0] = (float)(s / (double)e[1]);
 }
 
