@@ -220,6 +220,7 @@ enum Slot {
   S_JAC,
   S_WOLD,
   S_MG,
+  S_MGSPLIT,  // multigrid: split fields of the smoothed levels
   S_DIRECT,
   S_POS,
   S_ANGVEL,
@@ -241,7 +242,9 @@ enum Slot {
   S_NUM
 };
 
-// A captured multigrid cycle, replayed while the grid and buffers are unchanged.
+// Captured multigrid cycles, replayed while the grid and buffers are unchanged: the iterate and the refinement's correction
+// each go to and fro between two buffers, and a first correction starts from none.
+constexpr int kMgGraphs = 8;
 struct MgGraphCache {
   cudaGraphExec_t exec = nullptr;
   Geom g;
@@ -256,7 +259,8 @@ struct Net;
 struct Ctx {
   vg_config cfg;
   nn::Net* net = nullptr;   // attached warm-start network (not owned)
-  MgGraphCache mg_graph[2];  // phase-1 and phase-2 cycle graphs
+  MgGraphCache mg_graph[kMgGraphs];  // cycle graphs, replaced in turn
+  int mg_graph_next = 0;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
   std::string err;

@@ -285,67 +285,6 @@ __device__ __forceinline__ void rbgs_point(const Geom& g, float r2x, float r2y, 
   }
 }
 
-// Point red-black Gauss-Seidel on L e = r (FP32).  One thread per component
-// of an interior point of `color`: threadIdx.x runs along a row over
-// (point j, component c) pairs -- x = 1 + parity + 2 j, components adjacent --
-// so a warp reads ~11 points' worth of consecutive floats of the AoS field
-// instead of 32 points 24 bytes apart; y and z come from the block index
-// (launch_rows), so no thread divides by a grid size.  zero_first: e is zero
-// before this sweep, so the red points take -r H directly.
-__global__ void __launch_bounds__(256) k_rbgs(Geom g, float r2x, float r2y, float r2z, float H,
-                                              float* __restrict__ e, const float* __restrict__ r, unsigned color,
-                                              int zero_first) {
-  pdl_entry();
-  const unsigned nx = g.np[0], ny = g.np[1];
-  const unsigned jc = blockIdx.x * blockDim.x + threadIdx.x;
-  const unsigned y = blockIdx.y * blockDim.y + threadIdx.y + 1, z = blockIdx.z + 1;
-  const unsigned j = jc / 3u, c = jc - 3u * j;
-  const unsigned x = 1u + ((color + 1u + y + z) & 1u) + 2u * j;
-  if (y + 1 >= ny || x + 1 >= nx) return;
-  const unsigned k = x + nx * (y + ny * z);
-  const unsigned sy = nx, sz = nx * ny;
-  float v;
-  if (zero_first) {
-    v = sor_value(0.f, __fmul_rn(-r[3 * k + c], H));
-  } else {
-    const float sx = __fadd_rn(e[3 * (k + 1) + c], e[3 * (k - 1) + c]);
-    const float syv = __fadd_rn(e[3 * (k + sy) + c], e[3 * (k - sy) + c]);
-    const float szv = __fadd_rn(e[3 * (k + sz) + c], e[3 * (k - sz) + c]);
-    v = sor_value(e[3 * k + c], gs_value(sx, syv, szv, r[3 * k + c], r2x, r2y, r2z, H));
-  }
-  e[3 * k + c] = v;
-}
-
-// The first pre-smoothing sweep from e = 0, both colours in one pass: red
-// points take -r H, black points the Gauss-Seidel update from those red
-// values (recomputed from r, the same float operations as the two half
-// sweeps, so the result is identical).  Threads over every interior (point,
-// component), as k_rbgs_add.
-__global__ void __launch_bounds__(256) k_rbgs_first(Geom g, float r2x, float r2y, float r2z, float H,
-                                                    float* __restrict__ e, const float* __restrict__ r) {
-  pdl_entry();
-  const unsigned nx = g.np[0], ny = g.np[1];
-  const unsigned jc = blockIdx.x * blockDim.x + threadIdx.x;
-  const unsigned y = blockIdx.y * blockDim.y + threadIdx.y + 1, z = blockIdx.z + 1;
-  const unsigned j = jc / 3u, c = jc - 3u * j;
-  const unsigned x = 1u + j;
-  if (y + 1 >= ny || x + 1 >= nx) return;
-  const unsigned k = x + nx * (y + ny * z), t = 3 * k + c;
-  float v;
-  if (((x + y + z) & 1u) == 0u) {
-    v = sor_value(0.f, __fmul_rn(-r[t], H));
-  } else {
-    const unsigned sy = nx, sz = nx * ny;
-    // red neighbours: omega (-r H) (boundary neighbours stay e = 0)
-    auto red = [&](unsigned n, bool in) { return in ? sor_value(0.f, __fmul_rn(-r[3 * n + c], H)) : 0.f; };
-    const float sx = __fadd_rn(red(k + 1, x + 2 < nx), red(k - 1, x > 1));
-    const float syv = __fadd_rn(red(k + sy, y + 2 < ny), red(k - sy, y > 1));
-    const float szv = __fadd_rn(red(k + sz, z + 2 < g.np[2]), red(k - sz, z > 1));
-    v = sor_value(0.f, gs_value(sx, syv, szv, r[t], r2x, r2y, r2z, H));
-  }
-  e[t] = v;
-}
-
 // Fused FP32 residual + full-weighting restriction at coarse interior point
 // (x, y, z): the fine residuals r - L e at the 27 fine points around
 // (2x, 2y, 2z) with weights 8/4/2/1 / 64, recomputed instead of writing the
@@ -380,66 +319,10 @@ __device__ __forceinline__ void residual_restrict_point(const Geom& F, const Geo
   rc[3 * k + 2] = __fmul_rn(acc[2], s);
 }
 
-// Global-memory form, tiled: a CTA owns kRTX x kRTY x kRTZ coarse points.  It
-// first computes the fine residuals r - L e of the (2 kRTX + 1) x (2 kRTY + 1)
-// x (2 kRTZ + 1) fine points around them into shared memory (coalesced along
-// fine rows, each fine residual evaluated once per tile instead of once per
-// coarse neighbour), then each (coarse point, component) sums its 27 fine
-// residuals in the order of residual_restrict_point.  Coarse boundary points
-// are never read, so they are not written.
+// The persistent solve's tiles: kRTX x kRTY x kRTZ coarse points from the fine residuals of the (2 kRTX + 1) x (2 kRTY + 1)
+// x (2 kRTZ + 1) points around them.
 constexpr int kRTX = 16, kRTY = 4, kRTZ = 2;
 constexpr int kRFX = 2 * kRTX + 1, kRFY = 2 * kRTY + 1, kRFZ = 2 * kRTZ + 1;
-__global__ void __launch_bounds__(256) k_residual_restrict(Geom F, Geom C, float r2x, float r2y, float r2z,
-                                                           const float* __restrict__ e, const float* __restrict__ r,
-                                                           float* __restrict__ rc) {
-  pdl_entry();
-  __shared__ float s_res[kRFX * kRFY * kRFZ * 3];
-  const unsigned cx0 = 1 + blockIdx.x * kRTX, cy0 = 1 + blockIdx.y * kRTY, cz0 = 1 + blockIdx.z * kRTZ;
-  const unsigned nx = F.np[0], ny = F.np[1], nz = F.np[2];
-  const unsigned sy = nx, sz = nx * ny;
-  // fine local (0, 0, 0) is fine (2 cx0 - 1, 2 cy0 - 1, 2 cz0 - 1)
-  for (unsigned p = threadIdx.x; p < (unsigned)(kRFX * kRFY * kRFZ); p += blockDim.x) {
-    const unsigned lx = p % kRFX, q = p / kRFX;
-    const unsigned ly = q % kRFY, lz = q / kRFY;
-    const unsigned fx = 2 * cx0 - 1 + lx, fy = 2 * cy0 - 1 + ly, fz = 2 * cz0 - 1 + lz;
-    float v[3] = {0.f, 0.f, 0.f};
-    if (fx + 1 < nx && fy + 1 < ny && fz + 1 < nz) {  // fx, fy, fz >= 1 by construction
-      const unsigned o = fx + sy * fy + sz * fz;
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const float lap = lap7(e[3 * o + c], e[3 * (o + 1) + c], e[3 * (o - 1) + c], e[3 * (o + sy) + c],
-                               e[3 * (o - sy) + c], e[3 * (o + sz) + c], e[3 * (o - sz) + c], r2x, r2y, r2z);
-        v[c] = __fsub_rn(r[3 * o + c], lap);
-      }
-    }
-    s_res[3 * p] = v[0];
-    s_res[3 * p + 1] = v[1];
-    s_res[3 * p + 2] = v[2];
-  }
-  __syncthreads();
-  // levels halve exactly, so the 27 fine points of a coarse interior point
-  // are all interior
-  for (unsigned i = threadIdx.x; i < (unsigned)(kRTX * kRTY * kRTZ * 3); i += blockDim.x) {
-    const unsigned c = i % 3u, p = i / 3u;
-    const unsigned lx = p % kRTX, q = p / kRTX;
-    const unsigned ly = q % kRTY, lz = q / kRTY;
-    const unsigned x = cx0 + lx, y = cy0 + ly, z = cz0 + lz;
-    if (x + 1 >= C.np[0] || y + 1 >= C.np[1] || z + 1 >= C.np[2]) continue;
-    const float* sr = s_res + 3 * ((2 * lx + 1) + kRFX * ((2 * ly + 1) + kRFY * (2 * lz + 1))) + c;
-    float acc = 0.f;
-#pragma unroll
-    for (int dz = -1; dz <= 1; ++dz)
-#pragma unroll
-      for (int dy = -1; dy <= 1; ++dy)
-#pragma unroll
-        for (int dx = -1; dx <= 1; ++dx) {
-          const float wt = (float)(8 >> (abs(dx) + abs(dy) + abs(dz)));
-          acc = __fmaf_rn(wt, sr[3 * (dx + kRFX * (dy + kRFY * dz))], acc);
-        }
-    rc[3 * (x + C.np[0] * (y + C.np[1] * z)) + c] = __fmul_rn(acc, 1.0f / 64.0f);
-  }
-}
-
 // e_fine += trilinear(e_coarse) at fine interior point (x, y, z).
 __device__ __forceinline__ void prolong_point(const Geom& F, const Geom& C, const float* __restrict__ ec,
                                               float* __restrict__ ef, unsigned x, unsigned y, unsigned z) {
@@ -462,130 +345,521 @@ __device__ __forceinline__ void prolong_point(const Geom& F, const Geom& C, cons
   ef[3 * k + 2] += a2 * wt;
 }
 
-// Global-memory form for small levels: one thread per coarse cell (cx .. cx+1) x (cy .. cy+1) x
-// (cz .. cz+1), all three components: it reads the cell's 8 corners once and
-// updates the 8 fine points (2 cx + ox, 2 cy + oy, 2 cz + oz) with the same
-// sums in the same order as prolong_point (fine boundary points skipped).
-__global__ void __launch_bounds__(256) k_prolong_cells(Geom F, Geom C, const float* __restrict__ ec,
-                                                     float* __restrict__ ef) {
-  pdl_entry();
-  const unsigned cx = blockIdx.x * blockDim.x + threadIdx.x;
-  const unsigned cy = blockIdx.y * blockDim.y + threadIdx.y, cz = blockIdx.z;
-  if (cx + 1 >= C.np[0] || cy + 1 >= C.np[1]) return;
-  const unsigned sy = C.np[0], sz = C.np[0] * C.np[1];
-  const unsigned c0 = cx + sy * cy + sz * cz;
-  float v[2][2][2][3];  // [iz][iy][ix][component]
-#pragma unroll
-  for (int iz = 0; iz < 2; ++iz)
-#pragma unroll
-    for (int iy = 0; iy < 2; ++iy)
-#pragma unroll
-      for (int ix = 0; ix < 2; ++ix)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) v[iz][iy][ix][c] = ec[3 * (c0 + ix + sy * iy + sz * iz) + c];
-  const unsigned fsy = F.np[0], fsz = F.np[0] * F.np[1];
-#pragma unroll
-  for (int oz = 0; oz < 2; ++oz)
-#pragma unroll
-    for (int oy = 0; oy < 2; ++oy)
-#pragma unroll
-      for (int ox = 0; ox < 2; ++ox) {
-        const unsigned X = 2 * cx + ox, Y = 2 * cy + oy, Z = 2 * cz + oz;
-        if (X == 0 || Y == 0 || Z == 0) continue;  // X <= nx - 2 etc. always
-        const float wt = 1.0f / (float)(1u << (ox + oy + oz));
-        const unsigned k = X + fsy * Y + fsz * Z;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          float a = 0.f;
-#pragma unroll
-          for (int iz = 0; iz <= oz; ++iz)
-#pragma unroll
-            for (int iy = 0; iy <= oy; ++iy)
-#pragma unroll
-              for (int ix = 0; ix <= ox; ++ix) a += v[iz][iy][ix][c];
-          ef[3 * k + c] += a * wt;
-        }
-      }
+
+// ------------------------------------------------------- split levels
+//
+// The fields of the smoothed levels are kept split: per component and colour (parity of x + y + z) a plane-by-plane array of
+// rows, row (y, z) holding that colour's points, x = 2 i + p at i with p = (colour + y + z) & 1.  An even number of cells per
+// axis is what makes a level a smoothed one, so nx = 2 m + 1; rows are padded to a multiple of four floats.  In a row the
+// points of even x and of odd x lie in the two colours' arrays, and a point's neighbours along y and z, which have the
+// other colour, at its own i.
+//
+// Why: a half sweep of red-black relaxation updates every other point.  On interleaved float[3] points it moved every
+// sector of e and r for half of the values and worked on scattered floats; split, it reads what it needs, four points of one
+// colour and component a thread as float4, and with the threads marching a few planes along z a value of the other colour
+// comes from L2 once and not three times.  The point arithmetic is unchanged, and so is every result.
+//
+// GB300, 129^3 (fields of 26 MB, mostly in the 129 MB L2), us a launch, interleaved -> split: half sweep 13.1 -> 9..7; first
+// sweep 30.6 -> 11.3; residual + restriction 26.2 -> 18.8; prolongation 18.3 -> 10.9; x += e and the residual 9.0 + 18.0 ->
+// 30 (one pass, but of five fields, which no longer fit the L2 together).
+struct SGeo {
+  unsigned nx, ny, nz, m, hx, groups;  // points, (nx - 1) / 2, floats of a row, float4 groups that hold interior points
+  size_t cs;                           // floats of one component and colour
+  float r2x, r2y, r2z, H;
+  unsigned pz;                         // floats of a plane
+};
+
+static SGeo split_geo(const Lev& L) {
+  SGeo g;
+  g.nx = L.g.np[0];
+  g.ny = L.g.np[1];
+  g.nz = L.g.np[2];
+  g.m = (g.nx - 1) / 2;
+  g.hx = (g.m + 1 + 3) / 4 * 4;
+  g.groups = (g.m + 3) / 4;
+  g.pz = g.hx * g.ny;
+  g.cs = (size_t)g.pz * g.nz;
+  g.r2x = L.r2x;
+  g.r2y = L.r2y;
+  g.r2z = L.r2z;
+  g.H = L.H;
+  return g;
 }
 
-// Global-memory form: a CTA of kPCX x kPCY x kPCZ threads, one per coarse
-// cell (cx .. cx+1) x (cy .. cy+1) x (cz .. cz+1).  Each thread reads its
-// cell's 8 corners once and forms the increments of the 8 fine points
-// (2 cx + ox, 2 cy + oy, 2 cz + oz), all three components, with the same sums
-// in the same order as prolong_point; the increments go through shared memory
-// so that the read-modify-write of the fine field runs along whole fine rows
-// (per-thread 24-byte runs would write every sector in pieces).  Fine
-// boundary points are skipped.
-template <int kPCX, int kPCY, int kPCZ>
-__global__ void __launch_bounds__(kPCX * kPCY * kPCZ) k_prolong_add(Geom F, Geom C, const float* __restrict__ ec,
-                                                                   float* __restrict__ ef) {
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ void st4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+
+// Launch shape over the interior rows of a level: blocks of (groups, rows), whole warps, `zs` planes per thread, three
+// components in the z index.
+struct SLaunch {
+  dim3 grid, block;
+  unsigned zs, nb;  // planes per thread; blocks
+};
+static SLaunch split_launch(const SGeo& g) {
+  const unsigned bx = std::min(32u, (g.groups + 3) / 4 * 4);
+  unsigned by = std::max(8u, 256u / bx / 8 * 8);
+  while (by > 8 && by - 8 >= g.ny - 2) by -= 8;
+  SLaunch L;
+  L.block = dim3(bx, by);
+  // marching planes saves reads of the plane before and behind; short marches keep enough threads on the chip
+  const double threads = 3.0 * g.groups * (g.ny - 2) * (g.nz - 2);
+  L.zs = threads > 1.2e6 ? 8 : threads > 4e5 ? 4 : threads > 1.5e5 ? 2 : 1;
+  L.grid = dim3((g.groups + bx - 1) / bx, (g.ny - 2 + by - 1) / by, 3 * ((g.nz - 2 + L.zs - 1) / L.zs));
+  L.nb = L.grid.x * L.grid.y * L.grid.z;
+  return L;
+}
+
+// The two x neighbours of four points of parity p of one colour, from the other colour's values oc at their places and the
+// value `ex` before (p = 0) or behind (p = 1) them.
+__device__ __forceinline__ void x_neighbours(unsigned p, float4 oc, float ex, float4& xm, float4& xp) {
+  xm = p ? oc : make_float4(ex, oc.x, oc.y, oc.z);
+  xp = p ? make_float4(oc.y, oc.z, oc.w, ex) : oc;
+}
+// That value's offset, and whether it lies in the row.
+__device__ __forceinline__ bool x_extra(const SGeo& g, unsigned p, unsigned i0, int& off) {
+  off = p ? 4 : -1;
+  return p ? i0 + 4 < g.hx : i0 > 0;
+}
+// Whether place i of a row holds an interior point of parity p.
+__device__ __forceinline__ bool x_interior(const SGeo& g, unsigned p, unsigned i) { return i + p >= 1 && i < g.m; }
+
+__device__ __forceinline__ float sweep_value(const SGeo& g, float own, float r, float xm, float xp, float ym, float yp,
+                                             float zm, float zp) {
+  return sor_value(own, gs_value(__fadd_rn(xp, xm), __fadd_rn(yp, ym), __fadd_rn(zp, zm), r, g.r2x, g.r2y, g.r2z, g.H));
+}
+
+// One colour's half sweep on L e = r.
+__global__ void __launch_bounds__(256) k_s_sweep(SGeo g, float* __restrict__ E, const float* __restrict__ R, unsigned col,
+                                                 unsigned zs) {
   pdl_entry();
-  constexpr int kPFX = 2 * kPCX * 3, kPFR = 2 * kPCY * 2 * kPCZ;  // floats per fine row, fine rows per CTA
-  __shared__ float s_inc[kPFR * kPFX];
-  const unsigned tx = threadIdx.x, ty = threadIdx.y, tz = threadIdx.z;
-  const unsigned cx0 = blockIdx.x * kPCX, cy0 = blockIdx.y * kPCY, cz0 = blockIdx.z * kPCZ;
-  const unsigned cx = cx0 + tx, cy = cy0 + ty, cz = cz0 + tz;
-  if (cx + 1 < C.np[0] && cy + 1 < C.np[1] && cz + 1 < C.np[2]) {
-    const unsigned sy = C.np[0], sz = C.np[0] * C.np[1];
-    const unsigned c0 = cx + sy * cy + sz * cz;
-    float v[2][2][2][3];  // [iz][iy][ix][component]
-#pragma unroll
-    for (int iz = 0; iz < 2; ++iz)
-#pragma unroll
-      for (int iy = 0; iy < 2; ++iy)
-#pragma unroll
-        for (int ix = 0; ix < 2; ++ix)
-#pragma unroll
-          for (int c = 0; c < 3; ++c) v[iz][iy][ix][c] = ec[3 * (c0 + ix + sy * iy + sz * iz) + c];
-#pragma unroll
-    for (int oz = 0; oz < 2; ++oz)
-#pragma unroll
-      for (int oy = 0; oy < 2; ++oy)
-#pragma unroll
-        for (int ox = 0; ox < 2; ++ox) {
-          const float wt = 1.0f / (float)(1u << (ox + oy + oz));
-          const unsigned row = (2 * ty + oy) + 2 * kPCY * (2 * tz + oz);
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            float a = 0.f;
-#pragma unroll
-            for (int iz = 0; iz <= oz; ++iz)
-#pragma unroll
-              for (int iy = 0; iy <= oy; ++iy)
-#pragma unroll
-                for (int ix = 0; ix <= ox; ++ix) a += v[iz][iy][ix][c];
-            s_inc[row * kPFX + 3 * (2 * tx + ox) + c] = a * wt;
-          }
-        }
+  const unsigned i0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x), y = blockIdx.y * blockDim.y + threadIdx.y + 1;
+  const unsigned c = blockIdx.z % 3u, z0 = 1 + blockIdx.z / 3u * zs, z1 = min(g.nz - 1, z0 + zs);
+  if (i0 >= 4 * g.groups || y + 1 >= g.ny) return;
+  const size_t o0 = (size_t)z0 * g.pz + y * g.hx + i0;
+  const float* o = E + (2 * c + (col ^ 1u)) * g.cs + o0;  // the other colour
+  float* e = E + (2 * c + col) * g.cs + o0;
+  const float* r = R + (2 * c + col) * g.cs + o0;
+  float4 om = ld4(o - g.pz), oc = ld4(o);
+  for (unsigned z = z0; z < z1; ++z, o += g.pz, e += g.pz, r += g.pz) {
+    const unsigned p = (col + y + z) & 1u;
+    const float4 op = ld4(o + g.pz), ym = ld4(o - g.hx), yp = ld4(o + g.hx), rv = ld4(r);
+    float4 ev = ld4(e), xm, xp;
+    int off;
+    const float ex = x_extra(g, p, i0, off) ? o[off] : 0.f;
+    x_neighbours(p, oc, ex, xm, xp);
+    if (x_interior(g, p, i0)) ev.x = sweep_value(g, ev.x, rv.x, xm.x, xp.x, ym.x, yp.x, om.x, op.x);
+    if (x_interior(g, p, i0 + 1)) ev.y = sweep_value(g, ev.y, rv.y, xm.y, xp.y, ym.y, yp.y, om.y, op.y);
+    if (x_interior(g, p, i0 + 2)) ev.z = sweep_value(g, ev.z, rv.z, xm.z, xp.z, ym.z, yp.z, om.z, op.z);
+    if (x_interior(g, p, i0 + 3)) ev.w = sweep_value(g, ev.w, rv.w, xm.w, xp.w, ym.w, yp.w, om.w, op.w);
+    st4(e, ev);
+    om = oc;
+    oc = op;
+  }
+}
+
+// The first pre-smoothing sweep from e = 0, both colours in one pass: red points take omega (-r H), black points the
+// update from those red values (recomputed from r, the same float operations as two half sweeps).
+__device__ __forceinline__ float first_red(const SGeo& g, float r) { return sor_value(0.f, __fmul_rn(-r, g.H)); }
+__device__ __forceinline__ float4 first_red4(const SGeo& g, float4 r) {
+  return make_float4(first_red(g, r.x), first_red(g, r.y), first_red(g, r.z), first_red(g, r.w));
+}
+__global__ void __launch_bounds__(256) k_s_first(SGeo g, float* __restrict__ E, const float* __restrict__ R, unsigned zs) {
+  pdl_entry();
+  const unsigned i0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x), y = blockIdx.y * blockDim.y + threadIdx.y + 1;
+  const unsigned c = blockIdx.z % 3u, z0 = 1 + blockIdx.z / 3u * zs, z1 = min(g.nz - 1, z0 + zs);
+  if (i0 >= 4 * g.groups || y + 1 >= g.ny) return;
+  const size_t o0 = (size_t)z0 * g.pz + y * g.hx + i0;
+  const float* rr = R + 2 * c * g.cs + o0;  // red
+  const float* rb = rr + g.cs;              // black
+  float* er = E + 2 * c * g.cs + o0;
+  float* eb = er + g.cs;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 om = z0 > 1 ? first_red4(g, ld4(rr - g.pz)) : zero, oc = first_red4(g, ld4(rr));
+  for (unsigned z = z0; z < z1; ++z, rr += g.pz, rb += g.pz, er += g.pz, eb += g.pz) {
+    const unsigned p = (1 + y + z) & 1u, q = p ^ 1u;  // parities of the black and the red points of the row
+    const float4 op = z + 2 < g.nz ? first_red4(g, ld4(rr + g.pz)) : zero;
+    const float4 ym = y > 1 ? first_red4(g, ld4(rr - g.hx)) : zero, yp = y + 2 < g.ny ? first_red4(g, ld4(rr + g.hx)) : zero;
+    const float4 rv = ld4(rb);
+    // the row's red values, zero on the boundary
+    float4 rc = oc, xm, xp, bv = zero;
+    if (!x_interior(g, q, i0)) rc.x = 0.f;
+    if (!x_interior(g, q, i0 + 1)) rc.y = 0.f;
+    if (!x_interior(g, q, i0 + 2)) rc.z = 0.f;
+    if (!x_interior(g, q, i0 + 3)) rc.w = 0.f;
+    int off;
+    const float ex = x_extra(g, p, i0, off) && x_interior(g, q, i0 + off) ? first_red(g, rr[off]) : 0.f;
+    x_neighbours(p, rc, ex, xm, xp);
+    if (x_interior(g, p, i0)) bv.x = sweep_value(g, 0.f, rv.x, xm.x, xp.x, ym.x, yp.x, om.x, op.x);
+    if (x_interior(g, p, i0 + 1)) bv.y = sweep_value(g, 0.f, rv.y, xm.y, xp.y, ym.y, yp.y, om.y, op.y);
+    if (x_interior(g, p, i0 + 2)) bv.z = sweep_value(g, 0.f, rv.z, xm.z, xp.z, ym.z, yp.z, om.z, op.z);
+    if (x_interior(g, p, i0 + 3)) bv.w = sweep_value(g, 0.f, rv.w, xm.w, xp.w, ym.w, yp.w, om.w, op.w);
+    st4(er, rc);
+    st4(eb, bv);
+    om = oc;
+    oc = op;
+  }
+}
+
+// A value of a split field at (x, y, z) of component c.
+__device__ __forceinline__ size_t split_at(const SGeo& g, unsigned c, unsigned x, unsigned y, unsigned z) {
+  return (2 * c + ((x + y + z) & 1u)) * g.cs + (size_t)z * g.pz + y * g.hx + (x >> 1);
+}
+
+// Residual r - L e and full-weighting restriction of one component: a CTA owns kQX x kQY x kQZ coarse points.  It first
+// computes the fine residuals of the (2 kQX + 1) x (2 kQY + 1) x (2 kQZ + 1) points around them into shared memory, even and
+// odd x apart, four points of one a thread; then each coarse point sums its 27 with the weights 8/4/2/1 / 64 in the order of
+// residual_restrict_point.  The coarse right-hand side is split, or interleaved on the coarsest level.  Levels halve exactly,
+// so the 27 fine points of a coarse interior point are interior.
+constexpr int kQX = 32, kQY = 4, kQZ = 4;
+constexpr int kQGroups = kQX / 4 + 1, kQRow = 4 * kQGroups, kQFY = 2 * kQY + 1, kQFZ = 2 * kQZ + 1;
+template <bool kSplitCoarse>
+__global__ void __launch_bounds__(256) k_s_restrict(SGeo g, SGeo C, const float* __restrict__ E, const float* __restrict__ R,
+                                                    float* __restrict__ rc) {
+  pdl_entry();
+  __shared__ __align__(16) float s_res[kQFZ * kQFY][2][kQRow];  // [row][odd x][i - ib]
+  const unsigned c = blockIdx.z % 3u, ib = blockIdx.x * kQX;
+  const unsigned cy0 = 1 + blockIdx.y * kQY, cz0 = 1 + blockIdx.z / 3u * kQZ;
+  for (unsigned it = threadIdx.x; it < (unsigned)(kQFZ * kQFY * 2 * kQGroups); it += 256) {
+    const unsigned k = it % kQGroups, q = it / kQGroups, odd = q & 1u, row = q >> 1;
+    const unsigned y = 2 * cy0 - 1 + row % kQFY, z = 2 * cz0 - 1 + row / kQFY, i0 = ib + 4 * k;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (y + 1 < g.ny && z + 1 < g.nz && i0 < g.m) {
+      const unsigned col = (odd + y + z) & 1u;
+      const size_t o = (size_t)z * g.pz + y * g.hx + i0;
+      const float* own = E + (2 * c + col) * g.cs + o;
+      const float* oth = E + (2 * c + (col ^ 1u)) * g.cs + o;
+      const float4 e = ld4(own), oc = ld4(oth), ym = ld4(oth - g.hx), yp = ld4(oth + g.hx), zm = ld4(oth - g.pz),
+                   zp = ld4(oth + g.pz), r = ld4(R + (2 * c + col) * g.cs + o);
+      int off;
+      const float ex = x_extra(g, odd, i0, off) ? oth[off] : 0.f;
+      float4 xm, xp;
+      x_neighbours(odd, oc, ex, xm, xp);
+      v.x = __fsub_rn(r.x, lap7(e.x, xp.x, xm.x, yp.x, ym.x, zp.x, zm.x, g.r2x, g.r2y, g.r2z));
+      v.y = __fsub_rn(r.y, lap7(e.y, xp.y, xm.y, yp.y, ym.y, zp.y, zm.y, g.r2x, g.r2y, g.r2z));
+      v.z = __fsub_rn(r.z, lap7(e.z, xp.z, xm.z, yp.z, ym.z, zp.z, zm.z, g.r2x, g.r2y, g.r2z));
+      v.w = __fsub_rn(r.w, lap7(e.w, xp.w, xm.w, yp.w, ym.w, zp.w, zm.w, g.r2x, g.r2y, g.r2z));
+    }
+    *reinterpret_cast<float4*>(&s_res[row][odd][4 * k]) = v;
   }
   __syncthreads();
-  // fine rows Y = 2 cy0 + (0 .. 2 kPCY - 1), Z = 2 cz0 + (0 .. 2 kPCZ - 1);
-  // fine x = 2 cx0 + (0 .. 2 kPCX - 1)
-  const unsigned nthreads = kPCX * kPCY * kPCZ, tid = tx + kPCX * (ty + kPCY * tz);
-  const unsigned X0 = 2 * cx0, Y0 = 2 * cy0, Z0 = 2 * cz0;
-  for (unsigned i = tid; i < (unsigned)(kPFR * kPFX); i += nthreads) {
-    const unsigned row = i / kPFX, col = i - row * kPFX;
-    const unsigned X = X0 + col / 3u, Y = Y0 + row % (2 * kPCY), Z = Z0 + row / (2 * kPCY);
-    if (X == 0 || Y == 0 || Z == 0 || X + 1 >= F.np[0] || Y + 1 >= F.np[1] || Z + 1 >= F.np[2]) continue;
-    ef[3 * (X + F.np[0] * (Y + F.np[1] * Z)) + col % 3u] += s_inc[i];
+  for (unsigned t = threadIdx.x; t < (unsigned)(kQX * kQY * kQZ); t += 256) {
+    const unsigned lx = t % kQX, ly = t / kQX % kQY, lz = t / (kQX * kQY);
+    const unsigned x = 1 + ib + lx, y = cy0 + ly, z = cz0 + lz;  // fine 2 x: even place lx + 1, odd places lx and lx + 1
+    if (x + 1 >= C.nx || y + 1 >= C.ny || z + 1 >= C.nz) continue;
+    float acc = 0.f;
+#pragma unroll
+    for (int dz = -1; dz <= 1; ++dz)
+#pragma unroll
+      for (int dy = -1; dy <= 1; ++dy) {
+        const float(*row)[kQRow] = s_res[(2 * lz + 1 + dz) * kQFY + 2 * ly + 1 + dy];
+        const int w = 8 >> (abs(dy) + abs(dz));
+        acc = __fmaf_rn((float)w * 0.5f, row[1][lx], acc);
+        acc = __fmaf_rn((float)w, row[0][lx + 1], acc);
+        acc = __fmaf_rn((float)w * 0.5f, row[1][lx + 1], acc);
+      }
+    acc = __fmul_rn(acc, 1.0f / 64.0f);
+    if (kSplitCoarse)
+      rc[split_at(C, c, x, y, z)] = acc;
+    else
+      rc[3 * (x + C.nx * (y + C.ny * (size_t)z)) + c] = acc;
   }
 }
 
-// Launch shape of the row kernels above over `items` (point, component)
-// pairs per row and the interior rows (ny - 2) x (nz - 2) of a level: rows of
-// up to 256 threads, rounded to whole warps; short rows stack in y.
-struct RowLaunch {
-  dim3 grid, block;
+// e_fine += trilinear(e_coarse) of one component: a thread owns four places of a fine row, even and odd x, and reads the one,
+// two or four coarse rows beside it; the sums in the order of prolong_point.
+template <bool kSplitCoarse>
+__global__ void __launch_bounds__(256) k_s_prolong(SGeo g, SGeo C, const float* __restrict__ ec, float* __restrict__ E) {
+  pdl_entry();
+  const unsigned i0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x), y = blockIdx.y * blockDim.y + threadIdx.y + 1;
+  const unsigned c = blockIdx.z % 3u, z = 1 + blockIdx.z / 3u;
+  if (i0 >= 4 * g.groups || y + 1 >= g.ny) return;
+  const unsigned oy = y & 1u, oz = z & 1u;
+  float a[4] = {0.f, 0.f, 0.f, 0.f}, b[4] = {0.f, 0.f, 0.f, 0.f};  // even x: coarse i; odd x: coarse i and i + 1
+  for (unsigned iz = 0; iz <= oz; ++iz)
+    for (unsigned iy = 0; iy <= oy; ++iy) {
+      const unsigned Y = (y >> 1) + iy, Z = (z >> 1) + iz;
+      float v[5];
+      if (kSplitCoarse) {
+        // coarse x = i0 .. i0 + 4 (i0 even): alternately of the two colours
+        const float* ra = ec + (2 * c + ((Y + Z) & 1u)) * C.cs + (size_t)Z * C.pz + Y * C.hx + (i0 >> 1);
+        const float* rb = ec + (2 * c + ((Y + Z + 1) & 1u)) * C.cs + (size_t)Z * C.pz + Y * C.hx + (i0 >> 1);
+        const float2 va = *reinterpret_cast<const float2*>(ra), vb = *reinterpret_cast<const float2*>(rb);
+        v[0] = va.x;
+        v[1] = vb.x;
+        v[2] = va.y;
+        v[3] = vb.y;
+        v[4] = (i0 >> 1) + 2 < C.hx ? ra[2] : 0.f;
+      } else {
+        const float* row = ec + 3 * ((size_t)C.nx * (Y + C.ny * (size_t)Z)) + c;
+#pragma unroll
+        for (unsigned k = 0; k < 5; ++k) v[k] = i0 + k < C.nx ? row[3 * (i0 + k)] : 0.f;
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        a[k] += v[k];
+        b[k] += v[k];
+        b[k] += v[k + 1];
+      }
+    }
+  const float wa = 1.0f / (float)(1u << (oy + oz)), wb = 0.5f * wa;
+  const size_t o = (size_t)z * g.pz + y * g.hx + i0;
+  float* even = E + (2 * c + ((y + z) & 1u)) * g.cs + o;
+  float* odd = E + (2 * c + ((y + z + 1) & 1u)) * g.cs + o;
+  float4 ve = ld4(even), vo = ld4(odd);
+  if (x_interior(g, 0, i0)) ve.x = __fmaf_rn(a[0], wa, ve.x);
+  if (x_interior(g, 0, i0 + 1)) ve.y = __fmaf_rn(a[1], wa, ve.y);
+  if (x_interior(g, 0, i0 + 2)) ve.z = __fmaf_rn(a[2], wa, ve.z);
+  if (x_interior(g, 0, i0 + 3)) ve.w = __fmaf_rn(a[3], wa, ve.w);
+  if (x_interior(g, 1, i0)) vo.x = __fmaf_rn(b[0], wb, vo.x);
+  if (x_interior(g, 1, i0 + 1)) vo.y = __fmaf_rn(b[1], wb, vo.y);
+  if (x_interior(g, 1, i0 + 2)) vo.z = __fmaf_rn(b[2], wb, vo.z);
+  if (x_interior(g, 1, i0 + 3)) vo.w = __fmaf_rn(b[3], wb, vo.w);
+  st4(even, ve);
+  st4(odd, vo);
+}
+
+// Block sums of two values into part[2 b + {0, 1}], as block_sum2, for any whole number of warps.
+__device__ __forceinline__ void split_sum2(float a32, float b32, double* __restrict__ part) {
+  __shared__ double s_a[8], s_b[8];
+  const unsigned tid = threadIdx.x + blockDim.x * threadIdx.y, warps = blockDim.x * blockDim.y / 32;
+  for (int o = 16; o > 0; o >>= 1) {
+    a32 += __shfl_xor_sync(0xffffffffu, a32, o);
+    b32 += __shfl_xor_sync(0xffffffffu, b32, o);
+  }
+  if ((tid & 31) == 0) {
+    s_a[tid >> 5] = (double)a32;
+    s_b[tid >> 5] = (double)b32;
+  }
+  __syncthreads();
+  if (tid == 0) {
+    double t1 = 0.0, t2 = 0.0;
+    for (unsigned w = 0; w < warps; ++w) {
+      t1 += s_a[w];
+      t2 += s_b[w];
+    }
+    const unsigned b = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
+    part[2 * b] = t1;
+    part[2 * b + 1] = t2;
+  }
+}
+
+// The iterate's values in a residual: x; x + e (the cycle's correction, whose sum is also written); or e alone (a first
+// correction, 0 + e).
+enum ResField { RES_X, RES_X_PLUS_E, RES_E };
+template <int kField>
+__device__ __forceinline__ float4 res_value(const float* x, const float* e, ptrdiff_t o) {
+  if (kField == RES_X) return ld4(x + o);
+  const float4 ev = ld4(e + o);
+  if (kField == RES_E) return ev;
+  const float4 xv = ld4(x + o);
+  return make_float4(__fadd_rn(xv.x, ev.x), __fadd_rn(xv.y, ev.y), __fadd_rn(xv.z, ev.z), __fadd_rn(xv.w, ev.w));
+}
+template <int kField>
+__device__ __forceinline__ float res_value1(const float* x, const float* e, ptrdiff_t o) {
+  return kField == RES_X ? x[o] : kField == RES_E ? e[o] : __fadd_rn(x[o], e[o]);
+}
+
+// Residual r = b - L v in FP32 (v: kField) at both colours of four places a thread, v itself to xn when it is a new sum, and
+// (kNorm) per-block sums of r^2 and b^2.  xn is another buffer than x, whose neighbours others still read; its boundary
+// values are the caller's.
+template <int kField, bool kNorm>
+__global__ void __launch_bounds__(256) k_s_residual(SGeo g, const float* __restrict__ x, const float* __restrict__ e,
+                                                    const float* __restrict__ b, float* __restrict__ xn,
+                                                    float* __restrict__ r, double* __restrict__ part, unsigned zs) {
+  pdl_entry();
+  const unsigned i0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x), y = blockIdx.y * blockDim.y + threadIdx.y + 1;
+  const unsigned c = blockIdx.z % 3u, z0 = 1 + blockIdx.z / 3u * zs, z1 = min(g.nz - 1, z0 + zs);
+  float rr = 0.f, bb = 0.f;
+  if (i0 < 4 * g.groups && y + 1 < g.ny) {
+    const size_t f0 = 2 * c * g.cs + (size_t)z0 * g.pz + y * g.hx + i0;
+    x += f0;
+    e += f0;
+    b += f0;
+    xn += f0;
+    r += f0;
+    const ptrdiff_t cs = (ptrdiff_t)g.cs, pz = (ptrdiff_t)g.pz, hx = (ptrdiff_t)g.hx;
+    // even and odd x of the planes before, at and behind; even x has colour (y + z) & 1
+    ptrdiff_t ec = ((y + z0) & 1u) ? cs : 0;  // offset of the even points' colour at plane z
+    float4 em = res_value<kField>(x, e, cs - ec - pz), om = res_value<kField>(x, e, ec - pz);
+    float4 e0 = res_value<kField>(x, e, ec), o0 = res_value<kField>(x, e, cs - ec);
+    for (unsigned z = z0; z < z1; ++z) {
+      const ptrdiff_t oc = cs - ec;
+      const float4 ep = res_value<kField>(x, e, oc + pz), op = res_value<kField>(x, e, ec + pz);
+      const float4 eym = res_value<kField>(x, e, oc - hx), oym = res_value<kField>(x, e, ec - hx);
+      const float4 eyp = res_value<kField>(x, e, oc + hx), oyp = res_value<kField>(x, e, ec + hx);
+      const float4 be = ld4(b + ec), bo = ld4(b + oc);
+      const float left = i0 ? res_value1<kField>(x, e, oc - 1) : 0.f;             // odd x before the four
+      const float right = i0 + 4 < g.hx ? res_value1<kField>(x, e, ec + 4) : 0.f;  // even x behind them
+      const float ev[5] = {e0.x, e0.y, e0.z, e0.w, right}, ov[5] = {left, o0.x, o0.y, o0.z, o0.w};
+      const float aem[4] = {em.x, em.y, em.z, em.w}, aep[4] = {ep.x, ep.y, ep.z, ep.w};
+      const float aom[4] = {om.x, om.y, om.z, om.w}, aop[4] = {op.x, op.y, op.z, op.w};
+      const float ey0[4] = {eym.x, eym.y, eym.z, eym.w}, ey1[4] = {eyp.x, eyp.y, eyp.z, eyp.w};
+      const float oy0[4] = {oym.x, oym.y, oym.z, oym.w}, oy1[4] = {oyp.x, oyp.y, oyp.z, oyp.w};
+      const float abe[4] = {be.x, be.y, be.z, be.w}, abo[4] = {bo.x, bo.y, bo.z, bo.w};
+      float re[4], ro[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        re[k] = __fsub_rn(abe[k], lap7(ev[k], ov[k + 1], ov[k], ey1[k], ey0[k], aep[k], aem[k], g.r2x, g.r2y, g.r2z));
+        ro[k] = __fsub_rn(abo[k], lap7(ov[k + 1], ev[k + 1], ev[k], oy1[k], oy0[k], aop[k], aom[k], g.r2x, g.r2y, g.r2z));
+        if (kNorm && x_interior(g, 0, i0 + k)) {
+          rr = fmaf(re[k], re[k], rr);
+          bb = fmaf(abe[k], abe[k], bb);
+        }
+        if (kNorm && x_interior(g, 1, i0 + k)) {
+          rr = fmaf(ro[k], ro[k], rr);
+          bb = fmaf(abo[k], abo[k], bb);
+        }
+      }
+      st4(r + ec, make_float4(re[0], re[1], re[2], re[3]));
+      st4(r + oc, make_float4(ro[0], ro[1], ro[2], ro[3]));
+      if (kField != RES_X) {
+        st4(xn + ec, e0);
+        st4(xn + oc, o0);
+      }
+      em = e0;
+      om = o0;
+      e0 = ep;
+      o0 = op;
+      x += pz;
+      e += pz;
+      b += pz;
+      xn += pz;
+      r += pz;
+      ec = cs - ec;
+    }
+  }
+  if (kNorm) split_sum2(rr, bb, part);
+}
+
+// The refinement residual r = b - L (hi + lo) to FP64-class accuracy (pair_residual), with hi = x or x + e (then written to
+// xn), and lo from a field or zero; a thread a point of one component and colour, along z.
+template <bool kAdd, bool kLo>
+__global__ void __launch_bounds__(256) k_s_residual_pair(SGeo g, PairCoef cf, const float* __restrict__ x,
+                                                         const float* __restrict__ e, const float* __restrict__ lo,
+                                                         const float* __restrict__ b, float* __restrict__ xn,
+                                                         float* __restrict__ r, double* __restrict__ part, unsigned zs) {
+  pdl_entry();
+  constexpr int kField = kAdd ? RES_X_PLUS_E : RES_X;
+  const unsigned i0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x), y = blockIdx.y * blockDim.y + threadIdx.y + 1;
+  const unsigned c = blockIdx.z % 3u, z0 = 1 + blockIdx.z / 3u * zs, z1 = min(g.nz - 1, z0 + zs);
+  float rr = 0.f;
+  if (i0 < 4 * g.groups && y + 1 < g.ny) {
+    for (unsigned col = 0; col < 2; ++col) {
+      const size_t o0 = (size_t)z0 * g.pz + y * g.hx + i0, own = (2 * c + col) * g.cs + o0, oth = (2 * c + (col ^ 1u)) * g.cs + o0;
+      ptrdiff_t o = 0;
+      const ptrdiff_t pz = (ptrdiff_t)g.pz, hx = (ptrdiff_t)g.hx;
+      const float *xo = x + oth, *eo = e + oth, *lo_o = lo + oth;
+      float4 hm = res_value<kField>(xo, eo, -pz), hc = res_value<kField>(xo, eo, 0);
+      const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+      float4 lm = kLo ? ld4(lo_o - pz) : zero, lc = kLo ? ld4(lo_o) : zero;
+      for (unsigned z = z0; z < z1; ++z, o += pz) {
+        const unsigned p = (col + y + z) & 1u;
+        const float4 hp = res_value<kField>(xo, eo, o + pz), hym = res_value<kField>(xo, eo, o - hx), hyp = res_value<kField>(xo, eo, o + hx);
+        const float4 lp = kLo ? ld4(lo_o + o + pz) : zero, lym = kLo ? ld4(lo_o + o - hx) : zero, lyp = kLo ? ld4(lo_o + o + hx) : zero;
+        const float4 h0 = res_value<kField>(x + own, e + own, o), l0 = kLo ? ld4(lo + own + o) : zero, bv = ld4(b + own + o);
+        int off;
+        const bool in = x_extra(g, p, i0, off);
+        float4 hxm, hxp, lxm, lxp;
+        x_neighbours(p, hc, in ? res_value1<kField>(xo, eo, o + off) : 0.f, hxm, hxp);
+        x_neighbours(p, lc, kLo && in ? lo_o[o + off] : 0.f, lxm, lxp);
+        float4 rv;
+#define VG_PAIR(k)                                                                                      \
+  {                                                                                                     \
+    const float h[7] = {h0.k, hxp.k, hxm.k, hyp.k, hym.k, hp.k, hm.k};                                  \
+    const float l[7] = {l0.k, lxp.k, lxm.k, lyp.k, lym.k, lp.k, lm.k};                                  \
+    rv.k = pair_residual(h, l, bv.k, cf);                                                               \
+  }
+        VG_PAIR(x) VG_PAIR(y) VG_PAIR(z) VG_PAIR(w)
+#undef VG_PAIR
+        if (x_interior(g, p, i0)) rr = fmaf(rv.x, rv.x, rr);
+        if (x_interior(g, p, i0 + 1)) rr = fmaf(rv.y, rv.y, rr);
+        if (x_interior(g, p, i0 + 2)) rr = fmaf(rv.z, rv.z, rr);
+        if (x_interior(g, p, i0 + 3)) rr = fmaf(rv.w, rv.w, rr);
+        st4(r + own + o, rv);
+        if (kAdd) st4(xn + own + o, h0);
+        hm = hc;
+        hc = hp;
+        lm = lc;
+        lc = lp;
+      }
+    }
+  }
+  split_sum2(rr, 0.f, part);
+}
+
+// a += b over split fields (n4 float4 groups).
+__global__ void __launch_bounds__(256) k_s_add(float4* __restrict__ a, const float4* __restrict__ b, size_t n4) {
+  pdl_entry();
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n4) return;
+  const float4 u = a[i], v = b[i];
+  a[i] = make_float4(__fadd_rn(u.x, v.x), __fadd_rn(u.y, v.y), __fadd_rn(u.z, v.z), __fadd_rn(u.w, v.w));
+}
+
+// Interleaved fields into split ones: the solution into x, its boundary values into x2 too, and the right-hand side; a warp a
+// row, component and parity after component and parity (the row's bytes stay in L1).
+__global__ void __launch_bounds__(256) k_s_in(SGeo g, const float* __restrict__ soln, const float* __restrict__ rhs,
+                                              float* __restrict__ x, float* __restrict__ x2, float* __restrict__ b) {
+  pdl_entry();
+  const unsigned row = blockIdx.x * 8 + threadIdx.x / 32, lane = threadIdx.x & 31;
+  if (row >= g.ny * g.nz) return;
+  const unsigned y = row % g.ny, z = row / g.ny;
+  const bool edge = y == 0 || z == 0 || y + 1 == g.ny || z + 1 == g.nz;
+  const float* sr = soln + 3 * (size_t)g.nx * row;
+  const float* br = rhs + 3 * (size_t)g.nx * row;
+  const size_t o = (size_t)z * g.pz + y * g.hx;
+  for (unsigned i = lane; i < g.hx; i += 32)
+#pragma unroll
+    for (unsigned p = 0; p < 2; ++p) {
+      const unsigned X = 2 * i + p;
+      const bool in = X < g.nx;
+#pragma unroll
+      for (unsigned c = 0; c < 3; ++c) {
+        const size_t at = (2 * c + ((p + y + z) & 1u)) * g.cs + o + i;
+        const float v = in ? sr[3 * X + c] : 0.f;
+        x[at] = v;
+        if (edge || X == 0 || X + 1 >= g.nx) x2[at] = v;
+        b[at] = in ? br[3 * X + c] : 0.f;
+      }
+    }
+}
+
+// The interleaved solution from the split fields: x, or x + d.
+template <bool kAdd>
+__global__ void __launch_bounds__(256) k_s_out(SGeo g, const float* __restrict__ x, const float* __restrict__ d,
+                                               float* __restrict__ soln) {
+  pdl_entry();
+  const unsigned row = blockIdx.x * 8 + threadIdx.x / 32, lane = threadIdx.x & 31;
+  if (row >= g.ny * g.nz) return;
+  const unsigned y = row % g.ny, z = row / g.ny;
+  float* sr = soln + 3 * (size_t)g.nx * row;
+  const size_t o = (size_t)z * g.pz + y * g.hx;
+  for (unsigned i = lane; i < 3 * g.nx; i += 32) {
+    const unsigned X = i / 3u, c = i - 3 * X;
+    const size_t at = (2 * c + ((X + y + z) & 1u)) * g.cs + o + (X >> 1);
+    sr[i] = kAdd ? __fadd_rn(x[at], d[at]) : x[at];
+  }
+}
+
+// Zero on the boundary (and in the rows' padding) of split fields: a correction is zero there, and only its interior is ever
+// written.  A thread a row, the fields in the launch's y.
+struct FaceList {
+  int n;
+  float* f[kMaxLayers + 2];
+  SGeo g[kMaxLayers + 2];
 };
-static RowLaunch launch_rows(unsigned items, unsigned ny, unsigned nz) {
-  const unsigned nb = (items + 255) / 256;
-  const unsigned bx = ((items + nb - 1) / nb + 31) / 32 * 32;
-  unsigned by = std::max(1u, 256u / bx);
-  while (by > 1 && by / 2 >= ny - 2) by >>= 1;
-  RowLaunch L;
-  L.block = dim3(bx, by, 1);
-  L.grid = dim3(nb, (ny - 2 + by - 1) / by, nz - 2);
-  return L;
+__global__ void __launch_bounds__(256) k_s_faces(const __grid_constant__ FaceList L) {
+  pdl_entry();
+  const SGeo& g = L.g[blockIdx.y];
+  const unsigned q = blockIdx.x * blockDim.x + threadIdx.x, y = q % g.ny, z = q / g.ny % g.nz, a = q / (g.ny * g.nz);
+  if (a >= 6) return;  // a = 2 c + colour
+  float* p = L.f[blockIdx.y] + a * g.cs + (size_t)z * g.pz + y * g.hx;
+  if (y == 0 || z == 0 || y + 1 == g.ny || z + 1 == g.nz) {
+    for (unsigned i = 0; i < g.hx; i += 4) st4(p + i, make_float4(0.f, 0.f, 0.f, 0.f));
+  } else {
+    if (((a + y + z) & 1u) == 0) p[0] = 0.f;  // x = 0
+    for (unsigned i = g.m; i < g.hx; ++i) p[i] = 0.f;
+  }
 }
 
 // The small levels of a V-cycle in one CTA, their e and r in shared memory:
@@ -1076,36 +1350,16 @@ struct MgBufs {
   ResLaunch rl;   // the residual kernels' launch over level 0
 };
 
-// One V(pre, post)-cycle on L e = R[level 0] (level 0's e and r in B; e
-// starts from zero).
-static vg_status enqueue_vcycle(Ctx* c, const MgPlan& P, const MgBufs& B, unsigned* nl) {
+// The coarsest level's exact solve, or the V-cycle of the small levels in one CTA: e from r of level first_small, both
+// interleaved.
+static vg_status enqueue_coarse(Ctx* c, const MgPlan& P, const MgBufs& B, float* E, float* R, unsigned* nl) {
   const int pre = 2, post = 2;
   const int fs = P.first_small;
-  for (int l = 0; l < fs; ++l) {
-    const Lev& L = P.lev[l];
-    float* e = B.E + 3 * L.base;
-    float* r = B.R + 3 * L.base;
-    const RowLaunch sw = launch_rows(3 * ((L.g.np[0] - 1) / 2), L.g.np[1], L.g.np[2]);  // one colour's points
-    const RowLaunch all = launch_rows(3 * (L.g.np[0] - 2), L.g.np[1], L.g.np[2]);     // every interior point
-    pdl_launch(c->stream, all.grid, all.block, 0, k_rbgs_first, L.g, L.r2x, L.r2y, L.r2z, L.H, e, r);
-    ++*nl;
-    for (int s = 1; s < pre; ++s)
-      for (unsigned col = 0; col < 2; ++col) {
-        pdl_launch(c->stream, sw.grid, sw.block, 0, k_rbgs, L.g, L.r2x, L.r2y, L.r2z, L.H, e, r, col, 0);
-        ++*nl;
-      }
-    const Lev& Cn = P.lev[l + 1];
-    const dim3 rg((Cn.g.np[0] - 2 + kRTX - 1) / kRTX, (Cn.g.np[1] - 2 + kRTY - 1) / kRTY,
-                  (Cn.g.np[2] - 2 + kRTZ - 1) / kRTZ);
-    pdl_launch(c->stream, rg, 256, 0, k_residual_restrict, L.g, Cn.g, L.r2x, L.r2y, L.r2z, e, r, B.R + 3 * Cn.base);
-    ++*nl;
-  }
   if (P.direct_global) {
     const Lev& L = P.lev[fs];
     const Geom& g = L.g;
+    // E and R also serve as ping-pong buffers in compact layout (3 N <= 3 points)
     const unsigned nxi = g.np[0] - 2, nyi = g.np[1] - 2, nzi = g.np[2] - 2, N = nxi * nyi * nzi;
-    float* E = B.E + 3 * L.base;  // ping-pong buffers in compact layout (3 N <= 3 points)
-    float* R = B.R + 3 * L.base;
     const unsigned nb = blocks_for(3 * N, 256);
     auto transform = [&](auto* X, auto* Y, auto* tab) {
       using T = typename std::remove_const<typename std::remove_pointer<decltype(tab)>::type>::type;
@@ -1160,8 +1414,8 @@ static vg_status enqueue_vcycle(Ctx* c, const MgPlan& P, const MgBufs& B, unsign
       off += (unsigned)(6 * L.g.points());
     }
     S.dst = P.direct ? (const float*)B.dst : nullptr;
-    S.r_in = B.R + 3 * P.lev[fs].base;
-    S.e_out = B.E + 3 * P.lev[fs].base;
+    S.r_in = R;
+    S.e_out = E;
     S.pre = pre;
     S.post = post;
     const Geom& cg = P.lev[P.nlev - 1].g;
@@ -1173,49 +1427,23 @@ static vg_status enqueue_vcycle(Ctx* c, const MgPlan& P, const MgBufs& B, unsign
     pdl_launch(c->stream, 1, 1024, P.small_smem, k_vcycle_small, S, B.cwork);
     ++*nl;
   }
-  for (int l = fs - 1; l >= 0; --l) {
-    const Lev& L = P.lev[l];
-    const Lev& Cn = P.lev[l + 1];
-    float* e = B.E + 3 * L.base;
-    float* r = B.R + 3 * L.base;
-    const RowLaunch sw = launch_rows(3 * ((L.g.np[0] - 1) / 2), L.g.np[1], L.g.np[2]);
-    // large levels through the shared-memory tile; small ones (few CTAs per
-    // tile) one thread per cell with direct updates, which measured faster there
-    if (Cn.g.points() >= (size_t)1 << 18) {
-      const dim3 pg((Cn.g.np[0] - 1 + 31) / 32, (Cn.g.np[1] - 1 + 3) / 4, (Cn.g.np[2] - 1 + 1) / 2);
-      pdl_launch(c->stream, pg, dim3(32, 4, 2), 0, k_prolong_add<32, 4, 2>, L.g, Cn.g, B.E + 3 * Cn.base, e);
-    } else {
-      const unsigned cells_x = Cn.g.np[0] - 1, pbx = cells_x >= 64 ? 64 : 32, pby = 256 / pbx;
-      const dim3 pg((cells_x + pbx - 1) / pbx, (Cn.g.np[1] - 1 + pby - 1) / pby, Cn.g.np[2] - 1);
-      pdl_launch(c->stream, pg, dim3(pbx, pby), 0, k_prolong_cells, L.g, Cn.g, B.E + 3 * Cn.base, e);
-    }
-    ++*nl;
-    for (int s = 0; s < post; ++s)
-      for (unsigned col = 0; col < 2; ++col) {
-        pdl_launch(c->stream, sw.grid, sw.block, 0, k_rbgs, L.g, L.r2x, L.r2y, L.r2z, L.H, e, r, col, 0);
-        ++*nl;
-      }
-  }
   VG_CUDA(c, cudaGetLastError());
   return VG_OK;
 }
 
-// One cycle on L x = rhs: V-cycle on the current residual R, x += e, then
-// R = rhs - L x in FP32 with its FP64-accumulated norm.
-// Cycle tails: the residual with its norm (the adaptive solve reads it), the
-// residual alone (a fixed schedule's next cycle needs R, not its norm), or
-// nothing (a fixed schedule's last cycle of a phase: the next step replaces R).
+// Cycle tails: the residual with its norm (the adaptive solve reads it), the residual alone (a fixed schedule's next cycle
+// needs R, not its norm), or nothing (a fixed schedule's last cycle of a phase: the next step replaces R).
 enum CycleTail { TAIL_NORM, TAIL_RESIDUAL, TAIL_NONE };
 
+// One cycle on L x = rhs of a hierarchy without smoothed levels (interleaved fields): the coarse solve on the residual R,
+// x += e, then R = rhs - L x in FP32 with its FP64-accumulated norm.
 static vg_status enqueue_cycle(Ctx* c, const MgPlan& P, const Geom& g, const MgBufs& B, float* x, const float* rhs,
                                unsigned* nl, CycleTail tail = TAIL_NORM) {
-  vg_status st = enqueue_vcycle(c, P, B, nl);
+  vg_status st = enqueue_coarse(c, P, B, B.E, B.R, nl);
   if (st != VG_OK) return st;
   const size_t n3 = 3 * g.points();
   const Lev& L0 = P.lev[0];
-  // x += e as a separate streaming pass: fused into the last half sweep it
-  // measured slower (x is not in L2 by then, and the sweep's gathers wait on it).
-  // x NULL: the correction stays in B.E (level 0) for the caller.
+  // x NULL: the correction stays in B.E for the caller.
   if (x) {
     add_f32(c, x, B.E, n3);
     ++*nl;
@@ -1232,51 +1460,55 @@ static vg_status enqueue_cycle(Ctx* c, const MgPlan& P, const Geom& g, const MgB
   return VG_OK;
 }
 
-// Capture (or reuse) the cycle graph for (x, rhs) in cache slot `slot`.
-static void cycle_graph(Ctx* c, const MgPlan& P, const Geom& g, const MgBufs& B, float* x, const float* rhs,
-                        int slot) {
-  MgGraphCache& G = c->mg_graph[slot];
-  const void* key[4] = {B.E, B.R, rhs, x};
-  if (G.exec && memcmp(&G.g, &g, sizeof(Geom)) == 0 && memcmp(G.key, key, sizeof(key)) == 0) return;
-  if (G.exec) {
-    cudaGraphExecDestroy(G.exec);
-    G.exec = nullptr;
-  }
-  cudaGraph_t graph = nullptr;
-  unsigned nl = 0;
-  if (cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-    const vg_status cst = enqueue_cycle(c, P, g, B, x, rhs, &nl);
-    const cudaError_t ce = cudaStreamEndCapture(c->stream, &graph);
-    if (cst == VG_OK && ce == cudaSuccess && graph && cudaGraphInstantiate(&G.exec, graph, 0) == cudaSuccess) {
-      G.g = g;
-      memcpy(G.key, key, sizeof(key));
-      G.launches = nl;
-    } else {
-      G.exec = nullptr;
+// Runs the work that `enqueue` puts on the stream, from a graph captured when the same (grid, buffers) came first; `key`
+// names every buffer that the cycle's kernels were given besides the workspace of its grid.
+template <class F>
+static vg_status run_cached(Ctx* c, const Geom& g, const void* const (&key)[4], F enqueue) {
+  MgGraphCache* G = nullptr;
+  for (MgGraphCache& q : c->mg_graph)
+    if (q.exec && memcmp(&q.g, &g, sizeof(Geom)) == 0 && memcmp(q.key, key, sizeof(key)) == 0) G = &q;
+  if (!G) {
+    G = &c->mg_graph[c->mg_graph_next];
+    c->mg_graph_next = (c->mg_graph_next + 1) % kMgGraphs;
+    if (G->exec) {
+      cudaGraphExecDestroy(G->exec);
+      G->exec = nullptr;
     }
-    if (graph) cudaGraphDestroy(graph);
+    cudaGraph_t graph = nullptr;
+    unsigned nl = 0;
+    if (cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+      const vg_status cst = enqueue(&nl);
+      const cudaError_t ce = cudaStreamEndCapture(c->stream, &graph);
+      if (cst == VG_OK && ce == cudaSuccess && graph && cudaGraphInstantiate(&G->exec, graph, 0) == cudaSuccess) {
+        G->g = g;
+        memcpy(G->key, key, sizeof(key));
+        G->launches = nl;
+      } else {
+        G->exec = nullptr;
+      }
+      if (graph) cudaGraphDestroy(graph);
+    }
+    cudaGetLastError();  // capture unavailable (e.g. the legacy stream): launch directly instead
   }
-  cudaGetLastError();  // capture unavailable (e.g. the legacy stream): launch directly instead
-}
-
-static vg_status run_cycle(Ctx* c, const MgPlan& P, const Geom& g, const MgBufs& B, float* x, const float* rhs,
-                           int slot) {
-  cycle_graph(c, P, g, B, x, rhs, slot);
-  MgGraphCache& G = c->mg_graph[slot];
-  if (G.exec) {
-    VG_CUDA(c, cudaGraphLaunch(G.exec, c->stream));
-    c->launches += G.launches;
+  if (G->exec) {
+    VG_CUDA(c, cudaGraphLaunch(G->exec, c->stream));
+    c->launches += G->launches;
     return VG_OK;
   }
   unsigned nl = 0;
-  const vg_status st = enqueue_cycle(c, P, g, B, x, rhs, &nl);
+  const vg_status st = enqueue(&nl);
   c->launches += nl;
   return st;
 }
 
-static vg_status read_norm(Ctx* c, const MgBufs& B, double* rr, double* bb) {
+static vg_status run_cycle(Ctx* c, const MgPlan& P, const Geom& g, const MgBufs& B, float* x, const float* rhs) {
+  const void* const key[4] = {B.E, rhs, x, nullptr};
+  return run_cached(c, g, key, [&](unsigned* nl) { return enqueue_cycle(c, P, g, B, x, rhs, nl); });
+}
+
+static vg_status read_norm(Ctx* c, const double* sums, double* rr, double* bb) {
   double h[2];
-  VG_CUDA(c, cudaMemcpyAsync(h, B.sums, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
+  VG_CUDA(c, cudaMemcpyAsync(h, sums, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
   VG_CUDA(c, cudaStreamSynchronize(c->stream));
   *rr = h[0];
   if (bb) *bb = h[1];
@@ -1348,7 +1580,23 @@ static vg_status direct_tables(Ctx* c, const Geom& lg, bool fp64, const void** o
   return VG_OK;
 }
 
-// Buffers of a solve on grid g (grow-only workspace slot S_MG).
+// Shared-memory limits of the coarse kernels: attributes are per device, set once for each device used.
+static void set_coarse_attributes(Ctx* c) {
+  static unsigned long long smem_set = 0;
+  const unsigned long long dev_bit = 1ull << (c->cfg.device & 63);
+  if (smem_set & dev_bit) return;
+  cudaFuncSetAttribute(k_vcycle_small, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  cudaFuncSetAttribute(k_dst_xy<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDstSmemMax);
+  cudaFuncSetAttribute(k_dst_xy<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDstSmemMax);
+  cudaFuncSetAttribute(k_dst_zz<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDstSmemMax);
+  cudaFuncSetAttribute(k_dst_zz<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDstSmemMax);
+  cudaFuncSetAttribute(k_dst_yx<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDstSmemMax);
+  cudaFuncSetAttribute(k_dst_yx<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDstSmemMax);
+  smem_set |= dev_bit;
+}
+
+// Buffers of a solve on grid g in interleaved fields (grow-only workspace slot S_MG): the persistent solve's, and those of a
+// hierarchy without smoothed levels.
 static vg_status setup_bufs(Ctx* c, const Geom& g, const MgPlan& P, MgBufs& B, float** etot, float** rir) {
   const size_t n0 = g.points();
   const ResLaunch rl = res_launch(g);
@@ -1375,19 +1623,7 @@ static vg_status setup_bufs(Ctx* c, const Geom& g, const MgPlan& P, MgBufs& B, f
     return st;
   *etot = (float*)(((uintptr_t)(B.cwork + 3 * coarse_pts) + 255) & ~(uintptr_t)255);  // IR correction
   *rir = *etot + 3 * n0;                                                                 // IR right-hand side
-  // kernel attributes are per device: set once for each device used
-  static unsigned long long smem_set = 0;
-  const unsigned long long dev_bit = 1ull << (c->cfg.device & 63);
-  if (!(smem_set & dev_bit)) {
-    cudaFuncSetAttribute(k_vcycle_small, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(k_dst_xy<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDstSmemMax);
-    cudaFuncSetAttribute(k_dst_xy<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDstSmemMax);
-    cudaFuncSetAttribute(k_dst_zz<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDstSmemMax);
-    cudaFuncSetAttribute(k_dst_zz<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDstSmemMax);
-    cudaFuncSetAttribute(k_dst_yx<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDstSmemMax);
-    cudaFuncSetAttribute(k_dst_yx<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDstSmemMax);
-    smem_set |= dev_bit;
-  }
+  set_coarse_attributes(c);
   return VG_OK;
 }
 
@@ -1421,13 +1657,317 @@ static PairCoef pair_coef(const Geom& g, const Lev& L0) {
   return cf;
 }
 
+// ---- the solve over split levels (hierarchies with smoothed levels)
+
+struct SplitBufs {
+  SGeo g[kMaxLayers];
+  SLaunch sl[kMaxLayers];
+  float *E[kMaxLayers], *R[kMaxLayers];  // correction and right-hand side of each smoothed level
+  float *X[2], *B, *T[3], *rir;          // level 0: the iterate twice, the right-hand side; refinement's corrections and residual
+  float *Ec, *Rc;                        // the coarse level's, interleaved
+  size_t n4;                             // float4 groups of a level-0 field
+  MgBufs mb;                             // sums, coarse workspace and tables
+};
+
+static vg_status setup_split(Ctx* c, const MgPlan& P, SplitBufs& S) {
+  if (P.small_smem > 200 * 1024) return fail(c, VG_TOO_LARGE, "multigrid: coarse levels exceed shared memory");
+  const int fs = P.first_small;
+  size_t bytes = 0;
+  auto take = [&](size_t n) {
+    const size_t at = bytes;
+    bytes += (n + 255) & ~(size_t)255;
+    return at;
+  };
+  size_t oE[kMaxLayers], oR[kMaxLayers], oF[7];
+  for (int l = 0; l < fs; ++l) {
+    S.g[l] = split_geo(P.lev[l]);
+    S.sl[l] = split_launch(S.g[l]);
+    const size_t f = 6 * S.g[l].cs * sizeof(float);
+    oE[l] = take(f);
+    oR[l] = take(f);
+    if (l == 0)
+      for (size_t& o : oF) o = take(f);
+  }
+  const size_t coarse = 3 * P.lev[fs].g.points(), last = 3 * P.lev[P.nlev - 1].g.points();
+  const size_t oEc = take(coarse * sizeof(float)), oRc = take(coarse * sizeof(float));
+  const size_t oP = take((2 * (size_t)S.sl[0].nb + 4) * sizeof(double)), oW = take(last * sizeof(double));
+  vg_status st = VG_OK;
+  char* mem = (char*)ws(c, S_MGSPLIT, bytes, &st);
+  if (st != VG_OK) return st;
+  for (int l = 0; l < fs; ++l) {
+    S.E[l] = (float*)(mem + oE[l]);
+    S.R[l] = (float*)(mem + oR[l]);
+  }
+  float* f[7];
+  for (int k = 0; k < 7; ++k) f[k] = (float*)(mem + oF[k]);
+  S.X[0] = f[0];
+  S.X[1] = f[1];
+  S.B = f[2];
+  for (int k = 0; k < 3; ++k) S.T[k] = f[3 + k];
+  S.rir = f[6];
+  S.Ec = (float*)(mem + oEc);
+  S.Rc = (float*)(mem + oRc);
+  S.n4 = 6 * S.g[0].cs / 4;
+  MgBufs& B = S.mb;
+  memset(&B, 0, sizeof(B));
+  B.part = (double*)(mem + oP);
+  B.sums = B.part + 2 * (size_t)S.sl[0].nb;
+  B.nb0 = S.sl[0].nb;
+  B.cwork = (double*)(mem + oW);
+  B.dst64 = P.direct_global && c->mg_coarse_fp64;
+  if (P.direct && (st = direct_tables(c, P.lev[P.nlev - 1].g, B.dst64, &B.dst, &B.d64a, &B.d64b)) != VG_OK)
+    return st;
+  set_coarse_attributes(c);
+  return VG_OK;
+}
+
+// One V(2,2)-cycle on L E[0] = r0 (E[0] starts from zero).
+static vg_status enqueue_vcycle(Ctx* c, const MgPlan& P, const SplitBufs& S, const float* r0, unsigned* nl) {
+  const int fs = P.first_small;
+  auto sweep = [&](int l, unsigned col) {
+    const SLaunch& L = S.sl[l];
+    pdl_launch(c->stream, L.grid, L.block, 0, k_s_sweep, S.g[l], S.E[l], l ? (const float*)S.R[l] : r0, col, L.zs);
+    ++*nl;
+  };
+  for (int l = 0; l < fs; ++l) {
+    const SLaunch& L = S.sl[l];
+    const float* r = l ? S.R[l] : r0;
+    pdl_launch(c->stream, L.grid, L.block, 0, k_s_first, S.g[l], S.E[l], r, L.zs);
+    ++*nl;
+    sweep(l, 0);
+    sweep(l, 1);
+    const unsigned* np = P.lev[l + 1].g.np;
+    const dim3 rg((np[0] - 2 + kQX - 1) / kQX, (np[1] - 2 + kQY - 1) / kQY, 3 * ((np[2] - 2 + kQZ - 1) / kQZ));
+    if (l + 1 < fs) {
+      pdl_launch(c->stream, rg, 256, 0, k_s_restrict<true>, S.g[l], S.g[l + 1], (const float*)S.E[l], r, S.R[l + 1]);
+    } else {
+      SGeo C = {};
+      C.nx = np[0];
+      C.ny = np[1];
+      C.nz = np[2];
+      pdl_launch(c->stream, rg, 256, 0, k_s_restrict<false>, S.g[l], C, (const float*)S.E[l], r, S.Rc);
+    }
+    ++*nl;
+  }
+  const vg_status st = enqueue_coarse(c, P, S.mb, S.Ec, S.Rc, nl);
+  if (st != VG_OK) return st;
+  for (int l = fs - 1; l >= 0; --l) {
+    const SLaunch& L = S.sl[l];
+    const dim3 pg(L.grid.x, L.grid.y, 3 * (S.g[l].nz - 2));
+    if (l + 1 < fs) {
+      pdl_launch(c->stream, pg, L.block, 0, k_s_prolong<true>, S.g[l], S.g[l + 1], (const float*)S.E[l + 1], S.E[l]);
+    } else {
+      SGeo C = {};
+      C.nx = P.lev[l + 1].g.np[0];
+      C.ny = P.lev[l + 1].g.np[1];
+      C.nz = P.lev[l + 1].g.np[2];
+      pdl_launch(c->stream, pg, L.block, 0, k_s_prolong<false>, S.g[l], C, (const float*)S.Ec, S.E[l]);
+    }
+    ++*nl;
+    for (int s = 0; s < 2; ++s)
+      for (unsigned col = 0; col < 2; ++col) sweep(l, col);
+  }
+  VG_CUDA(c, cudaGetLastError());
+  return VG_OK;
+}
+
+// r = b - L v (and v to xn), with its norm when `norm`.
+template <int kField>
+static void enqueue_residual(Ctx* c, const SplitBufs& S, const float* x, const float* b, float* xn, bool norm,
+                             unsigned* nl) {
+  const SLaunch& L = S.sl[0];
+  const float* e = S.E[0];
+  if (norm) {
+    pdl_launch(c->stream, L.grid, L.block, 0, k_s_residual<kField, true>, S.g[0], x, e, b, xn, S.R[0], S.mb.part, L.zs);
+  } else {
+    pdl_launch(c->stream, L.grid, L.block, 0, k_s_residual<kField, false>, S.g[0], x, e, b, xn, S.R[0], S.mb.part, L.zs);
+  }
+  ++*nl;
+}
+
+static void enqueue_norm(Ctx* c, const SplitBufs& S, int keep_b, unsigned* nl) {
+  pdl_launch(c->stream, 1, 1024, 0, k_sum_partials, S.mb.part, (int)S.mb.nb0, S.mb.sums, keep_b);
+  ++*nl;
+}
+
+// The accurate residual of x (kAdd: of x + e, written to xn) + lo into r, and its norm.
+template <bool kAdd, bool kLo>
+static void enqueue_pair(Ctx* c, const SplitBufs& S, const PairCoef& cf, const float* x, const float* lo, float* xn,
+                         float* r, unsigned* nl) {
+  const SLaunch& L = S.sl[0];
+  pdl_launch(c->stream, L.grid, L.block, 0, k_s_residual_pair<kAdd, kLo>, S.g[0], cf, x, (const float*)S.E[0], lo,
+             (const float*)S.B, xn, r, S.mb.part, L.zs);
+  ++*nl;
+  enqueue_norm(c, S, 1, nl);
+}
+
+// The solve's start: zero boundaries of the corrections, the split iterate and right-hand side, the first residual.
+static void enqueue_start(Ctx* c, const MgPlan& P, const SplitBufs& S, const float* soln3, const float* rhs3,
+                          unsigned* nl) {
+  FaceList F;
+  F.n = 0;
+  auto add = [&](float* f, const SGeo& g) {
+    F.f[F.n] = f;
+    F.g[F.n++] = g;
+  };
+  for (int l = 0; l < P.first_small; ++l) add(S.E[l], S.g[l]);
+  for (int k = 0; k < 3; ++k) add(S.T[k], S.g[0]);
+  pdl_launch(c->stream, dim3(blocks_for((size_t)6 * S.g[0].ny * S.g[0].nz, 256), F.n), 256, 0, k_s_faces, F);
+  pdl_launch(c->stream, blocks_for(S.g[0].ny * S.g[0].nz, 8), 256, 0, k_s_in, S.g[0], soln3, rhs3, S.X[0], S.X[1], S.B);
+  *nl += 2;
+  enqueue_residual<RES_X>(c, S, S.X[0], S.B, nullptr, true, nl);
+  enqueue_norm(c, S, 0, nl);
+}
+
+static void enqueue_out(Ctx* c, const SplitBufs& S, const float* x, const float* d, float* soln3, unsigned* nl) {
+  const unsigned nb = blocks_for(S.g[0].ny * S.g[0].nz, 8);
+  if (d)
+    pdl_launch(c->stream, nb, 256, 0, k_s_out<true>, S.g[0], x, d, soln3);
+  else
+    pdl_launch(c->stream, nb, 256, 0, k_s_out<false>, S.g[0], x, d, soln3);
+  ++*nl;
+}
+
+// run_multigrid_fixed over split levels.  Additions that the next kernel can make on the way are left to it: a cycle's
+// x += e to the residual that follows, a first correction's 0 + e to its readers.
+static vg_status split_fixed(Ctx* c, const Geom& g, const MgPlan& P, float* soln3, const float* rhs3) {
+  SplitBufs S;
+  vg_status st = setup_split(c, P, S);
+  if (st != VG_OK) return st;
+  const PairCoef cf = pair_coef(g, P.lev[0]);
+  const int k1 = c->mg_fixed_k1, k2 = c->mg_fixed_k2;
+  unsigned nl = 0;
+  enqueue_start(c, P, S, soln3, rhs3, &nl);
+  pdl_launch(c->stream, 1, 32, 0, k_relres, S.mb.sums, c->mg_relres_dev + 1);
+  ++nl;
+  int cur = 0;
+  for (int k = 0; k < k1; ++k) {
+    if ((st = enqueue_vcycle(c, P, S, S.R[0], &nl)) != VG_OK) return st;
+    if (k + 1 < k1)
+      enqueue_residual<RES_X_PLUS_E>(c, S, S.X[cur], S.B, S.X[cur ^ 1], false, &nl);
+    else
+      enqueue_pair<true, false>(c, S, cf, S.X[cur], nullptr, S.X[cur ^ 1], S.rir, &nl);
+    cur ^= 1;
+  }
+  const float* lo = nullptr;
+  if (k2 > 0) {
+    if ((st = enqueue_vcycle(c, P, S, S.rir, &nl)) != VG_OK) return st;
+    lo = S.E[0];
+    if (k2 > 1) {
+      int t = 0;
+      enqueue_residual<RES_E>(c, S, nullptr, S.rir, S.T[0], false, &nl);
+      for (int k = 1; k < k2; ++k) {
+        if ((st = enqueue_vcycle(c, P, S, S.R[0], &nl)) != VG_OK) return st;
+        if (k + 1 < k2) {
+          enqueue_residual<RES_X_PLUS_E>(c, S, S.T[t], S.rir, S.T[t ^ 1], false, &nl);
+          t ^= 1;
+        }
+      }
+      pdl_launch(c->stream, blocks_for(S.n4, 256), 256, 0, k_s_add, (float4*)S.T[t], (const float4*)S.E[0], S.n4);
+      ++nl;
+      lo = S.T[t];
+    }
+    enqueue_pair<false, true>(c, S, cf, S.X[cur], lo, nullptr, S.R[0], &nl);
+  }
+  pdl_launch(c->stream, 1, 32, 0, k_relres, S.mb.sums, c->mg_relres_dev);
+  ++nl;
+  enqueue_out(c, S, S.X[cur], lo, soln3, &nl);
+  c->launches += nl;
+  VG_CUDA(c, cudaGetLastError());
+  return VG_OK;
+}
+
+// run_multigrid over split levels; the cycles run from graphs.
+static vg_status split_adaptive(Ctx* c, const Geom& g, const MgPlan& P, float* soln3, const float* rhs3, double tol,
+                                int max_cycles, int* cycles, int* phase1, double* relres0, double* relres_out) {
+  SplitBufs S;
+  vg_status st = setup_split(c, P, S);
+  if (st != VG_OK) return st;
+  const PairCoef cf = pair_coef(g, P.lev[0]);
+  unsigned nl = 0;
+  enqueue_start(c, P, S, soln3, rhs3, &nl);
+  double rr = 0.0, bnorm2 = 0.0;
+  if ((st = read_norm(c, S.mb.sums, &rr, &bnorm2)) != VG_OK) return st;
+  const double bn = bnorm2 > 0.0 ? std::sqrt(bnorm2) : 1.0;
+  double relres = std::sqrt(rr) / bn;
+  *relres0 = relres;
+  int cyc = 0, cur = 0;
+  // a cycle from r0, then the residual of x + e (x NULL: of e) on right-hand side b, the sum to xn
+  auto cycle = [&](const float* r0, const float* x, const float* b, float* xn) -> vg_status {
+    const void* const key[4] = {S.E[0], r0, x, xn};
+    const vg_status cst = run_cached(c, g, key, [&](unsigned* n) -> vg_status {
+      const vg_status vst = enqueue_vcycle(c, P, S, r0, n);
+      if (vst != VG_OK) return vst;
+      if (x)
+        enqueue_residual<RES_X_PLUS_E>(c, S, x, b, xn, true, n);
+      else
+        enqueue_residual<RES_E>(c, S, nullptr, b, xn, true, n);
+      enqueue_norm(c, S, 1, n);
+      VG_CUDA(c, cudaGetLastError());
+      return VG_OK;
+    });
+    ++cyc;
+    return cst != VG_OK ? cst : read_norm(c, S.mb.sums, &rr, nullptr);
+  };
+  // Phase 1: FP32 cycles on the field itself while FP32 can represent the
+  // residual (relative residual above 1e-4).
+  const double switch_tol = std::max(tol, 1e-4);
+  while (relres > switch_tol && cyc < max_cycles) {
+    if ((st = cycle(S.R[0], S.X[cur], S.B, S.X[cur ^ 1])) != VG_OK) return st;
+    cur ^= 1;
+    relres = std::sqrt(rr) / bn;
+  }
+  *phase1 = cyc;
+  // Phase 2: iterative refinement (run_multigrid)
+  int lo = -1;  // the buffer in T that holds the accumulated corrections
+  for (;;) {
+    if (lo < 0)
+      enqueue_pair<false, false>(c, S, cf, S.X[cur], nullptr, nullptr, S.rir, &nl);
+    else
+      enqueue_pair<false, true>(c, S, cf, S.X[cur], S.T[lo], nullptr, S.rir, &nl);
+    if ((st = read_norm(c, S.mb.sums, &rr, nullptr)) != VG_OK) return st;
+    relres = std::sqrt(rr) / bn;
+    if (relres <= tol || cyc >= max_cycles) break;
+    const double inner_tol = std::max(0.9 * tol, 1e-4 * relres);
+    const int ta = lo == 0 ? 1 : 0, tb = 3 - ta - std::max(lo, 0) - (lo < 0 ? 2 : 0);
+    int t = ta;
+    double inner = relres;
+    bool first = true;
+    while (inner > inner_tol && cyc < max_cycles) {
+      if (first) {
+        st = cycle(S.rir, nullptr, S.rir, S.T[t]);
+      } else {
+        const int u = t == ta ? tb : ta;
+        st = cycle(S.R[0], S.T[t], S.rir, S.T[u]);
+        t = u;
+      }
+      if (st != VG_OK) return st;
+      first = false;
+      inner = std::sqrt(rr) / bn;
+    }
+    if (lo < 0) {
+      lo = t;
+    } else {
+      pdl_launch(c->stream, blocks_for(S.n4, 256), 256, 0, k_s_add, (float4*)S.T[lo], (const float4*)S.T[t], S.n4);
+      ++nl;
+    }
+  }
+  enqueue_out(c, S, S.X[cur], lo < 0 ? nullptr : S.T[lo], soln3, &nl);
+  c->launches += nl;
+  VG_CUDA(c, cudaGetLastError());
+  *cycles = cyc;
+  *relres_out = relres;
+  return VG_OK;
+}
+
 vg_status run_multigrid_fixed(Ctx* c, const Geom& g, float* soln3, const float* rhs3) {
   const MgPlan P = plan_levels(g);
+  if (!c->mg_relres_dev) return fail(c, VG_INVALID, "multigrid: no device slot for the residual");
+  if (P.first_small > 0) return split_fixed(c, g, P, soln3, rhs3);
   MgBufs B;
   float *etot = nullptr, *rir = nullptr;
   vg_status st = setup_bufs(c, g, P, B, &etot, &rir);
   if (st != VG_OK) return st;
-  if (!c->mg_relres_dev) return fail(c, VG_INVALID, "multigrid: no device slot for the residual");
   const size_t n0 = g.points();
   const unsigned nb0 = B.nb0;
   const Lev& L0 = P.lev[0];
@@ -1496,6 +2036,21 @@ vg_status run_multigrid_fixed(Ctx* c, const Geom& g, float* soln3, const float* 
 vg_status run_multigrid(Ctx* c, const Geom& g, float* soln3, const float* rhs3, double tol, int max_cycles,
                         int* cycles_out, double* relres0_out, double* relres_out) {
   const MgPlan P = plan_levels(g);
+  auto finish = [&](int cyc, int k1, double relres0, double relres) -> vg_status {
+    c->mg_last_k1 = k1;
+    c->mg_last_k2 = cyc - k1;
+    if (cycles_out) *cycles_out = cyc;
+    if (relres0_out) *relres0_out = relres0;
+    if (relres_out) *relres_out = relres;
+    if (relres > tol) return fail(c, VG_NOT_CONVERGED, "multigrid: cycle limit reached above tolerance");
+    return VG_OK;
+  };
+  if (P.first_small > 0) {
+    int cyc = 0, k1 = 0;
+    double r0 = 0.0, r1 = 0.0;
+    const vg_status sst = split_adaptive(c, g, P, soln3, rhs3, tol, max_cycles, &cyc, &k1, &r0, &r1);
+    return sst != VG_OK ? sst : finish(cyc, k1, r0, r1);
+  }
   const size_t n0 = g.points();
   MgBufs B;
   float *etot = nullptr, *rir = nullptr;
@@ -1512,7 +2067,7 @@ vg_status run_multigrid(Ctx* c, const Geom& g, float* soln3, const float* rhs3, 
   pdl_launch(c->stream, 1, 1024, 0, k_sum_partials, B.part, (int)nb0, B.sums, 0);
   c->launches += 2;
   double rr = 0.0, bnorm2 = 0.0;
-  if ((st = read_norm(c, B, &rr, &bnorm2)) != VG_OK) return st;
+  if ((st = read_norm(c, B.sums, &rr, &bnorm2)) != VG_OK) return st;
   const double bn = bnorm2 > 0.0 ? std::sqrt(bnorm2) : 1.0;
   double relres = std::sqrt(rr) / bn;
   const double relres0 = relres;
@@ -1521,9 +2076,9 @@ vg_status run_multigrid(Ctx* c, const Geom& g, float* soln3, const float* rhs3, 
   // residual (relative residual above 1e-4).
   const double switch_tol = std::max(tol, 1e-4);
   while (relres > switch_tol && cyc < max_cycles) {
-    if ((st = run_cycle(c, P, g, B, soln3, rhs3, 0)) != VG_OK) return st;
+    if ((st = run_cycle(c, P, g, B, soln3, rhs3)) != VG_OK) return st;
     ++cyc;
-    if ((st = read_norm(c, B, &rr, nullptr)) != VG_OK) return st;
+    if ((st = read_norm(c, B.sums, &rr, nullptr)) != VG_OK) return st;
     relres = std::sqrt(rr) / bn;
   }
   const int k1 = cyc;
@@ -1537,7 +2092,7 @@ vg_status run_multigrid(Ctx* c, const Geom& g, float* soln3, const float* rhs3, 
     pdl_launch(c->stream, B.rl.grid, B.rl.block, 0, k_residual_pair<true>, g, cf, B.rl.zs, soln3, B.lo, rhs3, rir, B.part);
     pdl_launch(c->stream, 1, 1024, 0, k_sum_partials, B.part, (int)nb0, B.sums, 1);
     c->launches += 2;
-    if ((st = read_norm(c, B, &rr, nullptr)) != VG_OK) return st;
+    if ((st = read_norm(c, B.sums, &rr, nullptr)) != VG_OK) return st;
     relres = std::sqrt(rr) / bn;
     if (relres <= tol || cyc >= max_cycles) break;
     // The FP32 residual of the correction equation tracks the accurate residual
@@ -1548,9 +2103,9 @@ vg_status run_multigrid(Ctx* c, const Geom& g, float* soln3, const float* rhs3, 
     VG_CUDA(c, cudaMemcpyAsync(B.R, rir, 3 * n0 * sizeof(float), cudaMemcpyDeviceToDevice, c->stream));
     double inner = relres;
     while (inner > inner_tol && cyc < max_cycles) {
-      if ((st = run_cycle(c, P, g, B, etot, rir, 1)) != VG_OK) return st;
+      if ((st = run_cycle(c, P, g, B, etot, rir)) != VG_OK) return st;
       ++cyc;
-      if ((st = read_norm(c, B, &rr, nullptr)) != VG_OK) return st;
+      if ((st = read_norm(c, B.sums, &rr, nullptr)) != VG_OK) return st;
       inner = std::sqrt(rr) / bn;
     }
     add_f32(c, B.lo, etot, 3 * n0);
@@ -1559,13 +2114,7 @@ vg_status run_multigrid(Ctx* c, const Geom& g, float* soln3, const float* rhs3, 
   add_f32(c, soln3, B.lo, 3 * n0);
   VG_LAUNCHED(c);
   VG_CUDA(c, cudaGetLastError());
-  c->mg_last_k1 = k1;
-  c->mg_last_k2 = cyc - k1;
-  if (cycles_out) *cycles_out = cyc;
-  if (relres0_out) *relres0_out = relres0;
-  if (relres_out) *relres_out = relres;
-  if (relres > tol) return fail(c, VG_NOT_CONVERGED, "multigrid: cycle limit reached above tolerance");
-  return VG_OK;
+  return finish(cyc, k1, relres0, relres);
 }
 
 // ------------------------------------------------------- persistent batched solve
