@@ -675,6 +675,7 @@ vg_status vg_destroy(vg_ctx* c) {
     if (G.exec) cudaGraphExecDestroy(G.exec);
   if (c->dflag) cudaFree(c->dflag);
   if (c->hflag) cudaFreeHost(c->hflag);
+  if (c->hnorm) cudaFreeHost(c->hnorm);
   if (c->mg_relres_dev) cudaFree(c->mg_relres_dev);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);

@@ -33,6 +33,7 @@
 #include <float.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <type_traits>
@@ -401,9 +402,11 @@ static SLaunch split_launch(const SGeo& g) {
   while (by > 8 && by - 8 >= g.ny - 2) by -= 8;
   SLaunch L;
   L.block = dim3(bx, by);
-  // marching planes saves reads of the plane before and behind; short marches keep enough threads on the chip
+  // marching planes saves reads of the plane before and behind; short marches keep enough threads on the chip.  Half sweep,
+  // us at 1 / 2 / 4 / 8 planes: 225 x 161 x 193 36.7 / 32.5 / 30.7 / 29.9, its whole solve best at 4; 129^3 (0.77 M threads
+  // at one plane) 10.7 / 9.2 / 9.9 / 10.9
   const double threads = 3.0 * g.groups * (g.ny - 2) * (g.nz - 2);
-  L.zs = threads > 1.2e6 ? 8 : threads > 4e5 ? 4 : threads > 1.5e5 ? 2 : 1;
+  L.zs = threads > 2e6 ? 4 : threads > 3e5 ? 2 : 1;
   L.grid = dim3((g.groups + bx - 1) / bx, (g.ny - 2 + by - 1) / by, 3 * ((g.nz - 2 + L.zs - 1) / L.zs));
   L.nb = L.grid.x * L.grid.y * L.grid.z;
   return L;
@@ -495,6 +498,7 @@ __global__ void __launch_bounds__(256) k_s_first(SGeo g, float* __restrict__ E, 
     if (x_interior(g, p, i0 + 3)) bv.w = sweep_value(g, 0.f, rv.w, xm.w, xp.w, ym.w, yp.w, om.w, op.w);
     st4(er, rc);
     st4(eb, bv);
+    if (i0 + 4 == g.m) (q ? eb : er)[4] = 0.f;  // x = nx - 1, behind the last group (of the even points)
     om = oc;
     oc = op;
   }
@@ -643,6 +647,48 @@ __device__ __forceinline__ void split_sum2(float a32, float b32, double* __restr
   }
 }
 
+// The adaptive solve's norms: k_sum_partials whose sums also go to pinned host memory ([0] r^2, [1] b^2), behind a sequence
+// number ([2]) that the host polls: a copy and a stream wait took about 12 us a norm more.  (Summing in the residual kernels
+// by their last block, instead of this launch of 4 us, made them 4 to 10 us longer: a fence and an atomic at every block's end.)
+__global__ void __launch_bounds__(1024) k_s_norm(const double* __restrict__ part, int nb, double* __restrict__ out2,
+                                                 int keep_b, unsigned long long* __restrict__ seq, volatile double* host) {
+  pdl_entry();
+  __shared__ double s1[32], s2[32];
+  double a1 = 0.0, a2 = 0.0;
+  for (int i = threadIdx.x; i < nb; i += 1024) {
+    a1 += part[2 * i];
+    a2 += part[2 * i + 1];
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    a1 += __shfl_xor_sync(0xffffffffu, a1, o);
+    a2 += __shfl_xor_sync(0xffffffffu, a2, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    s1[threadIdx.x >> 5] = a1;
+    s2[threadIdx.x >> 5] = a2;
+  }
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  a1 = s1[threadIdx.x];
+  a2 = s2[threadIdx.x];
+  for (int o = 16; o > 0; o >>= 1) {
+    a1 += __shfl_xor_sync(0xffffffffu, a1, o);
+    a2 += __shfl_xor_sync(0xffffffffu, a2, o);
+  }
+  if (threadIdx.x) return;
+  out2[0] = a1;
+  if (keep_b)
+    a2 = out2[1];
+  else
+    out2[1] = a2;
+  if (host) {
+    host[0] = a1;
+    host[1] = a2;
+    __threadfence_system();
+    host[2] = (double)++*seq;
+  }
+}
+
 // The iterate's values in a residual: x; x + e (the cycle's correction, whose sum is also written); or e alone (a first
 // correction, 0 + e).
 enum ResField { RES_X, RES_X_PLUS_E, RES_E };
@@ -715,6 +761,7 @@ __global__ void __launch_bounds__(256) k_s_residual(SGeo g, const float* __restr
       if (kField != RES_X) {
         st4(xn + ec, e0);
         st4(xn + oc, o0);
+        if (i0 + 4 == g.m) xn[ec + 4] = right;  // x = nx - 1
       }
       em = e0;
       om = o0;
@@ -796,32 +843,43 @@ __global__ void __launch_bounds__(256) k_s_add(float4* __restrict__ a, const flo
   a[i] = make_float4(__fadd_rn(u.x, v.x), __fadd_rn(u.y, v.y), __fadd_rn(u.z, v.z), __fadd_rn(u.w, v.w));
 }
 
-// Interleaved fields into split ones: the solution into x, its boundary values into x2 too, and the right-hand side; a warp a
-// row, component and parity after component and parity (the row's bytes stay in L1).
+// Interleaved fields into split ones: the solution into x, its boundary values into x2 too, and the right-hand side.  A warp a
+// row, 64 points at a time through shared memory.
 __global__ void __launch_bounds__(256) k_s_in(SGeo g, const float* __restrict__ soln, const float* __restrict__ rhs,
                                               float* __restrict__ x, float* __restrict__ x2, float* __restrict__ b) {
   pdl_entry();
-  const unsigned row = blockIdx.x * 8 + threadIdx.x / 32, lane = threadIdx.x & 31;
-  if (row >= g.ny * g.nz) return;
-  const unsigned y = row % g.ny, z = row / g.ny;
+  __shared__ float s_f[8][2][192];
+  const unsigned w = threadIdx.x / 32, row = blockIdx.x * 8 + w, lane = threadIdx.x & 31;
+  if (row >= g.ny * g.nz) return;  // whole warps
+  const unsigned y = row % g.ny, z = row / g.ny, n3 = 3 * g.nx;
   const bool edge = y == 0 || z == 0 || y + 1 == g.ny || z + 1 == g.nz;
-  const float* sr = soln + 3 * (size_t)g.nx * row;
-  const float* br = rhs + 3 * (size_t)g.nx * row;
+  const float* sr = soln + (size_t)n3 * row;
+  const float* br = rhs + (size_t)n3 * row;
   const size_t o = (size_t)z * g.pz + y * g.hx;
-  for (unsigned i = lane; i < g.hx; i += 32)
+  for (unsigned i0 = 0; i0 < g.hx; i0 += 32) {
 #pragma unroll
-    for (unsigned p = 0; p < 2; ++p) {
-      const unsigned X = 2 * i + p;
-      const bool in = X < g.nx;
-#pragma unroll
-      for (unsigned c = 0; c < 3; ++c) {
-        const size_t at = (2 * c + ((p + y + z) & 1u)) * g.cs + o + i;
-        const float v = in ? sr[3 * X + c] : 0.f;
-        x[at] = v;
-        if (edge || X == 0 || X + 1 >= g.nx) x2[at] = v;
-        b[at] = in ? br[3 * X + c] : 0.f;
-      }
+    for (unsigned k = 0; k < 6; ++k) {
+      const unsigned q = 6 * i0 + 32 * k + lane;
+      s_f[w][0][32 * k + lane] = q < n3 ? sr[q] : 0.f;
+      s_f[w][1][32 * k + lane] = q < n3 ? br[q] : 0.f;
     }
+    __syncwarp();
+    const unsigned i = i0 + lane;
+    if (i < g.hx)
+#pragma unroll
+      for (unsigned p = 0; p < 2; ++p) {
+        const unsigned X = 2 * i + p;
+#pragma unroll
+        for (unsigned c = 0; c < 3; ++c) {
+          const size_t at = (2 * c + ((p + y + z) & 1u)) * g.cs + o + i;
+          const float v = s_f[w][0][6 * lane + 3 * p + c];
+          x[at] = v;
+          if (edge || X == 0 || X + 1 >= g.nx) x2[at] = v;
+          b[at] = s_f[w][1][6 * lane + 3 * p + c];
+        }
+      }
+    __syncwarp();
+  }
 }
 
 // The interleaved solution from the split fields: x, or x + d.
@@ -841,25 +899,26 @@ __global__ void __launch_bounds__(256) k_s_out(SGeo g, const float* __restrict__
   }
 }
 
-// Zero on the boundary (and in the rows' padding) of split fields: a correction is zero there, and only its interior is ever
-// written.  A thread a row, the fields in the launch's y.
+// Zero in the boundary planes and rows (y, z) of split fields, where a correction is zero and only its interior is ever
+// written (its first and last points in x are written with the rows); a warp a row.  Also the norms' sequence number.
 struct FaceList {
   int n;
   float* f[kMaxLayers + 2];
   SGeo g[kMaxLayers + 2];
+  unsigned long long* seq;
+  unsigned long long seq0;
 };
 __global__ void __launch_bounds__(256) k_s_faces(const __grid_constant__ FaceList L) {
   pdl_entry();
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *L.seq = L.seq0;
   const SGeo& g = L.g[blockIdx.y];
-  const unsigned q = blockIdx.x * blockDim.x + threadIdx.x, y = q % g.ny, z = q / g.ny % g.nz, a = q / (g.ny * g.nz);
-  if (a >= 6) return;  // a = 2 c + colour
+  const unsigned q = blockIdx.x * 8 + threadIdx.x / 32, lane = threadIdx.x & 31, edges = 2 * g.ny + 2 * g.nz;
+  const unsigned a = q / edges, k = q % edges;  // a = 2 c + colour
+  if (a >= 6) return;
+  const unsigned z = k < g.ny ? 0 : k < 2 * g.ny ? g.nz - 1 : (k - 2 * g.ny) % g.nz;
+  const unsigned y = k < 2 * g.ny ? k % g.ny : k < 2 * g.ny + g.nz ? 0 : g.ny - 1;
   float* p = L.f[blockIdx.y] + a * g.cs + (size_t)z * g.pz + y * g.hx;
-  if (y == 0 || z == 0 || y + 1 == g.ny || z + 1 == g.nz) {
-    for (unsigned i = 0; i < g.hx; i += 4) st4(p + i, make_float4(0.f, 0.f, 0.f, 0.f));
-  } else {
-    if (((a + y + z) & 1u) == 0) p[0] = 0.f;  // x = 0
-    for (unsigned i = g.m; i < g.hx; ++i) p[i] = 0.f;
-  }
+  for (unsigned i = 4 * lane; i < g.hx; i += 128) st4(p + i, make_float4(0.f, 0.f, 0.f, 0.f));
 }
 
 // The small levels of a V-cycle in one CTA, their e and r in shared memory:
@@ -1666,6 +1725,8 @@ struct SplitBufs {
   float *X[2], *B, *T[3], *rir;          // level 0: the iterate twice, the right-hand side; refinement's corrections and residual
   float *Ec, *Rc;                        // the coarse level's, interleaved
   size_t n4;                             // float4 groups of a level-0 field
+  unsigned long long* seq;  // norms so far
+  double* host;             // pinned memory that they also go to, or null
   MgBufs mb;                             // sums, coarse workspace and tables
 };
 
@@ -1690,7 +1751,7 @@ static vg_status setup_split(Ctx* c, const MgPlan& P, SplitBufs& S) {
   }
   const size_t coarse = 3 * P.lev[fs].g.points(), last = 3 * P.lev[P.nlev - 1].g.points();
   const size_t oEc = take(coarse * sizeof(float)), oRc = take(coarse * sizeof(float));
-  const size_t oP = take((2 * (size_t)S.sl[0].nb + 4) * sizeof(double)), oW = take(last * sizeof(double));
+  const size_t oP = take((2 * (size_t)S.sl[0].nb + 8) * sizeof(double)), oW = take(last * sizeof(double));
   vg_status st = VG_OK;
   char* mem = (char*)ws(c, S_MGSPLIT, bytes, &st);
   if (st != VG_OK) return st;
@@ -1713,6 +1774,8 @@ static vg_status setup_split(Ctx* c, const MgPlan& P, SplitBufs& S) {
   B.part = (double*)(mem + oP);
   B.sums = B.part + 2 * (size_t)S.sl[0].nb;
   B.nb0 = S.sl[0].nb;
+  S.seq = (unsigned long long*)(B.sums + 4);
+  S.host = nullptr;
   B.cwork = (double*)(mem + oW);
   B.dst64 = P.direct_global && c->mg_coarse_fp64;
   if (P.direct && (st = direct_tables(c, P.lev[P.nlev - 1].g, B.dst64, &B.dst, &B.d64a, &B.d64b)) != VG_OK)
@@ -1771,23 +1834,24 @@ static vg_status enqueue_vcycle(Ctx* c, const MgPlan& P, const SplitBufs& S, con
   return VG_OK;
 }
 
-// r = b - L v (and v to xn), with its norm when `norm`.
-template <int kField>
-static void enqueue_residual(Ctx* c, const SplitBufs& S, const float* x, const float* b, float* xn, bool norm,
-                             unsigned* nl) {
-  const SLaunch& L = S.sl[0];
-  const float* e = S.E[0];
-  if (norm) {
-    pdl_launch(c->stream, L.grid, L.block, 0, k_s_residual<kField, true>, S.g[0], x, e, b, xn, S.R[0], S.mb.part, L.zs);
-  } else {
-    pdl_launch(c->stream, L.grid, L.block, 0, k_s_residual<kField, false>, S.g[0], x, e, b, xn, S.R[0], S.mb.part, L.zs);
-  }
+static void enqueue_norm(Ctx* c, const SplitBufs& S, int keep_b, unsigned* nl) {
+  pdl_launch(c->stream, 1, 1024, 0, k_s_norm, (const double*)S.mb.part, (int)S.mb.nb0, S.mb.sums, keep_b, S.seq,
+             (volatile double*)S.host);
   ++*nl;
 }
 
-static void enqueue_norm(Ctx* c, const SplitBufs& S, int keep_b, unsigned* nl) {
-  pdl_launch(c->stream, 1, 1024, 0, k_sum_partials, S.mb.part, (int)S.mb.nb0, S.mb.sums, keep_b);
+// r = b - L v (and v to xn), with its norm when `norm` (and ||b||^2 when `with_b`).
+template <int kField>
+static void enqueue_residual(Ctx* c, const SplitBufs& S, const float* x, const float* b, float* xn, bool norm,
+                             unsigned* nl, bool with_b = false) {
+  const SLaunch& L = S.sl[0];
+  const float* e = S.E[0];
+  if (norm)
+    pdl_launch(c->stream, L.grid, L.block, 0, k_s_residual<kField, true>, S.g[0], x, e, b, xn, S.R[0], S.mb.part, L.zs);
+  else
+    pdl_launch(c->stream, L.grid, L.block, 0, k_s_residual<kField, false>, S.g[0], x, e, b, xn, S.R[0], S.mb.part, L.zs);
   ++*nl;
+  if (norm) enqueue_norm(c, S, with_b ? 0 : 1, nl);
 }
 
 // The accurate residual of x (kAdd: of x + e, written to xn) + lo into r, and its norm.
@@ -1806,17 +1870,18 @@ static void enqueue_start(Ctx* c, const MgPlan& P, const SplitBufs& S, const flo
                           unsigned* nl) {
   FaceList F;
   F.n = 0;
+  F.seq = S.seq;
+  F.seq0 = c->norm_seq;
   auto add = [&](float* f, const SGeo& g) {
     F.f[F.n] = f;
     F.g[F.n++] = g;
   };
   for (int l = 0; l < P.first_small; ++l) add(S.E[l], S.g[l]);
   for (int k = 0; k < 3; ++k) add(S.T[k], S.g[0]);
-  pdl_launch(c->stream, dim3(blocks_for((size_t)6 * S.g[0].ny * S.g[0].nz, 256), F.n), 256, 0, k_s_faces, F);
+  pdl_launch(c->stream, dim3(blocks_for((size_t)12 * (S.g[0].ny + S.g[0].nz), 8), F.n), 256, 0, k_s_faces, F);
   pdl_launch(c->stream, blocks_for(S.g[0].ny * S.g[0].nz, 8), 256, 0, k_s_in, S.g[0], soln3, rhs3, S.X[0], S.X[1], S.B);
   *nl += 2;
-  enqueue_residual<RES_X>(c, S, S.X[0], S.B, nullptr, true, nl);
-  enqueue_norm(c, S, 0, nl);
+  enqueue_residual<RES_X>(c, S, S.X[0], S.B, nullptr, true, nl, true);
 }
 
 static void enqueue_out(Ctx* c, const SplitBufs& S, const float* x, const float* d, float* soln3, unsigned* nl) {
@@ -1877,17 +1942,41 @@ static vg_status split_fixed(Ctx* c, const Geom& g, const MgPlan& P, float* soln
   return VG_OK;
 }
 
+// The next norm of the solve, from pinned host memory as soon as the last block has written it.  The wait is a poll of that
+// memory; after every few thousand polls the stream is asked whether it has failed, or is done without the norm having come.
+static vg_status next_norm(Ctx* c, double* rr, double* bb) {
+  const double want = (double)++c->norm_seq;
+  volatile double* h = c->hnorm;
+  for (unsigned long long polls = 1; h[2] != want; ++polls) {
+    if (polls % 4096) continue;
+    const cudaError_t e = cudaStreamQuery(c->stream);
+    if (e == cudaErrorNotReady) continue;
+    VG_CUDA(c, e);
+    if (h[2] != want) return fail(c, VG_CUDA_ERROR, "multigrid: a residual norm was not written");
+  }
+  std::atomic_thread_fence(std::memory_order_acquire);
+  *rr = h[0];
+  if (bb) *bb = h[1];
+  if (!(*rr == *rr)) return fail(c, VG_NONFINITE, "multigrid: non-finite residual");
+  return VG_OK;
+}
+
 // run_multigrid over split levels; the cycles run from graphs.
 static vg_status split_adaptive(Ctx* c, const Geom& g, const MgPlan& P, float* soln3, const float* rhs3, double tol,
                                 int max_cycles, int* cycles, int* phase1, double* relres0, double* relres_out) {
   SplitBufs S;
   vg_status st = setup_split(c, P, S);
   if (st != VG_OK) return st;
+  if (!c->hnorm) {
+    VG_CUDA(c, cudaHostAlloc((void**)&c->hnorm, 64, cudaHostAllocDefault));
+    c->hnorm[2] = 0.0;
+  }
+  S.host = c->hnorm;
   const PairCoef cf = pair_coef(g, P.lev[0]);
   unsigned nl = 0;
   enqueue_start(c, P, S, soln3, rhs3, &nl);
   double rr = 0.0, bnorm2 = 0.0;
-  if ((st = read_norm(c, S.mb.sums, &rr, &bnorm2)) != VG_OK) return st;
+  if ((st = next_norm(c, &rr, &bnorm2)) != VG_OK) return st;
   const double bn = bnorm2 > 0.0 ? std::sqrt(bnorm2) : 1.0;
   double relres = std::sqrt(rr) / bn;
   *relres0 = relres;
@@ -1902,12 +1991,11 @@ static vg_status split_adaptive(Ctx* c, const Geom& g, const MgPlan& P, float* s
         enqueue_residual<RES_X_PLUS_E>(c, S, x, b, xn, true, n);
       else
         enqueue_residual<RES_E>(c, S, nullptr, b, xn, true, n);
-      enqueue_norm(c, S, 1, n);
       VG_CUDA(c, cudaGetLastError());
       return VG_OK;
     });
     ++cyc;
-    return cst != VG_OK ? cst : read_norm(c, S.mb.sums, &rr, nullptr);
+    return cst != VG_OK ? cst : next_norm(c, &rr, nullptr);
   };
   // Phase 1: FP32 cycles on the field itself while FP32 can represent the
   // residual (relative residual above 1e-4).
@@ -1925,7 +2013,7 @@ static vg_status split_adaptive(Ctx* c, const Geom& g, const MgPlan& P, float* s
       enqueue_pair<false, false>(c, S, cf, S.X[cur], nullptr, nullptr, S.rir, &nl);
     else
       enqueue_pair<false, true>(c, S, cf, S.X[cur], S.T[lo], nullptr, S.rir, &nl);
-    if ((st = read_norm(c, S.mb.sums, &rr, nullptr)) != VG_OK) return st;
+    if ((st = next_norm(c, &rr, nullptr)) != VG_OK) return st;
     relres = std::sqrt(rr) / bn;
     if (relres <= tol || cyc >= max_cycles) break;
     const double inner_tol = std::max(0.9 * tol, 1e-4 * relres);
