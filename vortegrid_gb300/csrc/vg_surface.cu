@@ -232,17 +232,24 @@ __global__ void __launch_bounds__(kStatThreads) k_stats_blocks(const float* __re
   }
 }
 
+// One warp over the blocks' partials (one thread took 61 us for 304 blocks, a warp 6).
 __global__ void k_stats_finish(const double* __restrict__ part, int nb, size_t n, float* __restrict__ st) {
   pdl_entry();
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
   double s = 0.0, s2 = 0.0;
   float lo = FLT_MAX, hi = -FLT_MAX;
-  for (int b = 0; b < nb; ++b) {
+  for (int b = threadIdx.x; b < nb; b += 32) {
     s += part[4 * b];
     s2 += part[4 * b + 1];
     lo = fminf(lo, (float)part[4 * b + 2]);
     hi = fmaxf(hi, (float)part[4 * b + 3]);
   }
+  for (int o = 16; o > 0; o >>= 1) {
+    s += __shfl_xor_sync(0xffffffffu, s, o);
+    s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+    lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+  }
+  if (threadIdx.x) return;
   st[0] = lo;
   st[1] = hi;
   st[3] = (float)(s2 / (double)n);  // mean of squares
@@ -352,95 +359,91 @@ __global__ void k_sdf_immediate(Geom g, const float* __restrict__ dens, float am
 // The points, their neighbours and the updates are those of the serial sweep,
 // in an order that respects every dependence, so the result is its own bit
 // for bit.
+//
+// Bound by the chain of 3 T - 2 dependent steps in a tile, each a barrier and
+// a shared-memory access by every thread of a diagonal plane.  Thread (j, k)
+// is at x = s - j - k in step s, so with rows of kRow and planes of kPlane
+// floats the lanes of a warp (16 j, 2 k) lie kRow - 1 and kPlane - 1 floats
+// apart: kRow - 1 odd and kPlane - 1 = 16 modulo 32 put all 32 in different
+// banks.  Rows of T + 1 floats without padding made every access 16-way
+// conflicted: 0.3 us a step, 752 us for the two sweeps of a 129^3 grid against
+// 414 us (smaller tiles, with fewer steps but more diagonals, came to 600 us
+// at best in that layout).
 constexpr int kSdfTile = 16;
 constexpr int kSdfThreads = kSdfTile * kSdfTile;  // one thread per (j, k) of a local diagonal plane
 __global__ void __launch_bounds__(kSdfThreads) k_sdf_sweep(Geom g, int diag, int backward, unsigned tiles_x,
                                                            float* __restrict__ sdf,
                                                            const unsigned char* __restrict__ pinned) {
   pdl_entry();
-  constexpr int T = kSdfTile, E = kSdfTile + 1;  // staged extent: the tile plus one backward layer
-  __shared__ float S[E * E * E];                 // S[(w + 1) E^2 + (v + 1) E + (u + 1)], u, v, w in [-1, T)
-  __shared__ unsigned char pin[T * T * T];
+  constexpr int T = kSdfTile;
+  constexpr int kRow = 18, kPlane = 337;  // see above: kRow - 1 odd, kPlane - 1 = 16 modulo 32
+  static_assert(T == 16, "rows are half a warp, their pins 16 bits");
+  __shared__ float S[(T + 1) * kPlane];  // S[(w + 1) kPlane + (v + 1) kRow + u + 1], u, v, w in [-1, T)
+  __shared__ unsigned short fixed_row[T * T];
   const int ty = blockIdx.x, tz = blockIdx.y;
   const int tx = diag - ty - tz;
   if (tx < 0 || tx >= (int)tiles_x) return;
   const int nx = g.np[0], ny = g.np[1], nz = g.np[2];
-  const long long sy = nx, sz = (long long)nx * ny;
-  // tile origin in sweep coordinates (distance from the sweep's first point)
+  // tile origin in sweep coordinates (distance from the sweep's first point); sweep point (u, v, w) is
+  // at first + dx u + dy v + dz w
   const int ox = tx * T, oy = ty * T, oz = tz * T;
-  auto gidx = [&](int u, int v, int w) -> long long {
-    const int x = backward ? nx - 1 - u : u, y = backward ? ny - 1 - v : v, z = backward ? nz - 1 - w : w;
-    return x + sy * y + sz * z;
-  };
-  // stage: the tile (u, v, w in [0, T)) and the backward faces (one of u, v, w = -1, the others in
-  // [0, T)); a neighbour before the grid's first point reads FLT_MAX, as in the serial sweep
-  // all of a thread's loads are issued before any is stored, so the staging
-  // costs one memory latency rather than one per element
-  constexpr int kStage = (E * E * E + kSdfThreads - 1) / kSdfThreads;
-  float val[kStage];
-  unsigned char pv[kStage];
+  const long long sy = nx, sz = (long long)nx * ny;
+  const long long dx = backward ? -1 : 1, dy = backward ? -sy : sy, dz = backward ? -sz : sz;
+  const long long first = backward ? sz * nz - 1 : 0;
+  const int j = threadIdx.x % T, k = threadIdx.x / T;
+  // stage: thread (j, k) takes the row elements u = j, v = k of all planes, so that loads run along x;
+  // then one element of each backward face.  A neighbour before the grid's first point reads FLT_MAX,
+  // as in the serial sweep.  All loads are issued before any is used: one memory latency.
+  const bool in_xy = ox + j < nx && oy + k < ny;
+  const long long row = first + dx * (ox + j) + dy * (oy + k) + dz * oz;
+  float val[T];
+  unsigned char pv[T];
 #pragma unroll
-  for (int q = 0; q < kStage; ++q) {
-    const int t = threadIdx.x + q * kSdfThreads;
-    val[q] = FLT_MAX;
-    pv[q] = 0;
-    if (t >= E * E * E) continue;
-    const int lu = t % E - 1, lv = (t / E) % E - 1, lw = t / (E * E) - 1;
-    if ((lu < 0) + (lv < 0) + (lw < 0) > 1) continue;  // edges and corners of the backward layer are never read
-    const int u = ox + lu, v = oy + lv, w = oz + lw;
-    if (u >= 0 && v >= 0 && w >= 0 && u < nx && v < ny && w < nz) {
-      const long long o = gidx(u, v, w);
-      val[q] = sdf[o];
-      pv[q] = pinned[o];
+  for (int w = 0; w < T; ++w) {
+    val[w] = FLT_MAX;
+    pv[w] = 1;
+    if (in_xy && oz + w < nz) {
+      val[w] = sdf[row + dz * w];
+      pv[w] = pinned[row + dz * w];
     }
   }
+  float sx = FLT_MAX, fy = FLT_MAX, fz = FLT_MAX;
+  if (ox > 0 && oy + j < ny && oz + k < nz) sx = sdf[first + dx * (ox - 1) + dy * (oy + j) + dz * (oz + k)];
+  if (oy > 0 && ox + j < nx && oz + k < nz) fy = sdf[first + dx * (ox + j) + dy * (oy - 1) + dz * (oz + k)];
+  if (oz > 0 && in_xy) fz = sdf[row - dz];
+  S[(k + 1) * kPlane + j + 1] = fy;
+  S[(k + 1) * kRow + j + 1] = fz;
+  unsigned mine = 0;  // bit w: this thread's staged element of plane w is updated and written back
 #pragma unroll
-  for (int q = 0; q < kStage; ++q) {
-    const int t = threadIdx.x + q * kSdfThreads;
-    if (t >= E * E * E) continue;
-    S[t] = val[q];
-    const int lu = t % E - 1, lv = (t / E) % E - 1, lw = t / (E * E) - 1;
-    if (lu >= 0 && lv >= 0 && lw >= 0) pin[lu + T * (lv + T * lw)] = pv[q];
+  for (int w = 0; w < T; ++w) {
+    S[(w + 1) * kPlane + (k + 1) * kRow + j + 1] = val[w];
+    const unsigned rows = __ballot_sync(0xffffffffu, pv[w]);  // two rows of 16 points
+    if (j == 0) fixed_row[w * T + k] = (unsigned short)(k & 1 ? rows >> 16 : rows);
+    if (!pv[w]) mine |= 1u << w;
   }
   __syncthreads();
-  const int j = threadIdx.x % T, kk = threadIdx.x / T;
+  // a thread walks its column (v = j, w = k) along x; its x neighbour is its own last value
+  const unsigned fixed = fixed_row[k * T + j];  // pinned, or outside the grid
+  float* col = S + (k + 1) * kPlane + (j + 1) * kRow + 1;
   for (int s = 0; s <= 3 * (T - 1); ++s) {
     // points (i, j, k) of the tile with i + j + k = s
-    const int i = s - j - kk;
+    const int i = s - j - k;
     if (i >= 0 && i < T) {
-      const int u = ox + i, v = oy + j, w = oz + kk;
-      if (u < nx && v < ny && w < nz && !pin[i + T * (j + T * kk)]) {
-        const int c = (kk + 1) * E * E + (j + 1) * E + (i + 1);
-        const float sx = S[c - 1], syv = S[c - E], szv = S[c - E * E];
-        const float ax = fabsf(sx), ay = fabsf(syv), az = fabsf(szv);
-        float nb, sp;
-        if (ax <= ay) {
-          if (ax <= az) {
-            nb = sx;
-            sp = g.cell[0];
-          } else {
-            nb = szv;
-            sp = g.cell[2];
-          }
-        } else if (ay <= az) {
-          nb = syv;
-          sp = g.cell[1];
-        } else {
-          nb = szv;
-          sp = g.cell[2];
-        }
-        float here = S[c];
-        update_sdf(here, __fadd_rn(nb, copysignf(sp, nb)));
-        S[c] = here;
-      }
+      float here = col[i];
+      const float syv = col[i - kRow], szv = col[i - kPlane];
+      const bool x_first = fabsf(sx) <= fabsf(syv);
+      const float xy = x_first ? sx : syv, sp_xy = x_first ? g.cell[0] : g.cell[1];
+      const bool xy_first = fabsf(xy) <= fabsf(szv);
+      const float nb = xy_first ? xy : szv, sp = xy_first ? sp_xy : g.cell[2];
+      const float cand = __fadd_rn(nb, copysignf(sp, nb));
+      if (!((fixed >> i) & 1u) && fabsf(cand) < fabsf(here)) col[i] = here = cand;
+      sx = here;
     }
     __syncthreads();
   }
-  for (int t = threadIdx.x; t < T * T * T; t += kSdfThreads) {
-    const int li = t % T, lj = (t / T) % T, lk = t / (T * T);
-    const int u = ox + li, v = oy + lj, w = oz + lk;
-    if (u < nx && v < ny && w < nz && !pin[t]) sdf[gidx(u, v, w)] = S[(lk + 1) * E * E + (lj + 1) * E + (li + 1)];
-  }
+#pragma unroll
+  for (int w = 0; w < T; ++w)
+    if ((mine >> w) & 1u) sdf[row + dz * w] = S[(w + 1) * kPlane + (k + 1) * kRow + j + 1];
 }
 
 __global__ void k_sdf_unreached(size_t pts, float* __restrict__ sdf) {
@@ -510,12 +513,12 @@ __global__ void k_mc_count(Geom g, const float* __restrict__ v, float iso, const
 }
 
 __global__ void k_mc_emit(Geom g, const float* __restrict__ v, float iso, const __grid_constant__ MCTable T,
-                          const unsigned* __restrict__ offsets, float* __restrict__ verts,
+                          const unsigned* __restrict__ offsets, size_t cap, float* __restrict__ verts,
                           float* __restrict__ normals) {
   pdl_entry();
   const size_t cx = g.np[0] - 1, cy = g.np[1] - 1, cells = cx * cy * (g.np[2] - 1);
   const size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= cells) return;
+  if (k >= cells || offsets[cells] > cap) return;  // no room: nothing is written
   const unsigned x = (unsigned)(k % cx), y = (unsigned)((k / cx) % cy), z = (unsigned)(k / (cx * cy));
   float val[8];
   const int mask = mc_mask(g, v, x + g.np[0] * (y + (size_t)g.np[1] * z), iso, val);
@@ -720,7 +723,7 @@ vg_status launch_signed_distance(Ctx* c, const Geom& g, const float* dens, float
     VG_LAUNCHED(c);
   } else {
     pdl_launch(c->stream, partial_blocks, kStatThreads, 0, k_stats_blocks, dens, pts, partials);
-    pdl_launch(c->stream, 1, 1, 0, k_stats_finish, (const double*)partials, partial_blocks, pts, stats);
+    pdl_launch(c->stream, 1, 32, 0, k_stats_finish, (const double*)partials, partial_blocks, pts, stats);
     c->launches += 2;
   }
   pdl_launch(c->stream, blocks_for(pts, 256), 256, 0, k_sdf_immediate, g, dens, ambient, (const float*)stats, sdf,
@@ -756,17 +759,18 @@ vg_status launch_marching_cubes(Ctx* c, const Geom& g, const float* v, float iso
   pdl_launch(c->stream, blocks_for(cells, 256), 256, 0, k_mc_count, g, v, iso, T, counts);
   VG_LAUNCHED(c);
   if ((st = exclusive_scan(c, counts, cells, offsets, true)) != VG_OK) return st;
+  // the triangles are made before the host knows their number: one wait, after which they are there
+  if (cap) {
+    pdl_launch(c->stream, blocks_for(cells, 128), 128, 0, k_mc_emit, g, v, iso, T, (const unsigned*)offsets, cap, verts,
+               normals);
+    VG_LAUNCHED(c);
+  }
   unsigned total = 0;
   VG_CUDA(c, cudaMemcpyAsync(&total, offsets + cells, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
   VG_CUDA(c, cudaStreamSynchronize(c->stream));
   *triangles = total;
   if (total > cap) return fail(c, VG_TOO_LARGE, "marching cubes: " + std::to_string(total) + " triangles, room for " +
                                                     std::to_string(cap));
-  if (total == 0) return VG_OK;
-  pdl_launch(c->stream, blocks_for(cells, 128), 128, 0, k_mc_emit, g, v, iso, T, (const unsigned*)offsets, verts,
-             normals);
-  VG_LAUNCHED(c);
-  VG_CUDA(c, cudaGetLastError());
   return VG_OK;
 }
 
