@@ -90,3 +90,64 @@ def test_body_sums_of_many_blocks(vg, ctx, n):
             parts += _collide(vg, ctx, p, torch.zeros_like(p), body)[0].astype(np.float64)
     whole = _collide(vg, ctx, ps, torch.zeros_like(ps), body)[0]
     assert abs(whole[0]) > 0 and abs(whole[0] - parts[0]) <= 3.6e-7 * abs(parts[0])
+
+
+def _some_bodies(nb):
+    """Moving spheres, solid boxes and hollow boxes by turns."""
+    out = []
+    for k in range(nb):
+        at = (0.5 - 0.2 * k, 0.1 * k, -0.3 + 0.1 * k)
+        kind = k % 3
+        out.append(_body(0 if kind == 1 else 1, at, (0.5, 0.1 * k, -0.2),
+                         (0.4, 0, 0) if kind == 1 else ((0.5, 0.7, 0.6) if kind == 0 else (1.9, 2.1, 2.0)),
+                         hollow=1.0 if kind == 2 else 0.0))
+    return out
+
+
+@pytest.mark.parametrize("nb", [1, 2, 3, 4, 5, 9, 16])
+def test_body_groups(vg, ctx, oracle_lib, nb):
+    """Bodies are taken four to a launch: any number of them leaves vortons
+    and tracers bit for bit as the oracle, also where a position or a velocity
+    is infinite or NaN (a NaN's payload is not compared)."""
+    n = 5000
+    rng = np.random.default_rng(nb)
+    pos = rng.uniform(-1.2, 1.2, (n, 3)).astype(np.float32)
+    vel = rng.normal(0, 0.5, (n, 3)).astype(np.float32)
+    w = rng.normal(0, 1.0, (n, 3)).astype(np.float32)
+    for k, bad in enumerate((np.inf, -np.inf, np.nan)):
+        pos[10 + k, k] = bad
+        pos[20 + k, (k + 1) % 3] = bad
+        vel[30 + k, k] = bad
+    size = np.full(n, 0.03, np.float32)
+    dens = rng.uniform(0.5, 2.0, n).astype(np.float32)
+    bodies = np.stack(_some_bodies(nb))
+
+    def same(got, ref):
+        a, b = got.cpu().numpy(), np.asarray(ref, np.float32)
+        a = a[:, :3] if a.ndim == 2 else a
+        nan = np.isnan(b)
+        assert np.array_equal(np.isnan(a), nan)
+        assert np.array_equal(a[~nan].view(np.uint32), b[~nan].view(np.uint32))
+
+    def quad(xyz, last=None):
+        q = np.zeros((n, 4), np.float32)
+        q[:, :3] = xyz
+        if last is not None:
+            q[:, 3] = last
+        return torch.from_numpy(q).cuda()
+
+    ps, v, a4, d = quad(pos, size), quad(vel), quad(w), torch.from_numpy(dens).cuda()
+    out, cnt = np.zeros((nb, 9), np.float32), np.zeros(nb, np.uint64)
+    ctx.check(vg.lib().vg_collide_vortons_device(ctx.h, vg._ptr(bodies), nb, vg._ptr(ps), vg._ptr(v), vg._ptr(a4),
+                                                 vg._ptr(d), n, 1.0, 1.0, vg._ptr(out), vg._ptr(cnt)), "vortons")
+    op, ov, ow, od, oout = oracle_lib.collide_vortons(pos, vel, w, size, dens, bodies)
+    for got, ref in ((ps, op), (v, ov), (a4, ow), (d, od)):
+        same(got, ref)
+    assert np.array_equal(cnt.astype(np.float64), oout[:, 8].astype(np.float64))
+    ps, v = quad(pos, size), quad(vel)
+    out = np.zeros((nb, 6), np.float32)
+    ctx.check(vg.lib().vg_collide_tracers_device(ctx.h, vg._ptr(bodies), nb, vg._ptr(ps), vg._ptr(v), vg._ptr(d), n,
+                                                 vg._ptr(out)), "tracers")
+    op, ov, _ = oracle_lib.collide_tracers(pos, vel, size, dens, bodies)
+    same(ps, op)
+    same(v, ov)

@@ -39,7 +39,7 @@ struct Body {
   int box;
   float parity, brad;
   float pos[3], vel[3], angvel[3], row[9];
-  float pn[6][3], pw[6];
+  float pw[6];
   float temperature, conductivity;
 };
 
@@ -72,9 +72,6 @@ bool load_body(const float* q, Body* b, std::string* err) {
   }
   const float half[3] = {q[20] * 0.5f, q[21] * 0.5f, q[22] * 0.5f};
   for (int a = 0; a < 3; ++a) {
-    for (int k = 0; k < 3; ++k) b->pn[2 * a][k] = b->pn[2 * a + 1][k] = 0.0f;
-    b->pn[2 * a][a] = 1.0f;
-    b->pn[2 * a + 1][a] = -1.0f;
     b->pw[2 * a] = b->pw[2 * a + 1] = half[a];
   }
   if (b->parity < 0.0f) {
@@ -121,12 +118,21 @@ __device__ __forceinline__ V3 xform(const Body& b, V3 v) {
             dot(mk(b.row[2], b.row[5], b.row[8]), v));
 }
 
+// A box's face normals: +x, -x, +y, -y, +z, -z.  With i known at compile time
+// the products with 1 and the repeated products with 0 (not dropped: they
+// carry infinities and NaN) cost nothing.
+__device__ __forceinline__ V3 face_normal(int i) {
+  const float s = i & 1 ? -1.0f : 1.0f;
+  return mk(i / 2 == 0 ? s : 0.0f, i / 2 == 1 ? s : 0.0f, i / 2 == 2 ? s : 0.0f);
+}
+
 // ConvexPolytope::ContactDistance (convexPolytope.cpp:97-144)
 __device__ float contact_distance(const Body& b, V3 q, int* idx) {
   const V3 r = xform_t(b, sub(q, from(b.pos)));
   float largest = -FLT_MAX;
+#pragma unroll
   for (int i = 0; i < 6; ++i) {
-    const float d = __fsub_rn(dot(r, from(b.pn[i])), b.pw[i]);
+    const float d = __fsub_rn(dot(r, face_normal(i)), b.pw[i]);
     if (d > largest) {
       largest = d;
       *idx = i;
@@ -140,10 +146,11 @@ __device__ float collision_distance(const Body& b, V3 q, V3 qv, int* idx) {
   const V3 r = xform_t(b, sub(q, from(b.pos)));
   const V3 rv = xform_t(b, sub(qv, from(b.vel)));
   float largest = -FLT_MAX;
+#pragma unroll
   for (int i = 0; i < 6; ++i) {
-    const float d = __fsub_rn(dot(r, from(b.pn[i])), b.pw[i]);
+    const float d = __fsub_rn(dot(r, face_normal(i)), b.pw[i]);
     if (d > largest) {
-      const float speed = __fmul_rn(dot(rv, from(b.pn[i])), b.parity);
+      const float speed = __fmul_rn(dot(rv, face_normal(i)), b.parity);
       if (speed <= 0.0f || d >= 0.0f || b.parity < 0.0f) {
         largest = d;
         *idx = i;
@@ -155,7 +162,7 @@ __device__ float collision_distance(const Body& b, V3 q, V3 qv, int* idx) {
 
 // ConvexPolytope::ContactPoint (convexPolytope.cpp:325-339)
 __device__ __forceinline__ V3 contact_point(const Body& b, V3 q, int idx, float dist, V3* n) {
-  *n = mul(xform(b, from(b.pn[idx])), b.parity);
+  *n = mul(xform(b, face_normal(idx)), b.parity);
   return sub(q, mul(*n, dist));
 }
 
@@ -174,9 +181,10 @@ __device__ void block_sums(float (&v)[K], float* __restrict__ out) {
     if (threadIdx.x < K) out[K * blockIdx.x + threadIdx.x] = 0.0f;
     return;
   }
-  for (int o = 16; o > 0; o >>= 1)
+  if (__any_sync(0xffffffffu, any))
+    for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-    for (int k = 0; k < K; ++k) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
+      for (int k = 0; k < K; ++k) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   if (lane == 0)
 #pragma unroll
@@ -233,8 +241,9 @@ __global__ void __launch_bounds__(kSumThreads) k_sum_blocks(const float* __restr
 }
 
 // The bodies of one call, in order (a kernel parameter).
+template <int NB>
 struct Bodies {
-  Body b[kMaxBodies];
+  Body b[NB];
 };
 
 // One body's CollideVortonsSlice for one vorton, on the vorton's state in
@@ -351,7 +360,8 @@ __device__ bool collide_vorton(const Body& B, float4& p4s, float4& v4s, float4& 
 // state stays in registers from body to body (each body sees the vorton as
 // the bodies before left it, as with one launch per body) and is written
 // once.  Per body, block partial sums at part + 6 blocks k.
-__global__ void __launch_bounds__(kBodyThreads) k_collide_vortons(const __grid_constant__ Bodies BB, int nb,
+template <int NB>
+__global__ void __launch_bounds__(kBodyThreads) k_collide_vortons(const __grid_constant__ Bodies<NB> BB,
                                                                   float4* __restrict__ ps, float4* __restrict__ vel,
                                                                   float4* __restrict__ w4, float* __restrict__ dens,
                                                                   int n, float ambient, float cp,
@@ -366,7 +376,8 @@ __global__ void __launch_bounds__(kBodyThreads) k_collide_vortons(const __grid_c
     d = dens[i];
   }
   bool changed = false;
-  for (int k = 0; k < nb; ++k) {
+#pragma unroll
+  for (int k = 0; k < NB; ++k) {
     float acc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (i < n) changed |= collide_vorton(BB.b[k], p4, v4, a4, d, ambient, cp, acc);
     block_sums<6>(acc, part + (size_t)6 * gridDim.x * k);
@@ -447,7 +458,8 @@ __device__ bool collide_tracer(const Body& B, float4& p4s, float4& v4s, const fl
 
 // CollideTracersSlice for every body in order, one tracer per thread, its
 // state in registers from body to body and written once (as k_collide_vortons).
-__global__ void __launch_bounds__(kBodyThreads) k_collide_tracers(const __grid_constant__ Bodies BB, int nb,
+template <int NB>
+__global__ void __launch_bounds__(kBodyThreads) k_collide_tracers(const __grid_constant__ Bodies<NB> BB,
                                                                   float4* __restrict__ ps, float4* __restrict__ vel,
                                                                   const float* __restrict__ dens, int n,
                                                                   float* __restrict__ part) {
@@ -458,7 +470,8 @@ __global__ void __launch_bounds__(kBodyThreads) k_collide_tracers(const __grid_c
     v4 = vel[i];
   }
   bool changed = false;
-  for (int k = 0; k < nb; ++k) {
+#pragma unroll
+  for (int k = 0; k < NB; ++k) {
     float acc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (i < n) changed |= collide_tracer(BB.b[k], p4, v4, dens, i, acc);
     block_sums<6>(acc, part + (size_t)6 * gridDim.x * k);
@@ -510,6 +523,28 @@ __global__ void k_embedded_fill(const unsigned* __restrict__ flag, const unsigne
   if (d) d[i] = d[s];
 }
 
+// The bodies in groups of up to four: launch(Bodies<NB>, first body).  A kernel
+// that knows its number of bodies reads their values as constant operands; with
+// an index in a loop they were loaded by instructions of their own, which
+// bound the kernels (2^22 tracers and three bodies: 212 us, now 143 us, bound by
+// instruction issue; most is the narrow phase of the lanes near a box).
+template <int NB, typename F>
+void launch_group(const Body* B, int k, const F& launch) {
+  Bodies<NB> g;
+  for (int i = 0; i < NB; ++i) g.b[i] = B[k + i];
+  launch(g, k);
+}
+
+template <typename F>
+void for_body_groups(const Body* B, int nb, const F& launch) {
+  for (int k = 0; k < nb; k += 4) switch (nb - k) {
+      case 1: launch_group<1>(B, k, launch); break;
+      case 2: launch_group<2>(B, k, launch); break;
+      case 3: launch_group<3>(B, k, launch); break;
+      default: launch_group<4>(B, k, launch); break;
+    }
+}
+
 vg_status load_bodies(Ctx* c, const float* bodies, int nb, Body* out) {
   if (nb < 0 || nb > kMaxBodies) return fail(c, VG_INVALID, "between 0 and 16 bodies");
   if (nb && !bodies) return VG_INVALID;
@@ -539,12 +574,12 @@ vg_status vg_collide_vortons_device(vg_ctx* c, const float* bodies, int nb, floa
   if (st != VG_OK) return st;
   float* part = (float*)(sums + 6 * kMaxBodies);
   if (nb) {
-    Bodies BB;
-    memcpy(BB.b, B, sizeof(BB.b));
-    k_collide_vortons<<<blocks, kBodyThreads, 0, c->stream>>>(BB, nb, (float4*)pos_size, (float4*)vel4,
-                                                             (float4*)angvel4, density, (int)n, ambient_density,
-                                                             specific_heat, part);
-    ++c->launches;
+    for_body_groups(B, nb, [&](const auto& g, int k) {
+      k_collide_vortons<<<blocks, kBodyThreads, 0, c->stream>>>(g, (float4*)pos_size, (float4*)vel4, (float4*)angvel4,
+                                                               density, (int)n, ambient_density, specific_heat,
+                                                               part + (size_t)6 * blocks * k);
+      ++c->launches;
+    });
     k_sum_blocks<6, true><<<dim3(6, nb), kSumThreads, 0, c->stream>>>(part, (int)blocks, sums);
     ++c->launches;
   }
@@ -589,11 +624,11 @@ vg_status vg_collide_tracers_device(vg_ctx* c, const float* bodies, int nb, floa
   if (st != VG_OK) return st;
   float* part = (float*)(sums + 6 * kMaxBodies);
   if (nb) {
-    Bodies BB;
-    memcpy(BB.b, B, sizeof(BB.b));
-    k_collide_tracers<<<blocks, kBodyThreads, 0, c->stream>>>(BB, nb, (float4*)pos_size, (float4*)vel4, density,
-                                                             (int)n, part);
-    ++c->launches;
+    for_body_groups(B, nb, [&](const auto& g, int k) {
+      k_collide_tracers<<<blocks, kBodyThreads, 0, c->stream>>>(g, (float4*)pos_size, (float4*)vel4, density, (int)n,
+                                                               part + (size_t)6 * blocks * k);
+      ++c->launches;
+    });
     k_sum_blocks<6, false><<<dim3(6, nb), kSumThreads, 0, c->stream>>>(part, (int)blocks, sums);
     ++c->launches;
   }

@@ -471,16 +471,19 @@ __host__ __device__ __forceinline__ int mc_corner(int c, int k) {
 __host__ __device__ __forceinline__ int mc_edge_a(int e) { return e < 8 ? e : e - 8; }
 __host__ __device__ __forceinline__ int mc_edge_b(int e) { return e < 8 ? ((e & 4) | ((e + 1) & 3)) : e - 4; }
 
-// VertexInterp (marchingCubes.cpp:228-250): an end point within 1e-5
-// (compared in double, as the reference's double literal makes it), else
-// p1 + mu (p2 - p1).
+// VertexInterp (marchingCubes.cpp:228-250): an end point within 1e-5, else
+// p1 + mu (p2 - p1).  The reference's literal makes it compare in double; the
+// largest float below that literal is 0.00001f, so x <= 0.00001f is the same
+// test on floats (the conversions to FP64 and its comparisons were most of
+// k_mc_emit's time).
+static_assert((double)0.00001f < 0.00001 && (double)(0.00001f * (1.0f + FLT_EPSILON)) > 0.00001, "neighbours of 1e-5");
 __device__ __forceinline__ void mc_interp(float iso, const float* p1, const float* p2, float v1, float v2,
                                           float* out) {
-  if ((double)fabsf(__fsub_rn(iso, v1)) < 0.00001) {
+  if (fabsf(__fsub_rn(iso, v1)) <= 0.00001f) {
     out[0] = p1[0], out[1] = p1[1], out[2] = p1[2];
-  } else if ((double)fabsf(__fsub_rn(iso, v2)) < 0.00001) {
+  } else if (fabsf(__fsub_rn(iso, v2)) <= 0.00001f) {
     out[0] = p2[0], out[1] = p2[1], out[2] = p2[2];
-  } else if ((double)fabsf(__fsub_rn(v1, v2)) < 0.00001) {
+  } else if (fabsf(__fsub_rn(v1, v2)) <= 0.00001f) {
     out[0] = p1[0], out[1] = p1[1], out[2] = p1[2];
   } else {
     const float mu = __fdiv_rn(__fsub_rn(iso, v1), __fsub_rn(v2, v1));
@@ -519,11 +522,12 @@ __global__ void k_mc_emit(Geom g, const float* __restrict__ v, float iso, const 
   const size_t cx = g.np[0] - 1, cy = g.np[1] - 1, cells = cx * cy * (g.np[2] - 1);
   const size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= cells || offsets[cells] > cap) return;  // no room: nothing is written
+  size_t out = offsets[k];
+  const int nt = (int)(offsets[k + 1] - out);  // 0 for most cells, whose corners are then not read
+  if (nt == 0) return;
   const unsigned x = (unsigned)(k % cx), y = (unsigned)((k / cx) % cy), z = (unsigned)(k / (cx * cy));
   float val[8];
   const int mask = mc_mask(g, v, x + g.np[0] * (y + (size_t)g.np[1] * z), iso, val);
-  const int nt = T.cnt[mask];
-  if (nt == 0) return;
   // corner positions min + index x spacing (marchingCubes.cpp:806-816)
   const float lo[3] = {__fadd_rn(__fmul_rn((float)x, g.cell[0]), g.mn[0]),
                        __fadd_rn(__fmul_rn((float)y, g.cell[1]), g.mn[1]),
@@ -543,7 +547,6 @@ __global__ void k_mc_emit(Geom g, const float* __restrict__ v, float iso, const 
       mc_interp(iso, pa, pb, val[a], val[b], vl[e]);
     }
   }
-  size_t out = offsets[k];
   for (int t = 0; t < nt; ++t, ++out) {
     const float* q0 = vl[T.tri[mask][3 * t]];
     const float* q1 = vl[T.tri[mask][3 * t + 1]];
