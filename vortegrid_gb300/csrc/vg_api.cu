@@ -377,7 +377,7 @@ static vg_status step_front(Ctx* c, StepState& s, const float* first_pos, const 
   // Cell lists serve the tree, the splat and PSE; the direct technique
   // without diffusion needs none.
   const int tech = c->cfg.velocity_technique;
-  s.cl = {nullptr, nullptr, nullptr};
+  s.cl = {nullptr, nullptr};
   if (tech != VG_VELOCITY_DIRECT || c->cfg.enable_diffusion) {
     if ((st = build_cell_lists(c, g, ps, n, &s.cl)) != VG_OK) return st;
   }

@@ -210,7 +210,6 @@ enum Slot {
   S_CELL,
   S_COUNT,
   S_START,
-  S_FILL,
   S_ITEMS,
   S_SCAN,
   S_TREE,
@@ -391,7 +390,6 @@ vg_status launch_direct(Ctx* c, int kind, bool ref, const float4* ps, const floa
 
 // Cell lists: stable counting sort of vortons by leaf cell (OffsetOfPosition).
 struct CellLists {
-  unsigned* cell;   // per vorton: leaf offset
   unsigned* start;  // per cell (+1): first item
   unsigned* items;  // vorton indices grouped by cell, ascending within a cell
 };
