@@ -542,7 +542,7 @@ static vg_status step_back(Ctx* c, StepState& s) {
   c->stats.kernels_launched = c->launches;
   c->grid = g;
   c->have_grid = true;
-  ++c->vel_gen;  // a new velocity grid (any by-cell copy is stale)
+  ++c->vel_gen;  // a new velocity grid (any float4 copy is stale)
   return VG_OK;
 }
 
@@ -755,8 +755,8 @@ static vg_status tracer_advect_enqueue(vg_ctx* c, const TracerJob& t, float dt) 
   vg_status st = VG_OK;
   const size_t m = t.m;
   const float* vel3 = (const float*)c->buf[S_VEL].p;
-  if (gather_by_cell(c->grid, m)) {
-    // float4 positions and velocities out of the records, the by-cell gather, and back
+  if (unpack_records(c->grid, m)) {
+    // float4 positions and velocities out of the records, the gather, and back
     pdl_launch(c->stream, blocks_for(m, 256), 256, 0, k_copy_pos3, t.stage, t.pitch, (int)m, t.p);
     if ((st = launch_gather_advect(c, c->grid, vel3, t.p, t.v, m, dt, true, nullptr, true)) != VG_OK) return st;
     pdl_launch(c->stream, blocks_for(m, 256), 256, 0, k_store_posvel, t.stage, t.pitch, (int)m, t.p, t.v);

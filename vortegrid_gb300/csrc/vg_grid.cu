@@ -465,65 +465,89 @@ __global__ void k_gather_advect_records(Geom g, const float* __restrict__ vel3, 
   r[5] = u[2];
 }
 
-// The velocity grid arranged by cell: the 8 corners of cell (x, y, z) as
-// float4 (u, v, w, 0), corners in interp's order (x fastest), so that a
-// tracer's gather is one 128-byte line instead of four scattered row pairs.
-__global__ void k_vel_cells(Geom g, const float* __restrict__ v3, float4* __restrict__ vc) {
+// The velocity grid as float4 points, for k_gather_advect_points.
+__global__ void k_vel_points(size_t pts, const float* __restrict__ v3, float4* __restrict__ vp) {
   pdl_entry();
-  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const size_t cx = g.np[0] - 1, cy = g.np[1] - 1;
-  const size_t cells = cx * cy * (size_t)(g.np[2] - 1);
-  if (t >= 8 * cells) return;
-  const size_t cell = t >> 3;
-  const unsigned q = (unsigned)(t & 7);
-  const size_t x = cell % cx, y = (cell / cx) % cy, z = cell / (cx * cy);
-  const size_t k = (x + (q & 1)) + (size_t)g.np[0] * ((y + ((q >> 1) & 1)) + (size_t)g.np[1] * (z + (q >> 2)));
-  vc[t] = make_float4(v3[3 * k], v3[3 * k + 1], v3[3 * k + 2], 0.f);
+  const size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < pts) vp[k] = make_float4(v3[3 * k], v3[3 * k + 1], v3[3 * k + 2], 0.f);
 }
 
-// k_gather_advect reading the by-cell copy: the same cell, weights and
-// trilinear sums as interp<3> on the grid (bit-identical).
-__global__ void k_gather_advect_cells(Geom g, const float4* __restrict__ vc, float4* __restrict__ pos,
-                                      float4* __restrict__ vel, int m, float dt, int evolve,
-                                      int* __restrict__ flag) {
+// k_gather_advect reading the float4 points: the same cell, weights and sums bit
+// for bit.  Eight lanes take the corners of a tracer, lane q corner q (x in bit
+// 0, y in bit 1, z in bit 2), for the eight tracers of those lanes in turn; the
+// sums along x, y and z are then exchanges between lanes 1, 2 and 4 apart, each
+// of which halves the number of tracers a lane holds, so that lane q ends with
+// its own tracer's.
+//
+// Bound by the first-level cache's lines a cycle: a tracer's corners lie in
+// four rows, and one load of eight lanes takes each row's line once, where a
+// thread that loads its tracer's corners itself takes one for every corner.
+// 2^22 tracers on 129^3 points: 88 us, and 7 us for the float4 points, against
+// 228 us from the three-float grid (a thread to a tracer, 24 loads) and 128 us + 84 us
+// from a copy of the grid with each cell's corners in a line of their own.
+__global__ void __launch_bounds__(256) k_gather_advect_points(Geom g, const float4* __restrict__ vp,
+                                                              float4* __restrict__ pos, float4* __restrict__ vel,
+                                                              int m, float dt, int evolve, int* __restrict__ flag) {
   pdl_entry();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= m) return;
-  float4 p = pos[i];
-  if (!inside_cells(g, p.x, p.y, p.z)) {
+  const bool valid = i < m;  // all lanes take part in the exchanges
+  float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (valid) p = pos[i];
+  const bool inside = valid && inside_cells(g, p.x, p.y, p.z);
+  const float pp[3] = {p.x, p.y, p.z};
+  unsigned idx[3] = {0, 0, 0};  // a lane without a tracer in the grid reads the first cell
+  float tw[3] = {0.f, 0.f, 0.f};
+  if (inside)
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      idx[a] = bin_axis(pp[a], g.mn[a], g.cpe[a]);
+      const float cmin = __fadd_rn(g.mn[a], __fmul_rn((float)idx[a], g.cell[a]));
+      tw[a] = __fmul_rn(__fsub_rn(pp[a], cmin), g.cpe[a]);
+    }
+  const unsigned nx = g.np[0], nxy = g.np[0] * g.np[1];
+  const unsigned base = idx[0] + nx * idx[1] + nxy * idx[2];
+  const int lane = threadIdx.x & 31, q = lane & 7, group = lane & 24;
+  const unsigned bx = q & 1, by = (q >> 1) & 1, bz = q >> 2;
+  const unsigned corner = bx + nx * by + nxy * bz;
+  float4 c[8];
+#pragma unroll
+  for (int r = 0; r < 8; ++r) c[r] = vp[__shfl_sync(0xffffffffu, base, group + r) + corner];
+  auto weight = [&](float t, unsigned bit, int from) {  // 1 - t or t of the tracer of lane `from`
+    const float w = __shfl_sync(0xffffffffu, t, from);
+    return bit ? w : __fsub_rn(1.0f, w);
+  };
+  auto times = [](float4 v, float w) {
+    return make_float4(__fmul_rn(v.x, w), __fmul_rn(v.y, w), __fmul_rn(v.z, w), 0.f);
+  };
+  // keeps one of two tracers' terms, by the lane's bit, and adds the partner's term of the same tracer
+  auto exchange = [](float4 t0, float4 t1, unsigned bit, int apart) {
+    const float4 keep = bit ? t1 : t0, give = bit ? t0 : t1;
+    return make_float4(__fadd_rn(keep.x, __shfl_xor_sync(0xffffffffu, give.x, apart)),
+                       __fadd_rn(keep.y, __shfl_xor_sync(0xffffffffu, give.y, apart)),
+                       __fadd_rn(keep.z, __shfl_xor_sync(0xffffffffu, give.z, apart)), 0.f);
+  };
+  float4 sx[4], sy[2];
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+    sx[r] = exchange(times(c[2 * r], weight(tw[0], bx, group + 2 * r)),
+                     times(c[2 * r + 1], weight(tw[0], bx, group + 2 * r + 1)), bx, 1);
+#pragma unroll
+  for (int r = 0; r < 2; ++r)
+    sy[r] = exchange(times(sx[2 * r], weight(tw[1], by, group + 4 * r + bx)),
+                     times(sx[2 * r + 1], weight(tw[1], by, group + 4 * r + 2 + bx)), by, 2);
+  const float4 u = exchange(times(sy[0], weight(tw[2], bz, group + 2 * by + bx)),
+                            times(sy[1], weight(tw[2], bz, group + 4 + 2 * by + bx)), bz, 4);
+  if (!valid) return;
+  if (!inside) {
     atomicOr(flag, (int)DF_OUT_OF_GRID);
     if (vel) vel[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     return;
   }
-  const float pp[3] = {p.x, p.y, p.z};
-  unsigned idx[3];
-  float tw[3], om[3];
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    idx[a] = bin_axis(pp[a], g.mn[a], g.cpe[a]);
-    const float cmin = __fadd_rn(g.mn[a], __fmul_rn((float)idx[a], g.cell[a]));
-    tw[a] = __fmul_rn(__fsub_rn(pp[a], cmin), g.cpe[a]);
-    om[a] = __fsub_rn(1.0f, tw[a]);
-  }
-  const size_t cell = idx[0] + (size_t)(g.np[0] - 1) * (idx[1] + (size_t)(g.np[1] - 1) * idx[2]);
-  float4 c[8];
-#pragma unroll
-  for (int q = 0; q < 8; ++q) c[q] = vc[8 * cell + q];
-  float u[3];
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    auto comp = [&](const float4& v) { return a == 0 ? v.x : (a == 1 ? v.y : v.z); };
-    const float y0 = __fadd_rn(__fmul_rn(__fadd_rn(__fmul_rn(om[0], comp(c[0])), __fmul_rn(tw[0], comp(c[1]))), om[1]),
-                               __fmul_rn(__fadd_rn(__fmul_rn(om[0], comp(c[2])), __fmul_rn(tw[0], comp(c[3]))), tw[1]));
-    const float y1 = __fadd_rn(__fmul_rn(__fadd_rn(__fmul_rn(om[0], comp(c[4])), __fmul_rn(tw[0], comp(c[5]))), om[1]),
-                               __fmul_rn(__fadd_rn(__fmul_rn(om[0], comp(c[6])), __fmul_rn(tw[0], comp(c[7]))), tw[1]));
-    u[a] = __fadd_rn(__fmul_rn(y0, om[2]), __fmul_rn(y1, tw[2]));
-  }
-  if (vel) vel[i] = make_float4(u[0], u[1], u[2], 0.f);
+  if (vel) vel[i] = make_float4(u.x, u.y, u.z, 0.f);
   if (evolve) {
-    p.x = __fadd_rn(p.x, __fmul_rn(u[0], dt));
-    p.y = __fadd_rn(p.y, __fmul_rn(u[1], dt));
-    p.z = __fadd_rn(p.z, __fmul_rn(u[2], dt));
+    p.x = __fadd_rn(p.x, __fmul_rn(u.x, dt));
+    p.y = __fadd_rn(p.y, __fmul_rn(u.y, dt));
+    p.z = __fadd_rn(p.z, __fmul_rn(u.z, dt));
     pos[i] = p;
   }
 }
@@ -728,10 +752,24 @@ vg_status launch_pse(Ctx* c, const Geom& g, const CellLists& cl, const float4* p
   return VG_OK;
 }
 
-bool gather_by_cell(const Geom& g, size_t m) {
+// Staged records are taken apart into float4 positions and velocities, and put
+// together again, for two tracers or more per cell of a grid of 2^17 cells.
+bool unpack_records(const Geom& g, size_t m) {
   if (g.np[0] < 2 || g.np[1] < 2 || g.np[2] < 2) return false;
   const size_t cells = (size_t)(g.np[0] - 1) * (g.np[1] - 1) * (size_t)(g.np[2] - 1);
   return cells >= ((size_t)1 << 17) && m >= 2 * cells;
+}
+
+// Tracers of the step's own grid gather from its float4 points where the copy
+// (made once per step) pays: it costs 4 ns per 1000 points, and saves 25 to
+// 35 ns per 1000 tracers.  2^18 tracers, copy included, against the three-float
+// grid: 9.3 against 10.7 us on 33^3 points, 10.2 against 15.6 on 65^3, 16.2
+// against 16.8 on 129^3 (eight points to a tracer); 2^20 tracers on 193^3
+// points (seven to a tracer) 62.5 against 64.1.
+static bool gather_points(const Geom& g, size_t m) {
+  const size_t pts = g.points();
+  return g.np[0] >= 2 && g.np[1] >= 2 && g.np[2] >= 2 && pts < ((size_t)1 << 31) && m >= ((size_t)1 << 18) &&
+         6 * m >= pts;
 }
 
 vg_status launch_gather_advect_records(Ctx* c, const Geom& g, const float* vel3, unsigned char* rec, size_t pitch,
@@ -746,29 +784,23 @@ vg_status launch_gather_advect_records(Ctx* c, const Geom& g, const float* vel3,
 }
 
 vg_status launch_gather_advect(Ctx* c, const Geom& g, const float* vel3, float4* pos, float4* vel, size_t m, float dt,
-                               bool evolve, const unsigned* order, bool by_cell) {
+                               bool evolve, const unsigned* order, bool step_grid) {
   if (m == 0) return VG_OK;
   if (m > 0x7fffffff) return fail(c, VG_TOO_LARGE, "advect: more than 2^31 particles");
-  const size_t cells = g.np[0] >= 2 && g.np[1] >= 2 && g.np[2] >= 2
-                           ? (size_t)(g.np[0] - 1) * (g.np[1] - 1) * (size_t)(g.np[2] - 1)
-                           : 0;
-  // Tracer groups of at least two per cell gather from the grid arranged by
-  // cell (made once per step; inside a graph capture always, so that every
-  // replay remakes it from that replay's grid) -- on grids of at least 2^17
-  // cells: a smaller grid stays in L1/L2 and the copy costs more than it saves
-  // (65,536 tracers on 32^3 cells: the step 1.6% slower with it).
-  if (by_cell && !order && gather_by_cell(g, m)) {
+  // (inside a graph capture the copy is always made, so that every replay
+  // remakes it from that replay's grid)
+  if (step_grid && !order && gather_points(g, m)) {
     vg_status st = VG_OK;
-    float4* vc = (float4*)ws(c, S_VELCELL, 8 * cells * sizeof(float4), &st);
+    float4* vp = (float4*)ws(c, S_VELPOINTS, g.points() * sizeof(float4), &st);
     if (st != VG_OK) return st;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     VG_CUDA(c, cudaStreamIsCapturing(c->stream, &cap));
-    if (cap != cudaStreamCaptureStatusNone || c->velcell_gen != c->vel_gen) {
-      pdl_launch(c->stream, blocks_for(8 * cells, 256), 256, 0, k_vel_cells, g, vel3, vc);
+    if (cap != cudaStreamCaptureStatusNone || c->velpoints_gen != c->vel_gen) {
+      pdl_launch(c->stream, blocks_for(g.points(), 256), 256, 0, k_vel_points, g.points(), vel3, vp);
       VG_LAUNCHED(c);
-      c->velcell_gen = cap != cudaStreamCaptureStatusNone ? ~0ull : c->vel_gen;
+      c->velpoints_gen = cap != cudaStreamCaptureStatusNone ? ~0ull : c->vel_gen;
     }
-    pdl_launch(c->stream, blocks_for(m, 256), 256, 0, k_gather_advect_cells, g, (const float4*)vc, pos, vel, (int)m,
+    pdl_launch(c->stream, blocks_for(m, 256), 256, 0, k_gather_advect_points, g, (const float4*)vp, pos, vel, (int)m,
                dt, evolve ? 1 : 0, outside_flag(c));
     VG_LAUNCHED(c);
     VG_CUDA(c, cudaGetLastError());

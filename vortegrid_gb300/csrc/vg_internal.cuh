@@ -237,7 +237,7 @@ enum Slot {
   S_MC,     // marching cubes: per-cell counts and offsets
   S_BODY,   // fluid-body collisions: per-block partial sums
   S_EMIT,   // emitters: jitter draws, records, deviation grid, flags
-  S_VELCELL,  // the velocity grid by cell (8 corners x float4) for large tracer groups
+  S_VELPOINTS,  // the velocity grid as float4 points, for large tracer groups
   S_NUM
 };
 
@@ -283,8 +283,8 @@ struct Ctx {
   // (step_evolved: a kernel of the step has done it)
   bool step_evolve = false, step_evolved = false;
   // generation of the step's velocity grid (counted on the host at each step)
-  // and the one the by-cell copy in buf[S_VELCELL] was made from
-  unsigned long long vel_gen = 0, velcell_gen = ~0ull;
+  // and the one the float4 copy in buf[S_VELPOINTS] was made from
+  unsigned long long vel_gen = 0, velpoints_gen = ~0ull;
   bool stats_pending = false;
   // Multigrid schedule.  mg_fixed_k1 > 0 runs a fixed schedule with no host
   // round trip (k1 FP32 cycles, then k2 refinement cycles), so that a step can
@@ -461,12 +461,12 @@ vg_status launch_pse(Ctx* c, const Geom& g, const CellLists& cl, const float4* p
                      float dt);
 vg_status launch_heat_pse(Ctx* c, const Geom& g, const CellLists& cl, const float4* ps, float* density, size_t n,
                           float kappa, float ambient, float dt);
-// by_cell: a tracer group of the step's own velocity grid (vel3 = buf[S_VEL]),
-// which may be gathered from a copy of the grid arranged by cell.
+// step_grid: a tracer group of the step's own velocity grid (vel3 = buf[S_VEL]),
+// which may be gathered from a float4 copy of the grid.
 vg_status launch_gather_advect(Ctx* c, const Geom& g, const float* vel3, float4* pos, float4* vel, size_t m,
-                               float dt, bool evolve, const unsigned* order = nullptr, bool by_cell = false);
-// Whether m tracers on grid g gather from the grid arranged by cell.
-bool gather_by_cell(const Geom& g, size_t m);
+                               float dt, bool evolve, const unsigned* order = nullptr, bool step_grid = false);
+// Whether m staged tracer records on grid g are gathered as float4 arrays.
+bool unpack_records(const Geom& g, size_t m);
 // The gather + Euler step in place on m staged particle records (position at
 // bytes 0-11, velocity at 12-23, pitch bytes apart).
 vg_status launch_gather_advect_records(Ctx* c, const Geom& g, const float* vel3, unsigned char* rec, size_t pitch,
