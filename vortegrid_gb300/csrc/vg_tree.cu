@@ -44,6 +44,10 @@ __device__ __forceinline__ float ref_vort_mag(float4 w) {
   return __fsqrt_rn(ref_dot_self(a, b, c));
 }
 
+// Two vortons at a time: a leaf's vortons cost two dependent memory latencies each
+// otherwise (14 us for the eight rings, now 8 us); four take registers that the
+// many empty leaves of a large grid pay for (75 us for 7 million, two 63 us).
+constexpr unsigned kLeafBatch = 2;
 __global__ void k_leaf(Geom g, const float4* __restrict__ ps, const float4* __restrict__ w,
                        const unsigned* __restrict__ start, const unsigned* __restrict__ items,
                        float4* __restrict__ out_pos, float4* __restrict__ out_w) {
@@ -52,19 +56,30 @@ __global__ void k_leaf(Geom g, const float4* __restrict__ ps, const float4* __re
   if (c >= g.points()) return;
   float px = 0.f, py = 0.f, pz = 0.f, wx = 0.f, wy = 0.f, wz = 0.f, size = 0.f, aux = FLT_MIN;
   const unsigned b = start[c], e = start[c + 1];
-  for (unsigned k = b; k < e; ++k) {
-    const unsigned i = items[k];
-    const float4 p = ps[i];
-    const float4 a = w[i];
-    const float mag = ref_vort_mag(a);
-    px = __fadd_rn(px, __fmul_rn(p.x, mag));
-    py = __fadd_rn(py, __fmul_rn(p.y, mag));
-    pz = __fadd_rn(pz, __fmul_rn(p.z, mag));
-    wx = __fadd_rn(wx, a.x);
-    wy = __fadd_rn(wy, a.y);
-    wz = __fadd_rn(wz, a.z);
-    size = p.w;
-    aux = __fadd_rn(aux, mag);
+  for (unsigned k = b; k < e; k += kLeafBatch) {  // a batch's loads at a time: two latencies for all of them
+    unsigned i[kLeafBatch];
+    float4 p[kLeafBatch], a[kLeafBatch];
+#pragma unroll
+    for (unsigned u = 0; u < kLeafBatch; ++u) i[u] = items[k + u < e ? k + u : k];
+#pragma unroll
+    for (unsigned u = 0; u < kLeafBatch; ++u)
+      if (k + u < e) {
+        p[u] = ps[i[u]];
+        a[u] = w[i[u]];
+      }
+#pragma unroll
+    for (unsigned u = 0; u < kLeafBatch; ++u) {
+      if (k + u >= e) break;
+      const float mag = ref_vort_mag(a[u]);
+      px = __fadd_rn(px, __fmul_rn(p[u].x, mag));
+      py = __fadd_rn(py, __fmul_rn(p[u].y, mag));
+      pz = __fadd_rn(pz, __fmul_rn(p[u].z, mag));
+      wx = __fadd_rn(wx, a[u].x);
+      wy = __fadd_rn(wy, a[u].y);
+      wz = __fadd_rn(wz, a[u].z);
+      size = p[u].w;
+      aux = __fadd_rn(aux, mag);
+    }
   }
   if (aux != FLT_MIN) {
     const float r = __fdiv_rn(1.0f, aux);
@@ -79,31 +94,49 @@ __global__ void k_leaf(Geom g, const float4* __restrict__ ps, const float4* __re
 // AggregateClusters for parent point k of layer P from its children in C
 // (decimation d): vorticity-weighted centroid, summed angular velocity, the
 // last child's nonzero size.
+constexpr unsigned kBatch = 4;
 __device__ __forceinline__ void aggregate_point(const Geom& P, const Geom& C, uint3 d, const float4* __restrict__ cpos,
                                                 const float4* __restrict__ cw, float4* __restrict__ ppos,
                                                 float4* __restrict__ pw, size_t k) {
-  const unsigned px = (unsigned)(k % P.np[0]);
-  const unsigned py = (unsigned)((k / P.np[0]) % P.np[1]);
-  const unsigned pz = (unsigned)(k / ((size_t)P.np[0] * P.np[1]));
+  const unsigned k32 = (unsigned)k;  // a tree's layers have fewer than 2^32 points
+  const unsigned px = k32 % P.np[0], py = k32 / P.np[0] % P.np[1], pz = k32 / P.np[0] / P.np[1];
   float x = 0.f, y = 0.f, z = 0.f, wx = 0.f, wy = 0.f, wz = 0.f, size = 0.f;
   if (px < P.np[0] - 1 && py < P.np[1] - 1 && pz < P.np[2] - 1) {
     float aux = FLT_MIN;
-    for (unsigned iz = 0; iz < d.z; ++iz)
-      for (unsigned iy = 0; iy < d.y; ++iy)
-        for (unsigned ix = 0; ix < d.x; ++ix) {
-          const size_t o = (px * d.x + ix) + (size_t)C.np[0] * ((py * d.y + iy) + (size_t)C.np[1] * (pz * d.z + iz));
-          const float4 p = cpos[o];
-          const float4 a = cw[o];
-          const float mag = ref_vort_mag(a);
-          x = __fadd_rn(x, __fmul_rn(p.x, mag));
-          y = __fadd_rn(y, __fmul_rn(p.y, mag));
-          z = __fadd_rn(z, __fmul_rn(p.z, mag));
-          wx = __fadd_rn(wx, a.x);
-          wy = __fadd_rn(wy, a.y);
-          wz = __fadd_rn(wz, a.z);
-          aux = __fadd_rn(aux, mag);
-          if (p.w != 0.0f) size = p.w;
+    // the children in z, y, x order, kBatch of them loaded at a time: one memory latency for the batch
+    const size_t o0 = px * d.x + (size_t)C.np[0] * (py * d.y + (size_t)C.np[1] * (pz * d.z));
+    const unsigned total = d.x * d.y * d.z;
+    unsigned ix = 0, iy = 0, iz = 0;
+    for (unsigned k0 = 0; k0 < total; k0 += kBatch) {
+      float4 p[kBatch], a[kBatch];
+#pragma unroll
+      for (unsigned u = 0; u < kBatch; ++u)
+        if (k0 + u < total) {
+          const size_t o = o0 + ix + (size_t)C.np[0] * (iy + (size_t)C.np[1] * iz);
+          p[u] = cpos[o];
+          a[u] = cw[o];
+          if (++ix == d.x) {
+            ix = 0;
+            if (++iy == d.y) {
+              iy = 0;
+              ++iz;
+            }
+          }
         }
+#pragma unroll
+      for (unsigned u = 0; u < kBatch; ++u) {
+        if (k0 + u >= total) break;
+        const float mag = ref_vort_mag(a[u]);
+        x = __fadd_rn(x, __fmul_rn(p[u].x, mag));
+        y = __fadd_rn(y, __fmul_rn(p[u].y, mag));
+        z = __fadd_rn(z, __fmul_rn(p[u].z, mag));
+        wx = __fadd_rn(wx, a[u].x);
+        wy = __fadd_rn(wy, a[u].y);
+        wz = __fadd_rn(wz, a[u].z);
+        aux = __fadd_rn(aux, mag);
+        if (p[u].w != 0.0f) size = p[u].w;
+      }
+    }
     const float r = __fdiv_rn(1.0f, aux);
     x = __fmul_rn(x, r);
     y = __fmul_rn(y, r);
@@ -124,8 +157,10 @@ __global__ void k_aggregate(Geom P, Geom C, uint3 d, const float4* __restrict__ 
 // The small top layers l0 .. depth-1 in one CTA, layer after layer (a barrier
 // between them makes each layer's writes visible to the next): the same cells
 // as one k_aggregate launch per layer, without a launch per few hundred points.
-constexpr size_t kTopLayerPoints = 4096;  // layers of at most this many points go to k_aggregate_top
-constexpr int kTopThreads = 1024;
+// Layers of up to 512 points, one to a thread: all layers up to 4,096 points took
+// 12 to 18 us, now 8 us and a launch of 4.7 us where there is one between.
+constexpr size_t kTopLayerPoints = 512;  // layers of at most this many points go to k_aggregate_top
+constexpr int kTopThreads = 512;
 __global__ void __launch_bounds__(kTopThreads) k_aggregate_top(const __grid_constant__ TreeParams T, int l0,
                                                                float4* __restrict__ sv_pos, float4* __restrict__ sv_w) {
   pdl_entry();
@@ -230,16 +265,22 @@ __device__ float3 tree_walk(const TreeParams& T, const float4* __restrict__ sp, 
 // FAST walk's per-cell constants for one call's spread factors sr, sc:
 // tp = (centroid, 1 / R), tw = (angular velocity x 2/3 R^3 sc, R^2), R =
 // size / 2 x sr -- what fast_accum derives from (sp, sw) at every pair.
+__device__ __forceinline__ void prepare_cell(float4& p, float4& a, float sr, float sc) {
+  const float radius = p.w * 0.5f * sr;
+  const float s = VG_TWO_THIRDS * radius * radius * radius * sc;
+  p.w = 1.0f / radius;
+  a = make_float4(a.x * s, a.y * s, a.z * s, radius * radius);
+}
+
 __global__ void k_tree_prep(const float4* __restrict__ sp, const float4* __restrict__ sw, size_t total, float sr,
                             float sc, float4* __restrict__ tp, float4* __restrict__ tw) {
   pdl_entry();
   const size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= total) return;
-  const float4 p = sp[k], a = sw[k];
-  const float radius = p.w * 0.5f * sr;
-  const float s = VG_TWO_THIRDS * radius * radius * radius * sc;
-  tp[k] = make_float4(p.x, p.y, p.z, 1.0f / radius);
-  tw[k] = make_float4(a.x * s, a.y * s, a.z * s, radius * radius);
+  float4 p = sp[k], a = sw[k];
+  prepare_cell(p, a, sr, sc);
+  tp[k] = p;
+  tw[k] = a;
 }
 
 // fast_accum's law from prepared constants (the same mathematics, the scale
@@ -271,15 +312,19 @@ __device__ __forceinline__ void prep_accum(float3& acc, float qx, float qy, floa
 // open cells that are not themselves opened add their monopoles, the opened
 // ones form the next layer's box.  Same cells as tree_walk, summed layer by
 // layer instead of depth first (FAST numerics sum in any order).
-template <int KIND>
-__device__ float3 tree_walk_fast(const TreeParams& T, const float4* __restrict__ tp, const float4* __restrict__ tw,
+//
+// kRawLeaf: the leaf layer's cells are prepared where they are read.  kLanes
+// neighbouring lanes walk for one query, each taking every kLanes-th row of a
+// layer's cells; all of them return the sum.
+template <int KIND, bool kRawLeaf, int kLanes>
+__device__ float3 tree_walk_fast(const TreeParams& T, const float4* __restrict__ sp, const float4* __restrict__ sw,
+                                 const float4* __restrict__ tp, const float4* __restrict__ tw,
                                  const float4* __restrict__ ps, const float4* __restrict__ w, int n, float qx,
                                  float qy, float qz, float sr, float sc) {
   float3 acc = make_float3(0.f, 0.f, 0.f);
-  if (T.depth <= 1) {  // no tree: direct sum (vortonSim.cpp:2125-2128)
-    for (int i = 0; i < n; ++i) fast_accum<KIND>(acc, qx, qy, qz, ps[i], w[i], sr, sc);
-    return acc;
-  }
+  const unsigned sub = threadIdx.x % kLanes;
+  if (T.depth <= 1)  // no tree: direct sum (vortonSim.cpp:2125-2128)
+    for (int i = (int)sub; i < n; i += kLanes) fast_accum<KIND>(acc, qx, qy, qz, ps[i], w[i], sr, sc);
   const float mfac = 0.0001f;
   const float q[3] = {qx, qy, qz};
   unsigned f0[3] = {0u, 0u, 0u}, fn[3] = {1u, 1u, 1u};  // open box of layer L: [f0, f0 + fn) per axis
@@ -311,33 +356,44 @@ __device__ float3 tree_walk_fast(const TreeParams& T, const float4* __restrict__
     // the layer's cells (fewer than 2^32 in a layer); a row's cells are
     // consecutive, visited up to 4 at a time with their loads issued
     // together; an opened cell's term is computed and dropped (acc kept)
-    const float4* __restrict__ lp = tp + T.base[L - 1];
-    const float4* __restrict__ lw = tw + T.base[L - 1];
+    const bool raw = kRawLeaf && L == 1;
+    const float4* __restrict__ lp = (raw ? sp : tp) + T.base[L - 1];
+    const float4* __restrict__ lw = (raw ? sw : tw) + T.base[L - 1];
     const unsigned sy = C.np[0], sz = C.np[0] * C.np[1];
-    for (unsigned iz = 0; iz < cn[2]; ++iz) {
-      const unsigned chz = c0[2] + iz;
-      const bool oz = any && chz - o0[2] < on[2];
-      for (unsigned iy = 0; iy < cn[1]; ++iy) {
-        const unsigned chy = c0[1] + iy;
-        const bool oyz = oz && chy - o0[1] < on[1];
-        const unsigned row = c0[0] + sy * chy + sz * chz;
-        for (unsigned ix0 = 0; ix0 < cn[0]; ix0 += 4) {
-          float4 cp[4], cw[4];
+    auto add_row = [&](unsigned iy, unsigned iz) {
+      const unsigned chy = c0[1] + iy, chz = c0[2] + iz;
+      const bool oyz = any && chz - o0[2] < on[2] && chy - o0[1] < on[1];
+      const unsigned row = c0[0] + sy * chy + sz * chz;
+      for (unsigned ix0 = 0; ix0 < cn[0]; ix0 += 4) {
+        float4 cp[4], cw[4];
 #pragma unroll
-          for (unsigned u = 0; u < 4; ++u)
-            if (ix0 + u < cn[0]) {
-              cp[u] = lp[row + ix0 + u];
-              cw[u] = lw[row + ix0 + u];
-            }
-#pragma unroll
-          for (unsigned u = 0; u < 4; ++u) {
-            const unsigned ix = ix0 + u;
-            if (ix >= cn[0]) break;
-            float3 next = acc;
-            prep_accum<KIND>(next, qx, qy, qz, cp[u], cw[u]);
-            if (!(oyz && c0[0] + ix - o0[0] < on[0])) acc = next;
+        for (unsigned u = 0; u < 4; ++u)
+          if (ix0 + u < cn[0]) {
+            cp[u] = lp[row + ix0 + u];
+            cw[u] = lw[row + ix0 + u];
           }
+#pragma unroll
+        for (unsigned u = 0; u < 4; ++u) {
+          const unsigned ix = ix0 + u;
+          if (ix >= cn[0]) break;
+          float3 next = acc;
+          if (raw) prepare_cell(cp[u], cw[u], sr, sc);
+          prep_accum<KIND>(next, qx, qy, qz, cp[u], cw[u]);
+          if (!(oyz && c0[0] + ix - o0[0] < on[0])) acc = next;
         }
+      }
+    };
+    if (kLanes == 1) {
+      for (unsigned iz = 0; iz < cn[2]; ++iz)
+        for (unsigned iy = 0; iy < cn[1]; ++iy) add_row(iy, iz);
+    } else {
+      for (unsigned iy = sub, iz = 0;; iy += kLanes) {
+        while (iy >= cn[1] && iz < cn[2]) {
+          iy -= cn[1];
+          ++iz;
+        }
+        if (iz >= cn[2]) break;
+        add_row(iy, iz);
       }
     }
     if (!any) break;
@@ -347,88 +403,112 @@ __device__ float3 tree_walk_fast(const TreeParams& T, const float4* __restrict__
       fn[a] = on[a];
     }
   }
+  // the query's lanes only: others may be at another query, or have none
+  const unsigned lanes = ((1u << kLanes) - 1u) << (threadIdx.x % 32 / kLanes * kLanes);
+#pragma unroll
+  for (int o = 1; o < kLanes; o <<= 1) {
+    acc.x += __shfl_xor_sync(lanes, acc.x, o);
+    acc.y += __shfl_xor_sync(lanes, acc.y, o);
+    acc.z += __shfl_xor_sync(lanes, acc.z, o);
+  }
   return acc;
 }
 
-// REFERENCE numerics walk the raw cells (sp, sw); FAST the prepared ones (tp, tw).
-template <int KIND, bool REF>
+// REFERENCE numerics walk the raw cells (sp, sw); FAST the prepared ones (tp, tw),
+// but with kRawLeaf the raw leaf cells.
+template <int KIND, bool REF, bool kRawLeaf, int kLanes>
 __device__ __forceinline__ float3 walk(const TreeParams& T, const float4* __restrict__ sp,
                                        const float4* __restrict__ sw, const float4* __restrict__ tp,
                                        const float4* __restrict__ tw, const float4* __restrict__ ps,
                                        const float4* __restrict__ w, int n, float qx, float qy, float qz, float sr,
                                        float sc) {
   if (REF) return tree_walk<KIND, true>(T, sp, sw, ps, w, n, qx, qy, qz, sr, sc);
-  return tree_walk_fast<KIND>(T, tp, tw, ps, w, n, qx, qy, qz, sr, sc);
+  return tree_walk_fast<KIND, kRawLeaf, kLanes>(T, sp, sw, tp, tw, ps, w, n, qx, qy, qz, sr, sc);
 }
 
-template <int KIND, bool REF>
+template <int KIND, bool REF, bool kRawLeaf, int kLanes>
 __global__ void __launch_bounds__(128) k_tree_eval(const __grid_constant__ TreeParams T, const float4* __restrict__ sp,
                                                     const float4* __restrict__ sw, const float4* __restrict__ tp,
                                                     const float4* __restrict__ tw, const float4* __restrict__ ps,
                                                     const float4* __restrict__ w, int n, const float4* __restrict__ q,
                                                     int m, float sr, float sc, float4* __restrict__ out) {
   pdl_entry();
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = (int)(((size_t)blockIdx.x * blockDim.x + threadIdx.x) / kLanes);
   if (j >= m) return;
   const float4 v = q[j];
-  const float3 r = walk<KIND, REF>(T, sp, sw, tp, tw, ps, w, n, v.x, v.y, v.z, sr, sc);
-  out[j] = make_float4(r.x, r.y, r.z, 0.f);
+  const float3 r = walk<KIND, REF, kRawLeaf, kLanes>(T, sp, sw, tp, tw, ps, w, n, v.x, v.y, v.z, sr, sc);
+  if (threadIdx.x % kLanes == 0) out[j] = make_float4(r.x, r.y, r.z, 0.f);
 }
 
-// Boundary points: z faces (nx*ny each), y faces (nx*(nz-2)), x faces ((ny-2)*(nz-2)).
-__device__ __forceinline__ bool face_point(const Geom& g, size_t t, unsigned& x, unsigned& y, unsigned& z) {
+// Boundary queries, row by row of nq: z faces (nq * ny each), y faces (nq * (nz - 2)),
+// then the points of the x faces ((ny - 2) * (nz - 2)).  step: points along x to a query of a row.
+struct BoundaryQueries {
+  size_t fz, fy, fx;  // queries of one face
+  unsigned nq, step;
+};
+
+BoundaryQueries boundary_queries(const Geom& g, bool copy_odd_x) {
+  BoundaryQueries b;
+  b.step = copy_odd_x ? 2 : 1;
+  b.nq = (g.np[0] + b.step - 1) / b.step;
+  const size_t iy = g.np[1] > 2 ? g.np[1] - 2 : 0, iz = g.np[2] > 2 ? g.np[2] - 2 : 0;
+  b.fz = (size_t)b.nq * g.np[1];
+  b.fy = b.nq * iz;
+  b.fx = iy * iz;
+  return b;
+}
+
+__device__ __forceinline__ bool face_point(const Geom& g, const BoundaryQueries& b, size_t t, unsigned& x, unsigned& y,
+                                           unsigned& z, bool& row) {
   const size_t nx = g.np[0], ny = g.np[1], nz = g.np[2];
-  const size_t fz = nx * ny;
-  if (t < 2 * fz) {
-    z = (t < fz) ? 0 : (unsigned)(nz - 1);
-    const size_t r = t % fz;
-    x = (unsigned)(r % nx);
-    y = (unsigned)(r / nx);
-    return nz > 1 || t < fz;
+  row = true;
+  if (t < 2 * b.fz) {
+    z = (t < b.fz) ? 0 : (unsigned)(nz - 1);
+    const size_t r = t % b.fz;
+    x = (unsigned)(r % b.nq) * b.step;
+    y = (unsigned)(r / b.nq);
+    return nz > 1 || t < b.fz;
   }
-  t -= 2 * fz;
-  const size_t iz = nz > 2 ? nz - 2 : 0;
-  const size_t fy = nx * iz;
-  if (t < 2 * fy) {
-    y = (t < fy) ? 0 : (unsigned)(ny - 1);
-    const size_t r = t % fy;
-    x = (unsigned)(r % nx);
-    z = (unsigned)(r / nx) + 1;
-    return ny > 1 || t < fy;
+  t -= 2 * b.fz;
+  if (t < 2 * b.fy) {
+    y = (t < b.fy) ? 0 : (unsigned)(ny - 1);
+    const size_t r = t % b.fy;
+    x = (unsigned)(r % b.nq) * b.step;
+    z = (unsigned)(r / b.nq) + 1;
+    return ny > 1 || t < b.fy;
   }
-  t -= 2 * fy;
-  const size_t iy = ny > 2 ? ny - 2 : 0;
-  const size_t fx = iy * iz;
-  if (t < 2 * fx) {
-    x = (t < fx) ? 0 : (unsigned)(nx - 1);
-    const size_t r = t % fx;
+  t -= 2 * b.fy;
+  row = false;
+  if (t < 2 * b.fx) {
+    x = (t < b.fx) ? 0 : (unsigned)(nx - 1);
+    const size_t r = t % b.fx, iy = ny - 2;
     y = (unsigned)(r % iy) + 1;
     z = (unsigned)(r / iy) + 1;
-    return nx > 1 || t < fx;
+    return nx > 1 || t < b.fx;
   }
   return false;
 }
 
-template <bool REF>
+// Vector potential of the tree at the grid's boundary points.  With copy_odd_x
+// (step 2) an odd x has the value of the point before it, which is walked for
+// once and written twice; on rows that only have their two x faces' points
+// the point before the last was not computed and still holds zero.
+template <bool REF, bool kRawLeaf, int kLanes>
 __global__ void __launch_bounds__(128) k_boundary_vecpot(const __grid_constant__ TreeParams T, Geom g,
                                                           const float4* __restrict__ sp, const float4* __restrict__ sw,
                                                           const float4* __restrict__ tp, const float4* __restrict__ tw,
                                                           const float4* __restrict__ ps, const float4* __restrict__ w,
-                                                          int n, int copy_odd_x, size_t nface,
-                                                          float* __restrict__ grid3) {
+                                                          int n, BoundaryQueries b, float* __restrict__ grid3) {
   pdl_entry();
-  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nface) return;
+  const size_t t = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / kLanes;
   unsigned x, y, z;
-  if (!face_point(g, t, x, y, z)) return;
-  const bool full_row = (z == 0 || z == g.np[2] - 1 || y == 0 || y == g.np[1] - 1);
+  bool row;
+  if (!face_point(g, b, t, x, y, z, row)) return;
   unsigned xq = x;
   bool zero = false;
-  if (copy_odd_x && (x & 1u)) {
-    // odd x reuses the preceding point's value; on rows that only visit the
-    // two x faces, x-1 was not computed and still holds zero
-    if (full_row || g.np[0] - 1 == 1)
-      xq = x - 1;
+  if (!row && b.step == 2 && (x & 1u)) {
+    if (x == 1)
+      xq = 0;
     else
       zero = true;
   }
@@ -438,12 +518,19 @@ __global__ void __launch_bounds__(128) k_boundary_vecpot(const __grid_constant__
     const float qx = __fadd_rn(g.mn[0], __fmul_rn((float)xq, __fmul_rn(g.cell[0], nudge)));
     const float qy = __fadd_rn(g.mn[1], __fmul_rn((float)y, __fmul_rn(g.cell[1], nudge)));
     const float qz = __fadd_rn(g.mn[2], __fmul_rn((float)z, __fmul_rn(g.cell[2], nudge)));
-    r = walk<1, REF>(T, sp, sw, tp, tw, ps, w, n, qx, qy, qz, 1.0f, 1.0f);
+    r = walk<1, REF, kRawLeaf, kLanes>(T, sp, sw, tp, tw, ps, w, n, qx, qy, qz, 1.0f, 1.0f);
   }
+  const unsigned sub = threadIdx.x % kLanes;
+  if (sub) return;
   const size_t o = x + (size_t)g.np[0] * (y + (size_t)g.np[1] * z);
   grid3[3 * o] = r.x;
   grid3[3 * o + 1] = r.y;
   grid3[3 * o + 2] = r.z;
+  if (row && b.step == 2 && x + 1 < g.np[0]) {
+    grid3[3 * o + 3] = r.x;
+    grid3[3 * o + 4] = r.y;
+    grid3[3 * o + 5] = r.z;
+  }
 }
 
 // Gather-form splat: point P accumulates from the 8 cells P - {0,1}^3 in
@@ -570,39 +657,62 @@ vg_status build_tree(Ctx* c, const Geom& g, const float4* ps, const float4* w, s
   return VG_OK;
 }
 
+// Whether m queries read the leaf layer's cells as they are and prepare them
+// themselves: the leaf layer has seven eighths of a tree's cells, few of which lie
+// next to a boundary point.  1.0 million vortons on 225 x 161 x 193 points (192,000
+// queries): 75 us of preparation and 67 us of walks, now 13 and 75 us; 129^3
+// (98,000): 26 and 47 us, now 4 and 57 us.  A query in every cell pays for the
+// preparation (65,536 vortons' velocity grid: 3 and 86 us, else 2 and 108 us).
+static bool raw_leaf(const Tree& t, size_t m) { return m < t.layer[0].points() / 8; }
+
 // The FAST walk's prepared cells (workspace slot S_TREEPREP) for spread
-// factors sr, sc; nothing when the tree has no layers (the walk then sums the
-// vortons directly).
-static vg_status tree_prep(Ctx* c, const Tree& t, float sr, float sc, float4** tp, float4** tw) {
+// factors sr, sc: tp, tw are indexed as sv_pos, sv_w, the leaf layer left out when
+// raw; nothing when the tree has no layers (the walk then sums the vortons
+// directly).
+static vg_status tree_prep(Ctx* c, const Tree& t, bool raw, float sr, float sc, float4** tp, float4** tw) {
   if (t.depth <= 1 || t.total == 0) return VG_OK;
+  const size_t first = raw ? t.base[1] : 0, count = t.total - first;
   vg_status st = VG_OK;
-  float4* buf = (float4*)ws(c, S_TREEPREP, 2 * t.total * sizeof(float4), &st);
+  float4* buf = (float4*)ws(c, S_TREEPREP, 2 * count * sizeof(float4), &st);
   if (st != VG_OK) return st;
-  *tp = buf;
-  *tw = buf + t.total;
-  pdl_launch(c->stream, blocks_for(t.total, 256), 256, 0, k_tree_prep, t.sv_pos, t.sv_w, t.total, sr, sc, *tp, *tw);
+  *tp = buf - first;
+  *tw = buf + count - first;
+  pdl_launch(c->stream, blocks_for(count, 256), 256, 0, k_tree_prep, t.sv_pos + first, t.sv_w + first, count, sr, sc,
+             buf, buf + count);
   VG_LAUNCHED(c);
   return VG_OK;
 }
+
+// Lanes to a query: four where the queries alone leave most of the chip idle.
+// 6,146 boundary points: 22.8 us with one lane, 9.8 us with four; 25,000 points
+// of a 65^3 grid: 56 and 33 us by themselves, but 32 such solves at a time 2.5 %
+// slower, so the line is below; 98,000: 60 and 58 us; 192,000: 78 and 83 us.
+static int walk_lanes(size_t m) { return m < 16384 ? 4 : 1; }
 
 vg_status launch_tree_eval(Ctx* c, int kind, bool ref, const Tree& t, const float4* ps, const float4* w, size_t n,
                            const float4* q, size_t m, float sr, float sc, float4* out) {
   if (m == 0) return VG_OK;
   const TreeParams T = make_params(t);
-  const unsigned blocks = blocks_for(m, 128);
   float4 *tp = nullptr, *tw = nullptr;
+  const bool raw = !ref && raw_leaf(t, m);
+  const int lanes = ref ? 1 : walk_lanes(m);
+  const unsigned blocks = blocks_for(lanes * m, 128);
   if (!ref) {
-    vg_status st = tree_prep(c, t, sr, sc, &tp, &tw);
+    vg_status st = tree_prep(c, t, raw, sr, sc, &tp, &tw);
     if (st != VG_OK) return st;
   }
-#define VG_TREE_LAUNCH(K, R) \
-  pdl_launch(c->stream, blocks, 128, 0, k_tree_eval<K, R>, T, t.sv_pos, t.sv_w, tp, tw, ps, w, (int)n, q, (int)m, sr, sc, out)
+  auto launch = [&](auto kernel) {
+    pdl_launch(c->stream, blocks, 128, 0, kernel, T, t.sv_pos, t.sv_w, tp, tw, ps, w, (int)n, q, (int)m, sr, sc, out);
+  };
   if (kind == 0) {
-    if (ref) VG_TREE_LAUNCH(0, true); else VG_TREE_LAUNCH(0, false);
+    if (ref) launch(k_tree_eval<0, true, false, 1>);
+    else if (lanes == 4) launch(raw ? k_tree_eval<0, false, true, 4> : k_tree_eval<0, false, false, 4>);
+    else launch(raw ? k_tree_eval<0, false, true, 1> : k_tree_eval<0, false, false, 1>);
   } else {
-    if (ref) VG_TREE_LAUNCH(1, true); else VG_TREE_LAUNCH(1, false);
+    if (ref) launch(k_tree_eval<1, true, false, 1>);
+    else if (lanes == 4) launch(raw ? k_tree_eval<1, false, true, 4> : k_tree_eval<1, false, false, 4>);
+    else launch(raw ? k_tree_eval<1, false, true, 1> : k_tree_eval<1, false, false, 1>);
   }
-#undef VG_TREE_LAUNCH
   VG_LAUNCHED(c);
   VG_CUDA(c, cudaGetLastError());
   return VG_OK;
@@ -611,19 +721,23 @@ vg_status launch_tree_eval(Ctx* c, int kind, bool ref, const Tree& t, const floa
 vg_status launch_boundary_vecpot(Ctx* c, const Tree& t, const Geom& g, const float4* ps, const float4* w, size_t n,
                                  bool copy_odd_x, bool ref, float* grid3) {
   const TreeParams T = make_params(t);
-  const size_t nx = g.np[0], ny = g.np[1], nz = g.np[2];
-  const size_t nface = 2 * nx * ny + 2 * nx * (nz > 2 ? nz - 2 : 0) + 2 * (ny > 2 ? ny - 2 : 0) * (nz > 2 ? nz - 2 : 0);
-  if (nface == 0) return VG_OK;
-  if (ref) {
-    pdl_launch(c->stream, blocks_for(nface, 128), 128, 0, k_boundary_vecpot<true>, 
-        T, g, t.sv_pos, t.sv_w, nullptr, nullptr, ps, w, (int)n, copy_odd_x ? 1 : 0, nface, grid3);
-  } else {
-    float4 *tp = nullptr, *tw = nullptr;
-    vg_status st = tree_prep(c, t, 1.0f, 1.0f, &tp, &tw);
+  const BoundaryQueries b = boundary_queries(g, copy_odd_x);
+  const size_t m = 2 * (b.fz + b.fy + b.fx);
+  if (m == 0) return VG_OK;
+  float4 *tp = nullptr, *tw = nullptr;
+  const bool raw = !ref && raw_leaf(t, m);
+  const int lanes = ref ? 1 : walk_lanes(m);
+  if (!ref) {
+    vg_status st = tree_prep(c, t, raw, 1.0f, 1.0f, &tp, &tw);
     if (st != VG_OK) return st;
-    pdl_launch(c->stream, blocks_for(nface, 128), 128, 0, k_boundary_vecpot<false>, 
-        T, g, t.sv_pos, t.sv_w, tp, tw, ps, w, (int)n, copy_odd_x ? 1 : 0, nface, grid3);
   }
+  auto launch = [&](auto kernel) {
+    pdl_launch(c->stream, blocks_for(lanes * m, 128), 128, 0, kernel, T, g, t.sv_pos, t.sv_w, tp, tw, ps, w, (int)n, b,
+               grid3);
+  };
+  if (ref) launch(k_boundary_vecpot<true, false, 1>);
+  else if (lanes == 4) launch(raw ? k_boundary_vecpot<false, true, 4> : k_boundary_vecpot<false, false, 4>);
+  else launch(raw ? k_boundary_vecpot<false, true, 1> : k_boundary_vecpot<false, false, 1>);
   VG_LAUNCHED(c);
   VG_CUDA(c, cudaGetLastError());
   return VG_OK;
