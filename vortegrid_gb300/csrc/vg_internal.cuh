@@ -260,7 +260,7 @@ struct Ctx {
   nn::Net* net = nullptr;   // attached warm-start network (not owned)
   MgGraphCache mg_graph[kMgGraphs];  // cycle graphs, replaced in turn
   int mg_graph_next = 0;
-  double* hnorm = nullptr;           // pinned: the adaptive solve's last residual norm (r^2, b^2, sequence number)
+  unsigned long long* hnorm = nullptr;  // pinned: the adaptive solve's last residual norm (r^2, b^2, its number, a check)
   unsigned long long norm_seq = 0;   // norms asked for so far
   cudaStream_t stream = nullptr;
   bool own_stream = false;

@@ -647,14 +647,22 @@ __device__ __forceinline__ void split_sum2(float a32, float b32, double* __restr
   }
 }
 
-// The adaptive solve's norms: k_sum_partials whose sums also go to pinned host memory ([0] r^2, [1] b^2), behind a sequence
-// number ([2]) that the host polls: a copy and a stream wait took about 12 us a norm more.  (Summing in the residual kernels
-// by their last block, instead of this launch of 4 us, made them 4 to 10 us longer: a fence and an atomic at every block's end.)
+// A solve's norms: the partial sums added up ([0] r^2, [1] b^2, kept when keep_b) and, for the adaptive solve, written to
+// pinned host memory that the host polls: both sums, the norm's number and a check word, so that the host takes the four
+// only when they belong together and no fence is needed between them.  A copy and a stream wait took 15 to 20 us a norm
+// more.  (Summing in the residual kernels by their last block, instead of this launch, made them 4 to 10 us longer: a fence
+// and an atomic at every block's end.)
 __global__ void __launch_bounds__(1024) k_s_norm(const double* __restrict__ part, int nb, double* __restrict__ out2,
-                                                 int keep_b, unsigned long long* __restrict__ seq, volatile double* host) {
+                                                 int keep_b, unsigned long long* __restrict__ seq,
+                                                 unsigned long long seq0, volatile unsigned long long* host) {
   pdl_entry();
   __shared__ double s1[32], s2[32];
-  double a1 = 0.0, a2 = 0.0;
+  double a1 = 0.0, a2 = 0.0, b2 = 0.0;
+  unsigned long long number = 0;
+  if (threadIdx.x == 0) {
+    if (keep_b) b2 = out2[1];
+    if (host) number = (keep_b ? *seq : seq0) + 1;  // the first norm of a solve is the one that sets b^2
+  }
   for (int i = threadIdx.x; i < nb; i += 1024) {
     a1 += part[2 * i];
     a2 += part[2 * i + 1];
@@ -676,17 +684,17 @@ __global__ void __launch_bounds__(1024) k_s_norm(const double* __restrict__ part
     a2 += __shfl_xor_sync(0xffffffffu, a2, o);
   }
   if (threadIdx.x) return;
-  out2[0] = a1;
-  if (keep_b)
-    a2 = out2[1];
-  else
-    out2[1] = a2;
+  if (keep_b) a2 = b2;
   if (host) {
-    host[0] = a1;
-    host[1] = a2;
-    __threadfence_system();
-    host[2] = (double)++*seq;
+    const unsigned long long r = __double_as_longlong(a1), b = __double_as_longlong(a2);
+    host[0] = r;
+    host[1] = b;
+    host[2] = number;
+    host[3] = r ^ b ^ number;
+    *seq = number;
   }
+  out2[0] = a1;
+  if (!keep_b) out2[1] = a2;
 }
 
 // The iterate's values in a residual: x; x + e (the cycle's correction, whose sum is also written); or e alone (a first
@@ -900,17 +908,14 @@ __global__ void __launch_bounds__(256) k_s_out(SGeo g, const float* __restrict__
 }
 
 // Zero in the boundary planes and rows (y, z) of split fields, where a correction is zero and only its interior is ever
-// written (its first and last points in x are written with the rows); a warp a row.  Also the norms' sequence number.
+// written (its first and last points in x are written with the rows); a warp a row.
 struct FaceList {
   int n;
   float* f[kMaxLayers + 2];
   SGeo g[kMaxLayers + 2];
-  unsigned long long* seq;
-  unsigned long long seq0;
 };
 __global__ void __launch_bounds__(256) k_s_faces(const __grid_constant__ FaceList L) {
   pdl_entry();
-  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *L.seq = L.seq0;
   const SGeo& g = L.g[blockIdx.y];
   const unsigned q = blockIdx.x * 8 + threadIdx.x / 32, lane = threadIdx.x & 31, edges = 2 * g.ny + 2 * g.nz;
   const unsigned a = q / edges, k = q % edges;  // a = 2 c + colour
@@ -1400,6 +1405,8 @@ struct MgBufs {
   float* lo;  // refinement: corrections accumulated on top of the FP32 iterate
   double* part;
   double* sums;
+  unsigned long long* seq;   // the adaptive solve: norms so far, on the device
+  unsigned long long* host;  // and the pinned memory that they go to
   double* cwork;
   const void* dst;  // the coarsest level's sine-transform tables when P.direct (float, or double with dst64)
   bool dst64;       // FP64 coarsest solve: double tables, and double ping-pong fields d64a, d64b (3 N each)
@@ -1408,6 +1415,12 @@ struct MgBufs {
   unsigned nb0;  // residual blocks (partial sums)
   ResLaunch rl;   // the residual kernels' launch over level 0
 };
+
+static void enqueue_norm(Ctx* c, const MgBufs& B, int keep_b, unsigned* nl) {
+  pdl_launch(c->stream, 1, 1024, 0, k_s_norm, (const double*)B.part, (int)B.nb0, B.sums, keep_b, B.seq, c->norm_seq,
+             (volatile unsigned long long*)B.host);
+  ++*nl;
+}
 
 // The coarsest level's exact solve, or the V-cycle of the small levels in one CTA: e from r of level first_small, both
 // interleaved.
@@ -1511,11 +1524,44 @@ static vg_status enqueue_cycle(Ctx* c, const MgPlan& P, const Geom& g, const MgB
     pdl_launch(c->stream, B.rl.grid, B.rl.block, 0, k_residual32n, g, L0.r2x, L0.r2y, L0.r2z, B.rl.zs, x, rhs, B.R, B.part);
     ++*nl;
   }
-  if (tail == TAIL_NORM) {
-    pdl_launch(c->stream, 1, 1024, 0, k_sum_partials, B.part, (int)B.nb0, B.sums, 1);
-    ++*nl;
-  }
+  if (tail == TAIL_NORM) enqueue_norm(c, B, 1, nl);
   VG_CUDA(c, cudaGetLastError());
+  return VG_OK;
+}
+
+// The pinned memory of the adaptive solve's norms; a number that no norm has had is in it.
+static vg_status norm_memory(Ctx* c, MgBufs& B) {
+  if (!c->hnorm) {
+    VG_CUDA(c, cudaHostAlloc((void**)&c->hnorm, 64, cudaHostAllocDefault));
+    for (int k = 0; k < 4; ++k) c->hnorm[k] = 0;
+  }
+  B.host = c->hnorm;
+  return VG_OK;
+}
+
+// The next norm of the solve, from pinned host memory as soon as k_s_norm has written it.  The wait is a poll of that
+// memory; after every few thousand polls the stream is asked whether it has failed, or is done without the norm having come.
+static vg_status next_norm(Ctx* c, double* rr, double* bb) {
+  const unsigned long long want = ++c->norm_seq;
+  volatile unsigned long long* h = c->hnorm;
+  unsigned long long r = 0, b = 0;
+  auto there = [&] {
+    if (h[2] != want) return false;
+    r = h[0];
+    b = h[1];
+    return h[3] == (r ^ b ^ want);
+  };
+  for (unsigned long long polls = 1; !there(); ++polls) {
+    if (polls % 4096) continue;
+    const cudaError_t e = cudaStreamQuery(c->stream);
+    if (e == cudaErrorNotReady) continue;
+    VG_CUDA(c, e);
+    if (!there()) return fail(c, VG_CUDA_ERROR, "multigrid: a residual norm was not written");
+    break;
+  }
+  memcpy(rr, &r, sizeof(r));
+  if (bb) memcpy(bb, &b, sizeof(b));
+  if (!(*rr == *rr)) return fail(c, VG_NONFINITE, "multigrid: non-finite residual");
   return VG_OK;
 }
 
@@ -1563,16 +1609,6 @@ static vg_status run_cached(Ctx* c, const Geom& g, const void* const (&key)[4], 
 static vg_status run_cycle(Ctx* c, const MgPlan& P, const Geom& g, const MgBufs& B, float* x, const float* rhs) {
   const void* const key[4] = {B.E, rhs, x, nullptr};
   return run_cached(c, g, key, [&](unsigned* nl) { return enqueue_cycle(c, P, g, B, x, rhs, nl); });
-}
-
-static vg_status read_norm(Ctx* c, const double* sums, double* rr, double* bb) {
-  double h[2];
-  VG_CUDA(c, cudaMemcpyAsync(h, sums, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
-  VG_CUDA(c, cudaStreamSynchronize(c->stream));
-  *rr = h[0];
-  if (bb) *bb = h[1];
-  if (!(h[0] == h[0])) return fail(c, VG_NONFINITE, "multigrid: non-finite residual");
-  return VG_OK;
 }
 
 // Tables of the exact coarsest-level solve: per axis the orthonormal DST-I
@@ -1672,6 +1708,8 @@ static vg_status setup_bufs(Ctx* c, const Geom& g, const MgPlan& P, MgBufs& B, f
   B.lo = (float*)(((uintptr_t)(B.R + 3 * P.total) + 255) & ~(uintptr_t)255);
   B.part = (double*)(((uintptr_t)(B.lo + 3 * n0) + 255) & ~(uintptr_t)255);
   B.sums = B.part + 2 * (size_t)nb0;
+  B.seq = (unsigned long long*)(B.sums + 2);
+  B.host = nullptr;
   B.cwork = B.sums + 4;
   B.nb0 = nb0;
   B.rl = rl;
@@ -1725,8 +1763,6 @@ struct SplitBufs {
   float *X[2], *B, *T[3], *rir;          // level 0: the iterate twice, the right-hand side; refinement's corrections and residual
   float *Ec, *Rc;                        // the coarse level's, interleaved
   size_t n4;                             // float4 groups of a level-0 field
-  unsigned long long* seq;  // norms so far
-  double* host;             // pinned memory that they also go to, or null
   MgBufs mb;                             // sums, coarse workspace and tables
 };
 
@@ -1774,8 +1810,7 @@ static vg_status setup_split(Ctx* c, const MgPlan& P, SplitBufs& S) {
   B.part = (double*)(mem + oP);
   B.sums = B.part + 2 * (size_t)S.sl[0].nb;
   B.nb0 = S.sl[0].nb;
-  S.seq = (unsigned long long*)(B.sums + 4);
-  S.host = nullptr;
+  B.seq = (unsigned long long*)(B.sums + 4);
   B.cwork = (double*)(mem + oW);
   B.dst64 = P.direct_global && c->mg_coarse_fp64;
   if (P.direct && (st = direct_tables(c, P.lev[P.nlev - 1].g, B.dst64, &B.dst, &B.d64a, &B.d64b)) != VG_OK)
@@ -1834,12 +1869,6 @@ static vg_status enqueue_vcycle(Ctx* c, const MgPlan& P, const SplitBufs& S, con
   return VG_OK;
 }
 
-static void enqueue_norm(Ctx* c, const SplitBufs& S, int keep_b, unsigned* nl) {
-  pdl_launch(c->stream, 1, 1024, 0, k_s_norm, (const double*)S.mb.part, (int)S.mb.nb0, S.mb.sums, keep_b, S.seq,
-             (volatile double*)S.host);
-  ++*nl;
-}
-
 // r = b - L v (and v to xn), with its norm when `norm` (and ||b||^2 when `with_b`).
 template <int kField>
 static void enqueue_residual(Ctx* c, const SplitBufs& S, const float* x, const float* b, float* xn, bool norm,
@@ -1851,7 +1880,7 @@ static void enqueue_residual(Ctx* c, const SplitBufs& S, const float* x, const f
   else
     pdl_launch(c->stream, L.grid, L.block, 0, k_s_residual<kField, false>, S.g[0], x, e, b, xn, S.R[0], S.mb.part, L.zs);
   ++*nl;
-  if (norm) enqueue_norm(c, S, with_b ? 0 : 1, nl);
+  if (norm) enqueue_norm(c, S.mb, with_b ? 0 : 1, nl);
 }
 
 // The accurate residual of x (kAdd: of x + e, written to xn) + lo into r, and its norm.
@@ -1862,7 +1891,7 @@ static void enqueue_pair(Ctx* c, const SplitBufs& S, const PairCoef& cf, const f
   pdl_launch(c->stream, L.grid, L.block, 0, k_s_residual_pair<kAdd, kLo>, S.g[0], cf, x, (const float*)S.E[0], lo,
              (const float*)S.B, xn, r, S.mb.part, L.zs);
   ++*nl;
-  enqueue_norm(c, S, 1, nl);
+  enqueue_norm(c, S.mb, 1, nl);
 }
 
 // The solve's start: zero boundaries of the corrections, the split iterate and right-hand side, the first residual.
@@ -1870,8 +1899,6 @@ static void enqueue_start(Ctx* c, const MgPlan& P, const SplitBufs& S, const flo
                           unsigned* nl) {
   FaceList F;
   F.n = 0;
-  F.seq = S.seq;
-  F.seq0 = c->norm_seq;
   auto add = [&](float* f, const SGeo& g) {
     F.f[F.n] = f;
     F.g[F.n++] = g;
@@ -1942,36 +1969,13 @@ static vg_status split_fixed(Ctx* c, const Geom& g, const MgPlan& P, float* soln
   return VG_OK;
 }
 
-// The next norm of the solve, from pinned host memory as soon as the last block has written it.  The wait is a poll of that
-// memory; after every few thousand polls the stream is asked whether it has failed, or is done without the norm having come.
-static vg_status next_norm(Ctx* c, double* rr, double* bb) {
-  const double want = (double)++c->norm_seq;
-  volatile double* h = c->hnorm;
-  for (unsigned long long polls = 1; h[2] != want; ++polls) {
-    if (polls % 4096) continue;
-    const cudaError_t e = cudaStreamQuery(c->stream);
-    if (e == cudaErrorNotReady) continue;
-    VG_CUDA(c, e);
-    if (h[2] != want) return fail(c, VG_CUDA_ERROR, "multigrid: a residual norm was not written");
-  }
-  std::atomic_thread_fence(std::memory_order_acquire);
-  *rr = h[0];
-  if (bb) *bb = h[1];
-  if (!(*rr == *rr)) return fail(c, VG_NONFINITE, "multigrid: non-finite residual");
-  return VG_OK;
-}
-
 // run_multigrid over split levels; the cycles run from graphs.
 static vg_status split_adaptive(Ctx* c, const Geom& g, const MgPlan& P, float* soln3, const float* rhs3, double tol,
                                 int max_cycles, int* cycles, int* phase1, double* relres0, double* relres_out) {
   SplitBufs S;
   vg_status st = setup_split(c, P, S);
   if (st != VG_OK) return st;
-  if (!c->hnorm) {
-    VG_CUDA(c, cudaHostAlloc((void**)&c->hnorm, 64, cudaHostAllocDefault));
-    c->hnorm[2] = 0.0;
-  }
-  S.host = c->hnorm;
+  if ((st = norm_memory(c, S.mb)) != VG_OK) return st;
   const PairCoef cf = pair_coef(g, P.lev[0]);
   unsigned nl = 0;
   enqueue_start(c, P, S, soln3, rhs3, &nl);
@@ -2143,8 +2147,8 @@ vg_status run_multigrid(Ctx* c, const Geom& g, float* soln3, const float* rhs3, 
   MgBufs B;
   float *etot = nullptr, *rir = nullptr;
   vg_status st = setup_bufs(c, g, P, B, &etot, &rir);
-  if (st != VG_OK) return st;
-  const unsigned nb0 = B.nb0;
+  if (st != VG_OK || (st = norm_memory(c, B)) != VG_OK) return st;
+  unsigned nl = 0;
   // e must be zero on every level's boundary (Dirichlet correction); the
   // kernels only ever write interior points.
   VG_CUDA(c, cudaMemsetAsync(B.E, 0, P.total * 3 * sizeof(float), c->stream));
@@ -2152,10 +2156,10 @@ vg_status run_multigrid(Ctx* c, const Geom& g, float* soln3, const float* rhs3, 
   const PairCoef cf = pair_coef(g, L0);
   pdl_launch(c->stream, B.rl.grid, B.rl.block, 0, k_residual32n, g, L0.r2x, L0.r2y, L0.r2z, B.rl.zs, soln3, rhs3, B.R,
                                                          B.part);
-  pdl_launch(c->stream, 1, 1024, 0, k_sum_partials, B.part, (int)nb0, B.sums, 0);
-  c->launches += 2;
+  enqueue_norm(c, B, 0, &nl);
+  ++c->launches;
   double rr = 0.0, bnorm2 = 0.0;
-  if ((st = read_norm(c, B.sums, &rr, &bnorm2)) != VG_OK) return st;
+  if ((st = next_norm(c, &rr, &bnorm2)) != VG_OK) return st;
   const double bn = bnorm2 > 0.0 ? std::sqrt(bnorm2) : 1.0;
   double relres = std::sqrt(rr) / bn;
   const double relres0 = relres;
@@ -2166,7 +2170,7 @@ vg_status run_multigrid(Ctx* c, const Geom& g, float* soln3, const float* rhs3, 
   while (relres > switch_tol && cyc < max_cycles) {
     if ((st = run_cycle(c, P, g, B, soln3, rhs3)) != VG_OK) return st;
     ++cyc;
-    if ((st = read_norm(c, B.sums, &rr, nullptr)) != VG_OK) return st;
+    if ((st = next_norm(c, &rr, nullptr)) != VG_OK) return st;
     relres = std::sqrt(rr) / bn;
   }
   const int k1 = cyc;
@@ -2178,9 +2182,9 @@ vg_status run_multigrid(Ctx* c, const Geom& g, float* soln3, const float* rhs3, 
   VG_CUDA(c, cudaMemsetAsync(B.lo, 0, 3 * n0 * sizeof(float), c->stream));
   for (;;) {
     pdl_launch(c->stream, B.rl.grid, B.rl.block, 0, k_residual_pair<true>, g, cf, B.rl.zs, soln3, B.lo, rhs3, rir, B.part);
-    pdl_launch(c->stream, 1, 1024, 0, k_sum_partials, B.part, (int)nb0, B.sums, 1);
-    c->launches += 2;
-    if ((st = read_norm(c, B.sums, &rr, nullptr)) != VG_OK) return st;
+    enqueue_norm(c, B, 1, &nl);
+    ++c->launches;
+    if ((st = next_norm(c, &rr, nullptr)) != VG_OK) return st;
     relres = std::sqrt(rr) / bn;
     if (relres <= tol || cyc >= max_cycles) break;
     // The FP32 residual of the correction equation tracks the accurate residual
@@ -2193,7 +2197,7 @@ vg_status run_multigrid(Ctx* c, const Geom& g, float* soln3, const float* rhs3, 
     while (inner > inner_tol && cyc < max_cycles) {
       if ((st = run_cycle(c, P, g, B, etot, rir)) != VG_OK) return st;
       ++cyc;
-      if ((st = read_norm(c, B.sums, &rr, nullptr)) != VG_OK) return st;
+      if ((st = next_norm(c, &rr, nullptr)) != VG_OK) return st;
       inner = std::sqrt(rr) / bn;
     }
     add_f32(c, B.lo, etot, 3 * n0);
@@ -2201,6 +2205,7 @@ vg_status run_multigrid(Ctx* c, const Geom& g, float* soln3, const float* rhs3, 
   }
   add_f32(c, soln3, B.lo, 3 * n0);
   VG_LAUNCHED(c);
+  c->launches += nl;
   VG_CUDA(c, cudaGetLastError());
   return finish(cyc, k1, relres0, relres);
 }
