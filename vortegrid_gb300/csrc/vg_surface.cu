@@ -64,7 +64,8 @@ __global__ void __launch_bounds__(128) k_density(Geom g, const float4* __restric
   const float one_over_cell_volume = __fdiv_rn(1.0f, __fmul_rn(__fmul_rn(g.cell[0], g.cell[1]), g.cell[2]));
   const float volume_ratio = __fmul_rn(vorton_volume, one_over_cell_volume);
   const unsigned nx = g.np[0], ny = g.np[1];
-  const unsigned X = (unsigned)(k % nx), Y = (unsigned)((k / nx) % ny), Z = (unsigned)(k / ((size_t)nx * ny));
+  unsigned X, Y, Z;
+  grid_index(k, nx, ny, X, Y, Z);
   unsigned cur[8], end[8];
 #pragma unroll
   for (int o = 0; o < 8; ++o) {
@@ -129,7 +130,8 @@ __global__ void k_gradient(Geom g, const float* __restrict__ v, float* __restric
   const size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= g.points()) return;
   const unsigned nx = g.np[0], ny = g.np[1];
-  const unsigned id[3] = {(unsigned)(k % nx), (unsigned)((k / nx) % ny), (unsigned)(k / ((size_t)nx * ny))};
+  unsigned id[3];
+  grid_index(k, nx, ny, id[0], id[1], id[2]);
   const size_t st[3] = {1, nx, (size_t)nx * ny};
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
@@ -315,7 +317,8 @@ __global__ void k_sdf_immediate(Geom g, const float* __restrict__ dens, float am
   if (k >= pts) return;
   const float denom = sdf_denominator(st, pts, ambient);
   const unsigned nx = g.np[0], ny = g.np[1], nz = g.np[2];
-  const unsigned x = (unsigned)(k % nx), y = (unsigned)((k / nx) % ny), z = (unsigned)(k / ((size_t)nx * ny));
+  unsigned x, y, z;
+  grid_index(k, nx, ny, x, y, z);
   const size_t nxy = (size_t)nx * ny;
   float here = FLT_MAX;
   bool pin = false;
@@ -510,7 +513,8 @@ __global__ void k_mc_count(Geom g, const float* __restrict__ v, float iso, const
   const size_t cx = g.np[0] - 1, cy = g.np[1] - 1, cells = cx * cy * (g.np[2] - 1);
   const size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= cells) return;
-  const size_t x = k % cx, y = (k / cx) % cy, z = k / (cx * cy);
+  unsigned x, y, z;
+  grid_index(k, (unsigned)cx, (unsigned)cy, x, y, z);
   float val[8];
   counts[k] = T.cnt[mc_mask(g, v, x + g.np[0] * (y + (size_t)g.np[1] * z), iso, val)];
 }
@@ -525,7 +529,8 @@ __global__ void k_mc_emit(Geom g, const float* __restrict__ v, float iso, const 
   size_t out = offsets[k];
   const int nt = (int)(offsets[k + 1] - out);  // 0 for most cells, whose corners are then not read
   if (nt == 0) return;
-  const unsigned x = (unsigned)(k % cx), y = (unsigned)((k / cx) % cy), z = (unsigned)(k / (cx * cy));
+  unsigned x, y, z;
+  grid_index(k, (unsigned)cx, (unsigned)cy, x, y, z);
   float val[8];
   const int mask = mc_mask(g, v, x + g.np[0] * (y + (size_t)g.np[1] * z), iso, val);
   // corner positions min + index x spacing (marchingCubes.cpp:806-816)

@@ -547,7 +547,8 @@ __global__ void __launch_bounds__(128) k_splat(Geom g, const float4* __restrict_
   const float vorton_volume = __fmul_rn(four_pi_over3, __fmul_rn(__fmul_rn(radius, radius), radius));
   const float corr = __fdiv_rn(__fmul_rn(scale, vorton_volume), cell_volume);
   const unsigned nx = g.np[0], ny = g.np[1], nz = g.np[2];
-  const unsigned X = (unsigned)(k % nx), Y = (unsigned)((k / nx) % ny), Z = (unsigned)(k / ((size_t)nx * ny));
+  unsigned X, Y, Z;
+  grid_index(k, nx, ny, X, Y, Z);
   unsigned cur[8], end[8];
 #pragma unroll
   for (int o = 0; o < 8; ++o) {
