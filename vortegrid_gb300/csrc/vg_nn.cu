@@ -134,6 +134,7 @@ struct PairSum {
 // Sum of squares of count values, one fixed partial per block (deterministic).
 template <typename T>
 __global__ void k_sumsq(const T* __restrict__ a, size_t count, double* __restrict__ partials) {
+  pdl_entry();
   PairSum s;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -162,6 +163,7 @@ __device__ __forceinline__ double warp_sum_partials(const double* __restrict__ p
 }
 
 __global__ void k_scales(const double* __restrict__ partials, int nb, double count, float h2k, float* scales) {
+  pdl_entry();
   const double s = warp_sum_partials(partials, nb);
   if (threadIdx.x != 0) return;
   double rms = sqrt(s / count);
@@ -175,6 +177,7 @@ __global__ void k_scales(const double* __restrict__ partials, int nb, double cou
 template <typename T>
 __global__ void k_pack_input(const T* __restrict__ rhs, const T* __restrict__ vp, int n, const float* __restrict__ scales,
                              __nv_bfloat16* __restrict__ x) {
+  pdl_entry();
   const size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t nv = (size_t)n * n * n;
   if (v >= nv) return;
@@ -211,6 +214,7 @@ __global__ void k_pack_input(const T* __restrict__ rhs, const T* __restrict__ vp
 // Interior points (all indices in 1..n-1) of the vector potential from the network output.
 __global__ void k_unpack_output(const float* __restrict__ out, int n, const float* __restrict__ scales,
                                 float* __restrict__ vp) {
+  pdl_entry();
   const size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= (size_t)n * n * n) return;
   const int i = (int)(v % n), j = (int)((v / n) % n), k = (int)(v / ((size_t)n * n));
@@ -229,6 +233,7 @@ __global__ void k_unpack_output(const float* __restrict__ out, int n, const floa
 template <typename T>
 __global__ void k_target_energy(const T* __restrict__ vp, int n, const float* __restrict__ scales,
                                 double* __restrict__ partials) {
+  pdl_entry();
   PairSum s;
   const int np = n + 1;
   const float s_t = scales[1];
@@ -257,6 +262,7 @@ __global__ void k_target_energy(const T* __restrict__ vp, int n, const float* __
 
 // e[1] = target energy (1 if zero), e[2] = 2 / e[1] (the loss gradient's scale)
 __global__ void k_finish_energy(const double* __restrict__ partials, int nb, float* e) {
+  pdl_entry();
   double s = warp_sum_partials(partials, nb);
   if (threadIdx.x != 0) return;
   if (!(s > 0.0) || !isfinite(s)) s = 1.0;
@@ -271,6 +277,7 @@ template <typename T>
 __global__ void k_loss_grad(const float* __restrict__ out, const T* __restrict__ vp, int n,
                             const float* __restrict__ scales, const float* __restrict__ e,
                             __nv_bfloat16* __restrict__ g, double* __restrict__ partials) {
+  pdl_entry();
   PairSum s;
   const size_t nv = (size_t)n * n * n;
   const int np = n + 1;
@@ -312,6 +319,7 @@ __global__ void k_loss_grad(const float* __restrict__ out, const T* __restrict__
 
 // e[0] = loss = sum of squared differences / target energy
 __global__ void k_finish_loss(const double* __restrict__ partials, int nb, float* e) {
+  pdl_entry();
   const double s = warp_sum_partials(partials, nb);
   if (threadIdx.x != 0) return;
   e[0] = (float)(s / (double)e[1]);
@@ -337,6 +345,7 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const float* f) {
 
 // 2x2x2 average pool: fine e^3 -> coarse (e/2)^3, C channels.
 __global__ void k_pool(const __nv_bfloat16* __restrict__ in, int ec, int C, __nv_bfloat16* __restrict__ out) {
+  pdl_entry();
   const int c8 = C / 8;
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t nvc = (size_t)ec * ec * ec;
@@ -362,6 +371,7 @@ __global__ void k_pool(const __nv_bfloat16* __restrict__ in, int ec, int C, __nv
 // g[v][c] = (y[v][c] > 0 ? 1 : kSlope) * sum over the 8 children of gin[child][c] (c < C1).
 __global__ void k_up_grad(const __nv_bfloat16* __restrict__ gin, int ccat, const __nv_bfloat16* __restrict__ y, int ec,
                           int C1, __nv_bfloat16* __restrict__ g) {
+  pdl_entry();
   const int c8 = C1 / 8;
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t nvc = (size_t)ec * ec * ec;
@@ -390,6 +400,7 @@ __global__ void k_up_grad(const __nv_bfloat16* __restrict__ gin, int ccat, const
 // g[v][c] = (e[v][c] > 0 ? 1 : kSlope) * (gin_cat[v][C1 + c] + gp[parent(v)][c] / 8).
 __global__ void k_skip_grad(const __nv_bfloat16* __restrict__ gcat, int ccat, int C1, const __nv_bfloat16* __restrict__ gp,
                             const __nv_bfloat16* __restrict__ e, int ef, int C, __nv_bfloat16* __restrict__ g) {
+  pdl_entry();
   const int c8 = C / 8;
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t nv = (size_t)ef * ef * ef;
@@ -410,6 +421,7 @@ __global__ void k_skip_grad(const __nv_bfloat16* __restrict__ gcat, int ccat, in
 
 // db[c] += sum over voxels of g[v][c].
 __global__ void k_colsum(const __nv_bfloat16* __restrict__ g, size_t nv, int C, float* __restrict__ db) {
+  pdl_entry();
   __shared__ float sh[256];
   const int lanes = blockDim.x / C;  // voxels handled side by side
   const int c = threadIdx.x % C, l = threadIdx.x / C;
@@ -485,7 +497,7 @@ vg_status pool(Ctx* c, const Net* N, int a_in, int a_out) {
   const int ec = N->dims(kActLevel[a_out]);
   const int C = kActC[a_in];
   const size_t cnt = (size_t)ec * ec * ec * (C / 8);
-  k_pool<<<blocks_for(cnt, 256), 256, 0, c->stream>>>(N->act[a_in], ec, C, N->act[a_out]);
+  pdl_launch(c->stream, blocks_for(cnt, 256), 256, 0, k_pool, N->act[a_in], ec, C, N->act[a_out]);
   VG_LAUNCHED(c);
   return VG_OK;
 }
@@ -526,7 +538,7 @@ vg_status backward(Ctx* c, Net* N) {
       if ((st = conv3_wgrad(c, layer_input(N, l), N->g[l], L.co, N->grad + N->wofs[l])) != VG_OK) return st;
       const int lanes = 256 / L.co;
       unsigned nb = (unsigned)std::min<size_t>((nv + lanes - 1) / lanes, 4 * (size_t)sm_count());
-      k_colsum<<<nb, 256, 0, c->stream>>>(N->g[l], nv, L.co, N->grad + N->bofs[l]);
+      pdl_launch(c->stream, nb, 256, 0, k_colsum, N->g[l], nv, L.co, N->grad + N->bofs[l]);
       VG_LAUNCHED(c);
     }
     if (l == 0) break;
@@ -552,7 +564,7 @@ vg_status backward(Ctx* c, Net* N) {
       if ((st = conv3_fwd(c, gi, wt, o)) != VG_OK) return st;
       const int ec = e / 2;
       const size_t cnt = (size_t)ec * ec * ec * (L.cup / 8);
-      k_up_grad<<<blocks_for(cnt, 256), 256, 0, c->stream>>>(N->gin[l], L.ci, N->act[kIn1[l]], ec, L.cup,
+      pdl_launch(c->stream, blocks_for(cnt, 256), 256, 0, k_up_grad, N->gin[l], L.ci, N->act[kIn1[l]], ec, L.cup,
                                                                N->g[l - 1]);
       VG_LAUNCHED(c);
     } else if (l == 2 || l == 4 || l == 6) {
@@ -565,7 +577,7 @@ vg_status backward(Ctx* c, Net* N) {
       const int ef = N->dims(kActLevel[skip_act]);
       const int C = kActC[skip_act];
       const size_t cnt = (size_t)ef * ef * ef * (C / 8);
-      k_skip_grad<<<blocks_for(cnt, 256), 256, 0, c->stream>>>(N->gin[user], kNet[user].ci, kNet[user].cup, N->gin[l],
+      pdl_launch(c->stream, blocks_for(cnt, 256), 256, 0, k_skip_grad, N->gin[user], kNet[user].ci, kNet[user].cup, N->gin[l],
                                                                  N->act[skip_act], ef, C, N->g[l - 1]);
       VG_LAUNCHED(c);
     } else {
@@ -601,10 +613,10 @@ vg_status check_grid(Ctx* c, const Net* N, const Geom& g) {
 template <typename T>
 vg_status prepare_input(Ctx* c, Net* N, const Geom& g, const T* rhs, const T* vp) {
   const size_t pts = g.points();
-  k_sumsq<T><<<kRedBlocks, 256, 0, c->stream>>>(rhs, pts * 3, N->partials);
-  k_scales<<<1, 32, 0, c->stream>>>(N->partials, kRedBlocks, (double)pts * 3, grid_h2(g) * N->out_scale, N->scales);
+  pdl_launch(c->stream, kRedBlocks, 256, 0, k_sumsq<T>, rhs, pts * 3, N->partials);
+  pdl_launch(c->stream, 1, 32, 0, k_scales, N->partials, kRedBlocks, (double)pts * 3, grid_h2(g) * N->out_scale, N->scales);
   const size_t nv = N->vox(0);
-  k_pack_input<T><<<blocks_for(nv, 256), 256, 0, c->stream>>>(rhs, vp, N->n, N->scales, N->act[A_X]);
+  pdl_launch(c->stream, blocks_for(nv, 256), 256, 0, k_pack_input<T>, rhs, vp, N->n, N->scales, N->act[A_X]);
   c->launches += 3;
   VG_CUDA(c, cudaGetLastError());
   return VG_OK;
@@ -616,11 +628,11 @@ vg_status backward_pair(Ctx* c, Net* N, const Geom& g, const T* rhs, const T* vp
   if ((st = prepare_input<T>(c, N, g, rhs, vp)) != VG_OK) return st;
   if ((st = forward(c, N)) != VG_OK) return st;
   const int n = N->n;
-  k_target_energy<T><<<kRedBlocks, 256, 0, c->stream>>>(vp, n, N->scales, N->partials);
-  k_finish_energy<<<1, 32, 0, c->stream>>>(N->partials, kRedBlocks, N->loss);
-  k_loss_grad<T><<<kRedBlocks, 256, 0, c->stream>>>(N->out, vp, n, N->scales, N->loss, N->g[kLayers - 1],
+  pdl_launch(c->stream, kRedBlocks, 256, 0, k_target_energy<T>, vp, n, N->scales, N->partials);
+  pdl_launch(c->stream, 1, 32, 0, k_finish_energy, N->partials, kRedBlocks, N->loss);
+  pdl_launch(c->stream, kRedBlocks, 256, 0, k_loss_grad<T>, N->out, vp, n, N->scales, N->loss, N->g[kLayers - 1],
                                                     N->partials);
-  k_finish_loss<<<1, 32, 0, c->stream>>>(N->partials, kRedBlocks, N->loss);
+  pdl_launch(c->stream, 1, 32, 0, k_finish_loss, N->partials, kRedBlocks, N->loss);
   c->launches += 4;
   if (!accumulate) VG_CUDA(c, cudaMemsetAsync(N->grad, 0, N->nparam * sizeof(float), c->stream));
   return backward(c, N);
@@ -727,7 +739,7 @@ vg_status guess(Ctx* c, Net* N, const Geom& g, const float* rhs, float* vp) {
   if ((st = prepare_input<float>(c, N, g, rhs, vp)) != VG_OK) return st;
   if ((st = forward(c, N)) != VG_OK) return st;
   const size_t nv = N->vox(0);
-  k_unpack_output<<<blocks_for(nv, 256), 256, 0, c->stream>>>(N->out, N->n, N->scales, vp);
+  pdl_launch(c->stream, blocks_for(nv, 256), 256, 0, k_unpack_output, N->out, N->n, N->scales, vp);
   VG_LAUNCHED(c);
   VG_CUDA(c, cudaGetLastError());
   return VG_OK;

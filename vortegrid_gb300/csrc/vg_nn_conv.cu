@@ -168,6 +168,7 @@ __device__ __forceinline__ void store_tile(const float (&acc)[kMT][CO_T / 8][4],
 template <int CO_T>
 __global__ void __launch_bounds__(kWarps * 32) k_conv3_fwd(const ConvIn in, const __nv_bfloat16* __restrict__ wt,
                                                            const ConvOut out) {
+  pdl_entry();
   extern __shared__ __align__(16) uint4 smem4[];
   const Tile T = make_tile(in.D, in.H, in.W);
   const int hx = T.tx + 2, hy = T.ty + 2, nh = hx * hy * (T.tz + 2);
@@ -266,6 +267,7 @@ template <int CO_T>
 __global__ void __launch_bounds__(kWarps * 32) k_conv3_fwd_resident(const ConvIn in,
                                                                     const __nv_bfloat16* __restrict__ wt,
                                                                     const ConvOut out, int ncog) {
+  pdl_entry();
   extern __shared__ __align__(16) uint4 smem4[];
   const Tile T = make_tile(in.D, in.H, in.W);
   const int hx = T.tx + 2, hy = T.ty + 2, nh = hx * hy * (T.tz + 2);
@@ -348,6 +350,7 @@ __global__ void __launch_bounds__(kWarps * 32) k_conv3_fwd_resident(const ConvIn
 
 __global__ void __launch_bounds__(kWarps * 32) k_conv3_wgrad(const ConvIn in, const __nv_bfloat16* __restrict__ dy,
                                                              int Co, float* __restrict__ dw) {
+  pdl_entry();
   __shared__ __align__(16) uint4 sdy[2 * kTileVox];
   __shared__ __align__(16) uint4 sx[2 * kMaxHalo];
   const Tile T = make_tile(in.D, in.H, in.W);
@@ -449,7 +452,7 @@ vg_status launch_resident(Ctx* c, const ConvIn& in, const __nv_bfloat16* wt, con
   const long items = (long)T.nx * T.ny * T.nz * ncog;
   long grid = std::min<long>(items, (long)std::max(per_sm, 1) * sm_count());
   grid = std::max<long>(ncog, grid / ncog * ncog);
-  k_conv3_fwd_resident<CO_T><<<(unsigned)grid, kWarps * 32, smem, c->stream>>>(in, wt, out, ncog);
+  pdl_launch(c->stream, (unsigned)grid, kWarps * 32, smem, k_conv3_fwd_resident<CO_T>, in, wt, out, ncog);
   VG_LAUNCHED(c);
   VG_CUDA(c, cudaGetLastError());
   return VG_OK;
@@ -490,13 +493,13 @@ vg_status conv3_fwd(Ctx* c, const ConvIn& in, const __nv_bfloat16* wt, const Con
   const dim3 grid((unsigned)tiles, (unsigned)(out.Co / co_t));
   if (co_t == 64) {
     set_fwd_smem_attr<64>();
-    k_conv3_fwd<64><<<grid, kWarps * 32, smem, c->stream>>>(in, wt, out);
+    pdl_launch(c->stream, grid, kWarps * 32, smem, k_conv3_fwd<64>, in, wt, out);
   } else if (co_t == 32) {
     set_fwd_smem_attr<32>();
-    k_conv3_fwd<32><<<grid, kWarps * 32, smem, c->stream>>>(in, wt, out);
+    pdl_launch(c->stream, grid, kWarps * 32, smem, k_conv3_fwd<32>, in, wt, out);
   } else {
     set_fwd_smem_attr<16>();
-    k_conv3_fwd<16><<<grid, kWarps * 32, smem, c->stream>>>(in, wt, out);
+    pdl_launch(c->stream, grid, kWarps * 32, smem, k_conv3_fwd<16>, in, wt, out);
   }
   VG_LAUNCHED(c);
   VG_CUDA(c, cudaGetLastError());
@@ -512,7 +515,7 @@ vg_status conv3_wgrad(Ctx* c, const ConvIn& in, const __nv_bfloat16* dy, int Co,
   int splits = (4 * sm_count() + blocks_cc - 1) / blocks_cc;
   if (splits > ntiles) splits = ntiles;
   if (splits < 1) splits = 1;
-  k_conv3_wgrad<<<dim3((unsigned)blocks_cc, (unsigned)splits), kWarps * 32, 0, c->stream>>>(in, dy, Co, dw);
+  pdl_launch(c->stream, dim3((unsigned)blocks_cc, (unsigned)splits), kWarps * 32, 0, k_conv3_wgrad, in, dy, Co, dw);
   VG_LAUNCHED(c);
   VG_CUDA(c, cudaGetLastError());
   return VG_OK;

@@ -134,6 +134,7 @@ struct UmmaPlan {
 template <int CO_T>
 __global__ void __launch_bounds__(kThreads, 2) k_conv3_umma(const ConvIn in, const __nv_bfloat16* __restrict__ wt,
                                                             const ConvOut out, const UmmaPlan P, int* __restrict__ err) {
+  pdl_entry();
   extern __shared__ __align__(1024) unsigned char smem[];
   constexpr int N = 3 * CO_T;
   constexpr unsigned kWPlane = 9u * N * 16u;  // 8 channels of a slice's weights
@@ -381,7 +382,7 @@ vg_status launch_umma(Ctx* c, const ConvIn& in, const __nv_bfloat16* wt, const C
   VG_CUDA(c, cudaFuncSetAttribute(k_conv3_umma<CO_T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   VG_CUDA(c, cudaFuncSetAttribute(k_conv3_umma<CO_T>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   const int grid = P.ncog * std::min(ctas, P.nxt * P.nyt * P.nz);
-  k_conv3_umma<CO_T><<<(unsigned)grid, kThreads, smem, c->stream>>>(in, wt, out, P, c->dflag);
+  pdl_launch(c->stream, (unsigned)grid, kThreads, smem, k_conv3_umma<CO_T>, in, wt, out, P, c->dflag);
   VG_LAUNCHED(c);
   VG_CUDA(c, cudaGetLastError());
   return VG_OK;

@@ -120,6 +120,7 @@ template <int LW>
 __global__ void __launch_bounds__(kThreads, 1) k_conv3_wgrad_rows(const ConvIn in, const __nv_bfloat16* __restrict__ dy,
                                                                   int Co, float* __restrict__ dw, float* __restrict__ db,
                                                                   int* __restrict__ err) {
+  pdl_entry();
   using S = Shape<LW>;
   constexpr int W = S::W, P = S::P, XR = S::XR;
   constexpr unsigned kXSlab = S::kXSlab;
@@ -369,7 +370,7 @@ vg_status launch_wgrad(Ctx* c, const ConvIn& in, const __nv_bfloat16* dy, int Co
   VG_CUDA(c, cudaFuncSetAttribute(k_conv3_wgrad_rows<LW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem));
   const int blocks = (Co / 16) * ((in.C1 + in.C2) / 16), steps = (in.H / (2 * S::P)) * in.D;
   const int splits = std::max(1, std::min(steps, sm_count() / blocks));
-  k_conv3_wgrad_rows<LW><<<dim3((unsigned)blocks, (unsigned)splits), kThreads, S::smem, c->stream>>>(in, dy, Co, dw, db,
+  pdl_launch(c->stream, dim3((unsigned)blocks, (unsigned)splits), kThreads, S::smem, k_conv3_wgrad_rows<LW>, in, dy, Co, dw, db,
                                                                                                     c->dflag);
   VG_LAUNCHED(c);
   VG_CUDA(c, cudaGetLastError());
