@@ -369,15 +369,19 @@ __global__ void k_sdf_immediate(Geom g, const float* __restrict__ dens, float am
 // floats the lanes of a warp (16 j, 2 k) lie kRow - 1 and kPlane - 1 floats
 // apart: kRow - 1 odd and kPlane - 1 = 16 modulo 32 put all 32 in different
 // banks.  Rows of T + 1 floats without padding made every access 16-way
-// conflicted: 0.3 us a step, 752 us for the two sweeps of a 129^3 grid against
-// 414 us (smaller tiles, with fewer steps but more diagonals, came to 600 us
-// at best in that layout).
+// conflicted: 0.3 us a step, 752 us for the two sweeps of a 129^3 grid; padded
+// 0.12 us and 414 us (smaller tiles, with fewer steps but more diagonals, came to
+// 600 us at best without padding; warps that pass their values on without a
+// barrier to 500 us).  The tile's own points were last written two launches ago
+// or earlier, so they are loaded before the wait for the previous diagonal, whose
+// launch lets this one start as soon as it runs itself: 380 us.  (All loads go
+// past the first-level cache, where a line read before the wait may hold old
+// values of a neighbouring tile.)
 constexpr int kSdfTile = 16;
 constexpr int kSdfThreads = kSdfTile * kSdfTile;  // one thread per (j, k) of a local diagonal plane
 __global__ void __launch_bounds__(kSdfThreads) k_sdf_sweep(Geom g, int diag, int backward, unsigned tiles_x,
                                                            float* __restrict__ sdf,
                                                            const unsigned char* __restrict__ pinned) {
-  pdl_entry();
   constexpr int T = kSdfTile;
   constexpr int kRow = 18, kPlane = 337;  // see above: kRow - 1 odd, kPlane - 1 = 16 modulo 32
   static_assert(T == 16, "rows are half a warp, their pins 16 bits");
@@ -386,6 +390,7 @@ __global__ void __launch_bounds__(kSdfThreads) k_sdf_sweep(Geom g, int diag, int
   const int ty = blockIdx.x, tz = blockIdx.y;
   const int tx = diag - ty - tz;
   if (tx < 0 || tx >= (int)tiles_x) return;
+  if (diag == 0) pdl_entry();  // the tile of the last launch, or no sweep's yet
   const int nx = g.np[0], ny = g.np[1], nz = g.np[2];
   // tile origin in sweep coordinates (distance from the sweep's first point); sweep point (u, v, w) is
   // at first + dx u + dy v + dz w
@@ -406,16 +411,10 @@ __global__ void __launch_bounds__(kSdfThreads) k_sdf_sweep(Geom g, int diag, int
     val[w] = FLT_MAX;
     pv[w] = 1;
     if (in_xy && oz + w < nz) {
-      val[w] = sdf[row + dz * w];
-      pv[w] = pinned[row + dz * w];
+      val[w] = __ldcg(sdf + row + dz * w);
+      pv[w] = __ldcg(pinned + row + dz * w);
     }
   }
-  float sx = FLT_MAX, fy = FLT_MAX, fz = FLT_MAX;
-  if (ox > 0 && oy + j < ny && oz + k < nz) sx = sdf[first + dx * (ox - 1) + dy * (oy + j) + dz * (oz + k)];
-  if (oy > 0 && ox + j < nx && oz + k < nz) fy = sdf[first + dx * (ox + j) + dy * (oy - 1) + dz * (oz + k)];
-  if (oz > 0 && in_xy) fz = sdf[row - dz];
-  S[(k + 1) * kPlane + j + 1] = fy;
-  S[(k + 1) * kRow + j + 1] = fz;
   unsigned mine = 0;  // bit w: this thread's staged element of plane w is updated and written back
 #pragma unroll
   for (int w = 0; w < T; ++w) {
@@ -424,6 +423,14 @@ __global__ void __launch_bounds__(kSdfThreads) k_sdf_sweep(Geom g, int diag, int
     if (j == 0) fixed_row[w * T + k] = (unsigned short)(k & 1 ? rows >> 16 : rows);
     if (!pv[w]) mine |= 1u << w;
   }
+  pdl_entry();
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  float sx = FLT_MAX, fy = FLT_MAX, fz = FLT_MAX;
+  if (ox > 0 && oy + j < ny && oz + k < nz) sx = __ldcg(sdf + first + dx * (ox - 1) + dy * (oy + j) + dz * (oz + k));
+  if (oy > 0 && ox + j < nx && oz + k < nz) fy = __ldcg(sdf + first + dx * (ox + j) + dy * (oy - 1) + dz * (oz + k));
+  if (oz > 0 && in_xy) fz = __ldcg(sdf + row - dz);
+  S[(k + 1) * kPlane + j + 1] = fy;
+  S[(k + 1) * kRow + j + 1] = fz;
   __syncthreads();
   // a thread walks its column (v = j, w = k) along x; its x neighbour is its own last value
   const unsigned fixed = fixed_row[k * T + j];  // pinned, or outside the grid
