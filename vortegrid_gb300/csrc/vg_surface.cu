@@ -66,33 +66,12 @@ __global__ void __launch_bounds__(128) k_density(Geom g, const float4* __restric
   const unsigned nx = g.np[0], ny = g.np[1];
   unsigned X, Y, Z;
   grid_index(k, nx, ny, X, Y, Z);
-  unsigned cur[8], end[8];
-#pragma unroll
-  for (int o = 0; o < 8; ++o) {
-    const unsigned ox = o & 1, oy = (o >> 1) & 1, oz = (o >> 2) & 1;
-    cur[o] = end[o] = 0;
-    if (X >= ox && Y >= oy && Z >= oz) {
-      const size_t c = (X - ox) + (size_t)nx * ((Y - oy) + (size_t)ny * (Z - oz));
-      cur[o] = start[c];
-      end[o] = start[c + 1];
-    }
-  }
+  CellMerge merge(start, items, nx, ny, X, Y, Z);
   float d = 0.f, contrib = 0.f;
   for (;;) {
-    unsigned best = 0xffffffffu;
-    int bo = -1;
-#pragma unroll
-    for (int o = 0; o < 8; ++o) {
-      if (cur[o] < end[o]) {
-        const unsigned v = items[cur[o]];
-        if (v < best) {
-          best = v;
-          bo = o;
-        }
-      }
-    }
+    unsigned best;
+    const int bo = merge.next(items, best);
     if (bo < 0) break;
-    cur[bo]++;
     const float4 p = ps[best];
     const float pp[3] = {p.x, p.y, p.z};
     float tw[3], om[3];

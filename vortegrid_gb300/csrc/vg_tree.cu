@@ -546,37 +546,15 @@ __global__ void __launch_bounds__(128) k_splat(Geom g, const float4* __restrict_
   const float radius = __fmul_rn(ps[0].w, 0.5f);
   const float vorton_volume = __fmul_rn(four_pi_over3, __fmul_rn(__fmul_rn(radius, radius), radius));
   const float corr = __fdiv_rn(__fmul_rn(scale, vorton_volume), cell_volume);
-  const unsigned nx = g.np[0], ny = g.np[1], nz = g.np[2];
+  const unsigned nx = g.np[0], ny = g.np[1];
   unsigned X, Y, Z;
   grid_index(k, nx, ny, X, Y, Z);
-  unsigned cur[8], end[8];
-#pragma unroll
-  for (int o = 0; o < 8; ++o) {
-    const unsigned ox = o & 1, oy = (o >> 1) & 1, oz = (o >> 2) & 1;
-    cur[o] = end[o] = 0;
-    if (X >= ox && Y >= oy && Z >= oz) {
-      const size_t c = (X - ox) + (size_t)nx * ((Y - oy) + (size_t)ny * (Z - oz));
-      cur[o] = start[c];
-      end[o] = start[c + 1];
-    }
-  }
-  (void)nz;
+  CellMerge merge(start, items, nx, ny, X, Y, Z);
   float ax = 0.f, ay = 0.f, az = 0.f;
   for (;;) {
-    unsigned best = 0xffffffffu;
-    int bo = -1;
-#pragma unroll
-    for (int o = 0; o < 8; ++o) {
-      if (cur[o] < end[o]) {
-        const unsigned v = items[cur[o]];
-        if (v < best) {
-          best = v;
-          bo = o;
-        }
-      }
-    }
+    unsigned best;
+    const int bo = merge.next(items, best);
     if (bo < 0) break;
-    cur[bo]++;
     const float4 p = ps[best];
     const float4 a = w[best];
     // Accumulate (uniformGrid.h:1278-1342): this point is corner `bo` of the vorton's cell.
