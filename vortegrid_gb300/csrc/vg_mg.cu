@@ -2418,7 +2418,7 @@ __device__ __forceinline__ void slice_step(Slice& s, unsigned ipr, unsigned ny, 
   s.t += 32u * kPU;
 }
 
-// One colour's Gauss-Seidel half sweep (k_rbgs).
+// One colour's half sweep (k_s_sweep's arithmetic on interleaved fields).
 __device__ void p_rbgs(const Team& tm, const PLev& L, float* e, const float* r, unsigned col) {
   const unsigned nx = L.np[0], ny = L.np[1], sy = 3 * nx, sz = 3 * nx * ny;
   const unsigned ipr = 3 * ((nx - 1) / 2), safe = 3 * (1 + nx * (1 + ny));
@@ -2450,7 +2450,7 @@ __device__ void p_rbgs(const Team& tm, const PLev& L, float* e, const float* r, 
   }
 }
 
-// The first sweep from e = 0, both colours (k_rbgs_first).  Red items load
+// The first sweep from e = 0, both colours (as k_s_first).  Red items load
 // their own r in place of the neighbours they do not use.
 __device__ void p_rbgs_first(const Team& tm, const PLev& L, float* e, const float* r) {
   const unsigned nx = L.np[0], ny = L.np[1], nz = L.np[2], sy = 3 * nx, sz = 3 * nx * ny;
@@ -2563,7 +2563,7 @@ __device__ void p_residual_pair(const Team& tm, const PSim& S, float* r, double*
   if (arr) warp_add2(arr, nullptr, rr, 0.f);
 }
 
-// Fused residual + full-weighting restriction (k_residual_restrict), the
+// Fused residual + full-weighting restriction (as k_s_restrict), the
 // team's CTAs taking its tiles in turn.
 __device__ void p_restrict(const Team& tm, const PLev& F, const PLev& C, const float* e, const float* r, float* rc,
                            float* s_res) {
@@ -2616,7 +2616,7 @@ __device__ void p_restrict(const Team& tm, const PLev& F, const PLev& C, const f
   }
 }
 
-// e_fine += trilinear(e_coarse), one thread per coarse cell (k_prolong_cells).
+// e_fine += trilinear(e_coarse), one thread per coarse cell (as k_s_prolong).
 __device__ void p_prolong(const Team& tm, const PLev& F, const PLev& C, const float* ec, float* ef) {
   const unsigned ncx = C.np[0] - 1, ncy = C.np[1] - 1, cells = ncx * ncy * (C.np[2] - 1);
   const unsigned sy = C.np[0], sz = C.np[0] * C.np[1], fsy = F.np[0], fsz = F.np[0] * F.np[1];

@@ -1,4 +1,5 @@
-// BF16 tensor-core 3x3x3 convolutions for the learned warm start.
+// BF16 tensor-core 3x3x3 convolutions for the learned warm start, mma.sync forms:
+// for the edges that vg_nn_umma.cu and vg_nn_wgrad.cu (tcgen05) do not take.
 //
 // Products are BF16 x BF16 with FP32 accumulation (mma.sync.m16n8k16).
 //
