@@ -342,20 +342,21 @@ __global__ void k_sdf_immediate(Geom g, const float* __restrict__ dens, float am
 // in an order that respects every dependence, so the result is its own bit
 // for bit.
 //
-// Bound by the chain of 3 T - 2 dependent steps in a tile, each a barrier and
-// a shared-memory access by every thread of a diagonal plane.  Thread (j, k)
-// is at x = s - j - k in step s, so with rows of kRow and planes of kPlane
-// floats the lanes of a warp (16 j, 2 k) lie kRow - 1 and kPlane - 1 floats
-// apart: kRow - 1 odd and kPlane - 1 = 16 modulo 32 put all 32 in different
-// banks.  Rows of T + 1 floats without padding made every access 16-way
-// conflicted: 0.3 us a step, 752 us for the two sweeps of a 129^3 grid; padded
-// 0.12 us and 414 us (smaller tiles, with fewer steps but more diagonals, came to
-// 600 us at best without padding; warps that pass their values on without a
-// barrier to 500 us).  The tile's own points were last written two launches ago
-// or earlier, so they are loaded before the wait for the previous diagonal, whose
-// launch lets this one start as soon as it runs itself: 380 us.  (All loads go
-// past the first-level cache, where a line read before the wait may hold old
-// values of a neighbouring tile.)
+// Bound by the chain of 3 T - 2 dependent diagonal planes in a tile.  Thread (j, k)
+// walks its row along x, two planes to a barrier: its first point (x = a) has its
+// neighbours from before the barrier, its second point's y and z neighbours are
+// other threads' first points, which it works out itself from what those had
+// before the barrier.  A barrier to every plane took 0.12 us a plane.  The lanes of
+// a warp (16 j, 2 k) lie kRow - 1 and kPlane - 1 floats apart: kRow - 1 odd and
+// kPlane - 1 = 16 modulo 32 put all 32 in different banks (rows of T + 1 floats
+// without padding, every access 16-way conflicted, made a plane 0.3 us).  The
+// tile's own points were last written two launches ago or earlier, so they are
+// loaded before the wait for the previous diagonal, whose launch lets this one
+// start as soon as it runs itself.  (All loads go past the first-level cache, where
+// a line read before the wait may hold old values of a neighbouring tile.)  Two
+// sweeps of a 129^3 grid: 752 us unpadded, 414 padded, 380 loaded ahead, now 340.
+// Smaller tiles, with fewer planes but more diagonals, and warps that pass their
+// values on without a barrier were slower.
 constexpr int kSdfTile = 16;
 constexpr int kSdfThreads = kSdfTile * kSdfTile;  // one thread per (j, k) of a local diagonal plane
 __global__ void __launch_bounds__(kSdfThreads) k_sdf_sweep(Geom g, int diag, int backward, unsigned tiles_x,
@@ -364,7 +365,8 @@ __global__ void __launch_bounds__(kSdfThreads) k_sdf_sweep(Geom g, int diag, int
   constexpr int T = kSdfTile;
   constexpr int kRow = 18, kPlane = 337;  // see above: kRow - 1 odd, kPlane - 1 = 16 modulo 32
   static_assert(T == 16, "rows are half a warp, their pins 16 bits");
-  __shared__ float S[(T + 1) * kPlane];  // S[(w + 1) kPlane + (v + 1) kRow + u + 1], u, v, w in [-1, T)
+  // [(w + 1) kPlane + (v + 1) kRow + u + 1], u, v, w in [-1, T): the values so far, and those before the sweep
+  __shared__ float S[(T + 1) * kPlane], S0[(T + 1) * kPlane];
   __shared__ unsigned short fixed_row[T * T];
   const int ty = blockIdx.x, tz = blockIdx.y;
   const int tx = diag - ty - tz;
@@ -397,36 +399,47 @@ __global__ void __launch_bounds__(kSdfThreads) k_sdf_sweep(Geom g, int diag, int
   unsigned mine = 0;  // bit w: this thread's staged element of plane w is updated and written back
 #pragma unroll
   for (int w = 0; w < T; ++w) {
-    S[(w + 1) * kPlane + (k + 1) * kRow + j + 1] = val[w];
+    S[(w + 1) * kPlane + (k + 1) * kRow + j + 1] = S0[(w + 1) * kPlane + (k + 1) * kRow + j + 1] = val[w];
     const unsigned rows = __ballot_sync(0xffffffffu, pv[w]);  // two rows of 16 points
     if (j == 0) fixed_row[w * T + k] = (unsigned short)(k & 1 ? rows >> 16 : rows);
     if (!pv[w]) mine |= 1u << w;
   }
   pdl_entry();
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  float sx = FLT_MAX, fy = FLT_MAX, fz = FLT_MAX;
-  if (ox > 0 && oy + j < ny && oz + k < nz) sx = __ldcg(sdf + first + dx * (ox - 1) + dy * (oy + j) + dz * (oz + k));
+  float last = FLT_MAX, fy = FLT_MAX, fz = FLT_MAX;  // last: the x neighbour of the row's next point
+  if (ox > 0 && oy + j < ny && oz + k < nz) last = __ldcg(sdf + first + dx * (ox - 1) + dy * (oy + j) + dz * (oz + k));
   if (oy > 0 && ox + j < nx && oz + k < nz) fy = __ldcg(sdf + first + dx * (ox + j) + dy * (oy - 1) + dz * (oz + k));
   if (oz > 0 && in_xy) fz = __ldcg(sdf + row - dz);
-  S[(k + 1) * kPlane + j + 1] = fy;
-  S[(k + 1) * kRow + j + 1] = fz;
+  S[(k + 1) * kPlane + (j + 1) * kRow] = last;
+  S[(k + 1) * kPlane + j + 1] = S0[(k + 1) * kPlane + j + 1] = fy;
+  S[(k + 1) * kRow + j + 1] = S0[(k + 1) * kRow + j + 1] = fz;
   __syncthreads();
-  // a thread walks its column (v = j, w = k) along x; its x neighbour is its own last value
-  const unsigned fixed = fixed_row[k * T + j];  // pinned, or outside the grid
+  // rows (j, k), (j - 1, k) and (j, k - 1): the points not updated (pinned, outside the grid; a face's are none of the tile's)
+  const unsigned fixed = fixed_row[k * T + j], fixed_y = j ? fixed_row[k * T + j - 1] : 0xffffu,
+                 fixed_z = k ? fixed_row[(k - 1) * T + j] : 0xffffu;
   float* col = S + (k + 1) * kPlane + (j + 1) * kRow + 1;
-  for (int s = 0; s <= 3 * (T - 1); ++s) {
-    // points (i, j, k) of the tile with i + j + k = s
-    const int i = s - j - k;
-    if (i >= 0 && i < T) {
-      float here = col[i];
-      const float syv = col[i - kRow], szv = col[i - kPlane];
-      const bool x_first = fabsf(sx) <= fabsf(syv);
-      const float xy = x_first ? sx : syv, sp_xy = x_first ? g.cell[0] : g.cell[1];
-      const bool xy_first = fabsf(xy) <= fabsf(szv);
-      const float nb = xy_first ? xy : szv, sp = xy_first ? sp_xy : g.cell[2];
-      const float cand = __fadd_rn(nb, copysignf(sp, nb));
-      if (!((fixed >> i) & 1u) && fabsf(cand) < fabsf(here)) col[i] = here = cand;
-      sx = here;
+  const float* col0 = S0 + (k + 1) * kPlane + (j + 1) * kRow + 1;
+  const int two_z = k ? 2 * kPlane : kPlane;
+  auto update = [&](float xv, float yv, float zv, float here, bool is_fixed) {
+    const bool x_first = fabsf(xv) <= fabsf(yv);
+    const float xy = x_first ? xv : yv, sp_xy = x_first ? g.cell[0] : g.cell[1];
+    const bool xy_first = fabsf(xy) <= fabsf(zv);
+    const float nb = xy_first ? xy : zv, sp = xy_first ? sp_xy : g.cell[2];
+    const float cand = __fadd_rn(nb, copysignf(sp, nb));
+    return !is_fixed && fabsf(cand) < fabsf(here) ? cand : here;
+  };
+  for (int step = 0; step <= 3 * (T - 1); step += 2) {
+    // points a and b of row (j, k), on the diagonal planes step and step + 1
+    const int a = step - j - k, b = min(a + 1, T - 1);
+    if (a >= -1 && a < T) {
+      const float y_a = col[a - kRow], z_a = col[a - kPlane];
+      const float yy_b = col[b - 2 * kRow], yz_b = col[b - kRow - kPlane], zz_b = col[b - two_z];
+      const float here_a = col0[a], here_b = col0[b], here_y = col0[b - kRow], here_z = col0[b - kPlane];
+      // b's y and z neighbours, which their own threads update only now
+      const float y_b = update(y_a, yy_b, yz_b, here_y, (fixed_y >> b) & 1u);
+      const float z_b = update(z_a, yz_b, zz_b, here_z, (fixed_z >> b) & 1u);
+      if (a >= 0) col[a] = last = update(last, y_a, z_a, here_a, (fixed >> a) & 1u);
+      if (a + 1 < T) col[b] = last = update(last, y_b, z_b, here_b, (fixed >> b) & 1u);
     }
     __syncthreads();
   }
