@@ -862,7 +862,7 @@ static bool graph_step_possible(Ctx* c) {
 
 static vg_status step_records_body(vg_ctx* c, void* particles, size_t n, size_t stride, const float* extra_min,
                                    const float* extra_max, float dt, bool evolve, bool whole, size_t pitch,
-                                   unsigned char* stage, float4* ps, float4* w, float4* vel, bool pack_on_aux);
+                                   unsigned char* stage, float4* ps, float4* w, float4* vel, const TracerJob* tj);
 
 // vg_step, vg_step_evolve and vg_step_advect on host records (evolve: the
 // vortons move by velocity x dt before the records go back; tj: tracer
@@ -898,16 +898,8 @@ static vg_status step_records(vg_ctx* c, void* particles, size_t n, size_t strid
   }
   const char* what = tj ? "vg_step_advect" : evolve ? "vg_step_evolve" : "vg_step";
   auto enqueue = [&]() -> vg_status {
-    if (tj) {
-      // the tracer records go up on the second stream while the vortons step
-      // (after whatever the context's stream already holds)
-      VG_CUDA(c, cudaEventRecord(c->aux_ev0, c->stream));
-      VG_CUDA(c, cudaStreamWaitEvent(c->aux, c->aux_ev0, 0));
-      VG_CUDA(c, tracer_upload(*tj, c->aux));
-      VG_CUDA(c, cudaEventRecord(c->aux_ev1, c->aux));
-    }
     vg_status est = step_records_body(c, particles, n, stride, extra_min, extra_max, dt, evolve, whole, pitch, stage,
-                                      ps, w, vel, tj != nullptr);
+                                      ps, w, vel, tj);
     if (est == VG_OK && tj) {
       VG_CUDA(c, cudaStreamWaitEvent(c->stream, c->aux_ev1, 0));
       est = tracer_advect_enqueue(c, *tj, dt);
@@ -979,23 +971,31 @@ static vg_status step_records(vg_ctx* c, void* particles, size_t n, size_t strid
 // The vortons' part of step_records, enqueued on the context's stream.
 static vg_status step_records_body(vg_ctx* c, void* particles, size_t n, size_t stride, const float* extra_min,
                                    const float* extra_max, float dt, bool evolve, bool whole, size_t pitch,
-                                   unsigned char* stage, float4* ps, float4* w, float4* vel, bool pack_on_aux) {
+                                   unsigned char* stage, float4* ps, float4* w, float4* vel, const TracerJob* tj) {
   vg_status st = VG_OK;
   // record bytes [0, 56): position, velocity, orientation, angular velocity, density, size
   if (whole)
     VG_CUDA(c, cudaMemcpyAsync(stage, particles, n * stride, cudaMemcpyHostToDevice, c->stream));
   else
     VG_CUDA(c, cudaMemcpy2DAsync(stage, 56, particles, stride, 56, n, cudaMemcpyHostToDevice, c->stream));
+  if (tj) {
+    // the tracer records go up on the second stream while the vortons step, after the vortons' records: the copies
+    // share an engine, and with the tracers' first (65,536: 32 us) the step began after them
+    VG_CUDA(c, cudaEventRecord(c->aux_ev0, c->stream));
+    VG_CUDA(c, cudaStreamWaitEvent(c->aux, c->aux_ev0, 0));
+    VG_CUDA(c, tracer_upload(*tj, c->aux));
+    VG_CUDA(c, cudaEventRecord(c->aux_ev1, c->aux));
+  }
   pdl_launch(c->stream, blocks_for(n, 256), 256, 0, k_unpack_records, stage, pitch, (int)n, ps, w);
   VG_CUDA(c, cudaGetLastError());
   const float* rec0 = (const float*)particles;
   const float radius = rec0[13] * 0.5f;  // Particle::GetRadius of the first vorton
   st = run_step(c, ps, w, vel, n, rec0, radius, extra_min, extra_max, dt);
   if (st != VG_OK) return st;
-  // pack_on_aux: the vortons' records go back on the second stream while the
+  // with tracers the vortons' records go back on the second stream while the
   // tracers are advected on the first (aux_ev3 marks their return)
   cudaStream_t ps_stream = c->stream;
-  if (pack_on_aux) {
+  if (tj) {
     VG_CUDA(c, cudaEventRecord(c->aux_ev2, c->stream));
     VG_CUDA(c, cudaStreamWaitEvent(c->aux, c->aux_ev2, 0));
     ps_stream = c->aux;
@@ -1015,7 +1015,7 @@ static vg_status step_records_body(vg_ctx* c, void* particles, size_t n, size_t 
   else
     VG_CUDA(c, cudaMemcpy2DAsync((unsigned char*)particles + from, stride, stage + from, 56, 48 - from, n,
                                  cudaMemcpyDeviceToHost, ps_stream));
-  if (pack_on_aux) VG_CUDA(c, cudaEventRecord(c->aux_ev3, c->aux));
+  if (tj) VG_CUDA(c, cudaEventRecord(c->aux_ev3, c->aux));
   return VG_OK;
 }
 
