@@ -558,8 +558,8 @@ __global__ void __launch_bounds__(256) k_gather_advect_points(Geom g, const floa
                                                               float4* __restrict__ pos, float4* __restrict__ vel,
                                                               int m, float dt, int evolve, int* __restrict__ flag) {
   pdl_entry();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool valid = i < m;  // all lanes take part in the exchanges
+  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool valid = i < (unsigned)m;  // all lanes take part in the exchanges
   float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
   if (valid) p = pos[i];
   const bool inside = valid && inside_cells(g, p.x, p.y, p.z);
@@ -636,7 +636,7 @@ __global__ void __launch_bounds__(kBoxThreads) k_bbox(const float4* __restrict__
   pdl_entry();
   __shared__ unsigned sh[kBoxThreads / 32][6];
   float mn[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, mx[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < (unsigned)n; i += gridDim.x * blockDim.x) {
     const float4 p = pos[i];
     if (!(isfinite(p.x) && isfinite(p.y) && isfinite(p.z))) atomicOr(flag, (int)DF_NONFINITE);
     mn[0] = fminf(mn[0], p.x); mn[1] = fminf(mn[1], p.y); mn[2] = fminf(mn[2], p.z);

@@ -30,8 +30,8 @@ namespace {
 __global__ void k_bin(Geom g, const float4* __restrict__ pos, int n, unsigned* __restrict__ key,
                       unsigned* __restrict__ place, unsigned* __restrict__ count, unsigned ncells) {
   pdl_entry();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool valid = i < n;
+  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;  // n may be within a block of 2^31
+  const bool valid = i < (unsigned)n;
   unsigned off = 0xffffffffu;
   if (valid) {
     const float4 p = pos[i];
@@ -150,10 +150,10 @@ constexpr unsigned kMidCtas = 304, kBigCtas = 152;
 __global__ void k_place(int n, const unsigned* __restrict__ key, const unsigned* __restrict__ place,
                         const unsigned* __restrict__ start, uint2* __restrict__ slot) {
   pdl_entry();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= (unsigned)n) return;
   const unsigned k = key[i];
-  slot[start[k] + place[i]] = make_uint2(k, (unsigned)i);
+  slot[start[k] + place[i]] = make_uint2(k, i);
 }
 
 // big[0], big[1]: the numbers of mid and big cells; their offsets follow, mid ones from mid_list, big ones from big_list.
@@ -161,8 +161,8 @@ __global__ void k_order(int n, const uint2* __restrict__ slot, const unsigned* _
                         unsigned* __restrict__ items, unsigned* __restrict__ big, unsigned* __restrict__ mid_list,
                         unsigned* __restrict__ big_list) {
   pdl_entry();
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= n) return;
+  const unsigned p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= (unsigned)n) return;
   const uint2 me = slot[p];
   const unsigned s = start[me.x], e = start[me.x + 1], m = e - s;
   if (m <= kCountMax) {
@@ -171,7 +171,7 @@ __global__ void k_order(int n, const uint2* __restrict__ slot, const unsigned* _
 #pragma unroll 4
       for (unsigned q = s; q < e; ++q) rank += slot[q].y < me.y;
     items[s + rank] = me.y;
-  } else if ((unsigned)p == s) {
+  } else if (p == s) {
     if (m <= kSortMax)
       mid_list[atomicAdd(&big[0], 1u)] = me.x;
     else
