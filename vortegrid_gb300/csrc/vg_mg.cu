@@ -623,27 +623,28 @@ __global__ void __launch_bounds__(256) k_s_prolong(SGeo g, SGeo C, const float* 
 }
 
 // Block sums of two values into part[2 b + {0, 1}], as block_sum2, for any whole number of warps.
+template <bool kBoth>
 __device__ __forceinline__ void split_sum2(float a32, float b32, double* __restrict__ part) {
   __shared__ double s_a[8], s_b[8];
   const unsigned tid = threadIdx.x + blockDim.x * threadIdx.y, warps = blockDim.x * blockDim.y / 32;
   for (int o = 16; o > 0; o >>= 1) {
     a32 += __shfl_xor_sync(0xffffffffu, a32, o);
-    b32 += __shfl_xor_sync(0xffffffffu, b32, o);
+    if (kBoth) b32 += __shfl_xor_sync(0xffffffffu, b32, o);
   }
   if ((tid & 31) == 0) {
     s_a[tid >> 5] = (double)a32;
-    s_b[tid >> 5] = (double)b32;
+    if (kBoth) s_b[tid >> 5] = (double)b32;
   }
   __syncthreads();
   if (tid == 0) {
     double t1 = 0.0, t2 = 0.0;
     for (unsigned w = 0; w < warps; ++w) {
       t1 += s_a[w];
-      t2 += s_b[w];
+      if (kBoth) t2 += s_b[w];
     }
     const unsigned b = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
     part[2 * b] = t1;
-    part[2 * b + 1] = t2;
+    if (kBoth) part[2 * b + 1] = t2;
   }
 }
 
@@ -652,24 +653,27 @@ __device__ __forceinline__ void split_sum2(float a32, float b32, double* __restr
 // only when they belong together and no fence is needed between them.  A copy and a stream wait took 15 to 20 us a norm
 // more.  (Summing in the residual kernels by their last block, instead of this launch, made them 4 to 10 us longer: a fence
 // and an atomic at every block's end.)
-__global__ void __launch_bounds__(1024) k_s_norm(const double* __restrict__ part, int nb, double* __restrict__ out2,
+// Bound by FP64 additions, 16 cycles a warp: 1,024 threads with five additions each in the trees took 6.6 us at 129^3 and
+// 5.1 at 33^3, 256 threads take 4.5 and 3.0 (128 threads the same at 129^3).
+constexpr int kNormThreads = 256;
+__global__ void __launch_bounds__(kNormThreads) k_s_norm(const double* __restrict__ part, int nb, double* __restrict__ out2,
                                                  int keep_b, unsigned long long* __restrict__ seq,
                                                  unsigned long long seq0, volatile unsigned long long* host) {
   pdl_entry();
-  __shared__ double s1[32], s2[32];
+  __shared__ double s1[kNormThreads / 32], s2[kNormThreads / 32];
   double a1 = 0.0, a2 = 0.0, b2 = 0.0;
   unsigned long long number = 0;
   if (threadIdx.x == 0) {
     if (keep_b) b2 = out2[1];
     if (host) number = (keep_b ? *seq : seq0) + 1;  // the first norm of a solve is the one that sets b^2
   }
-  for (int i = threadIdx.x; i < nb; i += 1024) {
+  for (int i = threadIdx.x; i < nb; i += kNormThreads) {
     a1 += part[2 * i];
-    a2 += part[2 * i + 1];
+    if (!keep_b) a2 += part[2 * i + 1];
   }
   for (int o = 16; o > 0; o >>= 1) {
     a1 += __shfl_xor_sync(0xffffffffu, a1, o);
-    a2 += __shfl_xor_sync(0xffffffffu, a2, o);
+    if (!keep_b) a2 += __shfl_xor_sync(0xffffffffu, a2, o);
   }
   if ((threadIdx.x & 31) == 0) {
     s1[threadIdx.x >> 5] = a1;
@@ -677,11 +681,12 @@ __global__ void __launch_bounds__(1024) k_s_norm(const double* __restrict__ part
   }
   __syncthreads();
   if (threadIdx.x >= 32) return;
-  a1 = s1[threadIdx.x];
-  a2 = s2[threadIdx.x];
-  for (int o = 16; o > 0; o >>= 1) {
+  a1 = threadIdx.x < kNormThreads / 32 ? s1[threadIdx.x] : 0.0;
+  a2 = threadIdx.x < kNormThreads / 32 ? s2[threadIdx.x] : 0.0;
+#pragma unroll
+  for (int o = kNormThreads / 64; o > 0; o >>= 1) {
     a1 += __shfl_xor_sync(0xffffffffu, a1, o);
-    a2 += __shfl_xor_sync(0xffffffffu, a2, o);
+    if (!keep_b) a2 += __shfl_xor_sync(0xffffffffu, a2, o);
   }
   if (threadIdx.x) return;
   if (keep_b) a2 = b2;
@@ -757,11 +762,11 @@ __global__ void __launch_bounds__(256) k_s_residual(SGeo g, const float* __restr
         ro[k] = __fsub_rn(abo[k], lap7(ov[k + 1], ev[k + 1], ev[k], oy1[k], oy0[k], aop[k], aom[k], g.r2x, g.r2y, g.r2z));
         if (kNorm && x_interior(g, 0, i0 + k)) {
           rr = fmaf(re[k], re[k], rr);
-          bb = fmaf(abe[k], abe[k], bb);
+          if (kField == RES_X) bb = fmaf(abe[k], abe[k], bb);
         }
         if (kNorm && x_interior(g, 1, i0 + k)) {
           rr = fmaf(ro[k], ro[k], rr);
-          bb = fmaf(abo[k], abo[k], bb);
+          if (kField == RES_X) bb = fmaf(abo[k], abo[k], bb);
         }
       }
       st4(r + ec, make_float4(re[0], re[1], re[2], re[3]));
@@ -783,7 +788,7 @@ __global__ void __launch_bounds__(256) k_s_residual(SGeo g, const float* __restr
       ec = cs - ec;
     }
   }
-  if (kNorm) split_sum2(rr, bb, part);
+  if (kNorm) split_sum2<kField == RES_X>(rr, bb, part);  // ||b||^2 is asked of a solve's first residual only
 }
 
 // The refinement residual r = b - L (hi + lo) to FP64-class accuracy (pair_residual), with hi = x or x + e (then written to
@@ -839,7 +844,7 @@ __global__ void __launch_bounds__(256) k_s_residual_pair(SGeo g, PairCoef cf, co
       }
     }
   }
-  split_sum2(rr, 0.f, part);
+  split_sum2<false>(rr, 0.f, part);
 }
 
 // a += b over split fields (n4 float4 groups).
@@ -1417,7 +1422,7 @@ struct MgBufs {
 };
 
 static void enqueue_norm(Ctx* c, const MgBufs& B, int keep_b, unsigned* nl) {
-  pdl_launch(c->stream, 1, 1024, 0, k_s_norm, (const double*)B.part, (int)B.nb0, B.sums, keep_b, B.seq, c->norm_seq,
+  pdl_launch(c->stream, 1, kNormThreads, 0, k_s_norm, (const double*)B.part, (int)B.nb0, B.sums, keep_b, B.seq, c->norm_seq,
              (volatile unsigned long long*)B.host);
   ++*nl;
 }
