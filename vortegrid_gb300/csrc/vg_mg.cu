@@ -240,33 +240,6 @@ __global__ void __launch_bounds__(kRedThreads) k_residual_pair(Geom g, PairCoef 
   block_sum2(rr, 0.f, part);
 }
 
-// Sum the per-block partials in a fixed order (one block); with keep_b the
-// ||b||^2 slot is left as phase 1's first residual wrote it.
-__global__ void __launch_bounds__(1024) k_sum_partials(const double* __restrict__ part, int nb,
-                                                       double* __restrict__ out2, int keep_b) {
-  pdl_entry();
-  __shared__ double s1[1024], s2[1024];
-  double a1 = 0.0, a2 = 0.0;
-  for (int i = threadIdx.x; i < nb; i += blockDim.x) {
-    a1 += part[2 * i];
-    a2 += part[2 * i + 1];
-  }
-  s1[threadIdx.x] = a1;
-  s2[threadIdx.x] = a2;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if ((int)threadIdx.x < s) {
-      s1[threadIdx.x] += s1[threadIdx.x + s];
-      s2[threadIdx.x] += s2[threadIdx.x + s];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    out2[0] = s1[0];
-    if (!keep_b) out2[1] = s2[0];
-  }
-}
-
 __device__ __forceinline__ void rbgs_point(const Geom& g, float r2x, float r2y, float r2z, float H,
                                            float* __restrict__ e, const float* __restrict__ r, size_t k,
                                            bool zero_first) {
@@ -2066,16 +2039,15 @@ vg_status run_multigrid_fixed(Ctx* c, const Geom& g, float* soln3, const float* 
   vg_status st = setup_bufs(c, g, P, B, &etot, &rir);
   if (st != VG_OK) return st;
   const size_t n0 = g.points();
-  const unsigned nb0 = B.nb0;
   const Lev& L0 = P.lev[0];
   const PairCoef cf = pair_coef(g, L0);
   unsigned nl = 0;
   VG_CUDA(c, cudaMemsetAsync(B.E, 0, P.total * 3 * sizeof(float), c->stream));
   pdl_launch(c->stream, B.rl.grid, B.rl.block, 0, k_residual32n, g, L0.r2x, L0.r2y, L0.r2z, B.rl.zs, soln3, rhs3, B.R,
                                                          B.part);
-  pdl_launch(c->stream, 1, 1024, 0, k_sum_partials, B.part, (int)nb0, B.sums, 0);
+  enqueue_norm(c, B, 0, &nl);
   pdl_launch(c->stream, 1, 32, 0, k_relres, B.sums, c->mg_relres_dev + 1);
-  nl += 3;
+  nl += 2;
   for (int k = 0; k < c->mg_fixed_k1; ++k)
     if ((st = enqueue_cycle(c, P, g, B, soln3, rhs3, &nl, k + 1 < c->mg_fixed_k1 ? TAIL_RESIDUAL : TAIL_NONE)) != VG_OK)
       return st;
@@ -2087,14 +2059,14 @@ vg_status run_multigrid_fixed(Ctx* c, const Geom& g, float* soln3, const float* 
     // same float operations on the same values (0 + e = e exactly).
     pdl_launch(c->stream, B.rl.grid, B.rl.block, 0, k_residual_pair<false>, g, cf, B.rl.zs, (const float*)soln3,
                (const float*)nullptr, rhs3, c->mg_fixed_k2 ? B.R : rir, B.part);
-    pdl_launch(c->stream, 1, 1024, 0, k_sum_partials, B.part, (int)nb0, B.sums, 1);
-    nl += 2;
+    enqueue_norm(c, B, 1, &nl);
+    ++nl;
     if (c->mg_fixed_k2 == 1) {
       if ((st = enqueue_cycle(c, P, g, B, nullptr, rhs3, &nl, TAIL_NONE)) != VG_OK) return st;
       pdl_launch(c->stream, B.rl.grid, B.rl.block, 0, k_residual_pair<true>, g, cf, B.rl.zs, (const float*)soln3,
                  (const float*)B.E, rhs3, rir, B.part);
-      pdl_launch(c->stream, 1, 1024, 0, k_sum_partials, B.part, (int)nb0, B.sums, 1);
-      nl += 2;
+      enqueue_norm(c, B, 1, &nl);
+      ++nl;
     }
     pdl_launch(c->stream, 1, 32, 0, k_relres, B.sums, c->mg_relres_dev);
     ++nl;
@@ -2108,8 +2080,8 @@ vg_status run_multigrid_fixed(Ctx* c, const Geom& g, float* soln3, const float* 
   }
   VG_CUDA(c, cudaMemsetAsync(B.lo, 0, 3 * n0 * sizeof(float), c->stream));
   pdl_launch(c->stream, B.rl.grid, B.rl.block, 0, k_residual_pair<true>, g, cf, B.rl.zs, soln3, B.lo, rhs3, rir, B.part);
-  pdl_launch(c->stream, 1, 1024, 0, k_sum_partials, B.part, (int)nb0, B.sums, 1);
-  nl += 3;
+  enqueue_norm(c, B, 1, &nl);
+  nl += 2;
   if (c->mg_fixed_k2 > 0) {
     VG_CUDA(c, cudaMemsetAsync(etot, 0, 3 * n0 * sizeof(float), c->stream));
     VG_CUDA(c, cudaMemcpyAsync(B.R, rir, 3 * n0 * sizeof(float), cudaMemcpyDeviceToDevice, c->stream));
@@ -2119,8 +2091,8 @@ vg_status run_multigrid_fixed(Ctx* c, const Geom& g, float* soln3, const float* 
         return st;
     add_f32(c, B.lo, etot, 3 * n0);
     pdl_launch(c->stream, B.rl.grid, B.rl.block, 0, k_residual_pair<true>, g, cf, B.rl.zs, soln3, B.lo, rhs3, rir, B.part);
-    pdl_launch(c->stream, 1, 1024, 0, k_sum_partials, B.part, (int)nb0, B.sums, 1);
-    nl += 3;
+    enqueue_norm(c, B, 1, &nl);
+    nl += 2;
   }
   pdl_launch(c->stream, 1, 32, 0, k_relres, B.sums, c->mg_relres_dev);
   add_f32(c, soln3, B.lo, 3 * n0);
