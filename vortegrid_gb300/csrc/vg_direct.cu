@@ -123,6 +123,11 @@ __global__ void __launch_bounds__(kThreads) k_direct_fast(const float4* __restri
 
 constexpr int kPairTPT = 8;
 constexpr int kPairThreads = 256;
+// Sources of k_direct_pair's shared-memory tile (80 bytes each), or all of a
+// CTA's where there are fewer.  32,768 sources and 200,003 targets: 3,520 us with
+// tiles of 256, 3,516 of 512, 3,512 of 1,392.  The memory is dynamic: as a static
+// array of 256 the same loop took 3,732 us (one of its 128 registers spilled).
+constexpr int kPairTile = 512;
 
 // How a k_direct_pair launch divides its targets and sources.  Targets
 // [0, pts) may be the points of a grid: in the first `rows` grid rows (as
@@ -142,6 +147,7 @@ struct PairPlan {
   int row_ctas, row_ks, row_chunk;
   int pts, m;             // targets: grid points [0, pts), then qg[0, m - pts)
   int gen_ctas, gen_ks, gen_chunk;
+  int tile;               // sources of a shared-memory tile
 };
 
 // Position of the gridpoint (x, y, z): the velocity step's gridpoint positions,
@@ -214,8 +220,8 @@ __device__ __forceinline__ void pair_general(const float4* __restrict__ ps, cons
   }
   const int k0 = kc * P.gen_chunk;
   const int k1 = min(n, k0 + P.gen_chunk);
-  for (int tile = k0; tile < k1; tile += kTile) {
-    const int cnt = min(kTile, k1 - tile);
+  for (int tile = k0; tile < k1; tile += P.tile) {
+    const int cnt = min(P.tile, k1 - tile);
     __syncthreads();
     stage_pair_tile(ps, w, tile, cnt, sr, sc, sh);
     __syncthreads();
@@ -286,8 +292,8 @@ __device__ __forceinline__ void pair_rows(const float4* __restrict__ ps, const f
   const float2 qy = make_float2(qyv, qyv), qz = make_float2(qzv, qzv);
   const int k0 = kc * P.row_chunk;
   const int k1 = min(n, k0 + P.row_chunk);
-  for (int tile = k0; tile < k1; tile += kTile) {
-    const int cnt = min(kTile, k1 - tile);
+  for (int tile = k0; tile < k1; tile += P.tile) {
+    const int cnt = min(P.tile, k1 - tile);
     __syncthreads();
     stage_pair_tile(ps, w, tile, cnt, sr, sc, sh);
     __syncthreads();
@@ -351,7 +357,7 @@ __global__ void __launch_bounds__(kPairThreads, 2)
                   const float4* __restrict__ qg, PairPlan P, float* __restrict__ partial_rows,
                   float* __restrict__ partial_gen, float4* __restrict__ out) {
   pdl_entry();
-  __shared__ float4 sh[5 * kTile];
+  extern __shared__ float4 sh[];
   const int row_total = P.row_ctas * P.row_ks;
   if ((int)blockIdx.x < row_total)
     pair_rows(ps, w, n, sr, sc, P, (int)blockIdx.x, sh, partial_rows, out);
@@ -512,6 +518,11 @@ int direct_split(int kind, size_t n, size_t m, unsigned* tblocks_out, unsigned* 
 // CTA's time is its chunk length times the class's packed operations per
 // source and thread (row CTAs 8 + 4 x 9 = 44, general CTAs 4 x 17 = 68), plus
 // a fixed set-up; more chunks cost more partial sums to reduce.
+void set_tile(PairPlan& P) {
+  const int longest = std::max(P.row_ctas ? P.row_chunk : 1, P.gen_ctas ? P.gen_chunk : 1);
+  P.tile = std::min(kPairTile, longest);
+}
+
 PairPlan plan_pair(size_t n, size_t m, const Geom* grid) {
   PairPlan P = {};
   if (grid) {
@@ -562,6 +573,7 @@ PairPlan plan_pair(size_t n, size_t m, const Geom* grid) {
   P.row_ks = P.row_ctas ? (int)((n + P.row_chunk - 1) / P.row_chunk) : 1;
   P.gen_chunk = (int)((n + kg - 1) / kg);
   P.gen_ks = P.gen_ctas ? (int)((n + P.gen_chunk - 1) / P.gen_chunk) : 1;
+  set_tile(P);
   return P;
 }
 
@@ -574,9 +586,10 @@ cudaError_t launch_pair_plan(Launch launch, const PairPlan& P, const float4* ps,
   float* pr = reduce ? partial : nullptr;
   float* pg = reduce ? partial + (P.row_ctas ? (size_t)P.row_ks * P.pts * 4 : 0) : nullptr;
   const unsigned ctas = (unsigned)(P.row_ctas * P.row_ks + P.gen_ctas * P.gen_ks);
-  cudaError_t e = launch(dim3(ctas), dim3(kPairThreads), k_direct_pair, ps, w, n, sr, sc, qg, P, pr, pg, out);
+  cudaError_t e = launch(dim3(ctas), dim3(kPairThreads), (size_t)5 * P.tile * sizeof(float4), k_direct_pair, ps, w, n, sr, sc, qg, P,
+             pr, pg, out);
   if (e != cudaSuccess || !reduce) return e;
-  return launch(dim3(blocks_for((size_t)P.m, 128)), dim3(128), k_reduce_pair, (const float4*)pr, (const float*)pg,
+  return launch(dim3(blocks_for((size_t)P.m, 128)), dim3(128), 0, k_reduce_pair, (const float4*)pr, (const float*)pg,
                 P, out, split ? split->grid3 : (float*)nullptr, split ? (int)split->pts : 0,
                 split ? split->vel : (float4*)nullptr, split ? split->evolve_pos : (float4*)nullptr,
                 split ? split->evolve_dt : 0.f);
@@ -623,7 +636,9 @@ vg_status launch_direct(Ctx* c, int kind, bool ref, const float4* ps, const floa
       if (st != VG_OK) return st;
     }
     cudaStream_t s = c->stream;
-    auto launch = [s](dim3 g, dim3 b, auto kernel, auto... args) { return pdl_launch(s, g, b, 0, kernel, args...); };
+    auto launch = [s](dim3 g, dim3 b, size_t smem, auto kernel, auto... args) {
+      return pdl_launch(s, g, b, smem, kernel, args...);
+    };
     const float4* qg = (grid && split->after_grid) ? split->after_grid : q + P.pts;
     VG_CUDA(c, launch_pair_plan(launch, P, ps, w, (int)n, sr, sc, qg, partial, out, split));
     c->launches += reduce ? 2 : 1;
@@ -676,10 +691,11 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratch
 // A plain launch whose own error code is returned (no stream-wide error query
 // that could report, and clear, an error some other code left behind).
 template <typename... KArgs, typename... Args>
-cudaError_t launch_plain(cudaStream_t s, dim3 grid, dim3 block, void (*kernel)(KArgs...), Args... args) {
+cudaError_t launch_plain(cudaStream_t s, dim3 grid, dim3 block, size_t smem, void (*kernel)(KArgs...), Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
@@ -736,6 +752,7 @@ extern "C" vg_status vg_direct_noalloc(void* stream, int kind, const float* pos_
       P.gen_chunk = (int)((n + k - 1) / k);
       P.gen_ks = (int)((n + P.gen_chunk - 1) / P.gen_chunk);
     }
+    set_tile(P);
   } else {
     chunk = direct_split(kind, n, m, &tblocks, &ksplit);
     while (ksplit > 1 && (size_t)ksplit * m * 3 * sizeof(float) > room) {
@@ -754,18 +771,20 @@ extern "C" vg_status vg_direct_noalloc(void* stream, int kind, const float* pos_
   const float4* q = (const float4*)q4;
   float4* out = (float4*)out4;
   if (kind == 0) {
-    auto launch = [st](dim3 g, dim3 b, auto kernel, auto... args) { return launch_plain(st, g, b, kernel, args...); };
+    auto launch = [st](dim3 g, dim3 b, size_t smem, auto kernel, auto... args) {
+      return launch_plain(st, g, b, smem, kernel, args...);
+    };
     e = launch_pair_plan(launch, P, ps, w, (int)n, spread_range, spread_circ, q, partial, out, nullptr);
     if (e != cudaSuccess) return noalloc_fail(e, "k_direct_pair / k_reduce_pair launch");
     return VG_OK;
   }
-  e = launch_plain(st, dim3(blocks_for(n, 256)), dim3(256), k_prep_sources<1>, ps, w, (int)n, spread_range,
+  e = launch_plain(st, dim3(blocks_for(n, 256)), dim3(256), 0, k_prep_sources<1>, ps, w, (int)n, spread_range,
                    spread_circ, s0, s1);
   if (e != cudaSuccess) return noalloc_fail(e, "k_prep_sources launch");
-  e = launch_plain(st, dim3(tblocks, ksplit), dim3(kThreads), k_direct_fast<1>, (const float4*)s0, (const float4*)s1,
+  e = launch_plain(st, dim3(tblocks, ksplit), dim3(kThreads), 0, k_direct_fast<1>, (const float4*)s0, (const float4*)s1,
                    (int)n, chunk, q, (int)m, partial);
   if (e != cudaSuccess) return noalloc_fail(e, "k_direct_fast launch");
-  e = launch_plain(st, dim3(blocks_for(m, 256)), dim3(256), k_reduce_partials, (const float*)partial, (int)ksplit,
+  e = launch_plain(st, dim3(blocks_for(m, 256)), dim3(256), 0, k_reduce_partials, (const float*)partial, (int)ksplit,
                    (int)m, out);
   if (e != cudaSuccess) return noalloc_fail(e, "k_reduce_partials launch");
   return VG_OK;
