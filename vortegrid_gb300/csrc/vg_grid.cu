@@ -322,37 +322,40 @@ __global__ void k_pse_gather(const float4* __restrict__ ps, const float4* __rest
 // as its longest particle, not the sum of its longest lists -- that loads the
 // next one's values before it uses this one's.  Slots ascend with the particles'
 // indices within a cell, so the order of two particles of a cell is that of
-// their slots.  k_pse, 10^6 vortons at 225 x 161 x 193: 177 -> 118 us, 262,144 at
+// their slots.  kLanes neighbouring lanes take a particle's lists in turn; the
+// caller adds their sums (sum_lanes).  k_pse, 10^6 vortons at 225 x 161 x 193: 177 -> 118 us, 262,144 at
 // 129^3: 57 -> 36 us, 32 sets of 32,768: 65 -> 26 us each.
 constexpr int kPseThreads = 128;
-template <bool kAll, typename Load, typename Body>
+template <bool kAll, int kLanes, typename Load, typename Body>
 __device__ __forceinline__ void for_neighbours(int nx, int ny, int nz, int cx, int cy, int cz, unsigned t,
                                                const unsigned* __restrict__ start, const Load& load,
                                                const Body& body) {
-  constexpr int kSide = kAll ? 8 : 4;
-  __shared__ uint2 lists[2 * kSide - 1][kPseThreads];
-  uint2 range[2 * kSide - 1];
+  constexpr int kSide = kAll ? 8 : 4, kLists = 2 * kSide - 1, kMine = (kLists + kLanes - 1) / kLanes;
+  __shared__ uint2 lists[kMine][kPseThreads];
+  uint2 range[kMine];
 #pragma unroll
-  for (int r = 0; r < 2 * kSide - 1; ++r) {
+  for (int q = 0; q < kMine; ++q) {
+    const int r = q * kLanes + (int)(threadIdx.x % kLanes);
     const int s = r < kSide ? -1 : 1, k = r < kSide ? r : r - kSide + 1;
     const int ox = s * (kAll ? (k & 1) : (k == 1)), oy = s * (kAll ? ((k >> 1) & 1) : (k == 2));
     const int oz = s * (kAll ? ((k >> 2) & 1) : (k == 3));
     const int ncx = cx + ox, ncy = cy + oy, ncz = cz + oz;
     // the lower of the two cells has to be one that the reference's loop visits
     const int lx = s == 1 ? cx : ncx, ly = s == 1 ? cy : ncy, lz = s == 1 ? cz : ncz;
-    range[r] = make_uint2(0, 0);
-    if (ncx >= 0 && ncy >= 0 && ncz >= 0 && ncx < nx && ncy < ny && ncz < nz && lx < nx - 1 && ly < ny - 1 &&
-        lz < nz - 1) {
+    range[q] = make_uint2(0, 0);
+    if (r < kLists && ncx >= 0 && ncy >= 0 && ncz >= 0 && ncx < nx && ncy < ny && ncz < nz && lx < nx - 1 &&
+        ly < ny - 1 && lz < nz - 1) {
       const size_t cell = (size_t)ncx + (size_t)nx * ((size_t)ncy + (size_t)ny * ncz);
-      range[r] = make_uint2(start[cell], start[cell + 1]);
+      range[q] = make_uint2(start[cell], start[cell + 1]);
     }
   }
   int cnt = 0, own = 0, lower = 0;  // lists kept, and of them the own cell's, and those up to the lower side's
 #pragma unroll
-  for (int r = 0; r < 2 * kSide - 1; ++r) {
-    if (range[r].x < range[r].y) lists[cnt++][threadIdx.x] = range[r];
+  for (int q = 0; q < kMine; ++q) {
+    const int r = q * kLanes + (int)(threadIdx.x % kLanes);
+    if (range[q].x < range[q].y) lists[cnt++][threadIdx.x] = range[q];
     if (r == 0) own = cnt;
-    if (r == kSide - 1) lower = cnt;
+    if (r < kSide) lower = cnt;
   }
   if (cnt == 0) return;
   int r = 0;
@@ -373,6 +376,22 @@ __device__ __forceinline__ void for_neighbours(int nx, int ny, int nz, int cx, i
   }
 }
 
+// A particle's sum over its lanes, for all of them.
+template <int kLanes>
+__device__ __forceinline__ float sum_lanes(float v) {
+  const unsigned mask = ((1u << kLanes) - 1u) << (threadIdx.x % 32 / kLanes * kLanes);
+#pragma unroll
+  for (int o = 1; o < kLanes; o <<= 1) v += __shfl_xor_sync(mask, v, o);
+  return v;
+}
+
+// Four lanes to a particle where the particles alone do not fill the chip: 3,001
+// vortons 18.2 us with one lane, 7.6 with four; 32,000 in a puff 114 and 48; 32
+// sets of 1,000 to 65,536 at a time 25 and 12 each; but 262,144 36.2 and 38.5 (heat
+// 19.0 and 22.9).
+int pse_lanes(size_t n) { return n < 131072 ? 4 : 1; }
+
+template <int kLanes>
 __global__ void __launch_bounds__(kPseThreads) k_pse(Geom g, const float4* __restrict__ pss, const float4* __restrict__ w0s,
                                              float4* __restrict__ w, int n, const unsigned* __restrict__ start,
                                              const unsigned* __restrict__ items, float nu, float dt) {
@@ -380,7 +399,7 @@ __global__ void __launch_bounds__(kPseThreads) k_pse(Geom g, const float4* __res
   // threads take the vortons in cell order, so a warp's vortons share their
   // neighbour cells and read them contiguously (each vorton's sums are the
   // same whichever thread runs them)
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = (int)(((size_t)blockIdx.x * blockDim.x + threadIdx.x) / kLanes);
   if (t >= n) return;
   const int i = (int)items[t];
   const float4 p = pss[t];
@@ -401,7 +420,7 @@ __global__ void __launch_bounds__(kPseThreads) k_pse(Geom g, const float4* __res
   struct Neighbour {
     float4 p, w;
   };
-  for_neighbours<true>(
+  for_neighbours<true, kLanes>(
       nx, ny, nz, cx, cy, cz, (unsigned)t, start, [&](unsigned slot) { return Neighbour{pss[slot], w0s[slot]}; },
       [&](const Neighbour& v, bool here) {
         const float range = 4.0f * (here ? p.w : v.p.w);
@@ -413,6 +432,10 @@ __global__ void __launch_bounds__(kPseThreads) k_pse(Geom g, const float4* __res
         ay = fmaf(frac, v.w.y - wi.y, ay);
         az = fmaf(frac, v.w.z - wi.z, az);
       });
+  ax = sum_lanes<kLanes>(ax);
+  ay = sum_lanes<kLanes>(ay);
+  az = sum_lanes<kLanes>(az);
+  if (threadIdx.x % kLanes) return;
   float vx = wi.x + ax, vy = wi.y + ay, vz = wi.z + az;
   if (here_ok) {
     const float f = nu * dt;
@@ -440,12 +463,13 @@ __global__ void k_heat_gather(const float4* __restrict__ ps, const float* __rest
   d0s[t] = d[j];
 }
 
+template <int kLanes>
 __global__ void __launch_bounds__(kPseThreads) k_heat_pse(Geom g, const float4* __restrict__ pss, const float* __restrict__ d0s,
                                                   float* __restrict__ d, int n, const unsigned* __restrict__ start,
                                                   const unsigned* __restrict__ items, float kappa, float ambient,
                                                   float dt) {
   pdl_entry();
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = (int)(((size_t)blockIdx.x * blockDim.x + threadIdx.x) / kLanes);
   if (t >= n) return;
   const int i = (int)items[t];
   const float4 p = pss[t];
@@ -465,7 +489,7 @@ __global__ void __launch_bounds__(kPseThreads) k_heat_pse(Geom g, const float4* 
     float4 p;
     float d;
   };
-  for_neighbours<false>(
+  for_neighbours<false, kLanes>(
       nx, ny, nz, cx, cy, cz, (unsigned)t, start, [&](unsigned slot) { return Neighbour{pss[slot], d0s[slot]}; },
       [&](const Neighbour& v, bool here) {
         const float range = 4.0f * (here ? p.w : v.p.w);
@@ -475,6 +499,8 @@ __global__ void __launch_bounds__(kPseThreads) k_heat_pse(Geom g, const float4* 
         const float ratio = fminf(fmaxf(twokdt * law, -0.5f), 0.5f);
         acc = fmaf(ratio, v.d - di, acc);
       });
+  acc = sum_lanes<kLanes>(acc);
+  if (threadIdx.x % kLanes) return;
   float v = di + acc;
   if (here_ok) v += fminf(fmaxf(kappa * dt, -0.5f), 0.5f) * (ambient - v);
   d[i] = v;
@@ -800,8 +826,9 @@ vg_status launch_heat_pse(Ctx* c, const Geom& g, const CellLists& cl, const floa
   float4* pss = (float4*)tmp;
   float* d0s = (float*)(pss + n);
   pdl_launch(c->stream, blocks_for(n, 256), 256, 0, k_heat_gather, ps, density, (int)n, cl.items, pss, d0s);
-  pdl_launch(c->stream, blocks_for(n, kPseThreads), kPseThreads, 0, k_heat_pse, g, pss, d0s, density, (int)n, cl.start, cl.items, kappa,
-                                                        ambient, dt);
+  const int lanes = pse_lanes(n);
+  pdl_launch(c->stream, blocks_for(lanes * n, kPseThreads), kPseThreads, 0, lanes == 4 ? k_heat_pse<4> : k_heat_pse<1>,
+             g, pss, d0s, density, (int)n, cl.start, cl.items, kappa, ambient, dt);
   c->launches += 2;
   VG_CUDA(c, cudaGetLastError());
   return VG_OK;
@@ -815,7 +842,9 @@ vg_status launch_pse(Ctx* c, const Geom& g, const CellLists& cl, const float4* p
   if (st != VG_OK) return st;
   float4* w0s = pss + n;
   pdl_launch(c->stream, blocks_for(n, 256), 256, 0, k_pse_gather, ps, w, (int)n, cl.items, pss, w0s);
-  pdl_launch(c->stream, blocks_for(n, kPseThreads), kPseThreads, 0, k_pse, g, pss, w0s, w, (int)n, cl.start, cl.items, nu, dt);
+  const int lanes = pse_lanes(n);
+  pdl_launch(c->stream, blocks_for(lanes * n, kPseThreads), kPseThreads, 0, lanes == 4 ? k_pse<4> : k_pse<1>, g, pss, w0s,
+             w, (int)n, cl.start, cl.items, nu, dt);
   c->launches += 2;
   VG_CUDA(c, cudaGetLastError());
   return VG_OK;
