@@ -318,7 +318,7 @@ constexpr int kMgGraphs = 8;
 struct MgGraphCache {
   cudaGraphExec_t exec = nullptr;
   Geom g;
-  const void* key[4] = {nullptr, nullptr, nullptr, nullptr};
+  const void* key[5] = {};  // the buffers and tables that the cycle's kernels were given
   unsigned launches = 0;
 };
 

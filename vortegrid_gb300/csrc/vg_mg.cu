@@ -1544,9 +1544,10 @@ static vg_status next_norm(Ctx* c, double* rr, double* bb) {
 }
 
 // Runs the work that `enqueue` puts on the stream, from a graph captured when the same (grid, buffers) came first; `key`
-// names every buffer that the cycle's kernels were given besides the workspace of its grid.
+// names every buffer that the cycle's kernels were given besides the workspace of its grid: the coarsest level's tables
+// (B.dst) too, which have a workspace of their own that another grid's solve may move.
 template <class F>
-static vg_status run_cached(Ctx* c, const Geom& g, const void* const (&key)[4], F enqueue) {
+static vg_status run_cached(Ctx* c, const Geom& g, const void* const (&key)[5], F enqueue) {
   MgGraphCache* G = nullptr;
   for (MgGraphCache& q : c->mg_graph)
     if (q.exec && memcmp(&q.g, &g, sizeof(Geom)) == 0 && memcmp(q.key, key, sizeof(key)) == 0) G = &q;
@@ -1585,7 +1586,7 @@ static vg_status run_cached(Ctx* c, const Geom& g, const void* const (&key)[4], 
 }
 
 static vg_status run_cycle(Ctx* c, const MgPlan& P, const Geom& g, const MgBufs& B, float* x, const float* rhs) {
-  const void* const key[4] = {B.E, rhs, x, nullptr};
+  const void* const key[5] = {B.E, rhs, x, B.dst, nullptr};
   return run_cached(c, g, key, [&](unsigned* nl) { return enqueue_cycle(c, P, g, B, x, rhs, nl); });
 }
 
@@ -1965,7 +1966,7 @@ static vg_status split_adaptive(Ctx* c, const Geom& g, const MgPlan& P, float* s
   int cyc = 0, cur = 0;
   // a cycle from r0, then the residual of x + e (x NULL: of e) on right-hand side b, the sum to xn
   auto cycle = [&](const float* r0, const float* x, const float* b, float* xn) -> vg_status {
-    const void* const key[4] = {S.E[0], r0, x, xn};
+    const void* const key[5] = {S.E[0], r0, x, xn, S.mb.dst};
     const vg_status cst = run_cached(c, g, key, [&](unsigned* n) -> vg_status {
       const vg_status vst = enqueue_vcycle(c, P, S, r0, n);
       if (vst != VG_OK) return vst;
