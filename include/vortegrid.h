@@ -210,7 +210,8 @@ vg_status vg_get_poisson_schedule(const vg_ctx* ctx, int* fp32_cycles, int* refi
  * (on = 0, the default) or FP64 tables and arithmetic (on = 1).  No
  * counterpart in the reference, whose cascade has no coarsest solve.  Cycles
  * captured earlier are recaptured; a step captured by the caller in a CUDA
- * graph must be captured again.  The batched persistent solve needs FP32. */
+ * graph must be captured again (as after a solve of another grid on the same
+ * context: there is one set of tables).  The batched persistent solve needs FP32. */
 vg_status vg_set_coarsest_fp64(vg_ctx* ctx, int on);
 /* Wait for the context's stream and report any error a device stage flagged
  * since the last synchronising call (VG_OUT_OF_GRID, VG_NONFINITE).  The

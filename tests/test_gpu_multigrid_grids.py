@@ -49,3 +49,36 @@ def test_grids_in_turn(order, fp64):
         for p, want in zip(problems, alone):
             for _ in range(2):
                 assert torch.equal(solve(ctx, *p).view(torch.int32), want.view(torch.int32))
+
+
+@pytest.mark.parametrize("n3,other", [((33, 33, 33), (25, 25, 25)), ((65, 49, 33), (17, 17, 17))])
+def test_record_frames_around_another_solve(n3, other):
+    """Frames of pinned records, replayed from a graph on a fixed schedule, with a
+    solve of a grid with smaller tables between them: bit for bit the frames of
+    pageable records, which always run directly."""
+    import vortegrid_gb300 as vg
+    from vortegrid_gb300 import workloads
+    pos, w, s = workloads.ring(1500, seed=4)
+    grid = vg.GridGeom.make([-1.5] * 3, [3.0] * 3, list(n3))
+    g2, start, rhs = problem(other)
+    out = []
+    for pinned in (False, True):
+        sim = vg.VortonSim(cfg=vg.default_config(fixed_grid=grid, device=0))
+        sim.set_poisson_schedule(3, 1)
+        v = vg.make_particles(pos, w, s)
+        if pinned:
+            keep = torch.empty(v.nbytes, dtype=torch.uint8, pin_memory=True)
+            rec = keep.numpy().view(v.dtype)
+            rec[...] = v
+            v = rec
+        frames = []
+        for k in range(9):
+            if k in (5, 7):
+                x, cyc, r = start.clone(), ctypes.c_int(), ctypes.c_double()
+                sim.check(vg.lib().vg_multigrid_device(sim.h, ctypes.byref(g2), vg._ptr(x), vg._ptr(rhs), 1e-6, 50,
+                                                       ctypes.byref(cyc), ctypes.byref(r), ctypes.byref(r)), "multigrid")
+            sim.UpdateAndEvolve(v, 1.0 / 60.0, k)
+            frames.append(np.ascontiguousarray(v["velocity"]).copy())
+        out.append(frames)
+    for k, (a, b) in enumerate(zip(*out)):
+        assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), k

@@ -794,6 +794,10 @@ struct vg::HostStepGraph {
   const void* net = nullptr;
   int k1 = 0, k2 = 0;
   bool coarse64 = false;
+  // the grid that the multigrid's coarse tables are for: a replay reads them, and another grid's solve writes others
+  unsigned tab_np[3];
+  double tab_r2[3];
+  bool tab_fp64 = false;
   void* bufs[S_NUM];
   size_t bytes[S_NUM];
 };
@@ -835,6 +839,9 @@ static void fill_key(Ctx* c, HostStepGraph* k, const void* vortons, size_t n, si
   k->k1 = c->mg_fixed_k1;
   k->k2 = c->mg_fixed_k2;
   k->coarse64 = c->mg_coarse_fp64;
+  memcpy(k->tab_np, c->mginv_np, sizeof(k->tab_np));
+  memcpy(k->tab_r2, c->mginv_r2, sizeof(k->tab_r2));
+  k->tab_fp64 = c->mginv_fp64;
   for (int i = 0; i < S_NUM; ++i) {
     k->bufs[i] = c->buf[i].p;
     k->bytes[i] = c->buf[i].bytes;
@@ -847,7 +854,8 @@ static bool same_key(const HostStepGraph& a, const HostStepGraph& b) {
          memcmp(&a.size0, &b.size0, sizeof(float)) == 0 && a.evolve == b.evolve &&
          a.has_extra == b.has_extra && memcmp(a.extra, b.extra, sizeof(a.extra)) == 0 &&
          memcmp(&a.cfg, &b.cfg, sizeof(vg_config)) == 0 && a.net == b.net && a.k1 == b.k1 && a.k2 == b.k2 &&
-         a.coarse64 == b.coarse64 && memcmp(a.bufs, b.bufs, sizeof(a.bufs)) == 0 &&
+         a.coarse64 == b.coarse64 && memcmp(a.tab_np, b.tab_np, sizeof(a.tab_np)) == 0 &&
+         memcmp(a.tab_r2, b.tab_r2, sizeof(a.tab_r2)) == 0 && a.tab_fp64 == b.tab_fp64 && memcmp(a.bufs, b.bufs, sizeof(a.bufs)) == 0 &&
          memcmp(a.bytes, b.bytes, sizeof(a.bytes)) == 0;
 }
 
