@@ -82,3 +82,26 @@ def test_record_frames_around_another_solve(n3, other):
         out.append(frames)
     for k, (a, b) in enumerate(zip(*out)):
         assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), k
+
+
+@pytest.mark.parametrize("n3", [(33, 33, 33), (65, 65, 65)])
+def test_norms_of_solves_from_zero(n3):
+    """From a start and boundary of zeros the first residual is the right-hand side,
+    so that both norms are the same number, as they are for a right-hand side of
+    zeros: each solve by its own norms, whichever came before."""
+    import vortegrid_gb300 as vg
+    grid, _, rhs = problem(n3)
+    zero = torch.zeros_like(rhs)
+    ctx = vg.Context(numerics=vg.NUMERICS_FAST)
+    want = None
+    for _ in range(50):
+        for b in (zero, rhs):
+            soln, cyc, r0, r1 = zero.clone(), ctypes.c_int(-1), ctypes.c_double(-1), ctypes.c_double(-1)
+            ctx.check(vg.lib().vg_multigrid_device(ctx.h, ctypes.byref(grid), vg._ptr(soln), vg._ptr(b), 1e-6, 50,
+                                                   ctypes.byref(cyc), ctypes.byref(r0), ctypes.byref(r1)), "multigrid")
+            if b is zero:
+                assert cyc.value == 0 and r0.value == r1.value == 0.0 and not soln.any()
+                continue
+            assert cyc.value > 0 and r0.value == 1.0 and 0 < r1.value <= 1e-6
+            want = soln.clone() if want is None else want
+            assert torch.equal(soln.view(torch.int32), want.view(torch.int32))

@@ -331,7 +331,7 @@ struct Ctx {
   nn::Net* net = nullptr;   // attached warm-start network (not owned)
   MgGraphCache mg_graph[kMgGraphs];  // cycle graphs, replaced in turn
   int mg_graph_next = 0;
-  unsigned long long* hnorm = nullptr;  // pinned: the adaptive solve's last residual norm (r^2, b^2, its number, a check)
+  unsigned long long* hnorm = nullptr;  // pinned: the adaptive solve's last residual norm (halves of r^2 and b^2, each with its number)
   unsigned long long norm_seq = 0;   // norms asked for so far
   cudaStream_t stream = nullptr;
   bool own_stream = false;

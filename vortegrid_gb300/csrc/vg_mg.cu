@@ -33,7 +33,6 @@
 #include <float.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <type_traits>
@@ -622,10 +621,11 @@ __device__ __forceinline__ void split_sum2(float a32, float b32, double* __restr
 }
 
 // A solve's norms: the partial sums added up ([0] r^2, [1] b^2, kept when keep_b) and, for the adaptive solve, written to
-// pinned host memory that the host polls: both sums, the norm's number and a check word, so that the host takes the four
-// only when they belong together and no fence is needed between them.  A copy and a stream wait took 15 to 20 us a norm
-// more.  (Summing in the residual kernels by their last block, instead of this launch, made them 4 to 10 us longer: a fence
-// and an atomic at every block's end.)
+// pinned host memory that the host polls: the halves of both sums, each in a word with the norm's number, so that every word
+// says by itself whether it is this norm's, in whatever order the words arrive and without a fence.  (A check word
+// r^2 ^ b^2 ^ number is the same for any two norms with r^2 = b^2, as every solve from zero begins with.)  A copy and a
+// stream wait took 15 to 20 us a norm more.  (Summing in the residual kernels by their last block, instead of this launch,
+// made them 4 to 10 us longer: a fence and an atomic at every block's end.)
 // Bound by FP64 additions, 16 cycles a warp: 1,024 threads with five additions each in the trees took 6.6 us at 129^3 and
 // 5.1 at 33^3, 256 threads take 4.5 and 3.0 (128 threads the same at 129^3).
 constexpr int kNormThreads = 256;
@@ -664,11 +664,11 @@ __global__ void __launch_bounds__(kNormThreads) k_s_norm(const double* __restric
   if (threadIdx.x) return;
   if (keep_b) a2 = b2;
   if (host) {
-    const unsigned long long r = __double_as_longlong(a1), b = __double_as_longlong(a2);
-    host[0] = r;
-    host[1] = b;
-    host[2] = number;
-    host[3] = r ^ b ^ number;
+    const unsigned long long r = __double_as_longlong(a1), b = __double_as_longlong(a2), tag = number & 0xffffffffu;
+    host[0] = r << 32 | tag;
+    host[1] = (r >> 32) << 32 | tag;
+    host[2] = b << 32 | tag;
+    host[3] = (b >> 32) << 32 | tag;
     *seq = number;
   }
   out2[0] = a1;
@@ -1521,13 +1521,14 @@ static vg_status norm_memory(Ctx* c, MgBufs& B) {
 // memory; after every few thousand polls the stream is asked whether it has failed, or is done without the norm having come.
 static vg_status next_norm(Ctx* c, double* rr, double* bb) {
   const unsigned long long want = ++c->norm_seq;
-  volatile unsigned long long* h = c->hnorm;
-  unsigned long long r = 0, b = 0;
+  unsigned long long w[4];
   auto there = [&] {
-    if (h[2] != want) return false;
-    r = h[0];
-    b = h[1];
-    return h[3] == (r ^ b ^ want);
+    bool all = true;
+    for (int k = 0; k < 4; ++k) {
+      w[k] = __atomic_load_n(c->hnorm + k, __ATOMIC_RELAXED);
+      all = all && (unsigned)w[k] == (unsigned)want;
+    }
+    return all;
   };
   for (unsigned long long polls = 1; !there(); ++polls) {
     if (polls % 4096) continue;
@@ -1537,8 +1538,14 @@ static vg_status next_norm(Ctx* c, double* rr, double* bb) {
     if (!there()) return fail(c, VG_CUDA_ERROR, "multigrid: a residual norm was not written");
     break;
   }
-  memcpy(rr, &r, sizeof(r));
-  if (bb) memcpy(bb, &b, sizeof(b));
+  auto value = [&](int k) {
+    const unsigned long long bits = w[k] >> 32 | w[k + 1] >> 32 << 32;
+    double v;
+    memcpy(&v, &bits, sizeof(v));
+    return v;
+  };
+  *rr = value(0);
+  if (bb) *bb = value(2);
   if (!(*rr == *rr)) return fail(c, VG_NONFINITE, "multigrid: non-finite residual");
   return VG_OK;
 }
