@@ -543,6 +543,7 @@ static vg_status step_back(Ctx* c, StepState& s) {
   c->grid = g;
   c->have_grid = true;
   ++c->vel_gen;  // a new velocity grid (any float4 copy is stale)
+  if (c->step_captured) c->vel_uncounted = true;
   return VG_OK;
 }
 
@@ -939,7 +940,9 @@ static vg_status step_records(vg_ctx* c, void* particles, size_t n, size_t strid
         cudaGraph_t graph = nullptr;
         cudaGraphExec_t exec = nullptr;
         if (cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+          const bool uncounted = c->vel_uncounted;
           const vg_status cst = enqueue();
+          c->vel_uncounted = uncounted;  // this graph's replays are counted
           const cudaError_t ce = cudaStreamEndCapture(c->stream, &graph);
           if (cst == VG_OK && ce == cudaSuccess && graph && cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess) {
             cudaGraphDestroy(graph);

@@ -893,7 +893,7 @@ vg_status launch_gather_advect(Ctx* c, const Geom& g, const float* vel3, float4*
     if (st != VG_OK) return st;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     VG_CUDA(c, cudaStreamIsCapturing(c->stream, &cap));
-    if (cap != cudaStreamCaptureStatusNone || c->velpoints_gen != c->vel_gen) {
+    if (cap != cudaStreamCaptureStatusNone || c->vel_uncounted || c->velpoints_gen != c->vel_gen) {
       pdl_launch(c->stream, blocks_for(g.points(), 256), 256, 0, k_vel_points, g.points(), vel3, vp);
       VG_LAUNCHED(c);
       c->velpoints_gen = cap != cudaStreamCaptureStatusNone ? ~0ull : c->vel_gen;

@@ -356,6 +356,10 @@ struct Ctx {
   // generation of the step's velocity grid (counted on the host at each step)
   // and the one the float4 copy in buf[S_VELPOINTS] was made from
   unsigned long long vel_gen = 0, velpoints_gen = ~0ull;
+  // a step of this context was captured by the batch or the caller, whose graph
+  // may write the velocity grid at any time without being counted: the copy is
+  // then made for every tracer group
+  bool vel_uncounted = false;
   bool stats_pending = false;
   // Multigrid schedule.  mg_fixed_k1 > 0 runs a fixed schedule with no host
   // round trip (k1 FP32 cycles, then k2 refinement cycles), so that a step can
