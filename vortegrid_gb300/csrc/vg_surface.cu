@@ -797,6 +797,7 @@ vg_status launch_marching_cubes(Ctx* c, const Geom& g, const float* v, float iso
     pdl_launch(c->stream, blocks_for(cells, 128), 128, 0, k_mc_emit, g, v, iso, T, (const unsigned*)offsets, cap, verts,
                normals);
     VG_LAUNCHED(c);
+    VG_CUDA(c, cudaGetLastError());
   }
   unsigned total = 0;
   VG_CUDA(c, cudaMemcpyAsync(&total, offsets + cells, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
