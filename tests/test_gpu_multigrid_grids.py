@@ -105,3 +105,20 @@ def test_norms_of_solves_from_zero(n3):
             assert cyc.value > 0 and r0.value == 1.0 and 0 < r1.value <= 1e-6
             want = soln.clone() if want is None else want
             assert torch.equal(soln.view(torch.int32), want.view(torch.int32))
+
+
+# planes x components beyond what a launch has blocks in z; four planes to a thread of the sweeps, and one
+@pytest.mark.parametrize("n3", [(17, 17, 22401), (5, 5, 22401)])
+def test_long_box(n3):
+    """The reported residual is the solution's own, in float64 (the stored floats'
+    residual is half an ulp of each of the seven values)."""
+    import vortegrid_gb300 as vg
+    grid, start, rhs = problem(n3)
+    x = solve(vg.Context(numerics=vg.NUMERICS_FAST), grid, start, rhs).double()
+    h = [1.0 / float(grid.cell_spacing[a]) ** 2 for a in range(3)]
+    c = x[1:-1, 1:-1, 1:-1]
+    lap = (h[0] * (x[1:-1, 1:-1, :-2] + x[1:-1, 1:-1, 2:] - 2 * c) + h[1] * (x[1:-1, :-2, 1:-1] + x[1:-1, 2:, 1:-1] - 2 * c) +
+           h[2] * (x[:-2, 1:-1, 1:-1] + x[2:, 1:-1, 1:-1] - 2 * c))
+    b = rhs.double()[1:-1, 1:-1, 1:-1]
+    stored = np.finfo(np.float32).eps * float(x.norm())
+    assert float((b - lap).norm()) <= 1e-6 * float(b.norm()) + 4 * sum(h) * stored

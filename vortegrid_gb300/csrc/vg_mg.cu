@@ -364,6 +364,8 @@ __device__ __forceinline__ void st4(float* p, float4 v) { *reinterpret_cast<floa
 
 // Launch shape over the interior rows of a level: blocks of (groups, rows), whole warps, `zs` planes per thread, three
 // components in the z index.
+constexpr unsigned kMaxGridZ = 65535;
+static_assert(kMaxGridZ % 3 == 0, "components in the z index");
 struct SLaunch {
   dim3 grid, block;
   unsigned zs, nb;  // planes per thread; blocks
@@ -379,6 +381,7 @@ static SLaunch split_launch(const SGeo& g) {
   // at one plane) 10.7 / 9.2 / 9.9 / 10.9
   const double threads = 3.0 * g.groups * (g.ny - 2) * (g.nz - 2);
   L.zs = threads > 2e6 ? 4 : threads > 3e5 ? 2 : 1;
+  while (3 * (size_t)((g.nz - 2 + L.zs - 1) / L.zs) > kMaxGridZ) L.zs *= 2;  // long boxes: as many blocks as a launch can have
   L.grid = dim3((g.groups + bx - 1) / bx, (g.ny - 2 + by - 1) / by, 3 * ((g.nz - 2 + L.zs - 1) / L.zs));
   L.nb = L.grid.x * L.grid.y * L.grid.z;
   return L;
@@ -542,56 +545,59 @@ __global__ void __launch_bounds__(256) k_s_restrict(SGeo g, SGeo C, const float*
 }
 
 // e_fine += trilinear(e_coarse) of one component: a thread owns four places of a fine row, even and odd x, and reads the one,
-// two or four coarse rows beside it; the sums in the order of prolong_point.
+// two or four coarse rows beside it; the sums in the order of prolong_point.  A block takes one plane, or every
+// (gridDim.z / 3)th one of a box with more planes than a launch has blocks.
 template <bool kSplitCoarse>
 __global__ void __launch_bounds__(256) k_s_prolong(SGeo g, SGeo C, const float* __restrict__ ec, float* __restrict__ E) {
   pdl_entry();
   const unsigned i0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x), y = blockIdx.y * blockDim.y + threadIdx.y + 1;
-  const unsigned c = blockIdx.z % 3u, z = 1 + blockIdx.z / 3u;
+  const unsigned c = blockIdx.z % 3u;
   if (i0 >= 4 * g.groups || y + 1 >= g.ny) return;
-  const unsigned oy = y & 1u, oz = z & 1u;
-  float a[4] = {0.f, 0.f, 0.f, 0.f}, b[4] = {0.f, 0.f, 0.f, 0.f};  // even x: coarse i; odd x: coarse i and i + 1
-  for (unsigned iz = 0; iz <= oz; ++iz)
-    for (unsigned iy = 0; iy <= oy; ++iy) {
-      const unsigned Y = (y >> 1) + iy, Z = (z >> 1) + iz;
-      float v[5];
-      if (kSplitCoarse) {
-        // coarse x = i0 .. i0 + 4 (i0 even): alternately of the two colours
-        const float* ra = ec + (2 * c + ((Y + Z) & 1u)) * C.cs + (size_t)Z * C.pz + Y * C.hx + (i0 >> 1);
-        const float* rb = ec + (2 * c + ((Y + Z + 1) & 1u)) * C.cs + (size_t)Z * C.pz + Y * C.hx + (i0 >> 1);
-        const float2 va = *reinterpret_cast<const float2*>(ra), vb = *reinterpret_cast<const float2*>(rb);
-        v[0] = va.x;
-        v[1] = vb.x;
-        v[2] = va.y;
-        v[3] = vb.y;
-        v[4] = (i0 >> 1) + 2 < C.hx ? ra[2] : 0.f;
-      } else {
-        const float* row = ec + 3 * ((size_t)C.nx * (Y + C.ny * (size_t)Z)) + c;
-#pragma unroll
-        for (unsigned k = 0; k < 5; ++k) v[k] = i0 + k < C.nx ? row[3 * (i0 + k)] : 0.f;
+  for (unsigned z = 1 + blockIdx.z / 3u; z + 1 < g.nz; z += gridDim.z / 3u) {
+    const unsigned oy = y & 1u, oz = z & 1u;
+    float a[4] = {0.f, 0.f, 0.f, 0.f}, b[4] = {0.f, 0.f, 0.f, 0.f};  // even x: coarse i; odd x: coarse i and i + 1
+    for (unsigned iz = 0; iz <= oz; ++iz)
+      for (unsigned iy = 0; iy <= oy; ++iy) {
+        const unsigned Y = (y >> 1) + iy, Z = (z >> 1) + iz;
+        float v[5];
+        if (kSplitCoarse) {
+          // coarse x = i0 .. i0 + 4 (i0 even): alternately of the two colours
+          const float* ra = ec + (2 * c + ((Y + Z) & 1u)) * C.cs + (size_t)Z * C.pz + Y * C.hx + (i0 >> 1);
+          const float* rb = ec + (2 * c + ((Y + Z + 1) & 1u)) * C.cs + (size_t)Z * C.pz + Y * C.hx + (i0 >> 1);
+          const float2 va = *reinterpret_cast<const float2*>(ra), vb = *reinterpret_cast<const float2*>(rb);
+          v[0] = va.x;
+          v[1] = vb.x;
+          v[2] = va.y;
+          v[3] = vb.y;
+          v[4] = (i0 >> 1) + 2 < C.hx ? ra[2] : 0.f;
+        } else {
+          const float* row = ec + 3 * ((size_t)C.nx * (Y + C.ny * (size_t)Z)) + c;
+  #pragma unroll
+          for (unsigned k = 0; k < 5; ++k) v[k] = i0 + k < C.nx ? row[3 * (i0 + k)] : 0.f;
+        }
+  #pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          a[k] += v[k];
+          b[k] += v[k];
+          b[k] += v[k + 1];
+        }
       }
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        a[k] += v[k];
-        b[k] += v[k];
-        b[k] += v[k + 1];
-      }
-    }
-  const float wa = 1.0f / (float)(1u << (oy + oz)), wb = 0.5f * wa;
-  const size_t o = (size_t)z * g.pz + y * g.hx + i0;
-  float* even = E + (2 * c + ((y + z) & 1u)) * g.cs + o;
-  float* odd = E + (2 * c + ((y + z + 1) & 1u)) * g.cs + o;
-  float4 ve = ld4(even), vo = ld4(odd);
-  if (x_interior(g, 0, i0)) ve.x = __fmaf_rn(a[0], wa, ve.x);
-  if (x_interior(g, 0, i0 + 1)) ve.y = __fmaf_rn(a[1], wa, ve.y);
-  if (x_interior(g, 0, i0 + 2)) ve.z = __fmaf_rn(a[2], wa, ve.z);
-  if (x_interior(g, 0, i0 + 3)) ve.w = __fmaf_rn(a[3], wa, ve.w);
-  if (x_interior(g, 1, i0)) vo.x = __fmaf_rn(b[0], wb, vo.x);
-  if (x_interior(g, 1, i0 + 1)) vo.y = __fmaf_rn(b[1], wb, vo.y);
-  if (x_interior(g, 1, i0 + 2)) vo.z = __fmaf_rn(b[2], wb, vo.z);
-  if (x_interior(g, 1, i0 + 3)) vo.w = __fmaf_rn(b[3], wb, vo.w);
-  st4(even, ve);
-  st4(odd, vo);
+    const float wa = 1.0f / (float)(1u << (oy + oz)), wb = 0.5f * wa;
+    const size_t o = (size_t)z * g.pz + y * g.hx + i0;
+    float* even = E + (2 * c + ((y + z) & 1u)) * g.cs + o;
+    float* odd = E + (2 * c + ((y + z + 1) & 1u)) * g.cs + o;
+    float4 ve = ld4(even), vo = ld4(odd);
+    if (x_interior(g, 0, i0)) ve.x = __fmaf_rn(a[0], wa, ve.x);
+    if (x_interior(g, 0, i0 + 1)) ve.y = __fmaf_rn(a[1], wa, ve.y);
+    if (x_interior(g, 0, i0 + 2)) ve.z = __fmaf_rn(a[2], wa, ve.z);
+    if (x_interior(g, 0, i0 + 3)) ve.w = __fmaf_rn(a[3], wa, ve.w);
+    if (x_interior(g, 1, i0)) vo.x = __fmaf_rn(b[0], wb, vo.x);
+    if (x_interior(g, 1, i0 + 1)) vo.y = __fmaf_rn(b[1], wb, vo.y);
+    if (x_interior(g, 1, i0 + 2)) vo.z = __fmaf_rn(b[2], wb, vo.z);
+    if (x_interior(g, 1, i0 + 3)) vo.w = __fmaf_rn(b[3], wb, vo.w);
+    st4(even, ve);
+    st4(odd, vo);
+  }
 }
 
 // Block sums of two values into part[2 b + {0, 1}], as block_sum2, for any whole number of warps.
@@ -1837,7 +1843,7 @@ static vg_status enqueue_vcycle(Ctx* c, const MgPlan& P, const SplitBufs& S, con
   if (st != VG_OK) return st;
   for (int l = fs - 1; l >= 0; --l) {
     const SLaunch& L = S.sl[l];
-    const dim3 pg(L.grid.x, L.grid.y, 3 * (S.g[l].nz - 2));
+    const dim3 pg(L.grid.x, L.grid.y, std::min(3 * (S.g[l].nz - 2), kMaxGridZ));
     if (l + 1 < fs) {
       pdl_launch(c->stream, pg, L.block, 0, k_s_prolong<true>, S.g[l], S.g[l + 1], (const float*)S.E[l + 1], S.E[l]);
     } else {
