@@ -68,6 +68,35 @@ __device__ __forceinline__ unsigned bin_axis(float p, float mn, float cpe) {
   return (unsigned)__float2int_rz(__fmul_rn(__fsub_rn(p, mn), cpe));
 }
 
+// s += x; the sum's rounding error, exactly (Knuth's TwoSum).
+__device__ __forceinline__ float two_sum(float& s, float x) {
+  const float t = __fadd_rn(s, x), b = __fsub_rn(t, s);
+  const float e = __fadd_rn(__fsub_rn(s, __fsub_rn(t, b)), __fsub_rn(x, b));
+  s = t;
+  return e;
+}
+
+// A running sum of n floats, or of their squares (split exactly by an FMA), as an
+// unevaluated triple of floats: the errors of the first part's additions are
+// summed in the second, whose own are summed in the third.  What is lost stays
+// below n^2 2^-72 of the sum of magnitudes, and value() rounds once: no less than
+// a running sum in FP64 (n 2^-53) for n below 2^19, without the FP64 pipe, whose
+// rate on GB300 is a 64th of FP32's.
+struct TripleSum {
+  float hi = 0.f, mid = 0.f, lo = 0.f;
+  __device__ __forceinline__ void add(float x) { lo = __fadd_rn(lo, two_sum(mid, two_sum(hi, x))); }
+  __device__ __forceinline__ void add_square(float v) {
+    const float p = __fmul_rn(v, v), q = __fmaf_rn(v, v, -p);
+    const float e1 = two_sum(mid, two_sum(hi, p)), e2 = two_sum(mid, q);
+    lo = __fadd_rn(lo, __fadd_rn(e1, e2));
+  }
+  __device__ __forceinline__ double value() const { return (double)hi + ((double)mid + (double)lo); }
+  // Of squares: whether none has left the range of floats.  A square or its
+  // remainder below the normal floats loses up to 2^-149: under 2^-53 of a sum of
+  // 10^-22 for up to 8 million of them.
+  __device__ __forceinline__ bool in_range() const { return hi > 1e-22f && hi < 1e36f; }
+};
+
 // Point (x, y, z) of offset k in a grid of nx x ny points a plane: two 32-bit
 // divisions for grids of fewer than 2^32 points (the plain form's 64-bit ones cost
 // a pass over 2 million points 2 us: curl 17.1 -> 15.3, splat 54.9 -> 52.7).
