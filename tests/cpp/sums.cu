@@ -1,5 +1,6 @@
 // Sums of runs of floats and of their squares by vg::TripleSum (csrc/vg_internal.cuh), a thread a run:
-// sums <in.bin> <out.bin>; in: int32 runs, int32 n, float values[runs][n]; out: double sum, sum of squares [runs][2].
+// sums <in.bin> <out.bin>; in: int32 runs, int32 n, float values[runs][n]; out: double sum, sum of squares,
+// whether the squares are in range [runs][3].
 #include <cstdio>
 #include <vector>
 
@@ -13,8 +14,9 @@ __global__ void k_sums(const float* v, int runs, int n, double* out) {
     s.add(v[(size_t)t * n + i]);
     q.add_square(v[(size_t)t * n + i]);
   }
-  out[2 * t] = s.value();
-  out[2 * t + 1] = q.value();
+  out[3 * t] = s.value();
+  out[3 * t + 1] = q.value();
+  out[3 * t + 2] = q.in_range();
 }
 
 int main(int argc, char** argv) {
@@ -26,7 +28,7 @@ int main(int argc, char** argv) {
   fclose(f);
   float* dv = nullptr;
   double* dout = nullptr;
-  std::vector<double> out(2 * (size_t)head[0]);
+  std::vector<double> out(3 * (size_t)head[0]);
   if (cudaMalloc(&dv, v.size() * 4) || cudaMalloc(&dout, out.size() * 8)) return 2;
   if (cudaMemcpy(dv, v.data(), v.size() * 4, cudaMemcpyHostToDevice)) return 2;
   k_sums<<<(head[0] + 127) / 128, 128>>>(dv, head[0], head[1], dout);

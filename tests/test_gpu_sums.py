@@ -26,7 +26,7 @@ def sums(tmp_path_factory):
             np.array(v.shape, np.int32).tofile(f)
             v.tofile(f)
         subprocess.check_call([exe, str(tmp / "in.bin"), str(tmp / "out.bin")])
-        return np.fromfile(tmp / "out.bin", np.float64).reshape(-1, 2)
+        return np.fromfile(tmp / "out.bin", np.float64).reshape(-1, 3)
     return run
 
 
@@ -37,8 +37,21 @@ def test_no_less_than_fp64(sums, n, spread):
     rng = np.random.default_rng(n)
     v = (rng.normal(0, 1, (300, n)) * 10.0 ** rng.uniform(-spread, spread, (300, n))).astype(np.float32)
     got = sums(v)
-    for row, (s, q) in zip(v.astype(np.float64), got):
+    for row, (s, q, _) in zip(v.astype(np.float64), got):
         exact, squares = math.fsum(row), math.fsum(row * row)  # squares of floats are exact in float64
         lost = n * n * 2.0 ** -72
         assert abs(s - exact) <= 2.0 ** -52 * abs(exact) + lost * math.fsum(abs(row))
         assert abs(q - squares) <= (2.0 ** -52 + lost) * squares
+
+
+def test_range_of_squares(sums):
+    """Sums that squares outside the range of floats may have spoilt are told from
+    the others, among them those of zeros alone."""
+    rows = {"zeros": (0.0, 0.0, True), "minus zero": (-0.0, 0.0, True), "ones": (1.0, 1.0, True),
+            "zeros and ones": (0.0, 1.0, True), "small": (0.0, 1e-20, False), "subnormal": (0.0, 1e-40, False),
+            "large": (1.0, 1e19, False), "infinite": (0.0, np.inf, False), "not a number": (0.0, np.nan, False)}
+    v = np.zeros((len(rows), 41), np.float32)
+    for k, (a, b, _) in enumerate(rows.values()):
+        v[k] = a
+        v[k, 20] = b
+    assert [bool(x) for x in sums(v)[:, 2]] == [r[2] for r in rows.values()]

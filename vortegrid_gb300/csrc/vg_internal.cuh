@@ -84,17 +84,20 @@ __device__ __forceinline__ float two_sum(float& s, float x) {
 // rate on GB300 is a 64th of FP32's.
 struct TripleSum {
   float hi = 0.f, mid = 0.f, lo = 0.f;
+  unsigned bits = 0;  // of all values squared
   __device__ __forceinline__ void add(float x) { lo = __fadd_rn(lo, two_sum(mid, two_sum(hi, x))); }
   __device__ __forceinline__ void add_square(float v) {
     const float p = __fmul_rn(v, v), q = __fmaf_rn(v, v, -p);
     const float e1 = two_sum(mid, two_sum(hi, p)), e2 = two_sum(mid, q);
     lo = __fadd_rn(lo, __fadd_rn(e1, e2));
+    bits |= __float_as_uint(v);
   }
   __device__ __forceinline__ double value() const { return (double)hi + ((double)mid + (double)lo); }
   // Of squares: whether none has left the range of floats.  A square or its
   // remainder below the normal floats loses up to 2^-149: under 2^-53 of a sum of
-  // 10^-22 for up to 8 million of them.
-  __device__ __forceinline__ bool in_range() const { return hi > 1e-22f && hi < 1e36f; }
+  // 10^-22 for up to 8 million of them.  Zeros alone are in range: a field that is
+  // zero outside some vortons has threads that see nothing else.
+  __device__ __forceinline__ bool in_range() const { return (hi > 1e-22f && hi < 1e36f) || (bits & 0x7fffffffu) == 0; }
 };
 
 // Point (x, y, z) of offset k in a grid of nx x ny points a plane: two 32-bit
