@@ -122,3 +122,25 @@ def test_long_box(n3):
     b = rhs.double()[1:-1, 1:-1, 1:-1]
     stored = np.finfo(np.float32).eps * float(x.norm())
     assert float((b - lap).norm()) <= 1e-6 * float(b.norm()) + 4 * sum(h) * stored
+
+
+@pytest.mark.parametrize("n3", [(65, 65, 65), (129, 65, 49), (193, 129, 129)])
+def test_norms_of_whole_numbers(n3):
+    """With unit cells and whole numbers the first residual is exact, and so are the sums
+    of three of its squares (below 2^24).  The norm is told to a part in 10^13: 17
+    additions to pairs of floats (2^-47 each), the blocks' sums in float64."""
+    import vortegrid_gb300 as vg
+    grid = vg.GridGeom.make([0.0] * 3, [float(k - 1) for k in n3], list(n3))
+    rng = np.random.default_rng(sum(n3))
+    shape = n3[::-1] + (3,)
+    x0, b = rng.integers(-60, 61, shape), rng.integers(-1000, 1001, shape)
+    c = x0[1:-1, 1:-1, 1:-1]
+    lap = (x0[1:-1, 1:-1, :-2] + x0[1:-1, 1:-1, 2:] + x0[1:-1, :-2, 1:-1] + x0[1:-1, 2:, 1:-1] + x0[:-2, 1:-1, 1:-1] +
+           x0[2:, 1:-1, 1:-1] - 6 * c)
+    inner = b[1:-1, 1:-1, 1:-1]
+    want = np.sqrt(float(((inner - lap) ** 2).sum())) / np.sqrt(float((inner ** 2).sum()))
+    soln, rhs = (torch.from_numpy(a.astype(np.float32)).cuda() for a in (x0, b))
+    ctx, cyc, r0, r1 = vg.Context(numerics=vg.NUMERICS_FAST), ctypes.c_int(), ctypes.c_double(), ctypes.c_double()
+    ctx.check(vg.lib().vg_multigrid_device(ctx.h, ctypes.byref(grid), vg._ptr(soln), vg._ptr(rhs), 1e-6, 50,
+                                           ctypes.byref(cyc), ctypes.byref(r0), ctypes.byref(r1)), "multigrid")
+    assert abs(r0.value - want) <= 2e-13 * want

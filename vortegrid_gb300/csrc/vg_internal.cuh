@@ -100,6 +100,22 @@ struct TripleSum {
   __device__ __forceinline__ bool in_range() const { return (hi > 1e-22f && hi < 1e36f) || (bits & 0x7fffffffu) == 0; }
 };
 
+// A long running sum of FP32 terms as a pair of floats: what is lost is below
+// n 2^-47 of the sum of magnitudes.  Sums that have left the range of floats are
+// infinite, as FP32 sums are.
+struct PairSum {
+  float hi = 0.f, lo = 0.f;
+  __device__ __forceinline__ void add(float x) { lo = __fadd_rn(lo, two_sum(hi, x)); }
+  // The sum over the warp, for all lanes.
+  __device__ __forceinline__ void add_lanes() {
+    for (int o = 16; o > 0; o >>= 1) {
+      const float h = __shfl_xor_sync(0xffffffffu, hi, o), l = __shfl_xor_sync(0xffffffffu, lo, o);
+      lo = __fadd_rn(__fadd_rn(lo, l), two_sum(hi, h));
+    }
+  }
+  __device__ __forceinline__ double value() const { return hi <= 3.402823466e38f ? (double)hi + (double)lo : (double)hi; }
+};
+
 // Point (x, y, z) of offset k in a grid of nx x ny points a plane: two 32-bit
 // divisions for grids of fewer than 2^32 points (the plain form's 64-bit ones cost
 // a pass over 2 million points 2 us: curl 17.1 -> 15.3, splat 54.9 -> 52.7).

@@ -602,16 +602,14 @@ __global__ void __launch_bounds__(256) k_s_prolong(SGeo g, SGeo C, const float* 
 
 // Block sums of two values into part[2 b + {0, 1}], as block_sum2, for any whole number of warps.
 template <bool kBoth>
-__device__ __forceinline__ void split_sum2(float a32, float b32, double* __restrict__ part) {
+__device__ __forceinline__ void split_sum2(PairSum a, PairSum b2, double* __restrict__ part) {
   __shared__ double s_a[8], s_b[8];
   const unsigned tid = threadIdx.x + blockDim.x * threadIdx.y, warps = blockDim.x * blockDim.y / 32;
-  for (int o = 16; o > 0; o >>= 1) {
-    a32 += __shfl_xor_sync(0xffffffffu, a32, o);
-    if (kBoth) b32 += __shfl_xor_sync(0xffffffffu, b32, o);
-  }
+  a.add_lanes();
+  if (kBoth) b2.add_lanes();
   if ((tid & 31) == 0) {
-    s_a[tid >> 5] = (double)a32;
-    if (kBoth) s_b[tid >> 5] = (double)b32;
+    s_a[tid >> 5] = a.value();
+    if (kBoth) s_b[tid >> 5] = b2.value();
   }
   __syncthreads();
   if (tid == 0) {
@@ -697,6 +695,19 @@ __device__ __forceinline__ float res_value1(const float* x, const float* e, ptrd
   return kField == RES_X ? x[o] : kField == RES_E ? e[o] : __fadd_rn(x[o], e[o]);
 }
 
+// Sum of the squares of a third of eight places' interior values (even and odd x): the FP32 part of a norm, three squares
+// long; a thread's thirds (up to 12), a warp and the blocks are added in pairs of floats and in FP64.
+__device__ __forceinline__ float squares(const SGeo& g, unsigned i0, const float (&even)[4], const float (&odd)[4], int third) {
+  float s = 0.f;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    if (q / 3 != third) continue;
+    const float v = x_interior(g, q / 4, i0 + q % 4) ? (q < 4 ? even : odd)[q % 4] : 0.f;
+    s = __fmaf_rn(v, v, s);
+  }
+  return s;
+}
+
 // Residual r = b - L v in FP32 (v: kField) at both colours of four places a thread, v itself to xn when it is a new sum, and
 // (kNorm) per-block sums of r^2 and b^2.  xn is another buffer than x, whose neighbours others still read; its boundary
 // values are the caller's.
@@ -707,7 +718,7 @@ __global__ void __launch_bounds__(256) k_s_residual(SGeo g, const float* __restr
   pdl_entry();
   const unsigned i0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x), y = blockIdx.y * blockDim.y + threadIdx.y + 1;
   const unsigned c = blockIdx.z % 3u, z0 = 1 + blockIdx.z / 3u * zs, z1 = min(g.nz - 1, z0 + zs);
-  float rr = 0.f, bb = 0.f;
+  PairSum rr, bb;
   if (i0 < 4 * g.groups && y + 1 < g.ny) {
     const size_t f0 = 2 * c * g.cs + (size_t)z0 * g.pz + y * g.hx + i0;
     x += f0;
@@ -739,13 +750,15 @@ __global__ void __launch_bounds__(256) k_s_residual(SGeo g, const float* __restr
       for (int k = 0; k < 4; ++k) {
         re[k] = __fsub_rn(abe[k], lap7(ev[k], ov[k + 1], ov[k], ey1[k], ey0[k], aep[k], aem[k], g.r2x, g.r2y, g.r2z));
         ro[k] = __fsub_rn(abo[k], lap7(ov[k + 1], ev[k + 1], ev[k], oy1[k], oy0[k], aop[k], aom[k], g.r2x, g.r2y, g.r2z));
-        if (kNorm && x_interior(g, 0, i0 + k)) {
-          rr = fmaf(re[k], re[k], rr);
-          if (kField == RES_X) bb = fmaf(abe[k], abe[k], bb);
-        }
-        if (kNorm && x_interior(g, 1, i0 + k)) {
-          rr = fmaf(ro[k], ro[k], rr);
-          if (kField == RES_X) bb = fmaf(abo[k], abo[k], bb);
+      }
+      if (kNorm) {
+        rr.add(squares(g, i0, re, ro, 0));
+        rr.add(squares(g, i0, re, ro, 1));
+        rr.add(squares(g, i0, re, ro, 2));
+        if (kField == RES_X) {
+          bb.add(squares(g, i0, abe, abo, 0));
+          bb.add(squares(g, i0, abe, abo, 1));
+          bb.add(squares(g, i0, abe, abo, 2));
         }
       }
       st4(r + ec, make_float4(re[0], re[1], re[2], re[3]));
@@ -771,9 +784,12 @@ __global__ void __launch_bounds__(256) k_s_residual(SGeo g, const float* __restr
 }
 
 // The refinement residual r = b - L (hi + lo) to FP64-class accuracy (pair_residual), with hi = x or x + e (then written to
-// xn), and lo from a field or zero; a thread a point of one component and colour, along z.
+// xn), and lo from a field or zero; a thread takes four places of one component's row, one colour after the other, along z.
+// Launch bounds: blocks on an SM against values in registers.  225 x 161 x 193, with lo / without, us: 135 / 99 with as many
+// registers as the compiler takes (78 / 73: blocks of 224 threads just miss a fourth), 118 / 89 so (some spill); 129^3 47 / 33,
+// 44 / 31.
 template <bool kAdd, bool kLo>
-__global__ void __launch_bounds__(256) k_s_residual_pair(SGeo g, PairCoef cf, const float* __restrict__ x,
+__global__ void __launch_bounds__(256, kLo ? 3 : 4) k_s_residual_pair(SGeo g, PairCoef cf, const float* __restrict__ x,
                                                          const float* __restrict__ e, const float* __restrict__ lo,
                                                          const float* __restrict__ b, float* __restrict__ xn,
                                                          float* __restrict__ r, double* __restrict__ part, unsigned zs) {
@@ -781,7 +797,7 @@ __global__ void __launch_bounds__(256) k_s_residual_pair(SGeo g, PairCoef cf, co
   constexpr int kField = kAdd ? RES_X_PLUS_E : RES_X;
   const unsigned i0 = 4 * (blockIdx.x * blockDim.x + threadIdx.x), y = blockIdx.y * blockDim.y + threadIdx.y + 1;
   const unsigned c = blockIdx.z % 3u, z0 = 1 + blockIdx.z / 3u * zs, z1 = min(g.nz - 1, z0 + zs);
-  float rr = 0.f;
+  PairSum rr;
   if (i0 < 4 * g.groups && y + 1 < g.ny) {
     for (unsigned col = 0; col < 2; ++col) {
       const size_t o0 = (size_t)z0 * g.pz + y * g.hx + i0, own = (2 * c + col) * g.cs + o0, oth = (2 * c + (col ^ 1u)) * g.cs + o0;
@@ -810,10 +826,10 @@ __global__ void __launch_bounds__(256) k_s_residual_pair(SGeo g, PairCoef cf, co
   }
         VG_PAIR(x) VG_PAIR(y) VG_PAIR(z) VG_PAIR(w)
 #undef VG_PAIR
-        if (x_interior(g, p, i0)) rr = fmaf(rv.x, rv.x, rr);
-        if (x_interior(g, p, i0 + 1)) rr = fmaf(rv.y, rv.y, rr);
-        if (x_interior(g, p, i0 + 2)) rr = fmaf(rv.z, rv.z, rr);
-        if (x_interior(g, p, i0 + 3)) rr = fmaf(rv.w, rv.w, rr);
+        const float vx = x_interior(g, p, i0) ? rv.x : 0.f, vy = x_interior(g, p, i0 + 1) ? rv.y : 0.f;
+        const float vz = x_interior(g, p, i0 + 2) ? rv.z : 0.f, vw = x_interior(g, p, i0 + 3) ? rv.w : 0.f;
+        rr.add(__fmaf_rn(vy, vy, __fmul_rn(vx, vx)));
+        rr.add(__fmaf_rn(vw, vw, __fmul_rn(vz, vz)));
         st4(r + own + o, rv);
         if (kAdd) st4(xn + own + o, h0);
         hm = hc;
@@ -823,7 +839,7 @@ __global__ void __launch_bounds__(256) k_s_residual_pair(SGeo g, PairCoef cf, co
       }
     }
   }
-  split_sum2<false>(rr, 0.f, part);
+  split_sum2<false>(rr, PairSum(), part);
 }
 
 // a += b over split fields (n4 float4 groups).
