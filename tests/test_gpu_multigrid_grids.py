@@ -144,3 +144,20 @@ def test_norms_of_whole_numbers(n3):
     ctx.check(vg.lib().vg_multigrid_device(ctx.h, ctypes.byref(grid), vg._ptr(soln), vg._ptr(rhs), 1e-6, 50,
                                            ctypes.byref(cyc), ctypes.byref(r0), ctypes.byref(r1)), "multigrid")
     assert abs(r0.value - want) <= 2e-13 * want
+
+
+@pytest.mark.parametrize("n3", [(33, 33, 33), (65, 65, 65)])
+def test_norms_out_of_range(n3):
+    """A right-hand side whose squares are beyond the floats is refused, and the
+    context solves the next one."""
+    import vortegrid_gb300 as vg
+    grid, start, rhs = problem(n3)
+    ctx, cyc, r = vg.Context(numerics=vg.NUMERICS_FAST), ctypes.c_int(), ctypes.c_double()
+
+    def status(x, b):
+        st = vg.lib().vg_multigrid_device(ctx.h, ctypes.byref(grid), vg._ptr(x), vg._ptr(b), 1e-6, 50, ctypes.byref(cyc),
+                                          ctypes.byref(r), ctypes.byref(r))
+        ctx.synchronize()
+        return st
+    assert status(torch.zeros_like(rhs), rhs * 1e20) == 3  # VG_NONFINITE
+    assert status(start.clone(), rhs) == 0

@@ -2028,6 +2028,8 @@ static vg_status split_adaptive(Ctx* c, const Geom& g, const MgPlan& P, float* s
     if ((st = next_norm(c, &rr, nullptr)) != VG_OK) return st;
     relres = std::sqrt(rr) / bn;
     if (relres <= tol || cyc >= max_cycles) break;
+    // norms of squares beyond the floats: no cycle could follow, nor an end
+    if (!std::isfinite(relres)) return fail(c, VG_NONFINITE, "multigrid: the residual's norm is out of range");
     const double inner_tol = std::max(0.9 * tol, 1e-4 * relres);
     const int ta = lo == 0 ? 1 : 0, tb = 3 - ta - std::max(lo, 0) - (lo < 0 ? 2 : 0);
     int t = ta;
@@ -2194,6 +2196,8 @@ vg_status run_multigrid(Ctx* c, const Geom& g, float* soln3, const float* rhs3, 
     if ((st = next_norm(c, &rr, nullptr)) != VG_OK) return st;
     relres = std::sqrt(rr) / bn;
     if (relres <= tol || cyc >= max_cycles) break;
+    // norms of squares beyond the floats: no cycle could follow, nor an end
+    if (!std::isfinite(relres)) return fail(c, VG_NONFINITE, "multigrid: the residual's norm is out of range");
     // The FP32 residual of the correction equation tracks the accurate residual
     // of soln3 + lo + e to ~1e-11 relative (its right-hand side is already below 1e-4),
     // so a tenth of the tolerance is margin enough for the FP64 check that follows.
