@@ -64,3 +64,24 @@ def test_full_cells(vg, ctx, sizes):
     rng = np.random.default_rng(len(sizes))
     cells = np.concatenate([np.full(m, 3 + 7 * k) for k, m in enumerate(sizes)] + [np.full(max(sizes) // 2, -1)])
     run(vg, ctx, (9, 8, 7), rng.permutation(cells))
+
+
+@pytest.mark.parametrize("sizes", [(100000,), (5000, 40000, 600, 8192, 513), (262144, 262145, 31, 8193), (1000003,)])
+@pytest.mark.parametrize("shuffled", [False, True])
+def test_large_cells(vg, ctx, sizes, shuffled):
+    """Cells that bitmaps order, one window and many, their chunks of slots shared
+    with other large cells, in index order and not, among scattered vortons."""
+    rng = np.random.default_rng(sum(sizes))
+    cells = np.concatenate([np.full(m, 5 + 11 * k) for k, m in enumerate(sizes)] + [rng.integers(100, 3000, 2000)])
+    run(vg, ctx, (17, 15, 13), rng.permutation(cells) if shuffled else cells)
+
+
+@pytest.mark.parametrize("others", [0, 900001])
+def test_many_vortons(vg, ctx, others):
+    """More than 2^20 vortons: large cells are sorted up to 8,192 vortons and ordered by bitmaps beyond."""
+    rng = np.random.default_rng(others + 1)
+    sizes = [513, 8192, 8193, 70000, 3000, 400000] + [9000] * 60
+    cells = np.concatenate([np.full(m, 7 * k) for k, m in enumerate(sizes)] + [rng.integers(600, 60000, others),
+                                                                              np.full(300000, -1)])
+    assert len(cells) > 1 << 20
+    run(vg, ctx, (65, 33, 31), rng.permutation(cells))

@@ -13,14 +13,16 @@
 //   4. k_order, one thread per slot, puts the cell's indices into ascending
 //      order -- the order in which the reference accumulates them -- by
 //      counting the smaller ones; cells of more than kCountMax vortons are left
-//      to k_order_large, which sorts up to kSortMax indices in shared memory and
-//      marks the indices of larger cells in a bitmap.
+//      to k_order_large, which marks their indices in bitmaps, a window of
+//      indices at a time (or sorts them in shared memory: few of many vortons).
 // The result does not depend on thread timing.
 //
 // Bound by launches and the latency of dependent accesses: seven small kernels,
 // 262,144 vortons on a 129^3 grid in 26 us.  (A stable radix sort by cell in two
 // passes of 11 bits, fifteen kernels, took 69 us; its scatter, three barriers to
 // every 256 keys of a tile, 13 us a pass.)
+#include <algorithm>
+
 #include "vg_internal.cuh"
 
 namespace vg {
@@ -144,8 +146,12 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_chunks(const unsigned* __
 // the first-level cache mostly; 512 of them take about 1 us.  kSortMax: 32 KB.
 constexpr unsigned kCountMax = 512, kSortMax = 8192;
 constexpr int kOrderThreads = 1024;
-constexpr unsigned kWindow = kSortMax * 32;  // indices of one bitmap
+constexpr unsigned kMaxWindowBits = 18, kMinWindowBits = 13;  // log2 of a bitmap's indices: 32 KB and 1 KB
+// Up to so many vortons a large cell's windows are few and bitmaps order it; of
+// more, cells of up to kSortMax are sorted (a bitmap's pass costs about 3 us).
+constexpr size_t kBitmapAll = (size_t)1 << 20;
 constexpr unsigned kMidCtas = 304, kBigCtas = 152;
+constexpr unsigned kChunk = 32;  // slots whose extreme indices k_order writes down: a warp's
 
 __global__ void k_place(int n, const unsigned* __restrict__ key, const unsigned* __restrict__ place,
                         const unsigned* __restrict__ start, uint2* __restrict__ slot) {
@@ -156,27 +162,42 @@ __global__ void k_place(int n, const unsigned* __restrict__ key, const unsigned*
   slot[start[k] + place[i]] = make_uint2(k, i);
 }
 
-// big[0], big[1]: the numbers of mid and big cells; their offsets follow, mid ones from mid_list, big ones from big_list.
-__global__ void k_order(int n, const uint2* __restrict__ slot, const unsigned* __restrict__ start,
+// big[0], big[1]: the numbers of mid cells (up to mid_max vortons) and of big
+// ones; their offsets follow in mid_list and big_list.  range: of a warp's slots
+// in such cells, the least and the greatest index.
+__global__ void k_order(int n, unsigned mid_max, const uint2* __restrict__ slot, const unsigned* __restrict__ start,
                         unsigned* __restrict__ items, unsigned* __restrict__ big, unsigned* __restrict__ mid_list,
-                        unsigned* __restrict__ big_list) {
+                        unsigned* __restrict__ big_list, uint2* __restrict__ range) {
   pdl_entry();
   const unsigned p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= (unsigned)n) return;
-  const uint2 me = slot[p];
-  const unsigned s = start[me.x], e = start[me.x + 1], m = e - s;
-  if (m <= kCountMax) {
+  const bool valid = p < (unsigned)n;
+  uint2 me = make_uint2(0, 0);
+  unsigned s = 0, e = 0;
+  if (valid) {
+    me = slot[p];
+    s = start[me.x];
+    e = start[me.x + 1];
+  }
+  const unsigned m = e - s;
+  const bool large = m > kCountMax;
+  if (large) {
+    if (p == s) {
+      if (m <= mid_max)
+        mid_list[atomicAdd(&big[0], 1u)] = me.x;
+      else
+        big_list[atomicAdd(&big[1], 1u)] = me.x;
+    }
+  } else if (valid) {
     unsigned rank = 0;
     if (m > 1)
 #pragma unroll 4
       for (unsigned q = s; q < e; ++q) rank += slot[q].y < me.y;
     items[s + rank] = me.y;
-  } else if (p == s) {
-    if (m <= kSortMax)
-      mid_list[atomicAdd(&big[0], 1u)] = me.x;
-    else
-      big_list[atomicAdd(&big[1], 1u)] = me.x;
   }
+  if (!__any_sync(0xffffffffu, large)) return;
+  const unsigned lo = __reduce_min_sync(0xffffffffu, large ? me.y : 0xffffffffu);
+  const unsigned hi = __reduce_max_sync(0xffffffffu, large ? me.y : 0u);
+  if ((threadIdx.x & 31) == 0) range[p / kChunk] = make_uint2(lo, hi);
 }
 
 // Bitonic sort of one cell's indices at a time (v: kSortMax values in shared memory).
@@ -204,48 +225,94 @@ __device__ __forceinline__ void order_mid(unsigned cta, unsigned ctas, const uin
   }
 }
 
-// One cell and one window of kWindow indices at a time: the cell's indices in
-// the window are marked in a bitmap (kSortMax words) and read off it, after those
-// before the window.
+// One cell and one window of indices at a time: the cell's indices in the window
+// are marked in a bitmap and read off it, after those before the window.  The
+// windows are as wide as leaves every CTA one.  Vortons get their places as
+// k_bin's blocks run, so that the indices of a chunk of slots lie close together:
+// by their range most chunks are before the window or behind it as a whole.
+// Whole builds, us, by a radix sort / windows of 2^18 that read all slots of their
+// cell, and a sort of every cell up to kSortMax / this: 10,000 vortons, half of
+// them in one cell 72 / 78 / 46; 100,000 in one cell 134 / 145 / 53; 16 million in
+// 64 cells 1,711 / 2,023 / 1,506, in one cell 11,231 / 3,135 / 2,168, in cells of
+// their own 994 / 623 / 634.
 __device__ __forceinline__ void order_big(unsigned cta, unsigned ctas, int n, const uint2* __restrict__ slot,
-                                          const unsigned* __restrict__ start, const unsigned* __restrict__ big,
-                                          const unsigned* __restrict__ big_list, unsigned* __restrict__ items,
-                                          unsigned* bits) {
-  constexpr unsigned kWords = kSortMax, kPer = kWords / kOrderThreads;
+                                          const uint2* __restrict__ range, const unsigned* __restrict__ start,
+                                          const unsigned* __restrict__ big, const unsigned* __restrict__ big_list,
+                                          unsigned* __restrict__ items, unsigned* bits) {
   __shared__ unsigned sh[32], warp_sum[32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x / 32;
-  const unsigned windows = ((unsigned)n + kWindow - 1) / kWindow;
-  const unsigned long long units = (unsigned long long)big[1] * windows;
+  const unsigned cells = big[1];
+  unsigned log = kMaxWindowBits;
+  auto windows_of = [&](unsigned b) { return ((unsigned)n + (1u << b) - 1) >> b; };
+  while (log > kMinWindowBits && (unsigned long long)cells * windows_of(log) < ctas) --log;
+  const unsigned window = 1u << log, words = window / 32, per = words > kOrderThreads ? words / kOrderThreads : 1;
+  const unsigned windows = windows_of(log);
+  const unsigned long long units = (unsigned long long)cells * windows;
   for (unsigned long long u = cta; u < units; u += ctas) {
-    const unsigned cell = big_list[u / windows], first = (unsigned)(u % windows) * kWindow;
-    const unsigned s = start[cell], e = start[cell + 1];
-    for (unsigned w = threadIdx.x; w < kWords; w += kOrderThreads) bits[w] = 0;
+    const unsigned cell = big_list[u / windows], first = (unsigned)(u % windows) << log;
+    const unsigned s = start[cell], e = start[cell + 1], c1 = (e - 1) / kChunk;
+    for (unsigned w = threadIdx.x; w < words; w += kOrderThreads) bits[w] = 0;
     __syncthreads();
     unsigned before = 0;
-#pragma unroll 4
-    for (unsigned q = s + threadIdx.x; q < e; q += kOrderThreads) {
-      const unsigned i = slot[q].y;
-      before += i < first;
-      if (i >= first && i - first < kWindow) atomicOr(&bits[(i - first) / 32], 1u << (i & 31));
+    // a warp looks at every 32nd chunk, 32 of them at a time, then at the slots of those that it has to, 8 at a time
+    for (unsigned c0 = s / kChunk + wid; c0 <= c1; c0 += kOrderThreads) {
+      const unsigned c = c0 + 32 * lane;
+      bool in = false;
+      if (c <= c1) {
+        const uint2 r = range[c];
+        if (r.y < first)
+          before += min(c * kChunk + kChunk, e) - max(c * kChunk, s);
+        else
+          in = r.x < first + window;
+      }
+      unsigned todo = __ballot_sync(0xffffffffu, in);
+      while (todo) {
+        constexpr int kAt = 8;
+        unsigned i[kAt];
+#pragma unroll
+        for (int k = 0; k < kAt; ++k, todo &= todo - 1) {
+          const unsigned q = (c0 + 32 * (__ffs(todo) - 1)) * kChunk + lane;
+          i[k] = todo && q >= s && q < e ? slot[q].y : 0xffffffffu;
+        }
+#pragma unroll
+        for (int k = 0; k < kAt; ++k) {
+          before += i[k] < first;
+          if (i[k] >= first && i[k] - first < window) atomicOr(&bits[(i[k] - first) / 32], 1u << (i[k] & 31));
+        }
+      }
     }
     before = block_sum<kOrderThreads>(before, sh);  // its barriers also end the marking
+    const unsigned w0 = threadIdx.x * per;  // this thread's words; none past the bitmap
     unsigned cnt = 0;
-#pragma unroll
-    for (unsigned w = 0; w < kPer; ++w) cnt += __popc(bits[threadIdx.x * kPer + w]);
+    if (w0 < words)
+      for (unsigned w = 0; w < per; ++w) cnt += __popc(bits[w0 + w]);
     const unsigned inc = warp_inclusive(cnt);
     if (lane == 31) warp_sum[wid] = inc;
     __syncthreads();
     const unsigned ws_ = warp_sum[lane], winc = warp_inclusive(ws_);
     unsigned at = s + before + __shfl_sync(0xffffffffu, winc - ws_, wid) + inc - cnt;
-    for (unsigned w = 0; w < kPer; ++w)
-      for (unsigned x = bits[threadIdx.x * kPer + w]; x; x &= x - 1)
-        items[at++] = first + (threadIdx.x * kPer + w) * 32 + __ffs(x) - 1;
+    if (__shfl_sync(0xffffffffu, winc, 31) > 4 * words) {  // a word a warp, its indices side by side
+      for (unsigned l = 0; l < 32; ++l) {
+        unsigned to = __shfl_sync(0xffffffffu, at, l);
+        const unsigned wl = (wid * 32 + l) * per;
+        if (wl >= words) break;
+        for (unsigned w = wl; w < wl + per; ++w) {
+          const unsigned x = bits[w];
+          if ((x >> lane) & 1u) items[to + __popc(x & ((1u << lane) - 1u))] = first + w * 32 + lane;
+          to += __popc(x);
+        }
+      }
+    } else if (w0 < words) {
+      for (unsigned w = w0; w < w0 + per; ++w)
+        for (unsigned x = bits[w]; x; x &= x - 1) items[at++] = first + w * 32 + __ffs(x) - 1;
+    }
     __syncthreads();
   }
 }
 
 // The cells that k_order left: the first mid_ctas CTAs take the mid ones, the others the big ones.
 __global__ void __launch_bounds__(kOrderThreads) k_order_large(int n, unsigned mid_ctas, const uint2* __restrict__ slot,
+                                                               const uint2* __restrict__ range,
                                                                const unsigned* __restrict__ start,
                                                                const unsigned* __restrict__ big,
                                                                const unsigned* __restrict__ mid_list,
@@ -256,7 +323,7 @@ __global__ void __launch_bounds__(kOrderThreads) k_order_large(int n, unsigned m
   if (blockIdx.x < mid_ctas)
     order_mid(blockIdx.x, mid_ctas, slot, start, big, mid_list, items, v);
   else
-    order_big(blockIdx.x - mid_ctas, gridDim.x - mid_ctas, n, slot, start, big, big_list, items, v);
+    order_big(blockIdx.x - mid_ctas, gridDim.x - mid_ctas, n, slot, range, start, big, big_list, items, v);
 }
 
 }  // namespace
@@ -286,16 +353,19 @@ vg_status build_cell_lists(Ctx* c, const Geom& g, const float4* ps, size_t n, Ce
   vg_status st = VG_OK;
   // one slot per grid point and one for vortons outside the grid
   const size_t slots = ncells + 1;
-  // S_CELL: slot (2 n), key and later items, place (n each), lists of the mid and the big cells
-  const size_t mids = n / (kCountMax + 1) + 1, bigs = n / (kSortMax + 1) + 1;
-  uint2* slot = (uint2*)ws(c, S_CELL, (4 * n + mids + bigs) * sizeof(unsigned), &st);
+  // cells of up to mid_max vortons are sorted, larger ones ordered by bitmaps
+  const unsigned mid_max = n > kBitmapAll ? kSortMax : kCountMax;
+  // S_CELL: slot (2 n), ranges (2 chunks), key and later items, place (n each), lists of the mid and the big cells
+  const size_t mids = n / (kCountMax + 1), bigs = n / (mid_max + 1), chunks = (n + kChunk - 1) / kChunk;
+  uint2* slot = (uint2*)ws(c, S_CELL, (4 * n + 2 * chunks + mids + bigs + 2) * sizeof(unsigned), &st);
   if (st != VG_OK) return st;
   // S_COUNT: count (slots), numbers of mid and big cells
   unsigned* count = (unsigned*)ws(c, S_COUNT, (slots + 2) * sizeof(unsigned), &st);
   if (st != VG_OK) return st;
   unsigned* start = (unsigned*)ws(c, S_START, (slots + 1) * sizeof(unsigned), &st);
   if (st != VG_OK) return st;
-  unsigned* key = (unsigned*)(slot + n);
+  uint2* range = slot + n;
+  unsigned* key = (unsigned*)(range + chunks);
   unsigned *place = key + n, *items = key, *mid_list = place + n, *big_list = mid_list + mids;
   unsigned* big = count + slots;
   VG_CUDA(c, cudaMemsetAsync(count, 0, (slots + 2) * sizeof(unsigned), c->stream));
@@ -309,14 +379,17 @@ vg_status build_cell_lists(Ctx* c, const Geom& g, const float4* ps, size_t n, Ce
     pdl_launch(c->stream, blocks_for(n, 256), 256, 0, k_place, (int)n, (const unsigned*)key, (const unsigned*)place,
                (const unsigned*)start, slot);
     VG_LAUNCHED(c);
-    pdl_launch(c->stream, blocks_for(n, 256), 256, 0, k_order, (int)n, (const uint2*)slot, (const unsigned*)start, items,
-               big, mid_list, big_list);
+    pdl_launch(c->stream, blocks_for(n, 256), 256, 0, k_order, (int)n, mid_max, (const uint2*)slot, (const unsigned*)start,
+               items, big, mid_list, big_list, range);
     VG_LAUNCHED(c);
   }
   if (n > kCountMax) {
-    const unsigned mid_ctas = (unsigned)(mids - 1 < kMidCtas ? mids - 1 : kMidCtas), big_ctas = n > kSortMax ? kBigCtas : 0;
+    const unsigned mid_ctas = n > kBitmapAll ? (unsigned)std::min<size_t>(mids, kMidCtas) : 0;
+    // as many as there can be windows of large cells
+    const unsigned big_ctas = (unsigned)std::min<size_t>(bigs * ((n >> kMinWindowBits) + 1), kBigCtas);
     pdl_launch(c->stream, mid_ctas + big_ctas, kOrderThreads, 0, k_order_large, (int)n, mid_ctas, (const uint2*)slot,
-               (const unsigned*)start, (const unsigned*)big, (const unsigned*)mid_list, (const unsigned*)big_list, items);
+               (const uint2*)range, (const unsigned*)start, (const unsigned*)big, (const unsigned*)mid_list,
+               (const unsigned*)big_list, items);
     VG_LAUNCHED(c);
   }
   VG_CUDA(c, cudaGetLastError());
