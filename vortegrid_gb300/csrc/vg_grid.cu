@@ -325,7 +325,15 @@ __global__ void k_pse_gather(const float4* __restrict__ ps, const float4* __rest
 // their slots.  kLanes neighbouring lanes take a particle's lists in turn; the
 // caller adds their sums (sum_lanes).  k_pse, 10^6 vortons at 225 x 161 x 193: 177 -> 118 us, 262,144 at
 // 129^3: 57 -> 36 us, 32 sets of 32,768: 65 -> 26 us each.
+//
+// In dense cells a warp's particles have the same lists, and finding the next one's place costs more than the longest
+// list does.  Warps with kDense particles a list or more on average (one lane to a particle) go list by list, the own
+// cell's apart because the particle itself is in it, four particles' loads at a time.  Whole calls, us, a loop to every
+// list as before / one loop / this: 600,000 vortons on 33^3 points (17 a cell) 444 / 493 / 362, 400,000 on 49 x 33 x 41
+// (6) 214 / 185 / 162, 1.5 million on 17^3 (305) 12,022 / 16,956 / 10,066; below kDense the same as one loop.  By a line
+// of their own, without the warp, particles near it took both loops: up to 30 % more.
 constexpr int kPseThreads = 128;
+constexpr unsigned kDense = 5;
 template <bool kAll, int kLanes, typename Load, typename Body>
 __device__ __forceinline__ void for_neighbours(int nx, int ny, int nz, int cx, int cy, int cz, unsigned t,
                                                const unsigned* __restrict__ start, const Load& load,
@@ -350,14 +358,33 @@ __device__ __forceinline__ void for_neighbours(int nx, int ny, int nz, int cx, i
     }
   }
   int cnt = 0, own = 0, lower = 0;  // lists kept, and of them the own cell's, and those up to the lower side's
+  unsigned total = 0;               // particles in them
 #pragma unroll
   for (int q = 0; q < kMine; ++q) {
     const int r = q * kLanes + (int)(threadIdx.x % kLanes);
     if (range[q].x < range[q].y) lists[cnt++][threadIdx.x] = range[q];
+    total += range[q].y - range[q].x;
     if (r == 0) own = cnt;
     if (r < kSide) lower = cnt;
   }
+  // the warp's lanes that are here: one loop for all of them
+  const unsigned active = __activemask();
+  const bool dense = kLanes == 1 && __reduce_add_sync(active, min(total, 1u << 20)) >= kDense * kLists * __popc(active);
   if (cnt == 0) return;
+  if (dense) {
+    for (int r = 0; r < cnt; ++r) {
+      const uint2 list = lists[r][threadIdx.x];
+      if (r < own) {
+        for (unsigned slot = list.x; slot < list.y; ++slot)
+          if (slot != t) body(load(slot), t < slot);
+      } else {
+        const bool here = r >= lower;
+#pragma unroll 4
+        for (unsigned slot = list.x; slot < list.y; ++slot) body(load(slot), here);
+      }
+    }
+    return;
+  }
   int r = 0;
   uint2 at = lists[0][threadIdx.x];
   auto value = load(at.x);
