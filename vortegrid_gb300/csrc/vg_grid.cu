@@ -604,12 +604,18 @@ __global__ void k_vel_points(size_t pts, const float* __restrict__ v3, float4* _
 // Bound by the first-level cache's lines a cycle: a tracer's corners lie in
 // four rows, and one load of eight lanes takes each row's line once, where a
 // thread that loads its tracer's corners itself takes one for every corner.
-// 2^22 tracers on 129^3 points: 88 us, and 7 us for the float4 points, against
-// 228 us from the three-float grid (a thread to a tracer, 24 loads) and 128 us + 84 us
+// 2^22 tracers on 129^3 points: 99 us, and 7 us for the float4 points, against
+// 228 us from the three-float grid (a thread to a tracer, 24 loads) and 136 us + 84 us
 // from a copy of the grid with each cell's corners in a line of their own.
-__global__ void __launch_bounds__(256) k_gather_advect_points(Geom g, const float4* __restrict__ vp,
-                                                              float4* __restrict__ pos, float4* __restrict__ vel,
-                                                              int m, float dt, int evolve, int* __restrict__ flag) {
+//
+// Neighbouring tracers in one line's cells need none of that: a warp in which fewer
+// than kFewLines lanes change the line loads by thread (tracers in the order of
+// their cells 63 us, all eight lanes 107; in one cell 49 and 90, from the
+// three-float grid 46).  Six blocks an SM: 40 registers, 48 else (69 and 56 us).
+constexpr int kFewLines = 16;
+__global__ void __launch_bounds__(256, 6) k_gather_advect_points(Geom g, const float4* __restrict__ vp,
+                                                                 float4* __restrict__ pos, float4* __restrict__ vel,
+                                                                 int m, float dt, int evolve, int* __restrict__ flag) {
   pdl_entry();
   const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
   const bool valid = i < (unsigned)m;  // all lanes take part in the exchanges
@@ -631,35 +637,50 @@ __global__ void __launch_bounds__(256) k_gather_advect_points(Geom g, const floa
   const int lane = threadIdx.x & 31, q = lane & 7, group = lane & 24;
   const unsigned bx = q & 1, by = (q >> 1) & 1, bz = q >> 2;
   const unsigned corner = bx + nx * by + nxy * bz;
-  float4 c[8];
+  float4 c[8], u;
+  // lanes whose tracer's cell lies in another line than the lane's before it; 8 points of a row to a line
+  const unsigned before = __shfl_up_sync(0xffffffffu, base, 1);
+  if (__popc(__ballot_sync(0xffffffffu, base >> 3 != before >> 3)) < kFewLines) {
+    if (!valid) return;
 #pragma unroll
-  for (int r = 0; r < 8; ++r) c[r] = vp[__shfl_sync(0xffffffffu, base, group + r) + corner];
-  auto weight = [&](float t, unsigned bit, int from) {  // 1 - t or t of the tracer of lane `from`
-    const float w = __shfl_sync(0xffffffffu, t, from);
-    return bit ? w : __fsub_rn(1.0f, w);
-  };
-  auto times = [](float4 v, float w) {
-    return make_float4(__fmul_rn(v.x, w), __fmul_rn(v.y, w), __fmul_rn(v.z, w), 0.f);
-  };
-  // keeps one of two tracers' terms, by the lane's bit, and adds the partner's term of the same tracer
-  auto exchange = [](float4 t0, float4 t1, unsigned bit, int apart) {
-    const float4 keep = bit ? t1 : t0, give = bit ? t0 : t1;
-    return make_float4(__fadd_rn(keep.x, __shfl_xor_sync(0xffffffffu, give.x, apart)),
-                       __fadd_rn(keep.y, __shfl_xor_sync(0xffffffffu, give.y, apart)),
-                       __fadd_rn(keep.z, __shfl_xor_sync(0xffffffffu, give.z, apart)), 0.f);
-  };
-  float4 sx[4], sy[2];
+    for (unsigned k = 0; k < 8; ++k) c[k] = vp[base + (k & 1) + nx * ((k >> 1) & 1) + nxy * (k >> 2)];
+    auto mix = [](float4 a, float4 b, float t) {  // (1 - t) a + t b
+      const float s = __fsub_rn(1.0f, t);
+      return make_float4(__fadd_rn(__fmul_rn(s, a.x), __fmul_rn(t, b.x)), __fadd_rn(__fmul_rn(s, a.y), __fmul_rn(t, b.y)),
+                         __fadd_rn(__fmul_rn(s, a.z), __fmul_rn(t, b.z)), 0.f);
+    };
+    u = mix(mix(mix(c[0], c[1], tw[0]), mix(c[2], c[3], tw[0]), tw[1]),
+            mix(mix(c[4], c[5], tw[0]), mix(c[6], c[7], tw[0]), tw[1]), tw[2]);
+  } else {
 #pragma unroll
-  for (int r = 0; r < 4; ++r)
-    sx[r] = exchange(times(c[2 * r], weight(tw[0], bx, group + 2 * r)),
-                     times(c[2 * r + 1], weight(tw[0], bx, group + 2 * r + 1)), bx, 1);
+    for (int r = 0; r < 8; ++r) c[r] = vp[__shfl_sync(0xffffffffu, base, group + r) + corner];
+    auto weight = [&](float t, unsigned bit, int from) {  // 1 - t or t of the tracer of lane `from`
+      const float w = __shfl_sync(0xffffffffu, t, from);
+      return bit ? w : __fsub_rn(1.0f, w);
+    };
+    auto times = [](float4 v, float w) {
+      return make_float4(__fmul_rn(v.x, w), __fmul_rn(v.y, w), __fmul_rn(v.z, w), 0.f);
+    };
+    // keeps one of two tracers' terms, by the lane's bit, and adds the partner's term of the same tracer
+    auto exchange = [](float4 t0, float4 t1, unsigned bit, int apart) {
+      const float4 keep = bit ? t1 : t0, give = bit ? t0 : t1;
+      return make_float4(__fadd_rn(keep.x, __shfl_xor_sync(0xffffffffu, give.x, apart)),
+                         __fadd_rn(keep.y, __shfl_xor_sync(0xffffffffu, give.y, apart)),
+                         __fadd_rn(keep.z, __shfl_xor_sync(0xffffffffu, give.z, apart)), 0.f);
+    };
+    float4 sx[4], sy[2];
 #pragma unroll
-  for (int r = 0; r < 2; ++r)
-    sy[r] = exchange(times(sx[2 * r], weight(tw[1], by, group + 4 * r + bx)),
-                     times(sx[2 * r + 1], weight(tw[1], by, group + 4 * r + 2 + bx)), by, 2);
-  const float4 u = exchange(times(sy[0], weight(tw[2], bz, group + 2 * by + bx)),
-                            times(sy[1], weight(tw[2], bz, group + 4 + 2 * by + bx)), bz, 4);
-  if (!valid) return;
+    for (int r = 0; r < 4; ++r)
+      sx[r] = exchange(times(c[2 * r], weight(tw[0], bx, group + 2 * r)),
+                       times(c[2 * r + 1], weight(tw[0], bx, group + 2 * r + 1)), bx, 1);
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+      sy[r] = exchange(times(sx[2 * r], weight(tw[1], by, group + 4 * r + bx)),
+                       times(sx[2 * r + 1], weight(tw[1], by, group + 4 * r + 2 + bx)), by, 2);
+    u = exchange(times(sy[0], weight(tw[2], bz, group + 2 * by + bx)),
+                 times(sy[1], weight(tw[2], bz, group + 4 + 2 * by + bx)), bz, 4);
+    if (!valid) return;
+  }
   if (!inside) {
     atomicOr(flag, (int)DF_OUT_OF_GRID);
     if (vel) vel[i] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -887,10 +908,11 @@ bool unpack_records(const Geom& g, size_t m) {
 
 // Tracers of the step's own grid gather from its float4 points where the copy
 // (made once per step) pays: it costs 4 ns per 1000 points, and saves 25 to
-// 35 ns per 1000 tracers.  2^18 tracers, copy included, against the three-float
+// 35 ns per 1000 tracers in no order.  2^18 tracers, copy included, against the three-float
 // grid: 9.3 against 10.7 us on 33^3 points, 10.2 against 15.6 on 65^3, 16.2
 // against 16.8 on 129^3 (eight points to a tracer); 2^20 tracers on 193^3
-// points (seven to a tracer) 62.5 against 64.1.
+// points (seven to a tracer) 62.5 against 64.1.  Tracers in the order of their
+// cells gain nothing from it and pay the copy (10^6 on 129^3 24 us and 7).
 static bool gather_points(const Geom& g, size_t m) {
   const size_t pts = g.points();
   return g.np[0] >= 2 && g.np[1] >= 2 && g.np[2] >= 2 && pts < ((size_t)1 << 31) && m >= ((size_t)1 << 18) &&
