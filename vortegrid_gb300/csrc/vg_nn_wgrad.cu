@@ -266,12 +266,21 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3_wgrad_rows(const ConvIn i
       pb = pb + 1 == kXSlabs ? 0 : pb + 1;
     }
     if (want_db) {  // lanes of equal parity hold the same 8 channels
+      __shared__ float sh_db[kCopyThreads / 32][16];
 #pragma unroll
       for (int j = 0; j < 8; ++j)
         for (int o = 16; o > 1; o >>= 1) sum[j] += __shfl_xor_sync(0xffffffffu, sum[j], o);
       if (lane < 2)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) atomicAdd(db + co0 + c * 8 + j, sum[j]);
+        for (int j = 0; j < 8; ++j) sh_db[warp][c * 8 + j] = sum[j];
+      // one addition to db a CTA: its rounding is of the whole sum, so that one a warp made the error 1.4 times the column
+      // sum kernel's
+      asm volatile("bar.sync 1, %0;" ::"n"(kCopyThreads) : "memory");
+      if (tid < 16) {
+        float t = 0.f;
+        for (int w = 0; w < kCopyThreads / 32; ++w) t += sh_db[w][tid];
+        atomicAdd(db + co0 + tid, t);
+      }
     }
   } else if (warp == kMmaWarp) {
     // ---- MMAs.  Ring positions of X: xl the newest slab received (plane zt), xo the oldest not given back.
