@@ -511,6 +511,12 @@ int direct_split(int kind, size_t n, size_t m, unsigned* tblocks_out, unsigned* 
   return chunk;
 }
 
+// The plan's source tile, once its chunks are set.
+void set_tile(PairPlan& P) {
+  const int longest = std::max(P.row_ctas ? P.row_chunk : 1, P.gen_ctas ? P.gen_chunk : 1);
+  P.tile = std::min(kPairTile, longest);
+}
+
 // The source split of a k_direct_pair launch.  Each class of targets (grid
 // rows, general points) gets its own number of source chunks, chosen to
 // minimise the estimated time: the CTAs of both classes run in one wave
@@ -518,11 +524,6 @@ int direct_split(int kind, size_t n, size_t m, unsigned* tblocks_out, unsigned* 
 // CTA's time is its chunk length times the class's packed operations per
 // source and thread (row CTAs 8 + 4 x 9 = 44, general CTAs 4 x 17 = 68), plus
 // a fixed set-up; more chunks cost more partial sums to reduce.
-void set_tile(PairPlan& P) {
-  const int longest = std::max(P.row_ctas ? P.row_chunk : 1, P.gen_ctas ? P.gen_chunk : 1);
-  P.tile = std::min(kPairTile, longest);
-}
-
 PairPlan plan_pair(size_t n, size_t m, const Geom* grid) {
   PairPlan P = {};
   if (grid) {

@@ -329,7 +329,6 @@ enum Slot {
   S_CELL,
   S_COUNT,
   S_START,
-  S_ITEMS,
   S_SCAN,
   S_TREE,
   S_NEGVORT,
