@@ -332,9 +332,9 @@ __device__ __forceinline__ void prolong_point(const Geom& F, const Geom& C, cons
 // colour and component a thread as float4, and with the threads marching a few planes along z a value of the other colour
 // comes from L2 once and not three times.  The point arithmetic is unchanged, and so is every result.
 //
-// GB300, 129^3 (fields of 26 MB, mostly in the 129 MB L2), us a launch, interleaved -> split: half sweep 13.1 -> 9..7; first
-// sweep 30.6 -> 11.3; residual + restriction 26.2 -> 18.8; prolongation 18.3 -> 10.9; x += e and the residual 9.0 + 18.0 ->
-// 30 (one pass, but of five fields, which no longer fit the L2 together).
+// GB300, 129^3, us a launch within a solve (fields of 26 MB, mostly in the 129 MB L2), interleaved -> split: half sweep
+// 13.1 -> 6.7; first sweep 30.6 -> 10.6; residual + restriction 26.2 -> 18.6; prolongation 18.3 -> 11.1; x += e and the
+// residual 9.0 + 18.0 -> 26.4 (one pass, but of five fields, which no longer fit the L2 together).
 struct SGeo {
   unsigned nx, ny, nz, m, hx, groups;  // points, (nx - 1) / 2, floats of a row, float4 groups that hold interior points
   size_t cs;                           // floats of one component and colour
@@ -376,9 +376,10 @@ static SLaunch split_launch(const SGeo& g) {
   while (by > 8 && by - 8 >= g.ny - 2) by -= 8;
   SLaunch L;
   L.block = dim3(bx, by);
-  // marching planes saves reads of the plane before and behind; short marches keep enough threads on the chip.  Half sweep,
-  // us at 1 / 2 / 4 / 8 planes: 225 x 161 x 193 36.7 / 32.5 / 30.7 / 29.9, its whole solve best at 4; 129^3 (0.77 M threads
-  // at one plane) 10.7 / 9.2 / 9.9 / 10.9
+  // marching planes saves reads of the plane before and behind; short marches keep enough threads on the chip.  Half sweep
+  // within a solve, us at 1 / 2 / 4 / 8 planes: 225 x 161 x 193 (2.55 M threads at one plane) 35.0 / 30.6 / 28.4 / 26.9, but
+  // the whole step best at 4 (3,418 / 3,334 / 3,130 / 3,235); 129^3 (0.77 M) 8.1 / 6.7 / 7.0 / 7.2; 65^3 (0.1 M)
+  // 2.8 / 3.2 / 4.2 / 6.4
   const double threads = 3.0 * g.groups * (g.ny - 2) * (g.nz - 2);
   L.zs = threads > 2e6 ? 4 : threads > 3e5 ? 2 : 1;
   while (3 * (size_t)((g.nz - 2 + L.zs - 1) / L.zs) > kMaxGridZ) L.zs *= 2;  // long boxes: as many blocks as a launch can have
@@ -631,7 +632,7 @@ __device__ __forceinline__ void split_sum2(PairSum a, PairSum b2, double* __rest
 // stream wait took 15 to 20 us a norm more.  (Summing in the residual kernels by their last block, instead of this launch,
 // made them 4 to 10 us longer: a fence and an atomic at every block's end.)
 // Bound by FP64 additions, 16 cycles a warp: 1,024 threads with five additions each in the trees took 6.6 us at 129^3 and
-// 5.1 at 33^3, 256 threads take 4.5 and 3.0 (128 threads the same at 129^3).
+// 5.1 at 33^3, 256 threads take 4.3 and 2.6 (128 threads the same at 129^3).
 constexpr int kNormThreads = 256;
 __global__ void __launch_bounds__(kNormThreads) k_s_norm(const double* __restrict__ part, int nb, double* __restrict__ out2,
                                                  int keep_b, unsigned long long* __restrict__ seq,
@@ -785,11 +786,11 @@ __global__ void __launch_bounds__(256) k_s_residual(SGeo g, const float* __restr
 
 // The refinement residual r = b - L (hi + lo) to FP64-class accuracy (pair_residual), with hi = x or x + e (then written to
 // xn), and lo from a field or zero; a thread takes four places of one component's row, one colour after the other, along z.
-// Launch bounds: blocks on an SM against values in registers.  225 x 161 x 193, with lo / without, us: 135 / 99 with as many
-// registers as the compiler takes (78 / 73: blocks of 224 threads just miss a fourth), 118 / 89 so (some spill); 129^3 47 / 33,
-// 44 / 31.
+// Launch bounds: blocks on an SM against values in registers and loads in flight.  225 x 161 x 193, with lo / without, us:
+// 135 / 99 with as many registers as the compiler takes (78 / 73: blocks of 224 threads just miss a fourth), 119 / 89 so
+// (96 / 64); 129^3 47 / 33, 41 / 31.
 template <bool kAdd, bool kLo>
-__global__ void __launch_bounds__(256, kLo ? 3 : 4) k_s_residual_pair(SGeo g, PairCoef cf, const float* __restrict__ x,
+__global__ void __launch_bounds__(256, kLo ? 2 : 4) k_s_residual_pair(SGeo g, PairCoef cf, const float* __restrict__ x,
                                                          const float* __restrict__ e, const float* __restrict__ lo,
                                                          const float* __restrict__ b, float* __restrict__ xn,
                                                          float* __restrict__ r, double* __restrict__ part, unsigned zs) {
