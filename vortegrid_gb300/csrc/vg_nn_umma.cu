@@ -48,52 +48,6 @@ constexpr int kCols = 256;                        // tensor-memory columns of a 
 constexpr int kMaxPlanes = 16;
 constexpr size_t kSmemTwo = 113 * 1024, kSmemOne = 226 * 1024;  // shared memory of a CTA at two and at one per SM
 constexpr size_t kTail = (2 * kMaxSlabs + 2 * kMaxPlanes) * 8 + 64;
-constexpr unsigned long long kWaitNs = 2000000000ull;
-
-__device__ __forceinline__ unsigned su32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ bool try_wait(unsigned mbar, unsigned parity) {
-  unsigned done;
-  asm volatile(
-      "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
-      : "=r"(done)
-      : "r"(mbar), "r"(parity)
-      : "memory");
-  return done != 0;
-}
-
-__device__ __forceinline__ void wait_phase(unsigned mbar, unsigned parity, volatile int* abort_word) {
-  for (int k = 0; k < 512; ++k)
-    if (try_wait(mbar, parity)) return;
-  unsigned long long t0, t;
-  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
-  while (!*abort_word) {
-    for (int k = 0; k < 16; ++k)
-      if (try_wait(mbar, parity)) return;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-    if (t - t0 > kWaitNs) *abort_word = 1;
-  }
-}
-
-// One arrival for the warp, after all of its lanes.
-__device__ __forceinline__ void arrive(unsigned mbar) {
-  __syncwarp();
-  if ((threadIdx.x & 31) == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
-}
-
-__device__ __forceinline__ void commit_to(unsigned mbar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
-}
-
-__device__ __forceinline__ bool elect_one() {
-  unsigned r;
-  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(r));
-  return r != 0;
-}
-
-__device__ __forceinline__ void cp_async16(unsigned dst, const void* src, int src_bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
-}
 
 // No-swizzle K-major descriptors: the low word holds the address and the distance of the second 8 channels, the high word
 // the distance of 8-row groups (and the descriptor version).
@@ -113,15 +67,6 @@ __device__ __forceinline__ void mma(unsigned d, unsigned a_lo, unsigned b_lo, un
       "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n}" ::"r"(d),
       "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(kDescHiA), "r"(kDescHiB), "r"(acc)
       : "memory");
-}
-
-// 16 consecutive FP32 accumulator columns of this thread's TMEM lane.
-__device__ __forceinline__ void tmem_ld16(unsigned taddr, unsigned* r) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
 }
 
 struct UmmaPlan {

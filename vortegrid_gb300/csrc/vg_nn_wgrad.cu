@@ -37,52 +37,6 @@ constexpr int kCopyThreads = 256, kMmaWarp = kCopyThreads / 32 + 4, kThreads = k
 constexpr int kDrains = 3;
 constexpr int kXSlabs = 6, kYSlabs = 5;
 constexpr unsigned kYSlab = 256 * 3 * 32;  // bytes of a dY slab: 256 voxels, three copies
-constexpr unsigned long long kWaitNs = 2000000000ull;
-
-__device__ __forceinline__ unsigned s32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ bool try_wait(unsigned mbar, unsigned parity) {
-  unsigned done;
-  asm volatile(
-      "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
-      : "=r"(done)
-      : "r"(mbar), "r"(parity)
-      : "memory");
-  return done != 0;
-}
-
-// Waits for a phase, 2 s at most; a wait that runs out sets the abort word, which ends every later wait at once.
-__device__ __forceinline__ void wait_phase(unsigned mbar, unsigned parity, volatile int* abort_word) {
-  for (int k = 0; k < 512; ++k)
-    if (try_wait(mbar, parity)) return;
-  unsigned long long t0, t;
-  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
-  while (!*abort_word) {
-    for (int k = 0; k < 16; ++k)
-      if (try_wait(mbar, parity)) return;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-    if (t - t0 > kWaitNs) *abort_word = 1;
-  }
-}
-
-__device__ __forceinline__ void arrive_warp(unsigned mbar) {
-  __syncwarp();
-  if ((threadIdx.x & 31) == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
-}
-
-__device__ __forceinline__ void commit_to(unsigned mbar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
-}
-
-__device__ __forceinline__ bool elect_one() {
-  unsigned r;
-  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(r));
-  return r != 0;
-}
-
-__device__ __forceinline__ void cp16(unsigned dst, const void* src, int src_bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
-}
 
 // MN-major operands of 16-channel groups (32-byte rows, 32-byte swizzle): 8-voxel groups 256 bytes apart, channel groups
 // one x row (W x 32 bytes) apart.
@@ -98,13 +52,6 @@ __device__ __forceinline__ void mma_wgrad(unsigned d, unsigned a_lo, unsigned b_
       : "memory");
 }
 
-__device__ __forceinline__ void ld16(unsigned taddr, unsigned* r) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
-}
 __device__ __forceinline__ void st16_zero(unsigned taddr) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr),
                "r"(0)
@@ -134,9 +81,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3_wgrad_rows(const ConvIn i
   const int s0 = (int)((long long)steps * blockIdx.y / gridDim.y), s1 = (int)((long long)steps * (blockIdx.y + 1) / gridDim.y);
   if (s0 >= s1) return;  // the whole CTA
   const int drains = min(kDrains, s1 - s0);  // drain k (from 0) comes after the first (k + 1) / drains of the steps
-  const unsigned s_x = s32(smem), s_y = s_x + kXSlabs * kXSlab;
+  const unsigned s_x = su32(smem), s_y = s_x + kXSlabs * kXSlab;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kXSlabs * kXSlab + kYSlabs * kYSlab);
-  const unsigned b_xf = s32(bars), b_xe = b_xf + 8 * kXSlabs, b_yf = b_xe + 8 * kXSlabs, b_ye = b_yf + 8 * kYSlabs,
+  const unsigned b_xf = su32(bars), b_xe = b_xf + 8 * kXSlabs, b_yf = b_xe + 8 * kXSlabs, b_ye = b_yf + 8 * kYSlabs,
                  b_done = b_ye + 8 * kYSlabs, b_free = b_done + 8;
   unsigned* tslot = reinterpret_cast<unsigned*>(bars + 2 * kXSlabs + 2 * kYSlabs + 2);
   volatile int* abort_word = reinterpret_cast<volatile int*>(tslot + 1);
@@ -158,7 +105,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3_wgrad_rows(const ConvIn i
   for (unsigned i = tid; i < kYSlabs * kYSlab / 16; i += kThreads)
     reinterpret_cast<uint4*>(smem + kXSlabs * kXSlab)[i] = make_uint4(0, 0, 0, 0);
   if (warp == kMmaWarp) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(s32(tslot)));
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(su32(tslot)));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -211,7 +158,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3_wgrad_rows(const ConvIn i
           if (XR * W % 128 == 0 || v < XR * W) {
             const bool in_y = (unsigned)y < (unsigned)H;
             const __nv_bfloat16* p = plane + (in_y ? (y >> sh) * xrow_c + (x >> sh) * C : 0);
-            cp16(dst + i * 4096u, p, in_y ? 16 : 0);
+            cp_async16(dst + i * 4096u, p, in_y ? 16 : 0);
           }
         }
         asm volatile("cp.async.commit_group;\n" ::);
@@ -247,10 +194,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3_wgrad_rows(const ConvIn i
       asm volatile("cp.async.wait_group 2;\n" ::: "memory");
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       for (; pend > 2; --pend) {
-        arrive_warp(b_xf + 8 * pb);
+        arrive(b_xf + 8 * pb);
         pb = pb + 1 == kXSlabs ? 0 : pb + 1;
       }
-      arrive_warp(b_yf + 8 * yb_);
+      arrive(b_yf + 8 * yb_);
       if (++yb_ == kYSlabs) {
         yb_ = 0;
         yphase ^= 1;
@@ -264,7 +211,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3_wgrad_rows(const ConvIn i
     asm volatile("cp.async.wait_all;\n" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     for (; pend; --pend) {
-      arrive_warp(b_xf + 8 * pb);
+      arrive(b_xf + 8 * pb);
       pb = pb + 1 == kXSlabs ? 0 : pb + 1;
     }
     if (want_db) {  // lanes of equal parity hold the same 8 channels
@@ -350,7 +297,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3_wgrad_rows(const ConvIn i
         const int dz = j / 6, row = (j / 3) % 2, dx = j % 3, dyt = w4 - row;  // tap dy + 1 of this X row and dY row
         const unsigned at = tmem + ((unsigned)(w4 * 32) << 16) + 16 * j;
         unsigned r[16];
-        ld16(at, r);
+        tmem_ld16(at, r);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
         for (int q = 0; q < 16; ++q) asm volatile("" : "+r"(r[q]));
@@ -363,7 +310,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_conv3_wgrad_rows(const ConvIn i
       }
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::);
-      arrive_warp(b_free);
+      arrive(b_free);
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::);
