@@ -164,7 +164,8 @@ vg_status vg_step_evolve(vg_ctx* ctx, void* particles, size_t n, size_t stride, 
  * Poisson technique, a fixed multigrid schedule) with records in pinned host
  * memory capture their work as a CUDA graph on the second identical call and
  * replay it on later ones (identical: the same record pointers, counts,
- * strides, dt, extra box, first vorton's size, configuration and workspace). */
+ * strides, dt, extra box, first vorton's size, configuration, workspace and
+ * grid of the multigrid's tables). */
 vg_status vg_step_advect(vg_ctx* ctx, void* vortons, size_t n, size_t stride, const float* extra_min,
                          const float* extra_max, float dt, unsigned frame, int evolve_vortons, void* tracers,
                          size_t m, size_t tracer_stride);
