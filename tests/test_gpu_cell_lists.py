@@ -85,3 +85,14 @@ def test_many_vortons(vg, ctx, others):
                                                                               np.full(300000, -1)])
     assert len(cells) > 1 << 20
     run(vg, ctx, (65, 33, 31), rng.permutation(cells))
+
+
+@pytest.mark.parametrize("sizes", [(96, 97, 128, 129), (256, 257, 512, 513), (1024, 1025, 2048, 2049), (4096, 4097, 8192),
+                                   tuple(range(90, 135)) * 40, tuple(range(500, 525)) * 30,
+                                   tuple(range(1010, 1040)) * 20, tuple(range(1900, 2200, 3)) * 8])
+@pytest.mark.parametrize("shuffled", [False, True])
+def test_sorted_cells(vg, ctx, sizes, shuffled):
+    """Cells that a warp, a group of warps or a CTA sorts, at the edges of what a thread holds of
+    them, one each and more than there are warps, groups and CTAs."""
+    cells = np.repeat(3 * np.arange(len(sizes)), sizes)
+    run(vg, ctx, (17, 25, 15), np.random.default_rng(len(cells)).permutation(cells) if shuffled else cells)

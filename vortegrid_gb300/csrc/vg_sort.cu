@@ -13,8 +13,8 @@
 //   4. k_order, one thread per slot, puts the cell's indices into ascending
 //      order -- the order in which the reference accumulates them -- by
 //      counting the smaller ones; cells of more than kCountMax vortons are left
-//      to k_order_large, which marks their indices in bitmaps, a window of
-//      indices at a time (or sorts them in shared memory: few of many vortons).
+//      to k_order_large, where a warp, a group of warps or a CTA sorts their
+//      indices in registers or marks them in bitmaps, a window of indices at a time.
 // The result does not depend on thread timing.
 //
 // Bound by launches and the latency of dependent accesses: seven small kernels,
@@ -142,15 +142,18 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_chunks(const unsigned* __
 }
 
 // ---- a cell's indices in ascending order -------------------------------------
-// kCountMax: a thread's count costs as many loads as its cell has vortons, from
-// the first-level cache mostly; 512 of them take about 1 us.  kSortMax: 32 KB.
-constexpr unsigned kCountMax = 512, kSortMax = 8192;
-constexpr int kOrderThreads = 1024;
+// Up to kCountMax vortons each counts the smaller indices of its cell, as many
+// loads as the cell has vortons; up to kWarpMax a warp sorts them, up to kGroupMax
+// a quarter of a CTA, up to sort_max a CTA; bitmaps order larger cells.  Whole
+// builds of 10^6 vortons, us, by a radix sort / counts up to 512 and sorts in shared
+// memory / this: 82 a cell 114 / 79 / 81, 125 a cell 114 / 87 / 78, 455 a cell
+// 116 / 156 / 79, 578 a cell 117 / 152 / 84, 1,371 a cell 121 / 129 / 89, 2,915 a cell
+// 132 / 135 / 115.  With kCountMax 192, 125 a cell take 89; with 48, four million at 41
+// a cell take 172, not 165.  A CTA instead of a quarter for 1,371 a cell: 110.
+constexpr unsigned kCountMax = 96, kWarpMax = 1024, kGroupMax = 2048, kSortMax = 8192;
+constexpr int kOrderThreads = 1024, kGroup = 256;
 constexpr unsigned kMaxWindowBits = 18, kMinWindowBits = 13;  // log2 of a bitmap's indices: 32 KB and 1 KB
-// Up to so many vortons a large cell's windows are few and bitmaps order it; of
-// more, cells of up to kSortMax are sorted (a bitmap's pass costs about 3 us).
-constexpr size_t kBitmapAll = (size_t)1 << 20;
-constexpr unsigned kMidCtas = 304, kBigCtas = 152;
+constexpr unsigned kOrderCtas = 152;
 constexpr unsigned kChunk = 32;  // slots whose extreme indices k_order writes down: a warp's
 
 __global__ void k_place(int n, const unsigned* __restrict__ key, const unsigned* __restrict__ place,
@@ -162,12 +165,15 @@ __global__ void k_place(int n, const unsigned* __restrict__ key, const unsigned*
   slot[start[k] + place[i]] = make_uint2(k, i);
 }
 
-// big[0], big[1]: the numbers of mid cells (up to mid_max vortons) and of big
-// ones; their offsets follow in mid_list and big_list.  range: of a warp's slots
-// in such cells, the least and the greatest index.
-__global__ void k_order(int n, unsigned mid_max, const uint2* __restrict__ slot, const unsigned* __restrict__ start,
-                        unsigned* __restrict__ items, unsigned* __restrict__ big, unsigned* __restrict__ mid_list,
-                        unsigned* __restrict__ big_list, uint2* __restrict__ range) {
+// Lists of the cells that k_order leaves, and their lengths.
+struct LargeCells {
+  unsigned* count;    // of each list
+  unsigned* cell[4];  // for a warp, for a group, for a CTA, for bitmaps
+};
+
+// range: of a warp's slots in cells for bitmaps, the least and the greatest index.
+__global__ void k_order(int n, unsigned sort_max, const uint2* __restrict__ slot, const unsigned* __restrict__ start,
+                        unsigned* __restrict__ items, LargeCells large, uint2* __restrict__ range) {
   pdl_entry();
   const unsigned p = blockIdx.x * blockDim.x + threadIdx.x;
   const bool valid = p < (unsigned)n;
@@ -179,13 +185,17 @@ __global__ void k_order(int n, unsigned mid_max, const uint2* __restrict__ slot,
     e = start[me.x + 1];
   }
   const unsigned m = e - s;
-  const bool large = m > kCountMax;
-  if (large) {
+  const bool big = m > sort_max;
+  if (__any_sync(0xffffffffu, big)) {
+    const unsigned lo = __reduce_min_sync(0xffffffffu, big ? me.y : 0xffffffffu);
+    const unsigned hi = __reduce_max_sync(0xffffffffu, big ? me.y : 0u);
+    if ((threadIdx.x & 31) == 0) range[p / kChunk] = make_uint2(lo, hi);
+  }
+  if (m > kCountMax) {
     if (p == s) {
-      if (m <= mid_max)
-        mid_list[atomicAdd(&big[0], 1u)] = me.x;
-      else
-        big_list[atomicAdd(&big[1], 1u)] = me.x;
+      const int k = (m > kWarpMax) + (m > kGroupMax) + big;
+      (k < 2 ? k == 0 ? large.cell[0] : large.cell[1]
+             : k == 2 ? large.cell[2] : large.cell[3])[atomicAdd(&large.count[k], 1u)] = me.x;
     }
   } else if (valid) {
     unsigned rank = 0;
@@ -194,35 +204,78 @@ __global__ void k_order(int n, unsigned mid_max, const uint2* __restrict__ slot,
       for (unsigned q = s; q < e; ++q) rank += slot[q].y < me.y;
     items[s + rank] = me.y;
   }
-  if (!__any_sync(0xffffffffu, large)) return;
-  const unsigned lo = __reduce_min_sync(0xffffffffu, large ? me.y : 0xffffffffu);
-  const unsigned hi = __reduce_max_sync(0xffffffffu, large ? me.y : 0u);
-  if ((threadIdx.x & 31) == 0) range[p / kChunk] = make_uint2(lo, hi);
 }
 
-// Bitonic sort of one cell's indices at a time (v: kSortMax values in shared memory).
-__device__ __forceinline__ void order_mid(unsigned cta, unsigned ctas, const uint2* __restrict__ slot,
-                                          const unsigned* __restrict__ start, const unsigned* __restrict__ big,
-                                          const unsigned* __restrict__ mid_list, unsigned* __restrict__ items,
-                                          unsigned* v) {
-  for (unsigned b = cta; b < big[0]; b += ctas) {
-    const unsigned cell = mid_list[b], s = start[cell], m = start[cell + 1] - s;
-    unsigned pow2 = 2;
-    while (pow2 < m) pow2 *= 2;
-    for (unsigned i = threadIdx.x; i < pow2; i += kOrderThreads) v[i] = i < m ? slot[s + i].y : 0xffffffffu;
+// Barrier of the kThreads threads that sort a cell.
+template <int kThreads>
+__device__ __forceinline__ void sort_sync() {
+  if constexpr (kThreads == kOrderThreads)
     __syncthreads();
-    for (unsigned k = 2; k <= pow2; k *= 2)
-      for (unsigned j = k / 2; j > 0; j /= 2) {
-        for (unsigned t = threadIdx.x; t < pow2 / 2; t += kOrderThreads) {
-          const unsigned lo = 2 * t - (t & (j - 1)), hi = lo + j;
-          const unsigned a = v[lo], c = v[hi];
-          if ((a > c) == ((lo & k) == 0)) v[lo] = c, v[hi] = a;
-        }
-        __syncthreads();
-      }
-    for (unsigned i = threadIdx.x; i < m; i += kOrderThreads) items[s + i] = v[i];
-    __syncthreads();
+  else
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + (int)threadIdx.x / kThreads), "n"(kThreads) : "memory");
+}
+
+// Bound by the latency of a cell's chain (list, start, slots, then the exchanges),
+// hence few barriers: only pairs in different warps meet in shared memory.
+// Bitonic sort of m indices (up to kThreads R) from slot to items, R of them in a
+// thread's registers: thread t ends with those of ranks t R to t R + R - 1.  Pairs
+// R or more apart are exchanged between the lanes of a warp, those 32 R or more
+// apart by v (kThreads R values; unused for a warp).
+template <int kThreads, int R>
+__device__ __forceinline__ void sort_cell(int t, unsigned m, const uint2* __restrict__ slot,
+                                          unsigned* __restrict__ items, unsigned* v) {
+  unsigned x[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const unsigned i = r * kThreads + t;
+    x[r] = i < m ? slot[i].y : 0xffffffffu;  // no index: those of vortons are below 2^31
   }
+  auto pass = [&](int a, int b, bool up) {
+    const unsigned lo = min(x[a], x[b]), hi = max(x[a], x[b]);
+    x[a] = up ? lo : hi;
+    x[b] = up ? hi : lo;
+  };
+#pragma unroll
+  for (int k = 2; k < R; k *= 2)
+#pragma unroll
+    for (int j = k / 2; j > 0; j /= 2)
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (!(r & j)) pass(r, r + j, !(r & k));
+  // k, j: in threads from here on, runs of k sorted; the last run is all
+#pragma unroll 1
+  for (int k = 1; k <= kThreads; k *= 2) {
+    const bool up = !(t & k);
+#pragma unroll 1
+    for (int j = k / 2; j > 0; j /= 2) {
+      const bool low = up == !(t & j);
+      if (kThreads == 32 || j < 32) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const unsigned y = __shfl_xor_sync(0xffffffffu, x[r], j);
+          x[r] = low ? min(x[r], y) : max(x[r], y);
+        }
+      } else {
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r * kThreads + t] = x[r];
+        sort_sync<kThreads>();
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const unsigned y = v[r * kThreads + (t ^ j)];
+          x[r] = low ? min(x[r], y) : max(x[r], y);
+        }
+        sort_sync<kThreads>();
+      }
+    }
+#pragma unroll
+    for (int j = R / 2; j > 0; j /= 2)
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (!(r & j)) pass(r, r + j, up);
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if ((unsigned)(t * R + r) < m) items[t * R + r] = x[r];
 }
 
 // One cell and one window of indices at a time: the cell's indices in the window
@@ -231,17 +284,15 @@ __device__ __forceinline__ void order_mid(unsigned cta, unsigned ctas, const uin
 // k_bin's blocks run, so that the indices of a chunk of slots lie close together:
 // by their range most chunks are before the window or behind it as a whole.
 // Whole builds, us, by a radix sort / windows of 2^18 that read all slots of their
-// cell, and a sort of every cell up to kSortMax / this: 10,000 vortons, half of
-// them in one cell 72 / 78 / 46; 100,000 in one cell 134 / 145 / 53; 16 million in
-// 64 cells 1,711 / 2,023 / 1,506, in one cell 11,231 / 3,135 / 2,168, in cells of
-// their own 994 / 623 / 634.
+// cell, and a sort of every cell up to 8,192 / this: 10,000 vortons, half of them
+// outside 74 / 78 / 47; 100,000 in one cell 135 / 145 / 55; 16 million in 64 cells
+// 1,733 / 2,023 / 1,268, in one cell 11,277 / 3,135 / 1,481, scattered 1,018 / 623 / 628.
 __device__ __forceinline__ void order_big(unsigned cta, unsigned ctas, int n, const uint2* __restrict__ slot,
                                           const uint2* __restrict__ range, const unsigned* __restrict__ start,
-                                          const unsigned* __restrict__ big, const unsigned* __restrict__ big_list,
-                                          unsigned* __restrict__ items, unsigned* bits) {
+                                          unsigned cells, const unsigned* big_list, unsigned* __restrict__ items,
+                                          unsigned* bits) {
   __shared__ unsigned sh[32], warp_sum[32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x / 32;
-  const unsigned cells = big[1];
   unsigned log = kMaxWindowBits;
   auto windows_of = [&](unsigned b) { return ((unsigned)n + (1u << b) - 1) >> b; };
   while (log > kMinWindowBits && (unsigned long long)cells * windows_of(log) < ctas) --log;
@@ -310,20 +361,43 @@ __device__ __forceinline__ void order_big(unsigned cta, unsigned ctas, int n, co
   }
 }
 
-// The cells that k_order left: the first mid_ctas CTAs take the mid ones, the others the big ones.
-__global__ void __launch_bounds__(kOrderThreads) k_order_large(int n, unsigned mid_ctas, const uint2* __restrict__ slot,
+// The cells that k_order left.  Every thread works by the same counts, those
+// that its block read: they decide who meets at the barriers.
+__global__ void __launch_bounds__(kOrderThreads) k_order_large(int n, const uint2* __restrict__ slot,
                                                                const uint2* __restrict__ range,
                                                                const unsigned* __restrict__ start,
-                                                               const unsigned* __restrict__ big,
-                                                               const unsigned* __restrict__ mid_list,
-                                                               const unsigned* __restrict__ big_list,
-                                                               unsigned* __restrict__ items) {
+                                                               const LargeCells large, unsigned* __restrict__ items) {
   pdl_entry();
-  __shared__ unsigned v[kSortMax];
-  if (blockIdx.x < mid_ctas)
-    order_mid(blockIdx.x, mid_ctas, slot, start, big, mid_list, items, v);
-  else
-    order_big(blockIdx.x - mid_ctas, gridDim.x - mid_ctas, n, slot, range, start, big, big_list, items, v);
+  __shared__ unsigned v[kSortMax], count[4];
+  if (threadIdx.x < 4) count[threadIdx.x] = large.count[threadIdx.x];
+  __syncthreads();
+  const int t = threadIdx.x, lane = t & 31;
+  for (unsigned b = blockIdx.x + gridDim.x * (t / 32); b < count[0]; b += gridDim.x * (kOrderThreads / 32)) {
+    const unsigned cell = large.cell[0][b], s = start[cell], m = start[cell + 1] - s;
+    if (m <= 128)
+      sort_cell<32, 4>(lane, m, slot + s, items + s, nullptr);
+    else if (m <= 256)
+      sort_cell<32, 8>(lane, m, slot + s, items + s, nullptr);
+    else if (m <= 512)
+      sort_cell<32, 16>(lane, m, slot + s, items + s, nullptr);
+    else
+      sort_cell<32, 32>(lane, m, slot + s, items + s, nullptr);
+  }
+  static_assert(kGroupMax == 8 * kGroup && kSortMax == 8 * kOrderThreads, "eight indices a thread");
+  const int group = t / kGroup;
+  for (unsigned b = blockIdx.x + gridDim.x * group; b < count[1]; b += gridDim.x * (kOrderThreads / kGroup)) {
+    const unsigned cell = large.cell[1][b], s = start[cell], m = start[cell + 1] - s;
+    sort_cell<kGroup, 8>(t % kGroup, m, slot + s, items + s, v + kGroupMax * group);
+  }
+  __syncthreads();  // v is one from here on
+  for (unsigned b = blockIdx.x; b < count[2]; b += gridDim.x) {
+    const unsigned cell = large.cell[2][b], s = start[cell], m = start[cell + 1] - s;
+    if (m <= 4 * kOrderThreads)
+      sort_cell<kOrderThreads, 4>(t, m, slot + s, items + s, v);
+    else
+      sort_cell<kOrderThreads, 8>(t, m, slot + s, items + s, v);
+  }
+  order_big(blockIdx.x, gridDim.x, n, slot, range, start, count[3], large.cell[3], items, v);
 }
 
 }  // namespace
@@ -353,22 +427,31 @@ vg_status build_cell_lists(Ctx* c, const Geom& g, const float4* ps, size_t n, Ce
   vg_status st = VG_OK;
   // one slot per grid point and one for vortons outside the grid
   const size_t slots = ncells + 1;
-  // cells of up to mid_max vortons are sorted, larger ones ordered by bitmaps
-  const unsigned mid_max = n > kBitmapAll ? kSortMax : kCountMax;
-  // S_CELL: slot (2 n), ranges (2 chunks), key and later items, place (n each), lists of the mid and the big cells
-  const size_t mids = n / (kCountMax + 1), bigs = n / (mid_max + 1), chunks = (n + kChunk - 1) / kChunk;
-  uint2* slot = (uint2*)ws(c, S_CELL, (4 * n + 2 * chunks + mids + bigs + 2) * sizeof(unsigned), &st);
+  // A cell's bitmaps cost by the windows that all n indices fill, its sort by its
+  // own vortons: 262,144 vortons, 4,096 a cell 57 us by bitmaps, 69 sorted; 10^6, 2,915
+  // a cell 132 and 115, 4,629 a cell 119 and 127; two million, 5,830 a cell sorted 185
+  // (a radix sort 203).
+  const unsigned sort_max = (unsigned)std::clamp<size_t>(((n >> kMaxWindowBits) + 1) * 1024, kGroupMax, kSortMax);
+  // S_CELL: slot (2 n), ranges (2 chunks), key and later items, place (n each), the lists of large cells
+  const size_t chunks = (n + kChunk - 1) / kChunk;
+  const size_t of_warps = n / (kCountMax + 1), of_groups = n / (kWarpMax + 1), of_ctas = n / (kGroupMax + 1),
+               of_bitmaps = n / (sort_max + 1);
+  uint2* slot = (uint2*)ws(
+      c, S_CELL, (4 * n + 2 * chunks + of_warps + of_groups + of_ctas + of_bitmaps + 2) * sizeof(unsigned), &st);
   if (st != VG_OK) return st;
-  // S_COUNT: count (slots), numbers of mid and big cells
-  unsigned* count = (unsigned*)ws(c, S_COUNT, (slots + 2) * sizeof(unsigned), &st);
+  // S_COUNT: count (slots), the lists' lengths
+  unsigned* count = (unsigned*)ws(c, S_COUNT, (slots + 4) * sizeof(unsigned), &st);
   if (st != VG_OK) return st;
   unsigned* start = (unsigned*)ws(c, S_START, (slots + 1) * sizeof(unsigned), &st);
   if (st != VG_OK) return st;
   uint2* range = slot + n;
   unsigned* key = (unsigned*)(range + chunks);
-  unsigned *place = key + n, *items = key, *mid_list = place + n, *big_list = mid_list + mids;
-  unsigned* big = count + slots;
-  VG_CUDA(c, cudaMemsetAsync(count, 0, (slots + 2) * sizeof(unsigned), c->stream));
+  unsigned *place = key + n, *items = key;
+  LargeCells large = {count + slots, {place + n}};
+  large.cell[1] = large.cell[0] + of_warps;
+  large.cell[2] = large.cell[1] + of_groups;
+  large.cell[3] = large.cell[2] + of_ctas;
+  VG_CUDA(c, cudaMemsetAsync(count, 0, (slots + 4) * sizeof(unsigned), c->stream));
   if (n > 0) {
     pdl_launch(c->stream, blocks_for(n, 256), 256, 0, k_bin, g, ps, (int)n, key, place, count, (unsigned)ncells);
     VG_LAUNCHED(c);
@@ -379,17 +462,16 @@ vg_status build_cell_lists(Ctx* c, const Geom& g, const float4* ps, size_t n, Ce
     pdl_launch(c->stream, blocks_for(n, 256), 256, 0, k_place, (int)n, (const unsigned*)key, (const unsigned*)place,
                (const unsigned*)start, slot);
     VG_LAUNCHED(c);
-    pdl_launch(c->stream, blocks_for(n, 256), 256, 0, k_order, (int)n, mid_max, (const uint2*)slot, (const unsigned*)start,
-               items, big, mid_list, big_list, range);
+    pdl_launch(c->stream, blocks_for(n, 256), 256, 0, k_order, (int)n, sort_max, (const uint2*)slot, (const unsigned*)start,
+               items, large, range);
     VG_LAUNCHED(c);
   }
   if (n > kCountMax) {
-    const unsigned mid_ctas = n > kBitmapAll ? (unsigned)std::min<size_t>(mids, kMidCtas) : 0;
-    // as many as there can be windows of large cells
-    const unsigned big_ctas = (unsigned)std::min<size_t>(bigs * ((n >> kMinWindowBits) + 1), kBigCtas);
-    pdl_launch(c->stream, mid_ctas + big_ctas, kOrderThreads, 0, k_order_large, (int)n, mid_ctas, (const uint2*)slot,
-               (const uint2*)range, (const unsigned*)start, (const unsigned*)big, (const unsigned*)mid_list,
-               (const unsigned*)big_list, items);
+    // as many as there can be cells, or windows of those for bitmaps
+    const unsigned ctas =
+        (unsigned)std::min<size_t>(std::max(of_warps, of_bitmaps * ((n >> kMinWindowBits) + 1)), kOrderCtas);
+    pdl_launch(c->stream, ctas, kOrderThreads, 0, k_order_large, (int)n, (const uint2*)slot, (const uint2*)range,
+               (const unsigned*)start, large, items);
     VG_LAUNCHED(c);
   }
   VG_CUDA(c, cudaGetLastError());
