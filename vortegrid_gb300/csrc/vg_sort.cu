@@ -144,16 +144,17 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_chunks(const unsigned* __
 // ---- a cell's indices in ascending order -------------------------------------
 // Up to kCountMax vortons each counts the smaller indices of its cell, as many
 // loads as the cell has vortons; up to kWarpMax a warp sorts them, up to kGroupMax
-// a quarter of a CTA, up to sort_max a CTA; bitmaps order larger cells.  Whole
-// builds of 10^6 vortons, us, by a radix sort / counts up to 512 and sorts in shared
-// memory / this: 82 a cell 114 / 79 / 81, 125 a cell 114 / 87 / 78, 455 a cell
-// 116 / 156 / 79, 578 a cell 117 / 152 / 84, 1,371 a cell 121 / 129 / 89, 2,915 a cell
-// 132 / 135 / 115.  With kCountMax 192, 125 a cell take 89; with 48, four million at 41
-// a cell take 172, not 165.  A CTA instead of a quarter for 1,371 a cell: 110.
-constexpr unsigned kCountMax = 96, kWarpMax = 1024, kGroupMax = 2048, kSortMax = 8192;
-constexpr int kOrderThreads = 1024, kGroup = 256;
-constexpr unsigned kMaxWindowBits = 18, kMinWindowBits = 13;  // log2 of a bitmap's indices: 32 KB and 1 KB
-constexpr unsigned kOrderCtas = 152;
+// eight warps, up to sort_max a CTA; bitmaps order larger cells.  Whole builds of
+// 10^6 vortons, us, by a radix sort / counts up to 512 and sorts in shared memory /
+// this: 82 a cell 114 / 79 / 80, 125 a cell 114 / 87 / 80, 455 a cell 116 / 156 / 77,
+// 578 a cell 117 / 152 / 89, 1,371 a cell 121 / 129 / 94, 2,915 a cell 132 / 135 / 107.
+// With kCountMax 192, 125 a cell take 88; with 48, four million at 41 a cell take 172,
+// not 166.  CTAs of 512 threads: of 1,024 with as many registers each, one fills an
+// SM and waits for it to drain (32 steps at once on streams 0.9 % longer).
+constexpr unsigned kCountMax = 96, kWarpMax = 512, kGroupMax = 2048, kSortMax = 8192;
+constexpr int kOrderThreads = 512, kOrderWarps = kOrderThreads / 32, kGroup = 256;
+constexpr unsigned kMaxWindowBits = 18, kMinWindowBits = 12;  // log2 of a bitmap's indices: 32 KB and 512 B
+constexpr unsigned kOrderCtas = 304, kWindows = 152;
 constexpr unsigned kChunk = 32;  // slots whose extreme indices k_order writes down: a warp's
 
 __global__ void k_place(int n, const unsigned* __restrict__ key, const unsigned* __restrict__ place,
@@ -280,13 +281,14 @@ __device__ __forceinline__ void sort_cell(int t, unsigned m, const uint2* __rest
 
 // One cell and one window of indices at a time: the cell's indices in the window
 // are marked in a bitmap and read off it, after those before the window.  The
-// windows are as wide as leaves every CTA one.  Vortons get their places as
+// windows are as wide as leaves every SM one (304 of them instead of 152: 16 million
+// vortons in one cell 2,173 us, not 1,499: every window reads all ranges).  Vortons get their places as
 // k_bin's blocks run, so that the indices of a chunk of slots lie close together:
 // by their range most chunks are before the window or behind it as a whole.
 // Whole builds, us, by a radix sort / windows of 2^18 that read all slots of their
 // cell, and a sort of every cell up to 8,192 / this: 10,000 vortons, half of them
-// outside 74 / 78 / 47; 100,000 in one cell 135 / 145 / 55; 16 million in 64 cells
-// 1,733 / 2,023 / 1,268, in one cell 11,277 / 3,135 / 1,481, scattered 1,018 / 623 / 628.
+// outside 74 / 78 / 47; 100,000 in one cell 135 / 144 / 53; 16 million in 64 cells
+// 1,733 / 2,026 / 1,280, in one cell 11,277 / 3,132 / 1,499, scattered 1,018 / 623 / 628.
 __device__ __forceinline__ void order_big(unsigned cta, unsigned ctas, int n, const uint2* __restrict__ slot,
                                           const uint2* __restrict__ range, const unsigned* __restrict__ start,
                                           unsigned cells, const unsigned* big_list, unsigned* __restrict__ items,
@@ -295,7 +297,7 @@ __device__ __forceinline__ void order_big(unsigned cta, unsigned ctas, int n, co
   const int lane = threadIdx.x & 31, wid = threadIdx.x / 32;
   unsigned log = kMaxWindowBits;
   auto windows_of = [&](unsigned b) { return ((unsigned)n + (1u << b) - 1) >> b; };
-  while (log > kMinWindowBits && (unsigned long long)cells * windows_of(log) < ctas) --log;
+  while (log > kMinWindowBits && (unsigned long long)cells * windows_of(log) < min(ctas, kWindows)) --log;
   const unsigned window = 1u << log, words = window / 32, per = words > kOrderThreads ? words / kOrderThreads : 1;
   const unsigned windows = windows_of(log);
   const unsigned long long units = (unsigned long long)cells * windows;
@@ -305,9 +307,10 @@ __device__ __forceinline__ void order_big(unsigned cta, unsigned ctas, int n, co
     for (unsigned w = threadIdx.x; w < words; w += kOrderThreads) bits[w] = 0;
     __syncthreads();
     unsigned before = 0;
-    // a warp looks at every 32nd chunk, 32 of them at a time, then at the slots of those that it has to, 8 at a time
+    // a warp looks at every kOrderWarps-th chunk, 32 of them at a time, then at the slots of those that it has to,
+    // 8 at a time
     for (unsigned c0 = s / kChunk + wid; c0 <= c1; c0 += kOrderThreads) {
-      const unsigned c = c0 + 32 * lane;
+      const unsigned c = c0 + kOrderWarps * lane;
       bool in = false;
       if (c <= c1) {
         const uint2 r = range[c];
@@ -322,7 +325,7 @@ __device__ __forceinline__ void order_big(unsigned cta, unsigned ctas, int n, co
         unsigned i[kAt];
 #pragma unroll
         for (int k = 0; k < kAt; ++k, todo &= todo - 1) {
-          const unsigned q = (c0 + 32 * (__ffs(todo) - 1)) * kChunk + lane;
+          const unsigned q = (c0 + kOrderWarps * (__ffs(todo) - 1)) * kChunk + lane;
           i[k] = todo && q >= s && q < e ? slot[q].y : 0xffffffffu;
         }
 #pragma unroll
@@ -340,7 +343,7 @@ __device__ __forceinline__ void order_big(unsigned cta, unsigned ctas, int n, co
     const unsigned inc = warp_inclusive(cnt);
     if (lane == 31) warp_sum[wid] = inc;
     __syncthreads();
-    const unsigned ws_ = warp_sum[lane], winc = warp_inclusive(ws_);
+    const unsigned ws_ = lane < kOrderWarps ? warp_sum[lane] : 0, winc = warp_inclusive(ws_);
     unsigned at = s + before + __shfl_sync(0xffffffffu, winc - ws_, wid) + inc - cnt;
     if (__shfl_sync(0xffffffffu, winc, 31) > 4 * words) {  // a word a warp, its indices side by side
       for (unsigned l = 0; l < 32; ++l) {
@@ -369,33 +372,35 @@ __global__ void __launch_bounds__(kOrderThreads) k_order_large(int n, const uint
                                                                const LargeCells large, unsigned* __restrict__ items) {
   pdl_entry();
   __shared__ unsigned v[kSortMax], count[4];
-  if (threadIdx.x < 4) count[threadIdx.x] = large.count[threadIdx.x];
-  __syncthreads();
+  unsigned any = 0;
+  if (threadIdx.x < 4) count[threadIdx.x] = any = large.count[threadIdx.x];
+  if (!__syncthreads_or(any)) return;
   const int t = threadIdx.x, lane = t & 31;
-  for (unsigned b = blockIdx.x + gridDim.x * (t / 32); b < count[0]; b += gridDim.x * (kOrderThreads / 32)) {
+  for (unsigned b = blockIdx.x + gridDim.x * (t / 32); b < count[0]; b += gridDim.x * kOrderWarps) {
     const unsigned cell = large.cell[0][b], s = start[cell], m = start[cell + 1] - s;
     if (m <= 128)
       sort_cell<32, 4>(lane, m, slot + s, items + s, nullptr);
     else if (m <= 256)
       sort_cell<32, 8>(lane, m, slot + s, items + s, nullptr);
-    else if (m <= 512)
-      sort_cell<32, 16>(lane, m, slot + s, items + s, nullptr);
     else
-      sort_cell<32, 32>(lane, m, slot + s, items + s, nullptr);
+      sort_cell<32, 16>(lane, m, slot + s, items + s, nullptr);
   }
-  static_assert(kGroupMax == 8 * kGroup && kSortMax == 8 * kOrderThreads, "eight indices a thread");
+  static_assert(kGroupMax == 8 * kGroup && kSortMax == 16 * kOrderThreads, "what a thread holds");
   const int group = t / kGroup;
   for (unsigned b = blockIdx.x + gridDim.x * group; b < count[1]; b += gridDim.x * (kOrderThreads / kGroup)) {
     const unsigned cell = large.cell[1][b], s = start[cell], m = start[cell + 1] - s;
-    sort_cell<kGroup, 8>(t % kGroup, m, slot + s, items + s, v + kGroupMax * group);
+    if (m <= 4 * kGroup)
+      sort_cell<kGroup, 4>(t % kGroup, m, slot + s, items + s, v + kGroupMax * group);
+    else
+      sort_cell<kGroup, 8>(t % kGroup, m, slot + s, items + s, v + kGroupMax * group);
   }
   __syncthreads();  // v is one from here on
   for (unsigned b = blockIdx.x; b < count[2]; b += gridDim.x) {
     const unsigned cell = large.cell[2][b], s = start[cell], m = start[cell + 1] - s;
-    if (m <= 4 * kOrderThreads)
-      sort_cell<kOrderThreads, 4>(t, m, slot + s, items + s, v);
-    else
+    if (m <= 8 * kOrderThreads)
       sort_cell<kOrderThreads, 8>(t, m, slot + s, items + s, v);
+    else
+      sort_cell<kOrderThreads, 16>(t, m, slot + s, items + s, v);
   }
   order_big(blockIdx.x, gridDim.x, n, slot, range, start, count[3], large.cell[3], items, v);
 }
@@ -428,9 +433,9 @@ vg_status build_cell_lists(Ctx* c, const Geom& g, const float4* ps, size_t n, Ce
   // one slot per grid point and one for vortons outside the grid
   const size_t slots = ncells + 1;
   // A cell's bitmaps cost by the windows that all n indices fill, its sort by its
-  // own vortons: 262,144 vortons, 4,096 a cell 57 us by bitmaps, 69 sorted; 10^6, 2,915
-  // a cell 132 and 115, 4,629 a cell 119 and 127; two million, 5,830 a cell sorted 185
-  // (a radix sort 203).
+  // own vortons.  Whole builds, us, all sorted / all by bitmaps: 262,144 vortons, 4,096
+  // a cell 66 / 54; 600,000, 2,777 a cell 85 / 98, 4,800 a cell 107 / 94; 10^6, 2,915 a cell
+  // 106 / 134, 8,000 a cell 136 / 121; two million, 5,830 a cell 174 / 223.
   const unsigned sort_max = (unsigned)std::clamp<size_t>(((n >> kMaxWindowBits) + 1) * 1024, kGroupMax, kSortMax);
   // S_CELL: slot (2 n), ranges (2 chunks), key and later items, place (n each), the lists of large cells
   const size_t chunks = (n + kChunk - 1) / kChunk;
@@ -462,8 +467,8 @@ vg_status build_cell_lists(Ctx* c, const Geom& g, const float4* ps, size_t n, Ce
     pdl_launch(c->stream, blocks_for(n, 256), 256, 0, k_place, (int)n, (const unsigned*)key, (const unsigned*)place,
                (const unsigned*)start, slot);
     VG_LAUNCHED(c);
-    pdl_launch(c->stream, blocks_for(n, 256), 256, 0, k_order, (int)n, sort_max, (const uint2*)slot, (const unsigned*)start,
-               items, large, range);
+    pdl_launch(c->stream, blocks_for(n, 256), 256, 0, k_order, (int)n, sort_max, (const uint2*)slot,
+               (const unsigned*)start, items, large, range);
     VG_LAUNCHED(c);
   }
   if (n > kCountMax) {
